@@ -5,8 +5,10 @@
 //   1. SH -> DO   : SRCDO[p][c] = max(0, source in ordinate c)  (tensor-core
 //                   k_tc_gemm, or the factorized k_sh_to_do)
 //   2. sweeps     : downward ordinates, Lambertian bottom, upward ordinates;
-//                   boundary-plane chains (k_sweep_p1) beside the source
-//                   pass (k_sweep_prep), then the wavefront levels
+//                   with open boundaries the boundary-plane chains
+//                   (k_sweep_p1s), then the plane march (k_sweep_march);
+//                   else boundary-plane chains (k_sweep_p1) beside the
+//                   source pass (k_sweep_prep), then the wavefront levels
 //                   (k_sweep_levels, or one k_sweep per level); grids whose
 //                   wavefront is too deep are walked in the reference order
 //                   (k_sweep_seq)
@@ -17,8 +19,11 @@
 //                   delta-source, new truncation, next radiance truncation)
 //   5. k_accel_param, k_accelerate (CALC_ACCEL_SOLCRIT, ACCELERATE_SOLUTION)
 // Layouts are dense: [point][term] for the spherical-harmonic fields (terms
-// beyond a point's truncation are zero) and [point][column] for the
-// ordinate fields, columns grouped by hemisphere and trace octant.
+// beyond a point's truncation are zero); the ordinate fields are
+// [column][point] where the sweep runs column by column (the plane march,
+// the reference order), so that its rows are contiguous, and [point][column]
+// for the level schedule, whose items run over the columns of one point;
+// columns are grouped by hemisphere and trace octant.
 
 #include <cooperative_groups.h>
 #include <cuda.h>
@@ -34,6 +39,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/shdom_gb300.h"
@@ -54,7 +60,8 @@ namespace shdom {
 // Device error codes written to Dev::err (first error wins).
 enum {
   ERR_NONE = 0, ERR_SWEEP_NOFACE = 1, ERR_SWEEP_STEPS = 2, ERR_RAY_STEPS = 3, ERR_RAY_SO = 4, ERR_RAY_BELOW = 5,
-  ERR_TC_WAIT = 6  // a tensor-core transform gave up waiting on its pipeline
+  ERR_TC_WAIT = 6,  // a tensor-core transform gave up waiting on its pipeline
+  ERR_SWEEP_WAIT = 7  // a plane march gave up waiting on a neighbouring strip
 };
 
 __constant__ int c_face[6][4] = {{0, 2, 4, 6}, {1, 3, 5, 7}, {0, 1, 4, 5}, {2, 3, 6, 7}, {0, 1, 2, 3}, {4, 5, 6, 7}};
@@ -234,8 +241,10 @@ struct SweepArgs {
   const uint8_t *stk;              // polarized: Stokes component per column (null: all I)
   int *err;
   int npts, nang, ldo, is1d, nz, ny1, nx1;
+  size_t ps, cs;                   // strides of a point and of a column in srcdo / raddo
   float transmin;
   int oct_col0[8], oct_ncol[8];
+  __device__ __forceinline__ size_t at(int p, int col) const { return (size_t)p * ps + (size_t)col * cs; }
 };
 
 // One backward short-characteristic trace (BACK_INT_GRID3D_UNPOL,
@@ -265,7 +274,6 @@ struct RegLoad {
 };
 
 __device__ __forceinline__ void reg_load(const SweepArgs &a, int b, int pt, int col, RegLoad &x, bool upstream) {
-  const int ldo = a.ldo;
   const int iz = pt % a.nz;
   const int layer = (b & 4) ? iz - 1 : iz;
   x.pt = pt; x.col = col;
@@ -278,17 +286,16 @@ __device__ __forceinline__ void reg_load(const SweepArgs &a, int b, int pt, int 
     const int d = c_face[iface][k] ^ b;
     const int q = pt + ((d & 1) ? ox : 0) + ((d & 2) ? oy : 0) + ((d & 4) ? oz : 0);
     x.e[k] = __ldg(a.text + q);
-    x.s[k] = __ldg(a.srcdo + (size_t)q * ldo + col);
-    x.r[k] = upstream ? a.raddo[(size_t)q * ldo + col] : 0.f;
+    x.s[k] = __ldg(a.srcdo + a.at(q, col));
+    x.r[k] = upstream ? a.raddo[a.at(q, col)] : 0.f;
   }
   x.e1 = __ldg(a.text + pt);
-  x.s1 = __ldg(a.srcdo + (size_t)pt * ldo + col);
+  x.s1 = __ldg(a.srcdo + a.at(pt, col));
 }
 
 // Same inputs for a stored single-cell general trace.
 __device__ __forceinline__ void rec_load(const SweepArgs &a, const IrrRec &rec, int pt, int col, RegLoad &x,
                                          bool upstream) {
-  const int ldo = a.ldo;
   x.pt = pt; x.col = col;
   x.clamp = !a.stk || !a.stk[col];
   x.g = rec.g;
@@ -296,11 +303,11 @@ __device__ __forceinline__ void rec_load(const SweepArgs &a, const IrrRec &rec, 
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     x.e[k] = __ldg(a.text + q[k]);
-    x.s[k] = __ldg(a.srcdo + (size_t)q[k] * ldo + col);
-    x.r[k] = upstream ? a.raddo[(size_t)q[k] * ldo + col] : 0.f;
+    x.s[k] = __ldg(a.srcdo + a.at(q[k], col));
+    x.r[k] = upstream ? a.raddo[a.at(q[k], col)] : 0.f;
   }
   x.e1 = __ldg(a.text + pt);
-  x.s1 = __ldg(a.srcdo + (size_t)pt * ldo + col);
+  x.s1 = __ldg(a.srcdo + a.at(pt, col));
 }
 
 // Source integral over one cell (the reference's linear-in-tau source
@@ -444,7 +451,7 @@ __device__ __forceinline__ Trace trace_general(const SweepArgs &a, int b, int cl
   Trace t;
   t.radsrc = 0.f; t.tr = 1.f; t.status = ERR_SWEEP_STEPS; t.u = 0.f; t.v = 0.f;
   t.q[0] = t.q[1] = t.q[2] = t.q[3] = pt; t.f[0] = t.f[1] = t.f[2] = t.f[3] = 0.f;
-  const int ldo = a.ldo, n = a.npts;
+  const int n = a.npts;
   const float cx = a.col_cx[col], cy = a.col_cy[col], cz = a.col_cz[col];
   const float cxinv = cx != 0.f ? 1.f / cx : 1.0e6f, cyinv = cy != 0.f ? 1.f / cy : 1.0e6f, czinv = 1.f / cz;
   const int bitz = cz < 0.f;
@@ -454,7 +461,7 @@ __device__ __forceinline__ Trace trace_general(const SweepArgs &a, int b, int cl
   int cell = a.start[(size_t)b * n + pt];
   float xe = a.gridpos[3 * pt], ye = a.gridpos[3 * pt + 1], ze = a.gridpos[3 * pt + 2];
   float ext1 = a.text[pt];
-  float srcext1 = ext1 * a.srcdo[(size_t)pt * ldo + col];
+  float srcext1 = ext1 * a.srcdo[a.at(pt, col)];
   float rad = 0.f, tr = 1.f;
   const bool clamp = !a.stk || !a.stk[col];
   for (int guard = 0; guard < 65536; ++guard) {
@@ -480,8 +487,8 @@ __device__ __forceinline__ Trace trace_general(const SweepArgs &a, int b, int cl
     }
     const float e1 = a.text[i1], e2 = a.text[i2], e3 = a.text[i3], e4 = a.text[i4];
     const float ext0 = f1 * e1 + f2 * e2 + f3 * e3 + f4 * e4;
-    const float srcext0 = f1 * a.srcdo[(size_t)i1 * ldo + col] * e1 + f2 * a.srcdo[(size_t)i2 * ldo + col] * e2 +
-                          f3 * a.srcdo[(size_t)i3 * ldo + col] * e3 + f4 * a.srcdo[(size_t)i4 * ldo + col] * e4;
+    const float srcext0 = f1 * a.srcdo[a.at(i1, col)] * e1 + f2 * a.srcdo[a.at(i2, col)] * e2 +
+                          f3 * a.srcdo[a.at(i3, col)] * e3 + f4 * a.srcdo[a.at(i4, col)] * e4;
     float radsrc, transcell;
     cell_source(ext0, srcext0, ext1, srcext1, so, radsrc, transcell, clamp);
     rad += tr * radsrc;
@@ -622,7 +629,6 @@ __global__ void __launch_bounds__(P1_THREADS) k_sweep_p1(SweepArgs a, const Seg 
                                                          const int *__restrict__ p1off) {
   const int grp = blockIdx.x / P1_SPLIT, sid = blockIdx.x % P1_SPLIT;
   const int s0 = p1off[grp], s1 = p1off[grp + 1];
-  const int ldo = a.ldo;
   // staged items: the inputs of a single-face trace but the corner radiances
   RegLoad st[P1_STAGE];
   int sq[P1_STAGE][4];
@@ -667,11 +673,11 @@ __global__ void __launch_bounds__(P1_THREADS) k_sweep_p1(SweepArgs a, const Seg 
       int task, i, col;
       coords(ii, task, i, col);
 #pragma unroll
-      for (int c = 0; c < 4; ++c) x.r[c] = a.raddo[(size_t)q[c] * ldo + col];
+      for (int c = 0; c < 4; ++c) x.r[c] = a.raddo[a.at(q[c], col)];
       const Trace t = reg_trace(x, g.b, x.pt);
       float rad = t.radsrc;
       if (t.tr != 0.f) rad += t.tr * (t.f[0] * x.r[0] + t.f[1] * x.r[1] + t.f[2] * x.r[2] + t.f[3] * x.r[3]);
-      a.raddo[(size_t)x.pt * ldo + col] = rad;
+      a.raddo[a.at(x.pt, col)] = rad;
     };
     auto item_plain = [&](int ii) {
       int task, i, col;
@@ -690,10 +696,10 @@ __global__ void __launch_bounds__(P1_THREADS) k_sweep_p1(SweepArgs a, const Seg 
         if (t.status != ERR_NONE) atomicCAS(a.err, ERR_NONE, t.status);
         rad = t.radsrc;
         if (t.tr != 0.f)
-          rad += t.tr * (t.f[0] * a.raddo[(size_t)t.q[0] * ldo + col] + t.f[1] * a.raddo[(size_t)t.q[1] * ldo + col] +
-                         t.f[2] * a.raddo[(size_t)t.q[2] * ldo + col] + t.f[3] * a.raddo[(size_t)t.q[3] * ldo + col]);
+          rad += t.tr * (t.f[0] * a.raddo[a.at(t.q[0], col)] + t.f[1] * a.raddo[a.at(t.q[1], col)] +
+                         t.f[2] * a.raddo[a.at(t.q[2], col)] + t.f[3] * a.raddo[a.at(t.q[3], col)]);
       }
-      a.raddo[(size_t)pt * ldo + col] = rad;
+      a.raddo[a.at(pt, col)] = rad;
     };
     static_assert(P1_STAGE == 2, "the staged items are handled one by one below");
     if (threadIdx.x < items) {
@@ -747,7 +753,6 @@ __global__ void __launch_bounds__(P1_THREADS) k_sweep_p1r(SweepArgs a, const Seg
                                                           const TraceRec *__restrict__ recs) {
   const int grp = blockIdx.x / P1_SPLIT, sid = blockIdx.x % P1_SPLIT;
   const int s0 = p1off[grp], s1 = p1off[grp + 1];
-  const int ldo = a.ldo;
   // the group's level segments, in shared memory when they fit
   __shared__ Seg ssg[P1_SEGCAP];
   const bool local = s1 - s0 <= P1_SEGCAP;
@@ -771,12 +776,12 @@ __global__ void __launch_bounds__(P1_THREADS) k_sweep_p1r(SweepArgs a, const Seg
   auto combine = [&](const TraceRec &R, int pt, int col) {
     float rad = R.radsrc;
     if (R.tr != 0.f) {
-      const float r0 = a.raddo[(size_t)R.q.x * ldo + col], r1 = a.raddo[(size_t)R.q.y * ldo + col];
-      const float r2 = a.raddo[(size_t)R.q.z * ldo + col], r3 = a.raddo[(size_t)R.q.w * ldo + col];
+      const float r0 = a.raddo[a.at(R.q.x, col)], r1 = a.raddo[a.at(R.q.y, col)];
+      const float r2 = a.raddo[a.at(R.q.z, col)], r3 = a.raddo[a.at(R.q.w, col)];
       const float u = R.u, v = R.v;
       rad += R.tr * ((1.f - u) * (1.f - v) * r0 + (1.f - u) * v * r1 + u * (1.f - v) * r2 + u * v * r3);
     }
-    a.raddo[(size_t)pt * ldo + col] = rad;
+    a.raddo[a.at(pt, col)] = rad;
   };
   auto stage = [&](int si) {
     if (si >= s1) return;
@@ -826,7 +831,6 @@ struct P1Blk {
 __global__ void __launch_bounds__(256) k_p1_prep_s(SweepArgs a, const Seg *__restrict__ segs, int nseg, int n,
                                                    const int *__restrict__ seggrp, const int *__restrict__ p1slot,
                                                    TraceRec *__restrict__ out) {
-  const int ldo = a.ldo;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
     const int si = irr_seg_find(segs, nseg, j);
     const Seg g = segs[si];
@@ -854,7 +858,7 @@ __global__ void __launch_bounds__(256) k_p1_prep_s(SweepArgs a, const Seg *__res
       const float w = t.tr * f[k];
       if (w == 0.f) continue;
       if (a.bnd[t.q[k]] & hb) {
-        r.radsrc += w * a.raddo[(size_t)t.q[k] * ldo + col];  // preset: final
+        r.radsrc += w * a.raddo[a.at(t.q[k], col)];  // preset: final
       } else {
         sl[k] = slots[t.q[k]];
         if (sl[k] < 0) atomicCAS(a.err, ERR_NONE, ERR_SWEEP_NOFACE);  // not a phase-1 point of the group
@@ -874,7 +878,6 @@ __global__ void __launch_bounds__(P1S_THREADS) k_sweep_p1s(SweepArgs a, const Se
   __shared__ int sbase[P1_SEGCAP];
   const P1Blk B = blks[blockIdx.x];
   const int s0 = p1off[B.grp], s1 = p1off[B.grp + 1], ncs = B.ncs;
-  const int ldo = a.ldo;
   for (int t = threadIdx.x; t < s1 - s0; t += blockDim.x) { ssg[t] = p1segs[s0 + t]; sbase[t] = segbase[s0 + t]; }
   __syncthreads();
   TraceRec sr[P1_STAGE];
@@ -900,7 +903,7 @@ __global__ void __launch_bounds__(P1S_THREADS) k_sweep_p1s(SweepArgs a, const Se
       rad += R.tr * acc;
     }
     sv[slot * ncs + c] = rad;
-    a.raddo[(size_t)pt * ldo + col] = rad;
+    a.raddo[a.at(pt, col)] = rad;
   };
   auto stage = [&](int si) {
     if (si >= s1) return;
@@ -966,7 +969,7 @@ __device__ __forceinline__ void level_load(const SweepArgs &a, const Seg &g, int
     x.u = rec.g.y; x.v = rec.g.z;
   }
 #pragma unroll
-  for (int k = 0; k < 4; ++k) r[k] = a.raddo[(size_t)x.q[k] * a.ldo + x.col];
+  for (int k = 0; k < 4; ++k) r[k] = a.raddo[a.at(x.q[k], x.col)];
 }
 
 __device__ __forceinline__ void level_finish(const SweepArgs &a, const LevelItem &x, const float r[4]) {
@@ -974,7 +977,7 @@ __device__ __forceinline__ void level_finish(const SweepArgs &a, const LevelItem
   const float f0 = (1.f - u) * (1.f - v), f1 = (1.f - u) * v, f2 = u * (1.f - v), f3 = u * v;
   float rad = x.w.x;
   if (x.w.y != 0.f) rad += x.w.y * (f0 * r[0] + f1 * r[1] + f2 * r[2] + f3 * r[3]);
-  a.raddo[(size_t)x.pt * a.ldo + x.col] = rad;
+  a.raddo[a.at(x.pt, x.col)] = rad;
 }
 
 __device__ __forceinline__ int seg_find(const Seg *sg, int nseg, int i, int si) {
@@ -1029,215 +1032,460 @@ __global__ void __launch_bounds__(256) k_sweep_levels(SweepArgs a, const Seg *__
 // ------------------------------------------------------------ plane march
 // Phase 2 of a hemisphere whose (octant, face class) groups all march
 // (MarchGrp, planned on the host): each phase-2 point's regular trace stops
-// on a face in the previous plane along the group's class axis, so the
-// group's columns are swept plane by plane, every point of a plane
-// independent of the others.  One thread-block cluster per (group, column
-// slice): the cluster's CTAs split each plane into strips of rows along U.
-// A CTA keeps, for the previous and the current plane (two buffers swapped
-// every plane), its strip's radiances, ordinate sources times extinction
-// and extinctions in shared memory, plus one halo row on the upwind side
-// that the upwind CTA stores into it (distributed shared memory) when it
-// computes that row; the cluster meets at one cluster barrier per plane.
-// The source pass is fused: (radsrc, tr) of BACK_INT_GRID3D's cell
-// integral come from the ordinate source and extinction of the point
-// (loaded from global memory one plane ahead) and of the face corners (the
-// previous plane, in shared memory), with the arithmetic of reg_trace.
-// DRAM sees one read of the point's ordinate source and one write of its
-// radiance per item.
+// on a face in the previous plane along the group's class axis, so a column
+// is swept plane by plane, every point of a plane independent of the others.
+//
+// One thread-block cluster per column; its CTAs share out the rows of a plane
+// (strips along U, numbered by w, which grows towards the upwind side).  A
+// thread keeps one V position and up to RM consecutive rows for the whole
+// march, so the face weights of the x and y classes stay in registers and
+// the lerp along V of a row serves both rows it borders.
+//
+// rad = radsrc + tr * (face radiance), and (radsrc, tr), the cell integral
+// of BACK_INT_GRID3D, depend on the source alone.  So the loop is software
+// pipelined: in one step a thread combines plane t (a few instructions on
+// the previous plane's radiances) and forms (radsrc, tr) of plane t + 1 from
+// the source x extinction and extinction of plane t in shared memory and its
+// own of plane t + 1, loaded one plane ahead; the two are independent, and
+// one block barrier separates the steps.  (Forming both for the same plane,
+// one after the other, took twice the time per plane.)
+//
+// Radiances of the row above the strip come from the next CTA upwind, which
+// sends them into a ring of MRING halo rows in this CTA's shared memory with
+// st.async (the bytes are counted on an mbarrier, so no fence waits for the
+// global stores); a relaxed remote arrive returns the slot.  The strips run
+// as a pipeline, a plane or two apart, with no cluster-wide barrier per
+// plane.  The row above's source and extinction are read from memory.
+//
+// The ordinate fields are ordinate-major here (a point's stride is 1), so
+// the rows of the x and y classes are contiguous.  The planes of the z class
+// are nz apart: a thread takes four consecutive layers of its points at once
+// (16-byte loads into shared memory one group ahead, 16-byte stores).
+//
+// Every wait is bounded; a thread whose wait expires records the error and
+// goes on without waiting, and no CTA leaves before its cluster's last access.
+//
+// What bounds it: issue slots on the large grids (63% of the peak issue
+// rate at 96x96x48, 140 warp instructions per 32 point-ordinates where 60 of
+// the cell integral alone remain), the latency of a plane on small ones.
+// Measured per hemisphere, x and y classes plus z class, against the
+// point-major march with a cluster barrier per plane that it replaced:
+// 128x128x64 16 x 32 0.76 + 0.58 against 2.46 ms, 96x96x48 0.33 + 0.27
+// against 0.91, 64x64x32 8 x 16 0.060 + 0.045 against 0.276, 12x12x10
+// 0.014 + 0.014 against 0.099.  DRAM at 96x96x48: 1.2 times the bytes of the
+// source and the radiance, each once (2.9 times before).  Tried on the way:
+// fences in place of st.async (a plane waits for its global stores: 1.8
+// against 1.1 us a plane at 64x64x32), values one plane ahead in registers
+// instead of MDEPTH in shared memory (0.9 against 0.6 us of latency a plane),
+// and single 4-byte accesses for the z class (1.9 against 0.6 ms at
+// 128x128x64).
 struct MarchUnit {
-  int grp, c0, nc, tw;  // group, absolute columns [c0, c0+nc), rows per CTA
+  int grp, col;
 };
-constexpr int MT = 256;  // threads per CTA
-constexpr int MK = 16;   // (row, v) pairs per thread at most
+constexpr int MRING = 8;     // halo rows in flight between neighbouring strips
+constexpr int MMAXT = 512;   // threads per CTA at most
+constexpr int MROWS = 16;    // rows per thread at most
+constexpr int MWAIT = tc::kWaitLimit;
 
-// Shared memory of one CTA: the face geometry of the strip's columns
-// [nv][nc] (float4), then two plane buffers, each rad[tw+2][nv][nc],
-// se[tw+2][nv][nc] and ext[tw+2][nv] (rows -1 and tw are halo rows).
-__host__ __device__ inline size_t march_buf_floats(int tw, int nv, int nc) {
-  return (size_t)(tw + 2) * nv * (2 * nc + 1);
-}
-__host__ __device__ inline size_t march_smem_bytes(int tw, int nv, int nc) {
-  return sizeof(float) * (4 * (size_t)nv * nc + 2 * march_buf_floats(tw, nv, nc));
+constexpr int MDEPTH = 4;    // planes of the x and y classes in flight from memory (a power of two)
+
+__host__ __device__ inline size_t march_smem_bytes(int tw, int nv, int nz, bool z) {
+  const size_t n1 = (size_t)(tw + 1) * nv, nfix = 2 * (size_t)(tw + nv);
+  return 256 + sizeof(float) * ((z ? 16 * n1 + 8 * nfix + 4 * (size_t)nz : MDEPTH * (2 * n1 + nfix)) + (size_t)MRING * nv + 16 +
+                                2 * (size_t)tw * nv + 4 * n1);
 }
 
-__global__ void __launch_bounds__(MT, 2) k_sweep_march(SweepArgs a, const MarchGrp *__restrict__ grps,
-                                                       const MarchUnit *__restrict__ units) {
+// One float into another CTA's shared memory, 4 bytes counted on a barrier there.
+__device__ __forceinline__ void march_send(uint32_t dst, uint32_t bar, int cta, float x) {
+  asm volatile(
+      "{ .reg .b32 d, m; mapa.shared::cluster.u32 d, %0, %2; mapa.shared::cluster.u32 m, %1, %2;\n"
+      "  st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [d], %3, [m]; }" ::"r"(dst),
+      "r"(bar), "r"(cta), "r"(__float_as_uint(x))
+      : "memory");
+}
+// Arrives on the barrier at the same shared-memory address in another CTA of
+// the cluster.  Relaxed: it returns a halo slot whose values are already in
+// registers, and publishes nothing.
+__device__ __forceinline__ void march_arrive(uint32_t bar, int cta) {
+  asm volatile(
+      "{ .reg .b32 r; mapa.shared::cluster.u32 r, %0, %1; mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [r]; }" ::"r"(bar),
+      "r"(cta)
+      : "memory");
+}
+__device__ __forceinline__ void cp_async(float *dst, const float *src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async16(float *dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// a g + b f on both halves (packed FP32 pair operations).
+__device__ __forceinline__ float2 lerp2(float2 a, float2 b, float2 g, float2 f) {
+  float2 r;
+  asm("{ .reg .b64 ra, rb, rg, rf, rt;\n"
+      "  mov.b64 ra, {%2, %3}; mov.b64 rb, {%4, %5}; mov.b64 rg, {%6, %7}; mov.b64 rf, {%8, %9};\n"
+      "  mul.rn.f32x2 rt, ra, rg; fma.rn.f32x2 rt, rb, rf, rt; mov.b64 {%0, %1}, rt; }"
+      : "=f"(r.x), "=f"(r.y)
+      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(g.x), "f"(g.y), "f"(f.x), "f"(f.y));
+  return r;
+}
+
+// cell_source with one formula for all optical depths: the thin and the
+// thick source are both rs (s0 + s1 + (ext0 s1 - ext1 s0) X) with
+// rs = 1 / (ext0 + ext1), X = so / 6 up to tau = 2 and
+// 2 rs (1 - 2/tau + 2 T/A) past it; past tau = 4 (ext0, s0) are those of the
+// point four optical depths upwind.  Quotients as there (2 ulp).
+__device__ __forceinline__ void cell_source_march(float ext0, float se0, float ext1, float se1, float so, float &radsrc,
+                                                  float &tr, bool clamp) {
+  radsrc = 0.f;
+  tr = 1.f;
+  const float tau = 0.5f * (ext0 + ext1) * so;
+  if (tau == 0.f) return;  // clear: no source, full transmission
+  const float thin = tau * (1.f - 0.5f * tau * (1.f - 0.33333333333f * tau * (1.f - 0.25f * tau)));
+  const float ex = __expf(-tau);
+  const bool thick = tau >= 0.5f;
+  const float ab = thick ? 1.f - ex : thin;
+  tr = thick ? ex : 1.f - thin;
+  float x = 0.16666667f * so;
+  if (tau > 2.f) {
+    const float it = __fdividef(1.f, tau);
+    if (tau > 4.f) {
+      const float e = fmaf((ext0 - ext1) * 4.f, it, ext1);
+      if (ext0 > 0.f) se0 = __fdividef(se0 * e, ext0);
+      ext0 = e;
+    }
+    x = 2.f * __fdividef(1.f - 2.f * it + __fdividef(2.f * ex, ab), ext0 + ext1);
+  }
+  float src = __fdividef(se0 + se1 + (ext0 * se1 - ext1 * se0) * x, ext0 + ext1);
+  if (clamp) src = fmaxf(src, 0.f);
+  radsrc = src * ab;
+}
+
+template <int RM, bool ZC>
+__device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp &G, int col, unsigned char *msm, int cs, int rank) {
+  const int nV = G.nV, tw = (G.nU + cs - 1) / cs, w0 = rank * tw, nrow = max(0, min(tw, G.nU - w0));
+  const int N = tw * nV, N1 = N + nV, tid = threadIdx.x;
+  // shared memory: barriers; the points' own values on their way from memory
+  // (x and y classes: [MDEPTH planes][s, e][tw + 1][nV]; z class: [2 groups]
+  // [s, e][tw + 1][nV][4 layers]) and the final radiances of the fixed points
+  // ([..][2 per row, then the two edge rows]); the z class's face geometry;
+  // (source x ext, ext) pairs [2][tw + 1][nV], halo ring [MRING][nV],
+  // radiances [2][tw][nV].  The spare floats take the reads one position past
+  // a row of fixed points.
+  const int nfix = 2 * (tw + nV);
+  float *own = reinterpret_cast<float *>(msm + 256);
+  float *ownr = own + (ZC ? 16 : 2 * MDEPTH) * N1;
+  float4 *sgeo = reinterpret_cast<float4 *>(ownr + (ZC ? 8 : MDEPTH) * nfix);
+  float2 *sbuf = reinterpret_cast<float2 *>(sgeo + (ZC ? a.nz : 0)) + 2;
+  float *halo = reinterpret_cast<float *>(sbuf + 2 * N1) + 4;
+  float *rbuf = halo + MRING * nV + 4;
+  const uint32_t full0 = (uint32_t)__cvta_generic_to_shared(msm), empty0 = full0 + 8 * MRING;
+  const bool from_up = nrow > 0 && w0 + nrow < G.nU;   // the strip above is CTA rank + 1's
+  const bool push = rank > 0 && nrow > 0;              // our first row is CTA rank - 1's row above
+  if (nrow == 0) return;
+  const int ngrp = blockDim.x / nV, gi = tid / nV, v = tid - gi * nV;
+  const int R = (nrow + ngrp - 1) / ngrp, q0 = gi * R;  // rows [q0, q0 + kn) of the strip
+  const int kn = gi < ngrp ? max(0, min(R, nrow - q0)) : 0;
+  const int sdv = (G.b & (ZC ? 2 : 4)) ? -1 : 1;        // V offset of the upwind neighbour
+  // the face fraction along V is u and along U is v, or the other way round;
+  // from the stopping face's corners
+  const bool vu = G.dv[0] != G.dv[2], vflip = G.dv[0] != 0, uflip = G.du[0] != 0;
+  const bool clamp = !a.stk || !a.stk[col];
+  const float *__restrict__ src = a.srcdo + (size_t)col * a.cs;
+  float *rado = a.raddo + (size_t)col * a.cs;
+  const int ustep = G.upu > 0 ? G.su : -G.su;
+  const int p0 = (G.upu > 0 ? w0 + q0 : G.nU - 1 - (w0 + q0)) * G.su + v * G.sv;  // first row's point less the plane's
+  const int astep = G.da * G.sa;
+  const int last_fixed = (G.cls == 0 && G.xedge) || (G.cls == 1 && G.yedge);  // the last plane is fixed throughout: unread
+  const int nT = G.nA - last_fixed;
+  unsigned fix = 0;  // rows whose point is preset or phase 1 in every plane
+#pragma unroll
+  for (int j = 0; j < RM; ++j) {
+    const int w = w0 + q0 + j, u = G.upu > 0 ? w : G.nU - 1 - w;
+    const bool f = (!ZC && v == G.zfix) || (G.xedge && G.cls != 0 && (u == 0 || u == a.nx1 - 1)) ||
+                   (G.yedge && ((G.cls == 0 && (u == 0 || u == a.ny1 - 1)) || (ZC && (v == 0 || v == a.ny1 - 1))));
+    fix |= (unsigned)(f && j < kn) << j;
+  }
+  // where a fixed row's radiance is staged: by row at a fixed V position, else in an edge row
+  const bool vfix = ZC ? G.yedge && (v == 0 || v == a.ny1 - 1) : v == G.zfix;
+  auto fixslot = [&](int j) {
+    return vfix ? 2 * (q0 + j) + (ZC && v != 0 ? 1 : 0) : 2 * tw + (w0 + q0 + j == 0 ? 0 : nV) + v;
+  };
+  const bool pusher = push && q0 == 0 && kn > 0;
+  const bool above = from_up && kn > 0 && q0 + kn == nrow;  // the row above this thread's last is the next strip's
+  int lim = MWAIT;
+  auto expired = [&]() { lim = 0; atomicCAS(a.err, ERR_NONE, ERR_SWEEP_WAIT); };
+  auto push_row = [&](int t, float rad) {
+    if (t >= MRING && !tc::mbar_wait(empty0 + 8 * (t % MRING), (uint32_t)(t / MRING - 1) & 1u, lim)) expired();
+    march_send((uint32_t)__cvta_generic_to_shared(halo + (t % MRING) * nV + v), full0 + 8 * (t % MRING), rank - 1, rad);
+  };
+  // face weights: gx, fx along V (own position, upwind neighbour), gw, fw along U
+  const float4 *geo = reinterpret_cast<const float4 *>(a.geo) + col;
+  auto load_g = [&](int z) {
+    const int layer = (G.b & 4) ? z - 1 : z;
+    return layer >= 0 && layer < a.nz - 1 ? __ldg(geo + (size_t)layer * a.nang) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  float fx, gx, fw, gw, so;
+  auto weights = [&](const float4 &g) {
+    const float fv = vu ? g.y : g.z, fu = vu ? g.z : g.y;
+    fx = vflip ? 1.f - fv : fv; gx = vflip ? fv : 1.f - fv;
+    fw = uflip ? 1.f - fu : fu; gw = uflip ? fu : 1.f - fu;
+    so = g.x;
+  };
+  float radsrc[RM], tr[RM];
+  float cx = 0.f, cgx = 1.f, cw = 0.f, cgw = 1.f;  // weights of the plane being combined
+  // this thread's first row in the buffers of the previous and of the current plane
+  const int r0off = q0 * nV + v;
+  float *rprev = rbuf + r0off, *rcur = rprev + N;
+  float2 *sprev = sbuf + r0off, *scur = sprev + N1;
+  // Combines plane t from plane t - 1's radiances; put(j, rad) stores them.
+  auto combine_rows = [&](int t, auto full, const float *hal, auto &&put) {
+    float b0 = cgx * rprev[0] + cx * rprev[sdv];
+#pragma unroll
+    for (int j = 0; j < RM; ++j)
+      if (full.value || j < kn) {
+        const float *pn = rprev + (j + 1) * nV;
+        if (full.value ? j == RM - 1 : j == kn - 1) pn = hal;
+        const float b1 = cgx * pn[0] + cx * pn[sdv];
+        const float up = cgw * b0 + cw * b1;
+        const float rad = tr[j] != 0.f ? fmaf(tr[j], up, radsrc[j]) : radsrc[j];
+        rcur[j * nV] = rad;
+        put(j, rad);
+        if (j == 0 && pusher && t + 1 < nT) push_row(t, rad);
+        b0 = b1;
+      }
+  };
+  auto combine = [&](int t, auto &&put) {
+    // the row above this thread's last (a row of fixed points has none: any slot)
+    const float *hal = q0 + kn < nrow ? rprev + kn * nV : halo + ((t - 1) % MRING) * nV + v;
+    if (above && !tc::mbar_wait(full0 + 8 * ((t - 1) % MRING), (uint32_t)((t - 1) / MRING) & 1u, lim)) expired();
+    if (kn == RM) combine_rows(t, std::true_type{}, hal, put);
+    else if (kn > 0) combine_rows(t, std::false_type{}, hal, put);
+    float *x = rprev; rprev = rcur; rcur = x;
+  };
+  // Forms (radsrc, tr) of a plane from the previous plane's (source x ext,
+  // ext) and the points' own (row j: source o[j ostep], extinction oe
+  // further), which it stores; the radiances of fixed points (of[ofs slot])
+  // stand in for radsrc.
+  auto integrate_rows = [&](auto full, const float *o, int ostep, int oe) {
+    const float2 g2 = make_float2(gx, gx), f2 = make_float2(fx, fx), gu = make_float2(gw, gw), fu = make_float2(fw, fw);
+    float2 b0 = lerp2(sprev[0], sprev[sdv], g2, f2);
+#pragma unroll
+    for (int j = 0; j < RM; ++j)
+      if (full.value || j < kn) {
+        const float2 *p = sprev + (j + 1) * nV;
+        const float2 b1 = lerp2(p[0], p[sdv], g2, f2);
+        const float2 f = lerp2(b0, b1, gu, fu);
+        const float e = o[j * ostep + oe], se = o[j * ostep] * e;
+        scur[j * nV] = make_float2(se, e);
+        cell_source_march(f.y, f.x, e, se, so, radsrc[j], tr[j], clamp);
+        b0 = b1;
+      }
+  };
+  auto integrate = [&](const float *o, int ostep, int oe, const float *of, int ofs) {
+    if (kn == RM) integrate_rows(std::true_type{}, o, ostep, oe);
+    else if (kn > 0) integrate_rows(std::false_type{}, o, ostep, oe);
+    if (fix) {
+#pragma unroll
+      for (int j = 0; j < RM; ++j)
+        if ((fix >> j) & 1) { radsrc[j] = of[ofs * fixslot(j)]; tr[j] = 0.f; }
+    }
+    if (above) {
+      const float e = o[kn * ostep + oe];
+      scur[kn * nV] = make_float2(o[kn * ostep] * e, e);
+    }
+    float2 *x = sprev; sprev = scur; scur = x;
+  };
+  // the barrier before plane t - 1 is combined and plane t integrated; plane
+  // t - 2 has been combined, so the halo slot of plane t - 3 goes back
+  auto next_plane = [&](int t) {
+    __syncthreads();
+    if (tid == 0 && from_up && t >= 3 && t - 3 + MRING < nT - 1) {
+      tc::mbar_expect_tx(full0 + 8 * ((t - 3) % MRING), 4 * nV);
+      march_arrive(empty0 + 8 * ((t - 3) % MRING), rank + 1);
+    }
+  };
+  // plane 0 (the upwind boundary plane) is fixed
+  {
+    int p = G.a0 * G.sa + p0;
+#pragma unroll
+    for (int j = 0; j <= RM; ++j) {
+      if (j < RM) radsrc[j < RM ? j : 0] = tr[j < RM ? j : 0] = 0.f;
+      if (j < kn || (j == kn && above)) {
+        const float s = __ldg(src + p), e = __ldg(a.text + p);
+        sprev[j * nV] = make_float2(s * e, e);
+      }
+      if (j < kn) {
+        const float rad = rado[p];
+        rprev[j * nV] = rad;
+        if (pusher && j == 0 && nT > 1) push_row(0, rad);
+      }
+      p += ustep;
+    }
+  }
+  if constexpr (!ZC) {
+    weights(load_g(v));
+    cx = fx; cgx = gx; cw = fw; cgw = gw;
+    const int nl = kn + (above ? 1 : 0);
+    unsigned pf = (unsigned)((G.a0 + G.da) * G.sa + p0);  // first row's point in the plane fetched next
+    float *dst = own + r0off, *dfr = ownr;                 // and where its values go
+    auto fetch = [&](int t) {  // plane t's own values on their way (an empty group past the last plane)
+      if (t < nT) {
+        unsigned p = pf;
+#pragma unroll
+        for (int j = 0; j <= RM; ++j) {
+          if (j < nl) {
+            cp_async(dst + j * nV, src + p);
+            cp_async(dst + j * nV + N1, a.text + p);
+          }
+          p += ustep;
+        }
+        if (fix) {
+#pragma unroll
+          for (int j = 0; j < RM; ++j)
+            if ((fix >> j) & 1) cp_async(dfr + fixslot(j), rado + (pf + j * ustep));
+        }
+        pf += astep;
+        dst += 2 * N1;
+        dfr += nfix;
+        if ((t % MDEPTH) == 0) { dst = own + r0off; dfr = ownr; }  // slots of planes 1 .. MDEPTH, in turn
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+#pragma unroll 1
+    for (int t = 1; t < MDEPTH; ++t) fetch(t);
+    unsigned pc = (unsigned)(G.a0 * G.sa + p0);  // first row's point in plane t - 1
+    const float *o = own + r0off, *of = ownr;
+#pragma unroll 1
+    for (int t = 1; t <= nT; ++t) {  // combine plane t - 1, then integrate plane t
+      next_plane(t);
+      if (t > 1)
+        combine(t - 1, [&](int j, float rad) {
+          if (!((fix >> j) & 1)) rado[pc + j * ustep] = rad;
+        });
+      if (t < nT) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(MDEPTH - 2) : "memory");
+        integrate(o, nV, N1, of, 1);
+        o += 2 * N1;
+        of += nfix;
+        if ((t % MDEPTH) == 0) { o = own + r0off; of = ownr; }
+        fetch(t + MDEPTH - 1);
+      }
+      pc += astep;
+    }
+  } else {
+    // four layers (z & ~3 and the next three) of this thread's points at a
+    // time, staged in shared memory one group ahead; a combined radiance takes
+    // the place of its point's source, and the group is stored once its last
+    // plane is combined
+    const bool up = G.da > 0, vec = (a.nz & 3) == 0;
+    float *const fs = own + 4 * r0off;
+    for (int i = tid; i < a.nz; i += blockDim.x) sgeo[i] = load_g(i);
+    auto stage = [&](int zg) {
+      int p = p0 + 4 * zg;
+      float *d = fs + (zg & 1) * 8 * N1;
+#pragma unroll
+      for (int j = 0; j <= RM; ++j) {
+        if (j < kn || (j == kn && above)) {
+          if (vec) {
+            cp_async16(d, src + p);
+            cp_async16(d + 4 * N1, a.text + p);
+          } else {
+            for (int k = 0; k < 4; ++k)
+              if (4 * zg + k < a.nz) {
+                cp_async(d + k, src + p + k);
+                cp_async(d + 4 * N1 + k, a.text + p + k);
+              }
+          }
+        }
+        if (j < RM && ((fix >> j) & 1)) {
+          float *f = ownr + (zg & 1) * 4 * nfix + 4 * fixslot(j);
+          if (vec) cp_async16(f, rado + p);
+          else
+            for (int k = 0; k < 4; ++k)
+              if (4 * zg + k < a.nz) cp_async(f + k, rado + p + k);
+        }
+        p += ustep;
+        d += 4 * nV;
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    auto flush = [&](int zg) {
+      int p = p0 + 4 * zg;
+      const float *d = fs + (zg & 1) * 8 * N1;
+#pragma unroll
+      for (int j = 0; j < RM; ++j) {
+        if (j < kn && !((fix >> j) & 1)) {
+          if (vec && zg != (G.a0 >> 2)) {
+            *reinterpret_cast<float4 *>(rado + p) = *reinterpret_cast<const float4 *>(d);
+          } else {
+            for (int k = 0; k < 4; ++k)
+              if (4 * zg + k < a.nz && 4 * zg + k != G.a0) rado[p + k] = d[k];
+          }
+        }
+        p += ustep;
+        d += 4 * nV;
+      }
+    };
+    int z = G.a0;  // the layer of plane t
+    stage(z >> 2);
+    int zstaged = z >> 2, zhave = -1;  // the group staged last and the one in use
+#pragma unroll 1
+    for (int t = 0; t < nT; ++t) {  // combine plane t, then integrate plane t + 1
+      const int zn = z + G.da, zg = zn >> 2;
+      next_plane(t + 1);
+      if (t > 0) {
+        float *d = fs + ((z >> 2) & 1) * 8 * N1 + (z & 3);
+        combine(t, [&](int j, float rad) { d[4 * j * nV] = rad; });
+      }
+      if (t + 1 == nT) { flush(z >> 2); break; }
+      if (t > 0 && zg != z >> 2) flush(z >> 2);
+      weights(sgeo[zn]);
+      if (zg != zhave) {  // entering group zg: wait for it, then stage the one after
+        if (zg != zstaged) stage(zg);
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        zhave = zg;
+        zstaged = zg + (up ? 1 : -1);
+        if (zstaged >= 0 && 4 * zstaged < a.nz) stage(zstaged);
+      }
+      integrate(fs + (zg & 1) * 8 * N1 + (zn & 3), 4 * nV, 4 * N1, ownr + (zg & 1) * 4 * nfix + (zn & 3), 4);
+      cx = fx; cgx = gx; cw = fw; cgw = gw;
+      z = zn;
+    }
+  }
+}
+
+template <int RM, bool ZC>
+__global__ void __launch_bounds__(MMAXT) k_sweep_march(SweepArgs a, const MarchGrp *__restrict__ grps,
+                                                       const MarchUnit *__restrict__ units, int smem_words) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const int cs = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const MarchUnit U = units[blockIdx.x / cs];
   const MarchGrp G = grps[U.grp];
-  const int nc = U.nc, nV = G.nV, tw = U.tw, ldo = a.ldo;
-  const int u0 = rank * tw, nrow = max(0, min(tw, G.nU - u0));
-  extern __shared__ float4 msm4[];
-  float4 *sgeo = msm4;                                   // [nV][nc]
-  float *buf0 = reinterpret_cast<float *>(msm4 + (size_t)nV * nc);
-  const int bsz = (int)march_buf_floats(tw, nV, nc);
-  const int rsz = (tw + 2) * nV * nc;                    // one rad (or se) array
-  // this CTA's row that the downwind CTA (rank - upu) reads as its halo row,
-  // and the halo row's index in that CTA's buffers
-  const int cons = rank - G.upu;
-  const bool push = nrow > 0 && cons >= 0 && cons < cs && cons * tw < G.nU;
-  const int push_row = G.upu > 0 ? 0 : tw - 1;
-  const int halo_lr = G.upu > 0 ? tw : -1;
-  float *cons_buf0 = push ? cl.map_shared_rank(buf0, cons) : nullptr;
-  // thread -> column c and the strip's (row, v) pairs k0, k0 + tpc, ... (at most MK)
-  const int tpc = MT / nc, c = threadIdx.x % nc, k0 = threadIdx.x / nc;
-  const int col = U.c0 + c;
-  const bool clamp = !a.stk || !a.stk[col];
-  const bool pad = __ldg(a.col_cz + col) == 0.f;
-  const int kn = k0 < tpc ? max(0, (nrow * nV - k0 + tpc - 1) / tpc) : 0;
-  const int r0 = k0 / nV, v0 = k0 - r0 * nV;
-  const int ndn = G.cls == 0 ? a.nx1 : (G.cls == 1 ? a.ny1 : a.nz);  // extent of the class axis
-  auto plane_fixed = [&](int A) {
-    return pad || (G.cls == 2 && A == G.zfix) || (G.cls == 0 && G.xedge && (A == 0 || A == ndn - 1)) ||
-           (G.cls == 1 && G.yedge && (A == 0 || A == ndn - 1));
-  };
-  // per pair: fixed in every plane (from u, v alone), and whether the face
-  // corners lie inside the grid
-  unsigned uvfix = 0, valid = 0;
-  {
-    int r = r0, v = v0;
-#pragma unroll 1
-    for (int j = 0; j < kn; ++j) {
-      const int u = u0 + r;
-      const bool f = (G.cls != 2 && v == G.zfix) || (G.xedge && G.cls != 0 && (u == 0 || u == a.nx1 - 1)) ||
-                     (G.yedge && ((G.cls == 0 && (u == 0 || u == a.ny1 - 1)) ||
-                                  (G.cls == 2 && (v == 0 || v == a.ny1 - 1))));
-      bool ok = true;
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int uu = u + G.du[k], vv = v + G.dv[k];
-        ok = ok && uu >= 0 && uu < G.nU && vv >= 0 && vv < nV;
-      }
-      uvfix |= (unsigned)f << j;
-      valid |= (unsigned)ok << j;
-      v += tpc;
-      while (v >= nV) { v -= nV; ++r; }
-    }
+  extern __shared__ __align__(16) unsigned char msm[];
+  const uint32_t bar0 = (uint32_t)__cvta_generic_to_shared(msm);
+  // positions that nothing writes are read (and multiplied by zero) beside fixed points
+  for (int i = 64 + threadIdx.x; i < smem_words; i += blockDim.x) reinterpret_cast<float *>(msm)[i] = 0.f;
+  if (threadIdx.x == 0) {
+    const int tw = (G.nU + cs - 1) / cs;
+    for (int i = 0; i < 2 * MRING; ++i) tc::mbar_init(bar0 + 8 * i, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;");
+    if ((rank + 1) * tw < G.nU)
+      for (int i = 0; i < MRING; ++i) tc::mbar_expect_tx(bar0 + 8 * i, 4 * G.nV);
   }
-  // face geometry of the x and y classes: one entry per (v, column)
-  if (G.cls != 2) {
-    for (int i = threadIdx.x; i < nV * nc; i += MT) {
-      const int v = i / nc, cc = i - v * nc;
-      const int layer = (G.b & 4) ? v - 1 : v;
-      sgeo[i] = (layer >= 0 && layer < a.nz - 1)
-                    ? __ldg(reinterpret_cast<const float4 *>(a.geo) + (size_t)layer * a.nang + U.c0 + cc)
-                    : make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  // plane 0 (the upwind boundary plane) is fixed: radiance, source x extinction
-  // and extinction into buffer 0 (and its halo row into the downwind CTA's)
-  {
-    int r = r0, v = v0;
-#pragma unroll 1
-    for (int j = 0; j < kn; ++j) {
-      const int p = G.a0 * G.sa + (u0 + r) * G.su + v * G.sv;
-      const float rad = __ldg(a.raddo + (size_t)p * ldo + col), s = __ldg(a.srcdo + (size_t)p * ldo + col),
-                  e = __ldg(a.text + p);
-      const int sp = (r + 1) * nV + v, si = sp * nc + c;
-      buf0[si] = rad; buf0[rsz + si] = s * e; buf0[2 * rsz + sp] = e;
-      if (push && r == push_row) {
-        const int hp = (halo_lr + 1) * nV + v, hi = hp * nc + c;
-        cons_buf0[hi] = rad; cons_buf0[rsz + hi] = s * e; cons_buf0[2 * rsz + hp] = e;
-      }
-      v += tpc;
-      while (v >= nV) { v -= nV; ++r; }
-    }
-  }
-  // the point's own ordinate source and extinction (and, at fixed points,
-  // its final radiance), loaded one plane ahead
-  float ps[MK], pe[MK], pr[MK];
-  {
-    const int A = G.a0 + G.da;
-    const bool pf = G.nA > 1 && plane_fixed(A);
-    int r = r0, v = v0;
-#pragma unroll
-    for (int j = 0; j < MK; ++j) {
-      ps[j] = 0.f; pe[j] = 0.f; pr[j] = 0.f;
-      if (j < kn && G.nA > 1) {
-        const int p = A * G.sa + (u0 + r) * G.su + v * G.sv;
-        ps[j] = __ldg(a.srcdo + (size_t)p * ldo + col);
-        pe[j] = __ldg(a.text + p);
-        if (pf || ((uvfix >> j) & 1)) pr[j] = __ldg(a.raddo + (size_t)p * ldo + col);
-      }
-      v += tpc;
-      while (v >= nV) { v -= nV; ++r; }
-    }
-  }
-  float4 gz = make_float4(0.f, 0.f, 0.f, 0.f);
-  auto load_gz = [&](int A) {
-    const int layer = (G.b & 4) ? A - 1 : A;
-    return (G.cls == 2 && kn > 0 && layer >= 0 && layer < a.nz - 1)
-               ? __ldg(reinterpret_cast<const float4 *>(a.geo) + (size_t)layer * a.nang + col)
-               : make_float4(0.f, 0.f, 0.f, 0.f);
-  };
-  if (G.nA > 1) gz = load_gz(G.a0 + G.da);
-  // corner offsets relative to the point itself, in the previous plane's buffers
-  int qs[4], qe[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) { qe[k] = G.du[k] * nV + G.dv[k]; qs[k] = qe[k] * nc; }
-  // pair j sits at strip point k0 + j tpc: buffer point sp0 + j tpc, item si0 + j tpc nc
-  const int sp0 = k0 + nV, si0 = sp0 * nc + c, sstep = tpc * nc;
-  const int pb0 = (u0 + r0) * G.su + v0 * G.sv;  // pair 0's point index less the plane's
   cl.sync();
-  for (int t = 1; t < G.nA; ++t) {
-    const int A = G.a0 + t * G.da, An = A + G.da;
-    const bool more = t + 1 < G.nA;
-    const bool pf = plane_fixed(A), pfn = more && plane_fixed(An);
-    const float *prev = buf0 + ((t - 1) & 1) * bsz;
-    float *cur = buf0 + (t & 1) * bsz;
-    float *ccur = push ? cons_buf0 + (t & 1) * bsz : nullptr;
-    const float4 g2 = gz;
-    if (more) gz = load_gz(An);
-    // the plane's radiances from the previous plane, into shared memory,
-    // and each pair's inputs in the next plane into registers
-    const int Aoff = A * G.sa, step_n = G.da * G.sa;
-    {
-      int r = r0, v = v0, pb = pb0;
-#pragma unroll
-      for (int j = 0; j < MK; ++j) {
-        if (j < kn) {
-          const int sp = sp0 + j * tpc, si = si0 + j * sstep;
-          const float s1 = ps[j], e1 = pe[j];
-          float rad;
-          if (pf || ((uvfix >> j) & 1)) {
-            rad = pr[j];
-          } else if (!((valid >> j) & 1)) {
-            atomicCAS(a.err, ERR_NONE, ERR_SWEEP_NOFACE);
-            rad = 0.f;
-          } else {
-            const float4 g = G.cls == 2 ? g2 : sgeo[v * nc + c];
-            const float fu = g.y, fv = g.z;
-            const float f0 = (1.f - fu) * (1.f - fv), f1 = (1.f - fu) * fv, f2 = fu * (1.f - fv), f3 = fu * fv;
-            const float *pe_ = prev + 2 * rsz + sp, *ps_ = prev + rsz + si, *pr_ = prev + si;
-            const float ext0 = f0 * pe_[qe[0]] + f1 * pe_[qe[1]] + f2 * pe_[qe[2]] + f3 * pe_[qe[3]];
-            const float srcext0 = f0 * ps_[qs[0]] + f1 * ps_[qs[1]] + f2 * ps_[qs[2]] + f3 * ps_[qs[3]];
-            float radsrc, tr;
-            cell_source(ext0, srcext0, e1, e1 * s1, g.x, radsrc, tr, clamp);
-            rad = radsrc;
-            if (tr != 0.f) rad += tr * (f0 * pr_[qs[0]] + f1 * pr_[qs[1]] + f2 * pr_[qs[2]] + f3 * pr_[qs[3]]);
-          }
-          if (!(pf || ((uvfix >> j) & 1))) a.raddo[(size_t)(Aoff + pb) * ldo + col] = rad;
-          cur[si] = rad; cur[rsz + si] = s1 * e1; cur[2 * rsz + sp] = e1;
-          if (push && r == push_row) {
-            const int hp = (halo_lr + 1) * nV + v, hi = hp * nc + c;
-            ccur[hi] = rad; ccur[rsz + hi] = s1 * e1; ccur[2 * rsz + hp] = e1;
-          }
-          if (more) {
-            const int pn = Aoff + pb + step_n;
-            ps[j] = __ldg(a.srcdo + (size_t)pn * ldo + col);
-            pe[j] = __ldg(a.text + pn);
-            if (pfn || ((uvfix >> j) & 1)) pr[j] = __ldg(a.raddo + (size_t)pn * ldo + col);
-          }
-        }
-        v += tpc; pb += tpc * G.sv;
-        while (v >= nV) { v -= nV; ++r; pb += G.su - nV * G.sv; }
-      }
-    }
-    cl.sync();  // plane t is in every strip's current buffer and halo row; the previous buffers are free
-  }
+  march_column<RM, ZC>(a, G, U.col, msm, cs, rank);
+  cl.sync();  // no CTA leaves while another may still send into it or arrive on its barriers
 }
+
+// Cycles of the march that choose its cluster size and threads: issue slots
+// per row and warp, and per plane and warp, at the instructions per cycle
+// reached; the latency of a plane, and of each further row of a thread.
+// Fitted to 217 timings (six grids from 24x24x16 to 128x128x64, 1 to 16
+// CTAs per column, 64 to 512 threads; 29% rms), over which the choice is
+// within 17% of the best shape, 5% in the mean.
+constexpr double kMarchRow = 33, kMarchPlane = 184, kMarchIdle = 20, kMarchIpc = 1.97, kMarchLat = 633, kMarchRowLat = 575;
 
 // Sequential-order sweep for grids whose wavefront is too deep (periodic
 // wrap-around long characteristics chain points of one ordinate through the
@@ -1300,7 +1548,7 @@ __global__ void __launch_bounds__(SEQW) k_sweep_seq(SweepArgs a, const int *orde
   __shared__ float4 sc[2][SEQN];
   __shared__ short4 sd[2][SEQN];
   __shared__ int spt[3][SEQN];
-  const int col = col_begin + blockIdx.x, ldo = a.ldo, n = a.npts;
+  const int col = col_begin + blockIdx.x, n = a.npts;
   if (a.col_cz[col] == 0.f) return;  // padding ordinate
   const int b = col_octant(a, col);
   const int hb = (b & 4) ? 2 : 1;
@@ -1335,7 +1583,7 @@ __global__ void __launch_bounds__(SEQW) k_sweep_seq(SweepArgs a, const int *orde
             const float wt = R.tr * f[k];
             if (wt == 0.f) continue;
             if (a.bnd[q[k]] & hb) {  // a preset boundary point: final
-              wv += wt * a.raddo[(size_t)q[k] * ldo + col];
+              wv += wt * a.raddo[a.at(q[k], col)];
               continue;
             }
             const int rq = rk[q[k]];
@@ -1349,7 +1597,7 @@ __global__ void __launch_bounds__(SEQW) k_sweep_seq(SweepArgs a, const int *orde
             } else if (rq >= r0 - 2 * SEQN) {  // window w - 2: final, in the ring
               wv += wt * sval[pw * SEQN + (rq - (r0 - 2 * SEQN))];
             } else {
-              wv += wt * a.raddo[(size_t)q[k] * ldo + col];
+              wv += wt * a.raddo[a.at(q[k], col)];
             }
           }
         }
@@ -1365,7 +1613,7 @@ __global__ void __launch_bounds__(SEQW) k_sweep_seq(SweepArgs a, const int *orde
     const int pw = w & 1;
     for (int j = tid - t0; j < SEQN; j += nt) {
       const int pt = spt[w % 3][j];
-      if (pt >= 0) a.raddo[(size_t)pt * ldo + col] = sval[pw * SEQN + j];
+      if (pt >= 0) a.raddo[a.at(pt, col)] = sval[pw * SEQN + j];
     }
   };
   if (nwin > 0) prep(0, 0, SEQW);
@@ -1464,28 +1712,87 @@ __global__ void __launch_bounds__(256) k_do_to_sh_light(const float *__restrict_
   }
 }
 
+// The same on ordinate-major radiances: a block takes 32 points, lanes over
+// the points (consecutive, or nearly), its 8 warps a share of the columns
+// each; the partial sums meet in shared memory.
+__global__ void __launch_bounds__(256) k_do_to_sh_light_om(const float *__restrict__ raddo, size_t cs, int nang, int ncol_down,
+                                                            const int *__restrict__ pts, int npts_light,
+                                                            const float *__restrict__ t4, const float *__restrict__ fluxw,
+                                                            float *__restrict__ radiance, int nlm, float *__restrict__ fluxes) {
+  extern __shared__ float4 wsm4[];  // [nang][2]: the four l <= 1 weights, then (down, up) flux weights
+  __shared__ float part[6][8][32];
+  for (int c = threadIdx.x; c < nang; c += blockDim.x) {
+    const float w = __ldg(fluxw + c);
+    wsm4[2 * c] = make_float4(__ldg(t4 + c), __ldg(t4 + nang + c), __ldg(t4 + 2 * nang + c), __ldg(t4 + 3 * nang + c));
+    wsm4[2 * c + 1] = make_float4(c < ncol_down ? w : 0.f, c < ncol_down ? 0.f : w, 0.f, 0.f);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  const int p = i < npts_light ? __ldg(pts + i) : -1;
+  const int per = (nang + 7) / 8, c1 = min(nang, (wp + 1) * per);
+  float acc[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  if (p >= 0) {
+    const float *x = raddo + p;
+#pragma unroll 8
+    for (int c = wp * per; c < c1; ++c) {
+      const float v = __ldcs(x + (size_t)c * cs);  // read once: streamed past L1
+      const float4 t = wsm4[2 * c];
+      const float2 f = *reinterpret_cast<const float2 *>(&wsm4[2 * c + 1]);
+      acc[0] = fmaf(t.x, v, acc[0]); acc[1] = fmaf(t.y, v, acc[1]); acc[2] = fmaf(t.z, v, acc[2]);
+      acc[3] = fmaf(t.w, v, acc[3]); acc[4] = fmaf(f.x, v, acc[4]); acc[5] = fmaf(f.y, v, acc[5]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 6; ++r) part[r][wp][lane] = acc[r];
+  __syncthreads();
+  if (wp < 6) {
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += part[wp][k][lane];
+    if (p >= 0) {
+      if (wp < 4) radiance[(size_t)p * nlm + wp] = s;
+      else fluxes[2 * (size_t)p + wp - 4] = s;
+    }
+  }
+}
+
+// Transposes in [rows][cols] (row stride ldi) into out [cols][rows] (row stride ldo).
+__global__ void __launch_bounds__(256) k_transpose(const float *__restrict__ in, size_t ldi, float *__restrict__ out, size_t ldo,
+                                                   int rows, int cols) {
+  __shared__ float tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, nr = (rows + 31) / 32;
+  const int c0 = (int)(blockIdx.x / nr) * 32;
+  const size_t r0 = (size_t)(blockIdx.x % nr) * 32;
+  for (int k = ty; k < 32; k += 8)
+    if (r0 + k < (size_t)rows && c0 + tx < cols) tile[k][tx] = in[(r0 + k) * ldi + c0 + tx];
+  __syncthreads();
+  for (int k = ty; k < 32; k += 8)
+    if (c0 + k < cols && r0 + tx < (size_t)rows) out[(size_t)(c0 + k) * ldo + r0 + tx] = tile[tx][k];
+}
+
 // stk (polarized): Stokes component per column; the sky and the surface
 // emit unpolarized radiance, so the Q and U columns are preset to zero.
-__global__ void k_preset_top(const int *topp, int ntop, float *raddo, int ldo, int ncol_down, float skyrad,
+__global__ void k_preset_top(const int *topp, int ntop, float *raddo, size_t ps, size_t cs, int ncol_down, float skyrad,
                              const uint8_t *stk) {
   int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= ntop * ncol_down) return;
   int k = t / ncol_down, c = t - k * ncol_down;
-  raddo[(size_t)topp[k] * ldo + c] = (stk && stk[c]) ? 0.f : skyrad;
+  raddo[(size_t)topp[k] * ps + (size_t)c * cs] = (stk && stk[c]) ? 0.f : skyrad;
 }
 
 // FIXED/VARIABLE_LAMBERTIAN_BOUNDARY (src/polarized/shdomsub1.f:2438-2529):
 // the reflected direct beam and downwelling flux plus, with a thermal
 // source, the ground emission (1 - albedo) B (botplanck null otherwise).
 __global__ void k_lambertian(const int *botp, int nbot, const float *botalb, const float *dirflux, const float *fluxw,
-                             float *raddo, int nang, int ldo, int ncol_down, float *bcrad, const uint8_t *stk,
+                             float *raddo, int nang, size_t ps, size_t cs, int ncol_down, float *bcrad, const uint8_t *stk,
                              const float *botplanck) {
   int k = blockIdx.x;
   if (k >= nbot) return;
   int p = botp[k];
   __shared__ float red[256];
   float s = 0.f;
-  for (int c = threadIdx.x; c < ncol_down; c += blockDim.x) s += fluxw[c] * raddo[(size_t)p * ldo + c];
+  for (int c = threadIdx.x; c < ncol_down; c += blockDim.x) s += fluxw[c] * raddo[(size_t)p * ps + (size_t)c * cs];
   red[threadIdx.x] = s;
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {
@@ -1496,7 +1803,8 @@ __global__ void k_lambertian(const int *botp, int nbot, const float *botalb, con
   float b = opi * botalb[k] * (dirflux[p] + red[0]);
   if (botplanck) b += botplanck[k] * (1.f - botalb[k]);
   if (threadIdx.x == 0) bcrad[k] = b;
-  for (int c = ncol_down + threadIdx.x; c < nang; c += blockDim.x) raddo[(size_t)p * ldo + c] = (stk && stk[c]) ? 0.f : b;
+  for (int c = ncol_down + threadIdx.x; c < nang; c += blockDim.x)
+    raddo[(size_t)p * ps + (size_t)c * cs] = (stk && stk[c]) ? 0.f : b;
 }
 
 // Polarized transforms on the CUDA cores (the FP32 path): C[M][N] = A[M][K]
@@ -2055,14 +2363,14 @@ __device__ __forceinline__ void surface_brdf_d(int type, const float *par, float
 __global__ void __launch_bounds__(128) k_brdf_bottom(const int *__restrict__ botp, int nbot, const float *__restrict__ botpar,
                                                      int npar, int type, const BrdfOrd *__restrict__ dn, int ndn,
                                                      const BrdfOrd *__restrict__ up, int nup, const float *__restrict__ dirflux,
-                                                     float solarmu, float solaraz, float *raddo, int ldo, int nst,
+                                                     float solarmu, float solaraz, float *raddo, size_t ps, size_t cs, int nst,
                                                      const float *__restrict__ botplanck) {
   const int b = blockIdx.x;
   if (b >= nbot) return;
   const int p = botp[b];
   const float *par = botpar + (size_t)b * npar;
   const float opi = 0.318309886f;
-  const float *row = raddo + (size_t)p * ldo;
+  float *row = raddo + (size_t)p * ps;
   for (int u = threadIdx.x; u < nup; u += blockDim.x) {
     const BrdfOrd o = up[u];
     float R[3][3], out[3];
@@ -2073,7 +2381,7 @@ __global__ void __launch_bounds__(128) k_brdf_bottom(const int *__restrict__ bot
       surface_brdf_d(type, par, o.mu, o.phi, i.mu, i.phi, R);
       const int ci = (int)i.col, oi = (int)i.off;
       for (int k1 = 0; k1 < nst; ++k1) {
-        const float rin = row[ci + k1 * oi];
+        const float rin = row[(size_t)(ci + k1 * oi) * cs];
         for (int k = 0; k < nst; ++k) out[k] += i.w * R[k][k1] * rin;
       }
       if (botplanck) {  // polarized thermal emission, emissivity 1 - R11
@@ -2083,7 +2391,7 @@ __global__ void __launch_bounds__(128) k_brdf_bottom(const int *__restrict__ bot
       }
     }
     const int co = (int)o.col, oo = (int)o.off;
-    for (int k = 0; k < nst; ++k) raddo[(size_t)p * ldo + co + k * oo] = out[k];
+    for (int k = 0; k < nst; ++k) row[(size_t)(co + k * oo) * cs] = out[k];
   }
 }
 
@@ -2415,7 +2723,8 @@ struct RenderArgs {
   // bidirectional surface (brdf != 0): parameters at the bottom points, the
   // downward ordinates of the reflection sum and the ordinate radiances of
   // the last sweep (the downwelling radiances at the surface)
-  int brdf, nsfcpar, nbrdf_dn, ldo;
+  int brdf, nsfcpar, nbrdf_dn;
+  size_t ord_ps, ord_cs;  // strides of a point and of a column in raddo
   const float *botpar, *raddo;
   const float *botplanck;  // thermal source: B at the bottom points, else null
   const BrdfOrd *brdf_dn;
@@ -2437,7 +2746,7 @@ struct RenderArgs {
 __device__ __noinline__ void brdf_radiance_warp(const RenderArgs &a, int bi, float mu2, float phi2, int lane, int nst, float out[3]) {
   const float *par = a.botpar + (size_t)bi * a.nsfcpar;
   const int p = a.botp[bi];
-  const float *row = a.raddo + (size_t)p * a.ldo;
+  const float *row = a.raddo + (size_t)p * a.ord_ps;
   float acc[3] = {0.f, 0.f, 0.f}, R[3][3];
   if (lane == 0) {
     surface_brdf_d(a.brdf, par, mu2, phi2, a.solarmu, a.solaraz, R);
@@ -2448,7 +2757,7 @@ __device__ __noinline__ void brdf_radiance_warp(const RenderArgs &a, int bi, flo
     surface_brdf_d(a.brdf, par, mu2, phi2, i.mu, i.phi, R);
     const int ci = (int)i.col, oi = (int)i.off;
     for (int k1 = 0; k1 < nst; ++k1) {
-      const float rin = row[ci + k1 * oi];
+      const float rin = row[(size_t)(ci + k1 * oi) * a.ord_cs];
       for (int k = 0; k < nst; ++k) acc[k] += i.w * R[k][k1] * rin;
     }
     if (a.botplanck) {
@@ -3292,7 +3601,13 @@ struct Handle {
   DBuf<int> ns, nso, nr, errflag;
   DBuf<double> red;
   DBuf<AccelState> accel;
-  int ldo = 0;  // row stride of srcdo/raddo: nang rounded up to 4 (16-byte rows for TMA)
+  int ldo = 0;  // columns of srcdo/raddo: nang rounded up to 4 (16-byte rows for TMA)
+  // srcdo/raddo are ordinate-major (a column's points contiguous, padded to
+  // 32) when both hemispheres are swept column by column (the plane march or
+  // the reference order), else point-major for the level schedule
+  bool ord_major = false;
+  size_t ord_ps = 0, ord_cs = 0;  // strides of a point and of a column
+  DBuf<float> xf_rows;            // ordinate-major: point-major rows for the CUDA-core transforms
   // tensor-core transforms, per direction (0: SH -> DO, 1: DO -> SH)
   int xf_mode = 0;  // 0: 3xTF32 tensor cores, 1: single TF32 product, 2: CUDA-core factorized
   bool tc_ok[2] = {false, false};
@@ -3314,16 +3629,16 @@ struct Handle {
   int np1blk[2] = {0, 0};
   size_t p1smem[2] = {0, 0};
   DBuf<int> p1base[2], p1grp[2], p1slot[2];  // per segment: first slot, group; [group][point]: slot or -1
-  // plane-march phase 2 per hemisphere (k_sweep_march): units of (group,
-  // column slice), one cluster of mcs[h] CTAs each
+  // plane-march phase 2 per hemisphere (k_sweep_march): one cluster per
+  // column, the x and y classes' columns first
   bool march[2] = {false, false};
   bool march_off = false;  // sweep mode 3: the level schedule even where the march applies
   int render_single_scatter = 0, render_nosurface = 0;  // RENDER options of the following renders
   int tc_wait_limit = tc::kWaitLimit;  // polls of a tensor-core pipeline wait (0 only to test the abort path)
   DBuf<MarchGrp> mgrp[2];
   DBuf<MarchUnit> munit[2];
-  int mnunits[2] = {0, 0}, mcs[2] = {0, 0};
-  size_t msmem[2] = {0, 0};
+  struct MarchLaunch { int units = 0, cs = 0, threads = 0, rows = 0; size_t smem = 0; };
+  MarchLaunch mlaunch[2][2];  // [hemisphere][x and y classes, z class]
 
   bool initialized = false;
   int iters = 0;
@@ -3498,7 +3813,8 @@ static void make_map(CUtensorMap *m, const float *base, uint64_t inner, uint64_t
 // The tensor-core GEMM is instantiated for N tiles of 32..128 columns.
 template <int BN>
 static void tc_attr1() {
-  CK(cudaFuncSetAttribute(tc::k_tc_gemm<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes<BN>()));
+  CK(cudaFuncSetAttribute(tc::k_tc_gemm<BN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes<BN, false>()));
+  CK(cudaFuncSetAttribute(tc::k_tc_gemm<BN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tc::smem_bytes<BN, true>()));
 }
 static void tc_attr(int bn) {
   switch (bn) {
@@ -3510,7 +3826,10 @@ static void tc_attr(int bn) {
 template <int BN>
 static void tc_launch1(int nblocks, cudaStream_t st, const CUtensorMap &a, const CUtensorMap &bh,
                        const CUtensorMap &bl, int K, int ntn, int ntiles, const tc::Epilogue &g) {
-  tc::k_tc_gemm<BN><<<nblocks, tc::kThreads, tc::smem_bytes<BN>(), st>>>(a, bh, bl, K, ntn, ntiles, g);
+  if (g.Aord)
+    tc::k_tc_gemm<BN, true><<<nblocks, tc::kThreads, tc::smem_bytes<BN, true>(), st>>>(a, bh, bl, K, ntn, ntiles, g);
+  else
+    tc::k_tc_gemm<BN, false><<<nblocks, tc::kThreads, tc::smem_bytes<BN, false>(), st>>>(a, bh, bl, K, ntn, ntiles, g);
 }
 // Persistent launch: one CTA per SM (the pipeline fills the shared memory),
 // each walking its share of the ntiles = ntn x row-tile tiles.
@@ -3577,7 +3896,10 @@ static void setup_tc(Handle &H) {
     H.tc_bh[dir].upload(bh);
     H.tc_bl[dir].upload(bl);
     const float *a = dir == 0 ? H.source.p : H.raddo.p;
-    make_map(&H.tm_a[dir], a, (uint64_t)K, (uint64_t)P.npts, (uint64_t)lda, tc::BM);
+    if (dir == 1 && H.ord_major)  // A does not come by TMA (KM)
+      make_map(&H.tm_a[1], H.source.p, (uint64_t)nsh, (uint64_t)P.npts, (uint64_t)nsh, tc::BM);
+    else
+      make_map(&H.tm_a[dir], a, (uint64_t)K, (uint64_t)P.npts, (uint64_t)lda, tc::BM);
     make_map(&H.tm_bh[dir], H.tc_bh[dir].p, (uint64_t)kpad, (uint64_t)npad, (uint64_t)kpad, (uint32_t)bn);
     make_map(&H.tm_bl[dir], H.tc_bl[dir].p, (uint64_t)kpad, (uint64_t)npad, (uint64_t)kpad, (uint32_t)bn);
     H.tc_bn[dir] = bn; H.tc_ntiles[dir] = ntiles; H.tc_kpad[dir] = kpad;
@@ -3605,9 +3927,13 @@ static void setup_tc(Handle &H) {
       H.heavy.upload(hv); H.light.upload(lt);
       if (H.nheavy > 0) {
         H.src_c.alloc((size_t)H.nheavy * P.nlm);
-        H.rad_c.alloc((size_t)H.nheavy * H.ldo);
         make_map(&H.tm_ac[0], H.src_c.p, (uint64_t)P.nlm, (uint64_t)H.nheavy, (uint64_t)P.nlm, tc::BM);
-        make_map(&H.tm_ac[1], H.rad_c.p, (uint64_t)P.nang, (uint64_t)H.nheavy, (uint64_t)H.ldo, tc::BM);
+        if (H.ord_major) {
+          H.tm_ac[1] = H.tm_a[1];
+        } else {
+          H.rad_c.alloc((size_t)H.nheavy * H.ldo);
+          make_map(&H.tm_ac[1], H.rad_c.p, (uint64_t)P.nang, (uint64_t)H.nheavy, (uint64_t)H.ldo, tc::BM);
+        }
       }
     }
   }
@@ -3640,7 +3966,7 @@ static long long plan_device_bytes(const Plan &P) {
   b += vbytes(P.tms_iph) + vbytes(P.tms_w) + vbytes(P.phasetab) + vbytes(P.botalb) + vbytes(P.rad0);
   b += vbytes(P.thermal) + vbytes(P.botplanck) + vbytes(P.planckpt);
   const long long ldo = (P.nang + 3) & ~3;
-  b += 4LL * P.npts * (3LL * P.nst * P.nlm + 2 * ldo + 2 + 3) + 4LL * (long long)P.botp.size() + 64;
+  b += 4LL * P.npts * (3LL * P.nst * P.nlm + 2 + 3) + 8LL * ((P.npts + 31) & ~31) * ldo + 4LL * (long long)P.botp.size() + 64;
   if (P.nst == 3) b += vbytes(P.col_stk) + vbytes(P.coefp) + vbytes(P.phasetab2) + 8LL * P.nlm * 3 * P.nang;
   {  // gathered rows of the scattering points for the compacted transforms
     long long nh = 0;
@@ -3682,104 +4008,125 @@ static void fill_sizes(const Plan &P, shdom_sizes *o) {
   o->march_units_down = o->march_units_up = o->march_cluster_down = o->march_cluster_up = 0;
 }
 
-// Units and cluster shape of the plane march of each hemisphere that has
-// one.  Of 16-CTA and 8-CTA clusters the shape with more CTAs resident at
-// once is taken; the groups are split into column slices in proportion to
-// their work, about as many units as clusters fit on the device at once.
-// (Measured against two other plans: filling whole waves with twice as many
-// narrower units, and the fewest, widest units that fit; both were slower,
-// since a plane's time is mostly the latency of its dependent chain.)  A
-// hemisphere whose units cannot be launched on this device keeps the level
-// schedule.
-constexpr size_t kMarchSmemCap = 110 * 1024;  // two CTAs per SM
+// Cluster size and threads per CTA of the plane march of each hemisphere
+// that has one, for the x and y classes and for the z class.  A hemisphere
+// whose columns cannot be launched on this device keeps the level schedule.
+typedef void (*MarchKernel)(SweepArgs, const MarchGrp *, const MarchUnit *, int);
+constexpr int kMarchRows[6] = {1, 2, 3, 4, 6, MROWS};  // the kernel's rows per thread
+static int march_rows(int rows) {
+  int k = 0;
+  while (kMarchRows[k] < rows) ++k;
+  return k;
+}
+static MarchKernel march_kernel(int rows, bool z) {
+  static const MarchKernel xy[6] = {k_sweep_march<1, false>, k_sweep_march<2, false>, k_sweep_march<3, false>,
+                                    k_sweep_march<4, false>, k_sweep_march<6, false>, k_sweep_march<MROWS, false>};
+  static const MarchKernel zz[6] = {k_sweep_march<1, true>, k_sweep_march<2, true>, k_sweep_march<3, true>,
+                                    k_sweep_march<4, true>, k_sweep_march<6, true>, k_sweep_march<MROWS, true>};
+  return (z ? zz : xy)[march_rows(rows)];
+}
 
-static int march_max_clusters(int cs, size_t smem) {
+static cudaLaunchConfig_t march_config(int units, int cs, int threads, size_t smem, cudaStream_t st, cudaLaunchAttribute *at) {
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = cs; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)cs); cfg.blockDim = dim3(MT); cfg.dynamicSmemBytes = smem;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k_sweep_march, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
+  at->id = cudaLaunchAttributeClusterDimension;
+  at->val.clusterDim.x = cs; at->val.clusterDim.y = 1; at->val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)(units * cs)); cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = smem;
+  cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 1;
+  return cfg;
+}
+
+// The stopping face's corners are the four points of the 2 x 2 stencil
+// towards the upwind sides, one fraction along each transverse axis, and
+// the rows and positions that have no upwind neighbour are fixed points.
+static bool march_stencil_ok(const MarchGrp &g) {
+  const bool vu = g.dv[0] != g.dv[2];
+  for (int k = 0; k < 4; ++k) {
+    const bool k1 = k & 1, k2 = k & 2;  // corner k: second in v for k1, in u for k2
+    if ((g.dv[k] != g.dv[0]) != (vu ? k2 : k1) || (g.du[k] != g.du[0]) != (vu ? k1 : k2)) return false;
   }
-  return n;
+  const bool uend = g.cls == 0 ? g.yedge : g.xedge, vend = g.cls == 2 ? g.yedge : true;
+  return uend && vend;
 }
 
 static void setup_march(Handle &H) {
   Plan &P = H.P;
-  int dev = 0, clus = 0, maxsm = 0;
+  int dev = 0, clus = 0, maxsm = 0, smsm = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&clus, cudaDevAttrClusterLaunch, dev));
   CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  CK(cudaDeviceGetAttribute(&smsm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+  CK(cudaDeviceGetAttribute(&H.nsm, cudaDevAttrMultiProcessorCount, dev));
   H.march[0] = H.march[1] = false;
-  if (!clus || (size_t)maxsm < kMarchSmemCap) return;
-  CK(cudaFuncSetAttribute(k_sweep_march, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
-  const bool big = cudaFuncSetAttribute(k_sweep_march, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
-  if (!big) cudaGetLastError();
-  // resident clusters of each shape at the shared-memory cap; the shape with
-  // more CTAs resident at once is taken
-  int best_cs = 0, best_n = 0;
-  for (int cs : {16, 8}) {
-    if (cs > 8 && !big) continue;
-    const int n = march_max_clusters(cs, kMarchSmemCap);
-    if (n * cs > best_n * best_cs) { best_cs = cs; best_n = n; }
-  }
-  if (best_n < 1) return;
+  if (!clus) return;
   for (int h = 0; h < 2; ++h) {
     if (P.march[h].empty() || H.seq[h]) continue;
-    for (int cs : {best_cs, best_cs == 16 ? 8 : 0}) {
-      if (cs == 0) break;
-      const int nclusters = march_max_clusters(cs, kMarchSmemCap);
-      if (nclusters < 1) continue;
-      // Column slices per group in proportion to its work (planes x plane
-      // points x columns), about one unit per resident cluster, and at
-      // least as many as fit: every thread of a CTA takes one column and at
-      // most MK (row, v) pairs of its strip.
-      double tot = 0;
-      for (const MarchGrp &g : P.march[h]) tot += (double)g.nA * g.nU * g.nV * g.ncol;
-      std::vector<MarchUnit> units;
-      size_t smem = 0;
-      for (size_t gi = 0; gi < P.march[h].size(); ++gi) {
-        const MarchGrp &g = P.march[h][gi];
-        const double w = (double)g.nA * g.nU * g.nV * g.ncol;
-        int nsl = std::max(1, (int)std::floor(nclusters * w / tot));
-        nsl = std::min(nsl, g.ncol);
-        const int tw = (g.nU + cs - 1) / cs;
-        auto fits = [&](int nc) {
-          const int tpc = MT / nc;
-          return tpc >= 1 && (tw * g.nV + tpc - 1) / tpc <= MK && march_smem_bytes(tw, g.nV, nc) <= kMarchSmemCap;
-        };
-        while (nsl < g.ncol && !fits((g.ncol + nsl - 1) / nsl)) ++nsl;
-        if (!fits((g.ncol + nsl - 1) / nsl)) { units.clear(); break; }
-        const int base = g.ncol / nsl, extra = g.ncol % nsl;
-        int c0 = g.col0;
-        for (int k = 0; k < nsl; ++k) {
-          const int nc = base + (k < extra ? 1 : 0);
-          units.push_back(MarchUnit{(int)gi, c0, nc, tw});
-          smem = std::max(smem, march_smem_bytes(tw, g.nV, nc));
-          c0 += nc;
-        }
-      }
-      if (units.empty()) continue;
-      // longest units first (planes x pairs per thread), so that the units
-      // left for the second wave of clusters are the short ones
-      auto unit_time = [&](const MarchUnit &u) {
-        const MarchGrp &g = P.march[h][u.grp];
-        const int tpc = MT / u.nc;
-        return (long long)g.nA * ((u.tw * g.nV + tpc - 1) / tpc);
-      };
-      std::stable_sort(units.begin(), units.end(),
-                       [&](const MarchUnit &x, const MarchUnit &y) { return unit_time(x) > unit_time(y); });
-      std::vector<MarchGrp> grps(P.march[h].begin(), P.march[h].end());
-      H.mgrp[h].upload(grps);
-      H.munit[h].upload(units);
-      H.mnunits[h] = (int)units.size(); H.mcs[h] = cs; H.msmem[h] = smem;
-      H.march[h] = true;
-      break;
+    std::vector<MarchUnit> units[2];
+    bool ok = true;
+    for (size_t gi = 0; gi < P.march[h].size(); ++gi) {
+      const MarchGrp &g = P.march[h][gi];
+      ok = ok && march_stencil_ok(g);
+      for (int c = g.col0; c < g.col0 + g.ncol; ++c)
+        if (P.col_cz[c] != 0.f) units[g.cls == 2].push_back(MarchUnit{(int)gi, c});
     }
+    for (int k = 0; k < 2 && ok; ++k) {
+      Handle::MarchLaunch &L = H.mlaunch[h][k];
+      L.units = 0;
+      if (units[k].empty()) continue;
+      double best = 0;
+      bool found = false;
+      for (int cs : {1, 2, 4, 8, 16})
+        for (int nt = 64; nt <= MMAXT; nt += 32) {
+          size_t smem = 0;
+          int rows = 0;
+          double work = 0, longest = 0;
+          for (const MarchGrp &g : P.march[h]) {
+            if ((g.cls == 2) != (k == 1)) continue;
+            const int tw = (g.nU + cs - 1) / cs, ng = nt / g.nV;
+            if (ng < 1) { rows = MROWS + 1; break; }
+            const int r = (tw + ng - 1) / ng;
+            smem = std::max(smem, march_smem_bytes(tw, g.nV, P.nz, k == 1));
+            rows = std::max(rows, r);
+            // issue slots of a column's planes (cycles of one SM) and the latency of the chain of planes (cycles)
+            const double busy = std::min(nt / 32, ((tw + r - 1) / r * g.nV + 31) / 32);
+            work += (double)g.ncol * cs * g.nA * (busy * (kMarchRow * r + kMarchPlane) + (nt / 32 - busy) * kMarchIdle) / kMarchIpc;
+            longest = std::max(longest, (g.nA + 2.0 * (cs - 1)) * (kMarchLat + kMarchRowLat * r));
+          }
+          if (rows > MROWS || smem > (size_t)maxsm) continue;
+          cudaFuncAttributes fa;
+          CK(cudaFuncGetAttributes(&fa, march_kernel(rows, k == 1)));
+          const int wregs = (fa.numRegs + 7) / 8 * 8 * 32 * ((nt / 32 + 3) / 4 * 4);
+          const int resident = std::min({(int)((size_t)smsm / (smem + 1024)), 65536 / wregs, 2048 / nt, 32});
+          if (resident < 1) continue;
+          const double waves = std::ceil((double)units[k].size() * cs / ((double)resident * H.nsm));
+          const double t = std::max(work / H.nsm, waves * longest) + 0.09 * std::min(work / H.nsm, waves * longest);
+          if (found && t >= best) continue;
+          MarchKernel kn = march_kernel(rows, k == 1);
+          CK(cudaFuncSetAttribute(kn, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
+          if (cs > 8 && cudaFuncSetAttribute(kn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+            cudaGetLastError();
+            continue;
+          }
+          cudaLaunchAttribute at;
+          cudaLaunchConfig_t cfg = march_config(1, cs, nt, smem, nullptr, &at);
+          int n = 0;  // the launch must fit on this device
+          if (cudaOccupancyMaxActiveClusters(&n, kn, &cfg) != cudaSuccess || n < 1) {
+            cudaGetLastError();
+            continue;
+          }
+          best = t;
+          found = true;
+          L.cs = cs; L.threads = nt; L.rows = rows; L.smem = smem;
+        }
+      if (!found) { ok = false; break; }
+      L.units = (int)units[k].size();
+    }
+    if (!ok || (units[0].empty() && units[1].empty())) continue;
+    std::vector<MarchUnit> all(units[0]);
+    all.insert(all.end(), units[1].begin(), units[1].end());
+    std::vector<MarchGrp> grps(P.march[h].begin(), P.march[h].end());
+    H.mgrp[h].upload(grps);
+    H.munit[h].upload(all);
+    H.march[h] = true;
   }
 }
 
@@ -3999,7 +4346,15 @@ static void upload_plan(Handle &H) {
     H.brdf_dn.upload(dn); H.brdf_up.upload(up);
   }
   H.ldo = (P.nang + 3) & ~3;
-  const size_t nf = (size_t)P.npts * H.nst * P.nlm, nd = (size_t)P.npts * H.ldo;
+  setup_march(H);
+  // one hemisphere that the march cannot take puts both on the level schedule
+  for (int h = 0; h < 2; ++h)
+    if (!H.march[h] && !H.seq[h] && (P.seg_off[h].size() > 1 || P.p1off[h].size() > 1)) H.march[0] = H.march[1] = false;
+  H.ord_major = H.march[0] || H.march[1] || (H.seq[0] && H.seq[1]);
+  const size_t npad = ((size_t)P.npts + 31) & ~(size_t)31;
+  H.ord_ps = H.ord_major ? 1 : H.ldo;
+  H.ord_cs = H.ord_major ? npad : 1;
+  const size_t nf = (size_t)P.npts * H.nst * P.nlm, nd = npad * H.ldo;
   H.source.alloc(nf); H.delsource.alloc(nf); H.radiance.alloc(nf);
   H.srcdo.alloc(nd); H.raddo.alloc(nd);
   H.srcdo.zero(H.stream); H.raddo.zero(H.stream);
@@ -4045,10 +4400,10 @@ static void transforms_launch(Handle &H, int dir) {
   int blocks = std::min((P.npts + 7) / 8, 152 * 8);
   if (dir == 0) {
     CK(cudaFuncSetAttribute(k_sh_to_do<NMU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_sh_to_do<NMU><<<blocks, 256, smem, H.stream>>>(x, H.source.p, H.srcdo.p);
+    k_sh_to_do<NMU><<<blocks, 256, smem, H.stream>>>(x, H.source.p, H.ord_major ? H.xf_rows.p : H.srcdo.p);
   } else {
     CK(cudaFuncSetAttribute(k_do_to_sh<NMU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_do_to_sh<NMU><<<blocks, 256, smem, H.stream>>>(x, H.raddo.p, H.radiance.p);
+    k_do_to_sh<NMU><<<blocks, 256, smem, H.stream>>>(x, H.ord_major ? H.xf_rows.p : H.raddo.p, H.radiance.p);
   }
   CK(cudaGetLastError());
   H.launches += 1;
@@ -4066,7 +4421,9 @@ static void transform(Handle &H, int dir) {
     if (dir == 0) {
       g.N = P.nang; g.mode = 0; g.C = H.srcdo.p; g.ldc = H.ldo;
       g.stk = H.nst == 3 ? H.col_stk.p : nullptr;
+      g.ccs = H.ord_major ? H.ord_cs : 0;
     } else {
+      if (H.ord_major) { g.Aord = H.raddo.p; g.acs = H.ord_cs; }
       g.N = nsh; g.mode = 1; g.R = H.radiance.p; g.nlm = P.nlm; g.ldr = nsh; g.nr = H.nr.p; g.fluxes = H.fluxes.p;
       g.fluxw = H.col_fluxw.p; g.ncol_down = P.ncol_down;
     }
@@ -4079,23 +4436,31 @@ static void transform(Handle &H, int dir) {
       if (H.nheavy > 0) {
         const long long q = (long long)H.nheavy * (rowlen / 4);
         const int gb = (int)std::min<long long>((q + 255) / 256, 152 * 16);
-        k_gather_rows<<<gb, 256, 0, H.stream>>>(dir == 0 ? H.source.p : H.raddo.p, H.heavy.p, H.nheavy, rowlen,
-                                                 dir == 0 ? H.src_c.p : H.rad_c.p);
-        CK(cudaGetLastError());
+        if (!g.Aord) {
+          k_gather_rows<<<gb, 256, 0, H.stream>>>(dir == 0 ? H.source.p : H.raddo.p, H.heavy.p, H.nheavy, rowlen,
+                                                   dir == 0 ? H.src_c.p : H.rad_c.p);
+          CK(cudaGetLastError());
+          H.launches += 1;
+        }
         const int ntiles = ntn * ((H.nheavy + tc::BM - 1) / tc::BM);
         tc_launch(H.tc_bn[dir], H.nsm, H.stream, H.tm_ac[dir], H.tm_bh[dir], H.tm_bl[dir], dir == 0 ? P.nlm : P.nang,
                   ntn, ntiles, g);
         CK(cudaGetLastError());
         H.launches += 1;
       }
-      if (dir == 1 && H.nlight > 0) {
+      if (dir == 1 && H.nlight > 0 && H.ord_major) {
+        const int lb = (H.nlight + 31) / 32;
+        k_do_to_sh_light_om<<<lb, 256, 8 * P.nang * sizeof(float), H.stream>>>(
+            H.raddo.p, H.ord_cs, P.nang, P.ncol_down, H.light.p, H.nlight, H.t4.p, H.col_fluxw.p, H.radiance.p, P.nlm, H.fluxes.p);
+        CK(cudaGetLastError());
+        H.launches += 1;
+      } else if (dir == 1 && H.nlight > 0) {
         const int lb = std::min((H.nlight + 7) / 8, 152 * 16);
         k_do_to_sh_light<<<lb, 256, 6 * H.ldo * sizeof(float), H.stream>>>(H.raddo.p, H.ldo, P.nang, P.ncol_down, H.light.p, H.nlight, H.t4.p,
                                                     H.col_fluxw.p, H.radiance.p, P.nlm, H.fluxes.p);
         CK(cudaGetLastError());
         H.launches += 1;
       }
-      H.launches += 1;
       return;
     }
     const int ntiles = ntn * ((P.npts + tc::BM - 1) / tc::BM);
@@ -4105,30 +4470,56 @@ static void transform(Handle &H, int dir) {
     H.launches += 1;
     return;
   }
+  // CUDA-core transforms: on point-major rows (copied from or to the ordinate-major fields)
+  float *rows_in = H.raddo.p, *rows_out = H.srcdo.p;
+  auto copy_rows = [&](bool to_rows) {
+    const int n = H.P.npts, c = H.P.nang, tiles = ((n + 31) / 32) * ((c + 31) / 32);
+    if (to_rows)
+      k_transpose<<<tiles, 256, 0, H.stream>>>(H.raddo.p, H.ord_cs, H.xf_rows.p, H.ldo, c, n);
+    else
+      k_transpose<<<tiles, 256, 0, H.stream>>>(H.xf_rows.p, H.ldo, H.srcdo.p, H.ord_cs, n, c);
+    CK(cudaGetLastError());
+    H.launches += 1;
+  };
+  if (H.ord_major) {
+    if (!H.xf_rows.p) throw std::runtime_error("transform rows are not allocated");
+    rows_in = rows_out = H.xf_rows.p;
+    if (dir == 1) copy_rows(true);
+  }
   if (H.nst == 3) {  // FP32 dense transforms on the CUDA cores
     Plan &P = H.P;
     const int K = dir == 0 ? nsh : P.nang, N = dir == 0 ? P.nang : nsh;
     const dim3 grid((N + 63) / 64, (P.npts + 63) / 64);
     if (dir == 0)
-      k_dense_xf<<<grid, 256, 0, H.stream>>>(H.source.p, nsh, H.pol_t[0].p, K, N, P.npts, 0, H.srcdo.p, H.ldo,
+      k_dense_xf<<<grid, 256, 0, H.stream>>>(H.source.p, nsh, H.pol_t[0].p, K, N, P.npts, 0, rows_out, H.ldo,
                                               H.col_stk.p, nullptr, P.nlm);
     else
-      k_dense_xf<<<grid, 256, 0, H.stream>>>(H.raddo.p, H.ldo, H.pol_t[1].p, K, N, P.npts, 1, H.radiance.p, nsh,
+      k_dense_xf<<<grid, 256, 0, H.stream>>>(rows_in, H.ldo, H.pol_t[1].p, K, N, P.npts, 1, H.radiance.p, nsh,
                                               nullptr, H.nr.p, P.nlm);
     CK(cudaGetLastError());
     H.launches += 1;
     if (dir == 1) {
       const int fb = std::min((P.npts + 7) / 8, 152 * 16);
-      k_do_fluxes<<<fb, 256, 0, H.stream>>>(H.raddo.p, H.ldo, P.nang, P.ncol_down, H.col_fluxw.p, P.npts, H.fluxes.p);
+      k_do_fluxes<<<fb, 256, 0, H.stream>>>(rows_in, H.ldo, P.nang, P.ncol_down, H.col_fluxw.p, P.npts, H.fluxes.p);
       CK(cudaGetLastError());
       H.launches += 1;
     }
-    return;
+  } else {
+    const int nmu = H.P.nmu;
+    if (nmu <= 8) transforms_launch<8>(H, dir);
+    else if (nmu <= 16) transforms_launch<16>(H, dir);
+    else transforms_launch<32>(H, dir);
   }
-  const int nmu = H.P.nmu;
-  if (nmu <= 8) transforms_launch<8>(H, dir);
-  else if (nmu <= 16) transforms_launch<16>(H, dir);
-  else transforms_launch<32>(H, dir);
+  if (H.ord_major && dir == 0) copy_rows(false);
+}
+
+// Point-major rows for the CUDA-core transforms of ordinate-major fields
+// (the FP32 mode, and directions without a tensor-core transform).
+static void alloc_xf_rows(Handle &H) {
+  if (H.ord_major && !H.xf_rows.p && (H.xf_mode == 2 || !H.tc_ok[0] || !H.tc_ok[1])) {
+    H.xf_rows.alloc((size_t)H.P.npts * H.ldo);
+    H.xf_rows.zero(H.stream);
+  }
 }
 
 static SweepArgs sweep_args(Handle &H, int hemi) {
@@ -4138,6 +4529,7 @@ static SweepArgs sweep_args(Handle &H, int hemi) {
   a.bnd = H.bnd.p; a.rank = H.rank.p; a.start = H.start.p; a.level = H.level.p; a.text = H.text.p;
   a.srcdo = H.srcdo.p; a.raddo = H.raddo.p; a.col_cx = H.col_cx.p; a.col_cy = H.col_cy.p; a.col_cz = H.col_cz.p;
   a.tasks = H.tasks[hemi].p; a.err = H.errflag.p; a.npts = P.npts; a.nang = P.nang; a.ldo = H.ldo; a.is1d = P.is1d;
+  a.ps = H.ord_ps; a.cs = H.ord_cs;
   a.regular = H.regular.p; a.geo = H.geo.p; a.nz = P.nz; a.ny1 = P.ny1; a.nx1 = P.nx1;
   a.transmin = P.prob.transmin;
   a.irr = H.irr[hemi].p;
@@ -4170,7 +4562,6 @@ static void build_irr(Handle &H) {
     }
     for (int h = 0; h < 2; ++h) H.irr[h].view(G.irr[h]);
   }
-  setup_march(H);
   setup_p1s(H);
   if ((!H.march[0] && !H.seq[0] && P.seg_off[0].size() > 1) || (!H.march[1] && !H.seq[1] && P.seg_off[1].size() > 1))
     H.sweepw.alloc((size_t)P.npts * H.ldo);
@@ -4249,16 +4640,17 @@ static void sweep_hemisphere(Handle &H, int hemi) {
       H.launches += 1;
     }
     if (H.ktime_on) CK(cudaEventRecord(H.ev_k[hemi][1], H.stream));
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = H.mcs[hemi]; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.gridDim = dim3((unsigned)(H.mnunits[hemi] * H.mcs[hemi])); cfg.blockDim = dim3(MT);
-    cfg.dynamicSmemBytes = H.msmem[hemi]; cfg.stream = H.stream; cfg.attrs = at; cfg.numAttrs = 1;
     const MarchGrp *gp = H.mgrp[hemi].p;
     const MarchUnit *up = H.munit[hemi].p;
-    CK(cudaLaunchKernelEx(&cfg, k_sweep_march, a, gp, up));
-    H.launches += 1;
+    for (int k = 0; k < 2; ++k) {
+      const Handle::MarchLaunch &L = H.mlaunch[hemi][k];
+      if (!L.units) continue;
+      cudaLaunchAttribute at;
+      cudaLaunchConfig_t cfg = march_config(L.units, L.cs, L.threads, L.smem, H.stream, &at);
+      CK(cudaLaunchKernelEx(&cfg, march_kernel(L.rows, k == 1), a, gp, up, (int)(L.smem / 4)));
+      up += L.units;
+      H.launches += 1;
+    }
     if (H.ktime_on) CK(cudaEventRecord(H.ev_k[hemi][2], H.stream));
     return;
   }
@@ -4327,6 +4719,7 @@ static int check_device_error(Handle &H) {
   if (e == ERR_SWEEP_STEPS) m = "BACK_INT_GRID: trace exceeded the step limit";
   if (e == ERR_RAY_SO) m = "INTEGRATE_1RAY: SO<0";
   if (e == ERR_RAY_BELOW) m = "RENDER: Level below domain";
+  if (e == ERR_SWEEP_WAIT) m = "plane march: wait for a neighbouring strip expired";
   if (e == ERR_TC_WAIT) m = "tensor-core transform: pipeline wait expired";
   H.err = m;
   CK(cudaMemsetAsync(H.errflag.p, 0, sizeof(int), H.stream));
@@ -4414,6 +4807,7 @@ static int create_on_device(std::unique_ptr<shdom_handle> &H, int device, shdom_
     shdom::upload_plan(H->h);
     CK(cudaMemsetAsync(H->h.errflag.p, 0, sizeof(int), H->h.stream));
     shdom::build_irr(H->h);
+    shdom::alloc_xf_rows(H->h);
   } catch (const std::exception &e) {
     return fail(nullptr, e.what());
   }
@@ -4526,6 +4920,13 @@ int shdom_init_solution(shdom_handle *hh) {
     CK(cudaMemsetAsync(H.ns.p, 0, P.npts * sizeof(int), H.stream));
     CK(cudaMemsetAsync(H.nso.p, 0, P.npts * sizeof(int), H.stream));
     CK(cudaMemsetAsync(H.fluxes.p, 0, (size_t)P.npts * 2 * sizeof(float), H.stream));
+    // the sky's radiances at the top: no sweep writes them, so once is enough
+    if (const int t = (int)P.topp.size() * P.ncol_down) {
+      shdom::k_preset_top<<<(t + 255) / 256, 256, 0, H.stream>>>(H.topp.p, (int)P.topp.size(), H.raddo.p, H.ord_ps, H.ord_cs,
+                                                                 P.ncol_down, P.skyrad_bc, H.nst == 3 ? H.col_stk.p : nullptr);
+      CK(cudaGetLastError());
+      H.launches += 1;
+    }
     shdom::AccelState st{0.0, 1.0f, 0.0f};
     CK(cudaMemcpyAsync(H.accel.p, &st, sizeof(st), cudaMemcpyHostToDevice, H.stream));
     shdom::launch_source(H, 1, 0);
@@ -4565,23 +4966,17 @@ int shdom_solution_iterations(shdom_handle *hh, int maxiter, int *iters, float *
       if (timed) CK(cudaEventRecord(ev[0], H.stream));
       shdom::transform(H, 0);
       if (timed) CK(cudaEventRecord(ev[1], H.stream));
-      int ntop = (int)P.topp.size(), nbot = (int)P.botp.size();
-      if (ntop && P.ncol_down) {
-        int t = ntop * P.ncol_down;
-        shdom::k_preset_top<<<(t + 255) / 256, 256, 0, H.stream>>>(H.topp.p, ntop, H.raddo.p, H.ldo, P.ncol_down, P.skyrad_bc,
-                                                                   H.nst == 3 ? H.col_stk.p : nullptr);
-        H.launches += 1;
-      }
+      const int nbot = (int)P.botp.size();
       shdom::sweep_hemisphere(H, 0);
       if (nbot && P.brdf) {
         shdom::k_brdf_bottom<<<nbot, 128, 0, H.stream>>>(H.botp.p, nbot, H.botpar.p, P.nsfcpar, P.brdf, H.brdf_dn.p,
                                                           (int)P.brdf_dn.size(), H.brdf_up.p, (int)P.brdf_up.size(),
-                                                          H.dirflux.p, P.prob.solarmu, P.prob.solaraz, H.raddo.p, H.ldo,
+                                                          H.dirflux.p, P.prob.solarmu, P.prob.solaraz, H.raddo.p, H.ord_ps, H.ord_cs,
                                                           H.nst, H.botplanck.n ? H.botplanck.p : nullptr);
         H.launches += 1;
       } else if (nbot) {
         shdom::k_lambertian<<<nbot, 256, 0, H.stream>>>(H.botp.p, nbot, H.botalb.p, H.dirflux.p, H.col_fluxw.p, H.raddo.p,
-                                                         nang, H.ldo, P.ncol_down, H.bcrad.p, H.nst == 3 ? H.col_stk.p : nullptr,
+                                                         nang, H.ord_ps, H.ord_cs, P.ncol_down, H.bcrad.p, H.nst == 3 ? H.col_stk.p : nullptr,
                                                          H.botplanck.n ? H.botplanck.p : nullptr);
         H.launches += 1;
       }
@@ -4676,7 +5071,7 @@ static shdom::RenderArgs render_args(Handle &H, int nrays, const float *camx, co
   a.transcut = P.prob.transcut;
   a.coefp = H.nst == 3 ? H.coefp.p : nullptr;
   a.phasetab2 = H.nst == 3 ? H.phasetab2.p : nullptr;
-  a.brdf = P.brdf; a.nsfcpar = P.nsfcpar; a.nbrdf_dn = (int)P.brdf_dn.size(); a.ldo = H.ldo;
+  a.brdf = P.brdf; a.nsfcpar = P.nsfcpar; a.nbrdf_dn = (int)P.brdf_dn.size(); a.ord_ps = H.ord_ps; a.ord_cs = H.ord_cs;
   a.botpar = H.botpar.p; a.raddo = H.raddo.p; a.brdf_dn = H.brdf_dn.p;
   return a;
 }
@@ -5190,7 +5585,14 @@ int shdom_set_render_options(shdom_handle *hh, int single_scatter, int nosurface
 int shdom_set_transform_mode(shdom_handle *hh, int mode) {
   if (!hh) return fail(nullptr, "null handle");
   if (mode < 0 || mode > 2) return fail(hh, "shdom_set_transform_mode: mode must be 0, 1 or 2");
-  hh->h.xf_mode = mode;
+  Handle &H = hh->h;
+  DevGuard dg(H.device);
+  try {
+    H.xf_mode = mode;
+    shdom::alloc_xf_rows(H);
+  } catch (const std::exception &e) {
+    return fail(hh, e.what());
+  }
   return 0;
 }
 
@@ -5201,8 +5603,10 @@ int shdom_get_sizes(shdom_handle *hh, shdom_sizes *o) {
   o->launches = hh->h.launches;
   const shdom::Handle &H = hh->h;
   o->march = H.march_off ? 0 : ((H.march[0] ? 1 : 0) | (H.march[1] ? 2 : 0));
-  o->march_units_down = H.march[0] ? H.mnunits[0] : 0; o->march_units_up = H.march[1] ? H.mnunits[1] : 0;
-  o->march_cluster_down = H.march[0] ? H.mcs[0] : 0; o->march_cluster_up = H.march[1] ? H.mcs[1] : 0;
+  auto units = [&](int h) { return H.march[h] ? H.mlaunch[h][0].units + H.mlaunch[h][1].units : 0; };
+  auto clus = [&](int h) { return H.march[h] ? H.mlaunch[h][H.mlaunch[h][0].units ? 0 : 1].cs : 0; };
+  o->march_units_down = units(0); o->march_units_up = units(1);
+  o->march_cluster_down = clus(0); o->march_cluster_up = clus(1);
   return 0;
 }
 

@@ -40,6 +40,9 @@ struct Epilogue {
   int mode;          // 0: C = max(0, acc); 1: radiance (masked by nr), fluxes from A
   float *C;          // mode 0 output, row stride ldc
   int ldc;
+  size_t ccs;        // mode 0: column stride of C when it is ordinate-major (row stride 1), else 0
+  const float *Aord; // KM: the ordinate-major A operand (element (row, k) at Aord[k * acs + row])
+  size_t acs;
   float *R;          // mode 1 radiance [M][nlm]
   int nlm;
   const int *nr;
@@ -141,15 +144,17 @@ __device__ __forceinline__ void reg_fence16(uint32_t *r) {
 //                  next tile).
 // Summing the per-chunk partial products on the CUDA cores (round to
 // nearest) keeps the tensor-core accumulation chains 32 K-elements long.
-template <int BN>
+template <int BN, bool KM>
 struct Cfg {
   static constexpr int HALF = BN / 2;
   static constexpr int A_BYTES = BM * BK * 4, B_BYTES = BN * BK * 4;
   static constexpr int STAGE = 2 * A_BYTES + 2 * B_BYTES;
   static constexpr int kFluxTab = 16 * 1024;  // down and up flux weights, K padded to 32 (K <= 2048)
-  static constexpr int S = (227 * 1024 - 2048 - kFluxTab) / STAGE > 4 ? 4 : (227 * 1024 - 2048 - kFluxTab) / STAGE;
+  static constexpr int RAW = 4, kRaw = KM ? RAW * A_BYTES : 0;  // raw A tiles (KM)
+  static constexpr int kRoom = (227 * 1024 - 2048 - kFluxTab - kRaw) / STAGE;
+  static constexpr int S = kRoom > 4 ? 4 : kRoom;
   static constexpr uint32_t TCOLS = 2 * BN <= 256 ? 256u : 512u;
-  static constexpr size_t smem() { return (size_t)S * STAGE + 256 + kFluxTab + 1024; }
+  static constexpr size_t smem() { return (size_t)S * STAGE + 256 + kFluxTab + kRaw + 1024; }
 };
 constexpr int kThreads = 448;
 
@@ -160,12 +165,19 @@ __device__ __forceinline__ float tf32_rna_bits(float x) {
   return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
 }
 
-template <int BN>
+//
+// KM (the ordinate-to-harmonic direction on ordinate-major fields): A does
+// not come by TMA; each split thread copies its row's 32 values of a chunk
+// from global memory into its column of a raw [k][row] tile, RAW - 1 chunks
+// ahead (a warp's rows are consecutive points, or nearly so when A's rows
+// are the scattering points in order, so each copy is one contiguous line),
+// which also gathers the compacted rows without a pass of their own.
+template <int BN, bool KM>
 __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__ CUtensorMap tmA,
                                                          const __grid_constant__ CUtensorMap tmBh,
                                                          const __grid_constant__ CUtensorMap tmBl, int K, int ntn,
                                                          int ntiles, Epilogue g) {
-  using C = Cfg<BN>;
+  using C = Cfg<BN, KM>;
   constexpr int S = C::S, HALF = C::HALF, A_BYTES = C::A_BYTES, B_BYTES = C::B_BYTES, STAGE = C::STAGE;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base0 = saddr(smem_raw);
@@ -227,8 +239,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
         tile_origin(gc, m0, n0);
         const int kx = (gc % KB) * BK;
         const uint32_t st = sbase + s * STAGE;
-        mbar_expect_tx(full0 + 8 * s, A_BYTES + 2 * B_BYTES);
-        tma_load(st, &tmA, full0 + 8 * s, kx, m0);
+        mbar_expect_tx(full0 + 8 * s, (KM ? 0 : A_BYTES) + 2 * B_BYTES);
+        if (!KM) tma_load(st, &tmA, full0 + 8 * s, kx, m0);
         tma_load(st + 2 * A_BYTES, &tmBh, full0 + 8 * s, kx, n0);
         tma_load(st + 2 * A_BYTES + B_BYTES, &tmBl, full0 + 8 * s, kx, n0);
         issued = gc + 1;
@@ -286,14 +298,51 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
       tile_origin(0, m0, n0);
       flux = g.mode == 1 && n0 == 0;
     }
+    constexpr int RAW = C::RAW;
+    float *raw = reinterpret_cast<float *>(smem + S * STAGE + 256 + C::kFluxTab) + srow;  // KM: [RAW][BK][BM], this row's column
+    long long arow_pt = -1;
+    auto fetch = [&](int gc) {  // KM: chunk gc of this row on its way (an empty group past the last)
+      if (gc < G) {
+        const int c = gc % KB;
+        if (c == 0) {
+          int m0, n0;
+          tile_origin(gc, m0, n0);
+          const int r = m0 + srow;
+          arow_pt = r < g.M ? (g.rowmap ? (long long)g.rowmap[r] : (long long)r) : -1;
+        }
+        const float *ap = arow_pt >= 0 ? g.Aord + (size_t)(c * BK) * g.acs + arow_pt : g.Aord;
+        const int kn = arow_pt >= 0 ? min(BK, K - c * BK) : 0;
+        uint32_t d = saddr(raw + (gc % RAW) * (BK * BM));
+#pragma unroll
+        for (int u = 0; u < BK; ++u) {
+          const bool in = u < kn;
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + u * (BM * 4)),
+                       "l"(in ? ap + (size_t)u * g.acs : g.Aord), "r"(in ? 4 : 0)
+                       : "memory");
+        }
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    if (KM)
+      for (int i = 0; i < RAW - 1; ++i) fetch(i);
     for (int gc = 0; gc < G; ++gc) {
       const int s = gc % S, c = gc % KB;
+      float4 v[8];
+      if (KM) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(RAW - 2) : "memory");
+        const float *rw = raw + (gc % RAW) * (BK * BM);
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          v[u] = make_float4(rw[(4 * u) * BM], rw[(4 * u + 1) * BM], rw[(4 * u + 2) * BM], rw[(4 * u + 3) * BM]);
+        fetch(gc + RAW - 1);  // into the tile read a chunk ago
+      }
       const bool go = !*abort_flag && mbar_wait(full0 + 8 * s, (gc / S) & 1, g.wait_limit);
       if (!__all_sync(0xffffffffu, go)) { *abort_flag = 1; break; }
       uint8_t *arow = smem + s * STAGE + (srow >> 3) * 1024 + swz * 128;
-      float4 v[8];
+      if (!KM) {
 #pragma unroll
-      for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const float4 *>(arow + ((u ^ swz) << 4));
+        for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const float4 *>(arow + ((u ^ swz) << 4));
+      }
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         // u is the logical 16-byte unit of the row; (u ^ swz) its place in the 128-byte swizzle row
@@ -337,6 +386,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
         flux = g.mode == 1 && n0 == 0;  // one N tile of a row tile forms its fluxes
       }
     }
+    if (KM) asm volatile("cp.async.wait_group 0;" ::: "memory");  // no copy in flight when the shared memory is released
   } else {
     // ---------------------------------------------------------- accumulate
     const int lg = warp & 3, half = (warp - 6) >> 2;
@@ -372,7 +422,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
         if (arow < g.M) {
           const int row = g.rowmap ? g.rowmap[arow] : arow;
           const int cb = n0 + half * HALF;
-          if (g.mode == 0) {
+          if (g.mode == 0 && g.ccs) {
+            // ordinate-major: a warp's rows are consecutive (or nearly), so each column is one line
+            float *out = g.C + row;
+#pragma unroll
+            for (int j = 0; j < HALF; ++j) {
+              const int col = cb + j;
+              if (col < g.N) out[(size_t)col * g.ccs] = g.stk && g.stk[col] ? acc[j] : fmaxf(acc[j], 0.f);
+            }
+          } else if (g.mode == 0) {
             float *out = g.C + (size_t)row * g.ldc;
 #pragma unroll
             for (int j = 0; j < HALF; j += 4) {
@@ -415,8 +473,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::TCOLS));
 }
 
-template <int BN>
-inline size_t smem_bytes() { return Cfg<BN>::smem(); }
+template <int BN, bool KM>
+inline size_t smem_bytes() { return Cfg<BN, KM>::smem(); }
 
 }  // namespace tc
 }  // namespace shdom
