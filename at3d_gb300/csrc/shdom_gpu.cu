@@ -1492,147 +1492,219 @@ constexpr double kMarchRow = 33, kMarchPlane = 184, kMarchIdle = 20, kMarchIpc =
 // whole grid), in two kernels.
 //  * k_seq_prep: every (ordinate, point) trace of the hemisphere at once,
 //    since a trace depends on the source function only: its (radsrc, tr),
-//    the four corners of the face it stops on and the face coordinates, as
-//    a 32-byte record in [ordinate][rank] order.  The long characteristics
-//    (a row's first point crossing the wrap-around to the previous row, a
-//    chain of cells) run here in parallel instead of inside the walk.
-//  * k_sweep_seq: one block per ordinate walks the reference sweep order in
-//    windows of SEQN ranks.  One thread runs a window's chain in rank
-//    order, the item just before in a register (the usual dependency: the
-//    neighbour along the row) and the others in shared memory; a chain
-//    step is a few dependent instructions instead of a round of warp
-//    votes.  Meanwhile the other seven warps prepare the next window (read
-//    its records, coalesced; add its final dependencies; list the others
-//    with their weights) and write the window before back to the field.
-constexpr int SEQW = 256;  // threads of a walking block
-constexpr int SEQN = 512;  // ranks of a window
+//    the places of the four corners of the face it stops on in the walk and
+//    the face coordinates, as a 32-byte record at [ordinate][place].  Lanes
+//    run over points in memory order, so the fields are read in whole lines;
+//    a record is one sector.  Corners that are preset boundary points are
+//    folded into radsrc, since they are final before the sweep.
+//  * k_sweep_seq: one block per ordinate walks the points in windows of SEQN
+//    places; seven warps prepare the next window and write the one before
+//    back while one warp walks.
+//
+// Which faces are usable is a matter of the reference's sweep order (rank);
+// the walk itself may take any order in which corners come first.  The
+// reference visits the first two rows of a layer together, point by point,
+// which chains every item there to the ones 2 and 3 before it; the walk
+// takes layer by layer, row by row, upwind first.  k_seq_check confirms once
+// per grid that every corner comes earlier there (it did on every grid
+// tried); else, and with transmin < 1 (where faces depend on the medium),
+// the walk takes the rank order.
+//
+// The walk solves a chain v_i = w_i + a_i v_(i-1) + (corners at larger
+// distances).  The other corners are mostly at least a row back.  So the warp
+// takes the longest run of up to 32 items none of which has another corner
+// inside the run (a vote on each item's latest other corner; 22 to 29 items
+// on average from 20x14x12 to 100x80x4 points), gathers the others from
+// shared memory, and solves the run with a scan of affine maps: five shuffle
+// steps for a run instead of a dependent chain per item.  All weights are
+// non-negative with sums of at most one, so the products of a scan only
+// shrink.  Values of the last SEQRING places stay in shared memory (a layer
+// of the grid and more); older corners are read back from the records.
+//
+// What bounds it: the latency of a run on the one walking warp (about 400
+// cycles, 18 to 20 runs a window).  Measured per hemisphere, against one
+// thread walking item by item: 32x32x24 with 45 ordinates 0.177 against
+// 1.175 ms, 64x64x40 with 135 columns (I, Q, U) 0.97 against 7.57 ms; the
+// records 0.08 against 0.13 and 1.1 against 2.2 ms.  Tried: the rank order
+// with a scan of (v_(i-1), v_(i-2)) pairs for the interleaved rows (0.45 ms
+// at 32x32x24: 12 dependent steps a run) and with one late item per run
+// added afterwards (0.53 ms).
+constexpr int SEQW = 256;       // threads of a walking block
+constexpr int SEQN = 512;       // ranks of a window
+constexpr int SEQRING = 8192;   // ranks whose values stay in shared memory (a power of two)
+constexpr int SEQFAR = SEQRING - 2 * SEQN;  // corners further back than this are read from memory
+constexpr size_t kSeqSmem = sizeof(float) * SEQRING + 2 * (size_t)SEQN * (2 * sizeof(float4) + sizeof(short4));
 
-__device__ __forceinline__ int col_octant(const SweepArgs &a, int col) {
-  int b = 0;
-  for (int k = 0; k < 8; ++k)
-    if (a.oct_ncol[k] > 0 && col >= a.oct_col0[k] && col < a.oct_col0[k] + a.oct_ncol[k]) b = k;
-  return b;
+// A point's place in the walk of trace octant b, and back (lex: layer, row,
+// position, each upwind first; else the reference's rank).
+__device__ __forceinline__ int seq_place(const SweepArgs &a, int b, int pt, bool lex) {
+  if (!lex) return a.rank[(size_t)b * a.npts + pt];
+  const int iz = pt % a.nz, t = pt / a.nz, iy = t % a.ny1, ix = t / a.ny1;
+  const int x = (b & 1) ? ix : a.nx1 - 1 - ix, y = (b & 2) ? iy : a.ny1 - 1 - iy, z = (b & 4) ? iz : a.nz - 1 - iz;
+  return (z * a.ny1 + y) * a.nx1 + x;
+}
+__device__ __forceinline__ int seq_point(const SweepArgs &a, int b, int r, const int *__restrict__ order, bool lex) {
+  if (!lex) return __ldg(order + (size_t)b * a.npts + r);
+  const int x = r % a.nx1, t = r / a.nx1, y = t % a.ny1, z = t / a.ny1;
+  const int ix = (b & 1) ? x : a.nx1 - 1 - x, iy = (b & 2) ? y : a.ny1 - 1 - y, iz = (b & 4) ? z : a.nz - 1 - z;
+  return (ix * a.ny1 + iy) * a.nz + iz;
 }
 
-__global__ void __launch_bounds__(256) k_seq_prep(SweepArgs a, const int *__restrict__ order, int col_begin, int nc,
-                                                   TraceRec *__restrict__ rec) {
-  const int n = a.npts;
-  const long long total = (long long)nc * n;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int cl = (int)(i / n), r = (int)(i - (long long)cl * n);
-    const int col = col_begin + cl;
-    if (a.col_cz[col] == 0.f) continue;  // padding ordinate
-    const int b = col_octant(a, col);
-    const int hb = (b & 4) ? 2 : 1;
-    const int pt = order[(size_t)b * n + r];
-    if (a.bnd[pt] & hb) continue;  // preset boundary point
+// Whether every corner of the hemisphere's traces comes earlier in the lex walk (bad counts those that do not).
+__global__ void __launch_bounds__(256) k_seq_check(SweepArgs a, const int *__restrict__ col_oct, int col_begin, int *bad) {
+  const int col = col_begin + blockIdx.y;
+  if (a.col_cz[col] == 0.f) return;
+  const int b = __ldg(col_oct + col) - 1, hb = (b & 4) ? 2 : 1;
+  for (int pt = blockIdx.x * blockDim.x + threadIdx.x; pt < a.npts; pt += gridDim.x * blockDim.x) {
+    if (a.bnd[pt] & hb) continue;
     const Trace t = trace_point(a, b, pt, col);
-    if (t.status != ERR_NONE) atomicCAS(a.err, ERR_NONE, t.status);
-    TraceRec x;
-    x.radsrc = t.radsrc; x.tr = t.tr; x.u = t.u; x.v = t.v;
-    x.q = make_int4(t.q[0], t.q[1], t.q[2], t.q[3]);
-    rec[i] = x;
+    const int r = seq_place(a, b, pt, true);
+    for (int k = 0; k < 4; ++k)
+      if (!(a.bnd[t.q[k]] & hb) && t.f[k] != 0.f && seq_place(a, b, t.q[k], true) >= r) atomicAdd(bad, 1);
   }
 }
 
-__global__ void __launch_bounds__(SEQW) k_sweep_seq(SweepArgs a, const int *order, int col_begin,
-                                                    const TraceRec *__restrict__ rec) {
-  // sval: the values of the last two windows walked, by window parity (a
-  // ring of 2 SEQN).  Per item of a window being walked or prepared (by
-  // parity): the part from final dependencies, the weight of the item just
-  // before it, and up to four other dependencies (ring indices, weight 0 for
-  // none).  spt: the items' points, kept three windows for the write-back.
-  __shared__ float sval[2 * SEQN];
-  __shared__ float swv[2][SEQN], scp[2][SEQN];
-  __shared__ float4 sc[2][SEQN];
-  __shared__ short4 sd[2][SEQN];
-  __shared__ int spt[3][SEQN];
-  const int col = col_begin + blockIdx.x, n = a.npts;
+__global__ void __launch_bounds__(256) k_seq_prep(SweepArgs a, const int *__restrict__ col_oct, int col_begin, int lex,
+                                                   TraceRec *__restrict__ rec) {
+  const int n = a.npts;
+  const int col = col_begin + blockIdx.y;
   if (a.col_cz[col] == 0.f) return;  // padding ordinate
-  const int b = col_octant(a, col);
-  const int hb = (b & 4) ? 2 : 1;
-  const int *ord = order + (size_t)b * n, *rk = a.rank + (size_t)b * n;
-  const TraceRec *crec = rec + (size_t)blockIdx.x * n;
-  const int tid = threadIdx.x, warp = tid >> 5;
-  const int nwin = (n + SEQN - 1) / SEQN;
-  for (int j = tid; j < 2 * SEQN; j += SEQW) sval[j] = 0.f;
-
-  // window w's item list, by threads [t0, t0 + nt).  Dependencies: on a
-  // preset point or a window before w - 2, final in the field; on window
-  // w - 2, final in the ring; on window w - 1 or w, ring indices for the
-  // walk (window w - 1 may still be walking while w is prepared).
-  auto prep = [&](int w, int t0, int nt) {
-    const int r0 = w * SEQN, m = min(SEQN, n - r0), pw = w & 1;
-    for (int j = tid - t0; j < SEQN; j += nt) {
-      const int r = r0 + j;
-      float wv = 0.f, cp = 0.f;
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-      short d[4] = {0, 0, 0, 0};
-      int pt = -1;
-      if (j < m) {
-        const int p = ord[r];
-        if (!(a.bnd[p] & hb)) {
-          pt = p;
-          const TraceRec R = crec[r];
-          const int q[4] = {R.q.x, R.q.y, R.q.z, R.q.w};
-          const float f[4] = {(1.f - R.u) * (1.f - R.v), (1.f - R.u) * R.v, R.u * (1.f - R.v), R.u * R.v};
-          wv = R.radsrc;
+  const int b = __ldg(col_oct + col) - 1, hb = (b & 4) ? 2 : 1;
+  TraceRec *crec = rec + (size_t)blockIdx.y * n;
+  for (int pt = blockIdx.x * blockDim.x + threadIdx.x; pt < n; pt += gridDim.x * blockDim.x) {
+    const int r = seq_place(a, b, pt, lex);
+    if (r < 0) continue;
+    TraceRec x;
+    if (a.bnd[pt] & hb) {  // preset boundary point: its own value
+      x.radsrc = a.raddo[a.at(pt, col)]; x.tr = 0.f; x.u = 0.f; x.v = 0.f;
+      x.q = make_int4(-1, -1, -1, -1);
+    } else {
+      // a regular trace's corners are upwind neighbours: their places follow from the point's
+      const bool near = lex && a.regular[(size_t)b * n + pt];
+      const Trace t = trace_point(a, b, pt, col);
+      if (t.status != ERR_NONE) atomicCAS(a.err, ERR_NONE, t.status);
+      x.radsrc = t.radsrc; x.tr = t.tr; x.u = t.u; x.v = t.v;
+      int iface = 0;
+      if (near) {
+        const int iz = pt % a.nz, layer = (b & 4) ? iz - 1 : iz;
+        iface = (int)__ldg(a.geo + 4 * ((size_t)layer * a.nang + col) + 3);
+      }
+      int rq[4] = {-1, -1, -1, -1};
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float wt = R.tr * f[k];
-            if (wt == 0.f) continue;
-            if (a.bnd[q[k]] & hb) {  // a preset boundary point: final
-              wv += wt * a.raddo[a.at(q[k], col)];
-              continue;
-            }
-            const int rq = rk[q[k]];
-            if (rq >= r0) {  // this window
-              const int off = rq - r0;
-              if (off >= j) { atomicCAS(a.err, ERR_NONE, ERR_SWEEP_NOFACE); continue; }  // not rank-earlier
-              if (off == j - 1) cp += wt;
-              else { d[k] = (short)(pw * SEQN + off); c[k] = wt; }
-            } else if (rq >= r0 - SEQN) {  // window w - 1: walked just before this one
-              d[k] = (short)((pw ^ 1) * SEQN + (rq - (r0 - SEQN))); c[k] = wt;
-            } else if (rq >= r0 - 2 * SEQN) {  // window w - 2: final, in the ring
-              wv += wt * sval[pw * SEQN + (rq - (r0 - 2 * SEQN))];
-            } else {
-              wv += wt * a.raddo[a.at(q[k], col)];
-            }
-          }
+      for (int k = 0; k < 4; ++k) {
+        const float w = t.tr * t.f[k];
+        if (w == 0.f) continue;
+        if (a.bnd[t.q[k]] & hb) {
+          x.radsrc += w * a.raddo[a.at(t.q[k], col)];
+        } else if (near) {
+          const int dlt = c_face[iface][k] ^ b;
+          rq[k] = r - (dlt & 1) - ((dlt & 2) ? a.nx1 : 0) - ((dlt & 4) ? a.nx1 * a.ny1 : 0);
+        } else {
+          rq[k] = seq_place(a, b, t.q[k], lex);
+          if (rq[k] >= r) { rq[k] = -1; atomicCAS(a.err, ERR_NONE, ERR_SWEEP_NOFACE); }  // not earlier
         }
       }
-      spt[w % 3][j] = pt;
-      swv[pw][j] = wv; scp[pw][j] = cp;
-      sc[pw][j] = make_float4(c[0], c[1], c[2], c[3]);
-      sd[pw][j] = make_short4(d[0], d[1], d[2], d[3]);
+      x.q = make_int4(rq[0], rq[1], rq[2], rq[3]);
+    }
+    crec[r] = x;
+  }
+}
+
+__global__ void __launch_bounds__(SEQW) k_sweep_seq(SweepArgs a, const int *__restrict__ col_oct, const int *__restrict__ order, int col_begin,
+                                                    int lex, TraceRec *rec) {
+  // sval: the values of the last SEQRING places.  Per item of the window being
+  // walked and of the one being prepared, st: the part that is known, the
+  // weight of the item before and the latest of its other corners as a
+  // position in the window; up to four other corners (weights sc, 0 for none;
+  // ring positions sd).
+  extern __shared__ __align__(16) unsigned char sqm[];
+  float4 *st = reinterpret_cast<float4 *>(sqm), *sc = st + 2 * SEQN;
+  short4 *sd = reinterpret_cast<short4 *>(sc + 2 * SEQN);
+  float *sval = reinterpret_cast<float *>(sd + 2 * SEQN);
+  const int col = col_begin + blockIdx.x, n = a.npts;
+  if (a.col_cz[col] == 0.f) return;  // padding ordinate
+  const int b = __ldg(col_oct + col) - 1;
+  TraceRec *crec = rec + (size_t)blockIdx.x * n;
+  float *rado = a.raddo + (size_t)col * a.cs;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nwin = (n + SEQN - 1) / SEQN;
+  for (int j = tid; j < SEQRING; j += SEQW) sval[j] = 0.f;
+
+  // window w's items, by threads [t0, t0 + nt), nt at least SEQN / 3: the
+  // records of a thread's items are loaded before the first is used
+  auto prep = [&](int w, int t0, int nt) {
+    const int r0 = w * SEQN, m = min(SEQN, n - r0), o = (w & 1) * SEQN;
+    TraceRec rec3[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (const int j = tid - t0 + i * nt; j < m) rec3[i] = crec[r0 + j];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int j = tid - t0 + i * nt, r = r0 + j;
+      if (j >= m) break;
+      const TraceRec &R = rec3[i];
+      const int rq[4] = {R.q.x, R.q.y, R.q.z, R.q.w};
+      const float f[4] = {(1.f - R.u) * (1.f - R.v), (1.f - R.u) * R.v, R.u * (1.f - R.v), R.u * R.v};
+      float c[4] = {0.f, 0.f, 0.f, 0.f}, wv = R.radsrc, wa = 0.f;
+      short d[4] = {0, 0, 0, 0};
+      int latest = -1;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (rq[k] < 0) continue;
+        const float wt = R.tr * f[k];
+        const int dist = r - rq[k];
+        if (dist == 1) wa += wt;
+        else if (dist <= SEQFAR) { c[k] = wt; d[k] = (short)(rq[k] & (SEQRING - 1)); latest = max(latest, rq[k]); }
+        else wv += wt * crec[rq[k]].radsrc;  // written back windows ago
+      }
+      st[o + j] = make_float4(wv, wa, __int_as_float(latest - r0), 0.f);
+      sc[o + j] = make_float4(c[0], c[1], c[2], c[3]);
+      sd[o + j] = make_short4(d[0], d[1], d[2], d[3]);
     }
   };
-  // window w's radiances to the field, by threads [t0, t0 + nt)
+  // window w's radiances to the field (and to the records, for far corners), by threads [t0, t0 + nt)
   auto writeback = [&](int w, int t0, int nt) {
-    const int pw = w & 1;
-    for (int j = tid - t0; j < SEQN; j += nt) {
-      const int pt = spt[w % 3][j];
-      if (pt >= 0) a.raddo[a.at(pt, col)] = sval[pw * SEQN + j];
+    const int r0 = w * SEQN, m = min(SEQN, n - r0);
+    int pt[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+      if (const int j = tid - t0 + i * nt; j < m) pt[i] = seq_point(a, b, r0 + j, order, lex);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      const int j = tid - t0 + i * nt, r = r0 + j;
+      if (j >= m) break;
+      const float x = sval[r & (SEQRING - 1)];
+      rado[(size_t)pt[i] * a.ps] = x;
+      if (n > SEQFAR) crec[r].radsrc = x;
     }
   };
   if (nwin > 0) prep(0, 0, SEQW);
   __syncthreads();
+  float v1 = 0.f;  // the value one rank before the run
   for (int w = 0; w < nwin; ++w) {
     if (warp == 0) {
-      if (tid == 0) {  // the chain of window w in rank order, the item just before in a register
-        const int pw = w & 1, m = min(SEQN, n - w * SEQN);
-        float *out = sval + pw * SEQN;
-        float prev = 0.f;
-#pragma unroll 4
-        for (int i = 0; i < m; ++i) {
-          const float4 cc = sc[pw][i];
-          const short4 dd = sd[pw][i];
-          float v = swv[pw][i] + cc.x * sval[dd.x] + cc.y * sval[dd.y] + cc.z * sval[dd.z] + cc.w * sval[dd.w];
-          v = fmaf(scp[pw][i], prev, v);
-          out[i] = v;
-          prev = v;
+      const int r0 = w * SEQN, m = min(SEQN, n - r0), o = (w & 1) * SEQN;
+      // the items at s + lane, loaded a run ahead
+      float4 tt = st[o + min(lane, m - 1)], cc = sc[o + min(lane, m - 1)];
+      short4 dd = sd[o + min(lane, m - 1)];
+      for (int s = 0; s < m;) {
+        // the run ends before the first item with another corner inside it
+        const unsigned stop = __ballot_sync(0xffffffffu, __float_as_int(tt.z) >= s);
+        const int k = min(stop ? __ffs(stop) - 1 : 32, m - s);
+        const int slot = (r0 + s + lane) & (SEQRING - 1), ni = o + min(s + lane + k, m - 1);
+        float A = tt.y;
+        float T = fmaf(cc.y, sval[dd.y], fmaf(cc.x, sval[dd.x], tt.x)) + fmaf(cc.w, sval[dd.w], cc.z * sval[dd.z]);
+        tt = st[ni]; cc = sc[ni]; dd = sd[ni];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+          const float Au = __shfl_up_sync(0xffffffffu, A, off), Tu = __shfl_up_sync(0xffffffffu, T, off);
+          if (lane >= off) { T = fmaf(A, Tu, T); A *= Au; }
         }
+        const float x = fmaf(A, v1, T);
+        if (lane < k) sval[slot] = x;
+        v1 = __shfl_sync(0xffffffffu, x, k - 1);
+        s += k;
+        __syncwarp();
       }
     } else {  // meanwhile: prepare window w + 1, write back window w - 1
       if (w + 1 < nwin) prep(w + 1, 32, SEQW - 32);
@@ -3531,6 +3603,7 @@ struct DevGeom {
   DBuf<int> seg_off[2], level_items[2], p1off[2];
   DBuf<IrrRec> irr[2];
   bool irr_built = false;
+  bool seq_checked = false, seq_lex[2] = {false, false};  // the walk's order per hemisphere (k_seq_check)
   // block-local phase 1 (setup_p1s): per hemisphere, built once per grid and device
   bool p1s_built = false, p1s_ok[2] = {false, false};
   DBuf<P1Blk> p1blk[2];
@@ -4575,7 +4648,29 @@ static void build_irr(Handle &H) {
     size_t nrec = 0;
     for (int h = 0; h < 2; ++h)
       if (H.seq[h]) nrec = std::max(nrec, (size_t)P.npts * (h ? P.nang - P.ncol_down : P.ncol_down));
-    if (nrec) H.seqrec.alloc(nrec);
+    if (nrec) {
+      H.seqrec.alloc(nrec);
+      CK(cudaFuncSetAttribute(k_sweep_seq, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSeqSmem));
+      DevGeom &G = *H.geom;
+      std::lock_guard<std::mutex> lk(G.mu);
+      if (!G.seq_checked) {
+        DBuf<int> bad;
+        bad.alloc(2);
+        bad.zero(H.stream);
+        for (int h = 0; h < 2; ++h) {
+          const int c0 = h ? P.ncol_down : 0, nc = h ? P.nang - P.ncol_down : P.ncol_down;
+          if (!H.seq[h] || nc <= 0 || P.prob.transmin < 1.f) continue;
+          k_seq_check<<<dim3(std::min((P.npts + 255) / 256, H.nsm), nc), 256, 0, H.stream>>>(sweep_args(H, h), H.col_oct.p, c0, bad.p + h);
+          CK(cudaGetLastError());
+          H.launches += 1;
+        }
+        int n[2];
+        CK(cudaMemcpyAsync(n, bad.p, sizeof(n), cudaMemcpyDeviceToHost, H.stream));
+        CK(cudaStreamSynchronize(H.stream));
+        for (int h = 0; h < 2; ++h) G.seq_lex[h] = P.prob.transmin >= 1.f && n[h] == 0;
+        G.seq_checked = true;
+      }
+    }
   }
   {  // phase 1 runs on a high-priority stream so its blocks start before the source pass fills the SMs
     int lo = 0, hi = 0;
@@ -4596,11 +4691,10 @@ static void sweep_hemisphere(Handle &H, int hemi) {
   if (H.seq[hemi]) {
     const int c0 = hemi ? P.ncol_down : 0, nc = hemi ? P.nang - P.ncol_down : P.ncol_down;
     if (nc > 0) {
-      const long long total = (long long)nc * P.npts;
-      const int blocks = (int)std::min<long long>((total + 255) / 256, (long long)H.nsm * 8);
-      k_seq_prep<<<blocks, 256, 0, H.stream>>>(a, H.order.p, c0, nc, H.seqrec.p);
+      const int lex = H.geom->seq_lex[hemi];
+      k_seq_prep<<<dim3(std::min((P.npts + 255) / 256, H.nsm), nc), 256, 0, H.stream>>>(a, H.col_oct.p, c0, lex, H.seqrec.p);
       CK(cudaGetLastError());
-      k_sweep_seq<<<nc, SEQW, 0, H.stream>>>(a, H.order.p, c0, H.seqrec.p);
+      k_sweep_seq<<<nc, SEQW, kSeqSmem, H.stream>>>(a, H.col_oct.p, H.order.p, c0, lex, H.seqrec.p);
       CK(cudaGetLastError());
       H.launches += 2;
     }
