@@ -2895,12 +2895,13 @@ constexpr int RNLM = 1024;    // max spherical-harmonic terms for the per-ray ta
 // dot products of the new cell corners are split over groups of four lanes;
 // the path integration is evaluated uniformly by all lanes.
 // Real spherical harmonics Y_lm of one direction (mu, phi) into y[NLM] (the
-// j(l, m) term order of the solver), lane m of the warp running the upward
-// l recurrence of the normalised Wigner d^l_{m0}(mu) for its m.  FP32: the
+// j(l, m) term order of the solver), this lane running the upward l
+// recurrence of the normalised Wigner d^l_{m0}(mu) for m = first, first +
+// step, ...  FP32: the
 // values are stored as FP32 and dotted with FP32 coefficients.
-__device__ __forceinline__ void ylm_dir_warp(float *y, float x, float phf, int ml, int mm, int lane) {
+__device__ __forceinline__ void ylm_dir_lanes(float *y, float x, float phf, int ml, int mm, int first, int step) {
   const float fct = 0.3989422804014327f;  // 1/sqrt(2 pi)
-  for (int m = lane; m <= mm; m += 32) {
+  for (int m = first; m <= mm; m += step) {
     float c = 1.f, s = 0.f;
     if (m > 0) sincosf(m * phf, &s, &c);
     float dprev = 0.f, dcur;
@@ -2968,7 +2969,7 @@ __global__ void __launch_bounds__(RWARPS * 32) k_render(RenderArgs a) {
     return;
   }
   // Y_lm in the ray direction: lane m runs the l recurrence of its m
-  ylm_dir_warp(ydir[w], (float)mu2, (float)phi2, a.ml, a.mm, lane);
+  ylm_dir_lanes(ydir[w], (float)mu2, (float)phi2, a.ml, a.mm, lane, 32);
   __syncwarp();
   // t_l = sum_m Ydir(l,m) Ysun(l,m)
   for (int l = lane; l <= a.ml; l += 32) {
@@ -3640,7 +3641,8 @@ struct Handle {
   DBuf<int> g_interpptr, g_sjptr, g_sjiph, g_piph;
   DBuf<float> g_optwt, g_dextm, g_dalbm, g_dfj, g_albsp, g_sjw, g_legu, g_legs, g_fmix, g_scatj, g_legp, g_extp,
       g_albp, g_pphw;
-  DBuf<double> g_grad, g_beam, g_adj;
+  DBuf<double> g_grad, g_beam, g_adj, g_sunpath;
+  DBuf<uint8_t> g_flip;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   cudaEvent_t ev_caller[2] = {nullptr, nullptr};  // ordering against a caller's stream (device-buffer calls)
   cudaEvent_t ev_ext = nullptr;  // after the last render launched on a caller's stream
@@ -5336,7 +5338,13 @@ static void prepare_grad(Handle &H, int ipa) {
   H.g_dfj.upload(dfj); H.g_albsp.upload(albsp); H.g_sjptr.upload(sjptr); H.g_sjiph.upload(sjiph); H.g_sjw.upload(sjw);
   H.g_legu.upload(legu); H.g_legs.upload(legs); H.g_fmix.upload(fmix); H.g_scatj.upload(scatj); H.g_legp.upload(legp);
   H.g_extp.upload(ep); H.g_albp.upload(ap); H.g_piph.upload(piph); H.g_pphw.upload(phw);
-  H.g_grad.alloc((size_t)ng * 2); H.g_beam.alloc(npts);
+  H.g_grad.alloc((size_t)ng * 2); H.g_beam.alloc(npts); H.g_sunpath.alloc(ng);
+  if (!H.g_flip.p) {
+    H.g_flip.alloc(P.ncells);
+    shdom::k_cell_flip<<<(P.ncells + 255) / 256, 256, 0, H.stream>>>(H.gridptr.p, P.ncells, P.ny1, P.nz, H.g_flip.p);
+    CK(cudaGetLastError());
+    H.launches += 1;
+  }
   CK(cudaStreamSynchronize(cudaStreamLegacy));  // uploads land before the stream's kernels read them
   H.grad_ipa = ipa;
 }
@@ -5356,18 +5364,26 @@ static void levis_adjoint_device(Handle &H, int nrays, const float *dx, const fl
   G.piph = H.g_piph.p; G.pphw = H.g_pphw.p; G.adj = dadj; G.gradout = H.g_grad.p; G.beam = H.g_beam.p;
   G.botalb = H.botalb.p; G.npart = P.npart; G.maxnmicro = P.maxnmicro; G.ng = P.npx * P.npy * P.npz;
   G.scatmin = (float)P.scatmin;
+  G.cellflip = H.g_flip.p;
   CK(cudaMemsetAsync(H.g_grad.p, 0, H.g_grad.n * sizeof(double), H.stream));
   CK(cudaMemsetAsync(H.g_beam.p, 0, H.g_beam.n * sizeof(double), H.stream));
-  const int blocks = (nrays + shdom::GWARPS - 1) / shdom::GWARPS;
-  shdom::k_levis_adjoint<<<blocks, shdom::GWARPS * 32, 0, H.stream>>>(G);
+  constexpr int per = shdom::GWARPS * shdom::GRAYS;  // rays per block
+  const int blocks = (nrays + per - 1) / per;
+  const size_t smem = sizeof(float) * per * (((P.nlm + 3) & ~3) + 4 + 32);
+  CK(cudaFuncSetAttribute(shdom::k_levis_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  shdom::k_levis_adjoint<<<blocks, shdom::GWARPS * 32, smem, H.stream>>>(G);
   CK(cudaGetLastError());
   shdom::BeamArgs b;
-  b.gridpos = H.gridpos.p; b.zlev = H.zgrid.p; b.beam = H.g_beam.p; b.dextm = H.g_dextm.p; b.gradout = H.g_grad.p;
+  b.gridpos = H.gridpos.p; b.zlev = H.zgrid.p; b.beam = H.g_beam.p; b.sunpath = H.g_sunpath.p;
   b.npts = P.npts; b.npx = P.npx; b.npy = P.npy; b.npz = P.npz; b.bcflag = P.bcflag; b.ipflag = P.ipflag;
   b.delx = P.delx; b.dely = P.dely; b.solarmu = P.prob.solarmu; b.solaraz = P.prob.solaraz;
-  shdom::k_levis_beam<<<(P.npts + 255) / 256, 256, 0, H.stream>>>(b);
+  CK(cudaMemsetAsync(H.g_sunpath.p, 0, H.g_sunpath.n * sizeof(double), H.stream));
+  shdom::k_levis_beam<<<(P.npts + 127) / 128, 128, 0, H.stream>>>(b);
   CK(cudaGetLastError());
-  H.launches += 2;
+  const int ng = P.npx * P.npy * P.npz;
+  shdom::k_levis_beam_add<<<(2 * ng + 255) / 256, 256, 0, H.stream>>>(H.g_sunpath.p, H.g_dextm.p, ng, H.g_grad.p);
+  CK(cudaGetLastError());
+  H.launches += 3;
 }
 
 // Checks shared by the gradient entry points; builds the derivative tables

@@ -52,413 +52,421 @@ struct GradArgs {
   double *gradout;                         // [ng][2]
   double *beam;                            // [npts]
   const float *botalb;                     // surface albedo of the bottom points
+  const uint8_t *cellflip;                 // [ncells] parities of each cell's low corner (k_cell_flip)
   int npart, maxnmicro, ng;
   float scatmin;
 };
 
 constexpr int GWARPS = 4;
+constexpr int GRAYS = 4;   // rays per warp, eight lanes each
 
 // Exact single scatter of phase function iph at this ray's scattering angle.
 __device__ __forceinline__ float ss_phase(const RenderArgs &a, int sj, float sf, int iph) {
   return (1.f - sf) * a.phasetab[(size_t)sj * a.numphase + iph] + sf * a.phasetab[(size_t)(sj + 1) * a.numphase + iph];
 }
 
-// Sum over the four lanes of a corner group.  Only the group's lanes take
-// part, so it may be called where the groups of a warp have diverged (a
-// branch on the corner's point is uniform within its group).
-__device__ __forceinline__ float group_sum(float v) {
-  const unsigned gm = 0xfu << ((threadIdx.x & 31) & ~3u);
-  v += __shfl_xor_sync(gm, v, 1);
-  v += __shfl_xor_sync(gm, v, 2);
+// Sum over the eight lanes of a ray (every lane of the warp takes part).
+__device__ __forceinline__ double ray_sum(double v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  v += __shfl_xor_sync(0xffffffffu, v, 2);
+  v += __shfl_xor_sync(0xffffffffu, v, 4);
   return v;
 }
 
-template <bool GRAD>
-__device__ void levis_traverse(const GradArgs &G, int ray, const float *ydir, const float *tl, double rtot,
-                               double *rtot_out) {
+// Where a ray enters the grid, its direction and its single-scatter table position.
+struct LevisRay {
+  double x, y, z, c[3], ci[3], adj;
+  float mu, sf;
+  int cell, sj;  // cell < 0: nothing to traverse
+};
+
+__device__ LevisRay levis_ray(const GradArgs &G, int ray) {
   const RenderArgs &a = G.r;
-  const int lane = threadIdx.x & 31, grp = lane >> 2, gl = lane & 3;
   const double pi = 3.141592653589793;
-  double x0 = a.camx[ray], y0 = a.camy[ray], z0 = a.camz[ray], mu2 = a.cammu[ray], phi2 = a.camphi[ray];
-  const double muray = -mu2, phiray = phi2 - pi;
+  LevisRay r;
+  r.cell = -1; r.sj = 0; r.sf = 0.f; r.mu = 0.f; r.adj = 0.0;
+  for (int k = 0; k < 3; ++k) { r.c[k] = 0.0; r.ci[k] = 1e6; }
+  r.x = r.y = r.z = 0.0;
+  if (ray >= a.nrays) return r;
+  r.adj = G.adj[ray];
+  if (r.adj == 0.0) return r;
+  double x0 = a.camx[ray], y0 = a.camy[ray], z0 = a.camz[ray];
+  const double mu2 = a.cammu[ray], phi2 = a.camphi[ray], st = sqrt(1.0 - mu2 * mu2);
+  double sn, cn;
+  sincos(phi2 - pi, &sn, &cn);
+  r.mu = (float)mu2;
   const float ztop = a.zgrid[a.nz - 1];
   if (z0 > ztop) {
-    if (muray >= 0.0) { if (rtot_out) *rtot_out = 0.0; return; }
-    double r = (ztop - z0) / muray;
-    x0 += r * sqrt(1 - muray * muray) * cos(phiray);
-    y0 += r * sqrt(1 - muray * muray) * sin(phiray);
+    if (-mu2 >= 0.0) return r;
+    const double d = (ztop - z0) / -mu2;
+    x0 += d * st * cn;
+    y0 += d * st * sn;
     z0 = ztop;
   } else if (z0 < a.zgrid[0]) {
-    if (lane == 0) atomicCAS(a.err, ERR_NONE, ERR_RAY_BELOW);
-    if (rtot_out) *rtot_out = 0.0;
-    return;
+    if ((threadIdx.x & 7) == 0) atomicCAS(a.err, ERR_NONE, ERR_RAY_BELOW);
+    return r;
   }
-  const double adj = GRAD ? G.adj[ray] : 0.0;
-  int sj = 0;
-  float sf = 0.f;
   if (a.deltam) {
     double cosscat = (double)a.solarmu * mu2 + sqrt((1.0 - (double)a.solarmu * a.solarmu) * (1.0 - mu2 * mu2)) * cos((double)a.solaraz - phi2);
     cosscat = fmax(fmin(1.0, cosscat), -1.0);
-    float F = (float)((a.nscatangle - 1) * (acos(cosscat) / pi) + 1);
-    int J = min(a.nscatangle - 1, (int)F);
-    sf = F - J; sj = J - 1;
+    const float F = (float)((a.nscatangle - 1) * (acos(cosscat) / pi) + 1);
+    const int J = min(a.nscatangle - 1, (int)F);
+    r.sf = F - J; r.sj = J - 1;
   }
-  double cx = sqrt(1.0 - mu2 * mu2) * cos(phi2 - pi), cy = sqrt(1.0 - mu2 * mu2) * sin(phi2 - pi), cz = -mu2;
-  double cxinv, cyinv, czinv;
-  if (fabs(cx) > 1e-6) cxinv = 1.0 / cx; else { cx = 0; cxinv = 1e6; }
-  if (fabs(cy) > 1e-6) cyinv = 1.0 / cy; else { cy = 0; cyinv = 1e6; }
-  if (fabs(cz) > 1e-6) czinv = 1.0 / cz; else { cz = 0; czinv = 1e6; }
-  const int bitx = cx < 0, bity = cy < 0, bitz = cz < 0, ioct0 = bitx + 2 * bity + 4 * bitz;
-  const float xm = 0.5f * (a.xgrid[0] + a.xgrid[a.nx - 1]), ym = 0.5f * (a.ygrid[0] + a.ygrid[a.ny - 1]);
-  double xe = x0, ye = y0, ze = z0;
-  int cell = locate_cell(a, xe, ye, ze);
-  const double eps = 1.0e-5 * (a.gridpos[3 * a.gridptr[7] + 2] - a.gridpos[3 * a.gridptr[0] + 2]);
-  const double c12 = (double)0.08333333333f;
-  const int nl = a.ml + 1;
-  int oldp[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
-  float myJ = 0.f, myss = 0.f, myext = 0.f, g4[4] = {0.f, 0.f, 0.f, 0.f};
-  double transmit = 1.0, cumf = 0.0, racc = 0.0;
-  bool validrad = false;
-  int guard = 0;
-  while (!validrad && cell >= 0 && guard++ < (1 << 22)) {
-    const int *g = a.gridptr + 8 * (size_t)cell;
-    const int mypt = g[grp];
-    int reuse = -1;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) if (oldp[k] == mypt) reuse = k;
-    // values of the reused corner from the group that held it
-    const int srcl = reuse >= 0 ? 4 * reuse + gl : lane;
-    const float oJ = __shfl_sync(0xffffffffu, myJ, srcl), oss = __shfl_sync(0xffffffffu, myss, srcl);
-    const float oext = __shfl_sync(0xffffffffu, myext, srcl);
-    float og[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) og[i] = __shfl_sync(0xffffffffu, g4[i], srcl);
-    const bool need = reuse < 0;
-    const int ns = need ? a.ns[mypt] : 0;
-    float s = 0.f;
-    {
-      const float *S = a.source + (size_t)mypt * a.nlm;
-      for (int j = gl; j < ns; j += 4) s += S[j] * ydir[j];
+  r.c[0] = st * cn; r.c[1] = st * sn; r.c[2] = -mu2;
+  for (int k = 0; k < 3; ++k)
+    if (fabs(r.c[k]) > 1e-6) r.ci[k] = 1.0 / r.c[k]; else { r.c[k] = 0; r.ci[k] = 1e6; }
+  r.cell = locate_cell(a, x0, y0, z0);
+  r.x = x0; r.y = y0; r.z = z0;
+  return r;
+}
+
+// What one lane keeps of its corner: source J in the ray's direction, its
+// exact single scatter, and (GRAD) in gv the source gradient for the corner's
+// eight property neighbours, [neighbour][unknown] at a stride of the block
+// (COMPUTE_SOURCE_GRAD_1CELL).
+template <bool GRAD>
+__device__ void levis_corner(const GradArgs &G, const LevisRay &ray, int ip, const float *ydir, const float *tl, float &J,
+                             float &ss, float *gv) {
+  const RenderArgs &a = G.r;
+  const int nl = a.ml + 1, ns = a.ns[ip];
+  const float *S = a.source + (size_t)ip * a.nlm;
+  float s = 0.f;
+  if ((a.nlm & 3) == 0) {
+    float s1 = 0.f, s2 = 0.f, s3 = 0.f;
+    for (int j = 0; j < ns; j += 4) {  // terms past ns are stored as zero
+      const float4 v = *reinterpret_cast<const float4 *>(S + j), y = *reinterpret_cast<const float4 *>(ydir + j);
+      s = fmaf(v.x, y.x, s); s1 = fmaf(v.y, y.y, s1); s2 = fmaf(v.z, y.z, s2); s3 = fmaf(v.w, y.w, s3);
     }
-    s = group_sum(s);
-    // single scattering of the direct beam: with delta-M the exact term of
-    // the unscaled phase function replaces the truncated one in the source;
-    // without, the truncated term (from the series) is the single scatter
-    float ss = 0.f;
-    if (need) {
-      const float da = a.dirflux[mypt] * a.secmu0;
-      const float *cf = a.coef + (size_t)mypt * a.nl;
-      float sub = 0.f;
-      if (ns > 0) {
-        int ls = a.lofj[ns - 1];
-        for (int l = 0; l <= ls; ++l) sub += cf[l] * tl[l];
+    s = (s + s1) + (s2 + s3);
+  } else {
+    for (int j = 0; j < ns; ++j) s = fmaf(S[j], ydir[j], s);
+  }
+  // single scattering of the direct beam: with delta-M the exact term of
+  // the unscaled phase function replaces the truncated one in the source;
+  // without, the truncated term (from the series) is the single scatter
+  const float dirf = a.dirflux[ip], da = dirf * a.secmu0;
+  ss = 0.f;
+  float sub = 0.f;
+  if (ns > 0) {
+    const float *cf = a.coef + (size_t)ip * a.nl;
+    const int ls = a.lofj[ns - 1];
+    for (int l = 0; l <= ls; ++l) sub += cf[l] * tl[l];
+  }
+  if (a.deltam) {
+    s -= da * sub;
+    float add = 0.f;
+    for (int q = a.tms_ptr[ip]; q < a.tms_ptr[ip + 1]; ++q) add += a.tms_w[q] * ss_phase(a, ray.sj, ray.sf, a.tms_iph[q]);
+    ss = da * add;
+    s += ss;
+  } else if (GRAD) {
+    ss = da * sub;
+  }
+  J = s;
+  if constexpr (GRAD) {
+    float singscatj = 0.f;
+    if (a.deltam)
+      for (int q = G.sj_ptr[ip]; q < G.sj_ptr[ip + 1]; ++q) singscatj += G.sj_w[q] * ss_phase(a, ray.sj, ray.sf, G.sj_iph[q]);
+    const float *lt = G.legent_u + (size_t)ip * nl;
+    const float *Rp = a.nlm ? G.radiance + (size_t)ip * a.nlm : nullptr;
+    const int rns = G.nr[ip];
+    // sum_l f_l RY_l, RY_l = sum_m R(l, m) Ydir(l, m) over the point's
+    // radiance terms, for the series of the point less one (d2), of a
+    // property point less the point's (d1) and of the species (dj), each
+    // with the direct beam's term added without delta-M
+    const float beam = a.deltam ? 0.f : da;
+    auto dots = [&](const float *lp, float &d1, float &d2, float &dj) {
+      d1 = d2 = dj = 0.f;
+      const float *ls = G.npart == 1 ? lt : G.legent_s + (size_t)ip * nl;
+      for (int l = 0, j = 0; l < nl; ++l) {
+        const int jn = j + 2 * min(l, a.mm) + 1;
+        float ry = 0.f;
+        for (; j < jn; ++j)
+          if (j < rns) ry = fmaf(Rp[j], ydir[j], ry);
+        const float t = ry + beam * tl[l], f = lt[l];
+        d2 = fmaf(f - 1.f, t, d2);
+        d1 = fmaf(lp[l] - f, t, d1);
+        dj = fmaf(ls[l], t, dj);
       }
-      if (a.deltam) {
-        s -= da * sub;
-        float add = 0.f;
-        for (int q = a.tms_ptr[mypt]; q < a.tms_ptr[mypt + 1]; ++q) add += a.tms_w[q] * ss_phase(a, sj, sf, a.tms_iph[q]);
-        ss = da * add;
-        s += ss;
-      } else if (GRAD) {
-        ss = da * sub;
-      }
-    }
-    if (need) {
-      myJ = s; myss = ss; myext = a.text[mypt];
-      if (GRAD) {
-        // COMPUTE_SOURCE_GRAD_1CELL for the species at this point
-        const int ip = mypt;
-        const float secmu0 = a.secmu0, dirf = a.dirflux[ip];
-        float singscatj = 0.f;
-        if (a.deltam) {
-          float t = 0.f;
-          for (int q = G.sj_ptr[ip] + gl; q < G.sj_ptr[ip + 1]; q += 4) t += G.sj_w[q] * ss_phase(a, sj, sf, G.sj_iph[q]);
-          singscatj = group_sum(t);
-        }
-        // RY_l = sum_m R(l,m) Ydir(l,m) over the point's radiance terms; lane gl keeps l = gl, gl+4, ...
-        float ry[8];
-        const int rns = G.nr[ip];
-        const float *Rp = G.radiance + (size_t)ip * a.nlm;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int l = gl + 4 * i;
-          float v = 0.f;
-          if (l < nl) {
-            const int me = min(l, a.mm), j0 = (l <= a.mm) ? l * l : (2 * a.mm + 1) * l - a.mm * a.mm - a.mm;
-            for (int k = 0; k < 2 * me + 1; ++k) {
-              const int j = j0 + k;
-              if (j < rns) v += Rp[j] * ydir[j];
-            }
-          }
-          ry[i] = v;
-        }
-        auto dot_ry = [&](const float *f) {
-          float t = 0.f;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) { const int l = gl + 4 * i; if (l < nl) t += f[l] * ry[i]; }
-          return group_sum(t);
-        };
-        auto dot_tl = [&](const float *f) {
-          float t = 0.f;
-          for (int l = gl; l < nl; l += 4) t += f[l] * tl[l];
-          return group_sum(t);
-        };
+    };
+    const float albip = G.alb_sp[ip];
+    for (int nb = 0; nb < 8; ++nb) {
+      float v[2] = {0.f, 0.f};
+      const float xi = G.optinterpwt[(size_t)ip * 8 + nb];
+      if (xi >= 1e-7f) {  // (one of the eight where the grid point is a property point)
+        const int ib = G.interpptr[(size_t)ip * 8 + nb];
+        float d1, d2, dj;
+        dots(G.legenp_u + (size_t)ib * nl, d1, d2, dj);
         float sourcet;
-        const float albip = G.alb_sp[ip];
         if (G.npart == 1) {
           sourcet = (albip > 1e-8f) ? s / albip : 0.f;
         } else {
           sourcet = 0.f;
           if (G.scatterj[ip] > G.scatmin) {
-            const float *ls = G.legent_s + (size_t)ip * nl;
-            sourcet = dot_ry(ls);
-            if (!a.deltam) sourcet += dirf * secmu0 * dot_tl(ls);
-            else sourcet += dirf * singscatj * secmu0 / (1.f - G.fmix[ip]);
+            sourcet = dj;
+            if (a.deltam) sourcet += dirf * singscatj * a.secmu0 / (1.f - G.fmix[ip]);
           }
         }
         sourcet = fmaxf(0.f, sourcet);
-        const float *lt = G.legent_u + (size_t)ip * nl;
-        // D2 = sum_l (lt_l - 1) RY_l, the DFJ part of DSOURCE
-        float tmp[32];
-        for (int l = 0; l < nl; ++l) tmp[l] = lt[l] - 1.f;
-        const float d2 = dot_ry(tmp) + (a.deltam ? 0.f : dirf * secmu0 * dot_tl(tmp));
-#pragma unroll
-        for (int i = 0; i < 4; ++i) g4[i] = 0.f;
-        for (int nb = 0; nb < 8; ++nb) {
-          const float xi = G.optinterpwt[(size_t)ip * 8 + nb];
-          if (xi < 1e-7f) continue;
-          const int ib = G.interpptr[(size_t)ip * 8 + nb];
-          const float *lp = G.legenp_u + (size_t)ib * nl;
-          for (int l = 0; l < nl; ++l) tmp[l] = lp[l] - lt[l];
-          const float d1 = dot_ry(tmp) + (a.deltam ? 0.f : dirf * secmu0 * dot_tl(tmp));
-          float ssp = 0.f;
-          if (a.deltam)
-            for (int q = 0; q < G.maxnmicro; ++q) ssp += G.pphw[(size_t)ib * G.maxnmicro + q] * ss_phase(a, sj, sf, G.piph[(size_t)ib * G.maxnmicro + q] - 1);
-          const float ep = G.extp[ib], ap = G.albp[ib];
-#pragma unroll
-          for (int d = 0; d < 2; ++d) {
-            const float DE = d == 0 ? 1.f : 0.f, DA = d == 1 ? 1.f : 0.f;
-            const float DFJ = G.dfj[((size_t)ip * 8 + nb) * 2 + d];
-            const float dsource = (DE * ap + DA * ep) * d1 + DFJ * d2;
-            float v = xi * (sourcet * (albip * G.dextm[(size_t)ib * 2 + d] + G.dalbm[((size_t)ip * 8 + nb) * 2 + d]) + dsource);
-            // emission e (1 - albedo) B (src/polarized/shdomsub4.f:2009-2016), no temperature unknowns
-            if (G.planck)
-              v += xi * (G.planck[ip] * (1.f - albip) * G.dextm[(size_t)ib * 2 + d] -
-                         G.planck[ip] * G.dalbm[((size_t)ip * 8 + nb) * 2 + d]);
-            if (a.deltam) v += dirf * secmu0 * xi * (singscatj * DFJ + DA * (ssp - singscatj) * ep + DE * (ssp - singscatj) * ap);
-            if ((nb >> 1) == gl) g4[(nb & 1) * 2 + d] = v;
-          }
-        }
-      }
-    } else {
-      myJ = oJ; myss = oss; myext = oext;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) g4[i] = og[i];
-    }
-    float ext8[8], src8[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const float e = __shfl_sync(0xffffffffu, myext, 4 * k);
-      ext8[k] = e;
-      src8[k] = __shfl_sync(0xffffffffu, myJ, 4 * k) * e;
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) oldp[k] = g[k];
-    const int ip1 = g[0], ip2 = g[7];
-    const float *P1 = a.gridpos + 3 * ip1, *P2 = a.gridpos + 3 * ip2;
-    const float delx = P2[0] - P1[0], dely = P2[1] - P1[1], delz = P2[2] - P1[2];
-    const double idx = delx <= 0.f ? 1.0 : 1.0 / delx, idy = dely <= 0.f ? 1.0 : 1.0 / dely, idz = 1.0 / delz;
-    // Positions, path lengths and the trilinear weights are FP64, as in
-    // ADJOINT_INTEGRATE_1RAY; the interpolated extinction and source are
-    // single precision sums of FP64 products.  The weight terms of the
-    // gradient divide by the interpolated extinction, which cancels to
-    // nearly zero beside clouds and in the extrapolating open-boundary edge
-    // cells, so FP32 weights (relative error 1e-7 of terms of size 50/km)
-    // would not do there.
-    auto kernel8 = [&](double s, double fc[8]) {
-      const double u = (xe + s * cx - P1[0]) * idx, v = (ye + s * cy - P1[1]) * idy, w = (ze + s * cz - P1[2]) * idz;
-      fc[0] = (1 - w) * (1 - v) * (1 - u); fc[1] = (1 - w) * (1 - v) * u; fc[2] = (1 - w) * v * (1 - u); fc[3] = (1 - w) * v * u;
-      fc[4] = w * (1 - v) * (1 - u); fc[5] = w * (1 - v) * u; fc[6] = w * v * (1 - u); fc[7] = w * v * u;
-    };
-    // sum_k fc[k] val[k], each step rounded to single precision
-    auto interp = [](const double fc[8], const float val[8]) {
-      float acc = 0.f;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) acc = (float)((double)acc + fc[k] * (double)val[k]);
-      return acc;
-    };
-    double fc1[8], fc0[8];
-    kernel8(0.0, fc1);
-    float srcext1 = fmaxf(0.f, interp(fc1, src8));
-    float ext1 = interp(fc1, ext8);
-    const int cf = a.cellflags[cell];
-    const bool ipinx = (cf & 1) && !((a.bcflag & 1) && ((cx > 0 && xe < xm) || (cx < 0 && xe > xm)));
-    const bool ipiny = (cf & 2) && !((a.bcflag & 2) && ((cy > 0 && ye < ym) || (cy < 0 && ye > ym)));
-    const int iopp = g[7 - ioct0];
-    const double sox = ipinx ? 1e20 : (a.gridpos[3 * iopp] - xe) * cxinv;
-    const double soy = ipiny ? 1e20 : (a.gridpos[3 * iopp + 1] - ye) * cyinv;
-    const double soz = (a.gridpos[3 * iopp + 2] - ze) * czinv;
-    const double so = fmin(sox, fmin(soy, soz));
-    if (so < -eps) { if (lane == 0) atomicCAS(a.err, ERR_NONE, ERR_RAY_SO); break; }
-    double xn = xe + so * cx, yn = ye + so * cy, zn = ze + so * cz;
-    double fcn[8];
-    kernel8(so, fcn);
-    const float extn = interp(fcn, ext8);
-    const double taugrid = so * 0.5 * (ext1 + extn);
-    const int ntau = max(1, 1 + (int)(taugrid / a.tautol));
-    const double dels = so / ntau;
-    double accG = 0.0, accS = 0.0, accR = 0.0;  // per-cell weights of this lane's corner
-    const float ss8 = myss * myext;                // this corner's single scatter x extinction
-    for (int it = 1; it <= ntau; ++it) {
-      kernel8(it * dels, fc0);
-      float srcext0 = interp(fc0, src8);
-      const float ext0 = it != ntau ? interp(fc0, ext8) : extn;
-      srcext0 = fmaxf(0.f, srcext0);
-      const double ext = 0.5 * ((double)ext0 + (double)ext1);
-      double transcell;
-      if (ext != 0.0) {
-        const double tau = ext * dels;
-        const double abscell = tau * (1.0 - 0.5 * tau * (1.0 - 0.33333333333 * tau));
-        transcell = 1.0 - abscell;
-        const double corr = dels * (1.0 - 0.05 * ((double)ext1 - (double)ext0) * dels);
-        const double src = (0.5 * ((double)srcext0 + srcext1) + c12 * ((double)ext0 * srcext1 - (double)ext1 * srcext0) * corr) / ext;
-        const double fn = transmit * src * abscell;
-        if (GRAD) {
-          const double w0 = fc0[grp], w1 = fc1[grp];
-          const double wk = (0.5 * (w0 + w1) + c12 * ((double)ext0 * w1 - (double)ext1 * w0) * corr) / ext;
-          accG += transmit * abscell * wk;
-          // the single scatter is interpolated with each corner's term
-          // clamped at zero (SINGSCAT0/1 of ADJOINT_INTEGRATE_1RAY); the
-          // trilinear weights go negative where open-boundary edge cells
-          // extrapolate beyond the cell
-          const double s0 = fmaxf(0.f, (float)(w0 * ss8)), s1 = fmaxf(0.f, (float)(w1 * ss8));
-          accS += transmit * abscell * (0.5 * (s0 + s1) + c12 * ((double)ext0 * s1 - (double)ext1 * s0) * corr) / ext;
-          // radiance still to come from the start and from the end of this interval
-          const double pr1 = (rtot - cumf) / transmit;
-          const double tnext = transmit * transcell;
-          const double pr0 = (rtot - cumf - fn) / tnext;
-          double e0 = 0.0, e1 = 0.0;  // (COMPUTE_RADIANCE_DERIVATIVE_ADJOINT sums these in double)
-#pragma unroll
-          for (int k = 0; k < 8; ++k) { e0 += (double)ext8[k] * fc0[k]; e1 += (double)ext8[k] * fc1[k]; }
-          const double eavg = 0.5 * (e0 + e1);
-          if (eavg != 0.0) {
-            const double gb0 = -adj * pr0 * w0, gb1 = -adj * pr1 * w1;
-            double ag = (0.5 * (gb0 + gb1) + c12 * (e0 * gb1 - e1 * gb0) * dels * (1.0 - 0.05 * (e1 - e0) * dels)) / eavg;
-            accR += ag * transmit * abscell;
-          }
-        }
-        cumf += fn;
-        racc += fn;
-      } else {
-        transcell = 1.0;
-        accS = 0.0;
-      }
-      transmit *= transcell;
-      ext1 = ext0; srcext1 = srcext0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) fc1[k] = fc0[k];
-    }
-    if (GRAD) {
-      // source-gradient and attenuation terms for this lane's corner, property neighbours 2gl and 2gl+1
-      const int ip = mypt;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int nb = 2 * gl + h;
-        const float xi = G.optinterpwt[(size_t)ip * 8 + nb];
-        const int ib = G.interpptr[(size_t)ip * 8 + nb];
+        float ssp = 0.f;
+        if (a.deltam)
+          for (int q = 0; q < G.maxnmicro; ++q)
+            ssp += G.pphw[(size_t)ib * G.maxnmicro + q] * ss_phase(a, ray.sj, ray.sf, G.piph[(size_t)ib * G.maxnmicro + q] - 1);
+        const float ep = G.extp[ib], ap = G.albp[ib];
 #pragma unroll
         for (int d = 0; d < 2; ++d) {
-          const double v = adj * accG * (double)g4[h * 2 + d];
-          const float eg = G.dextm[(size_t)ib * 2 + d] * xi;
-          const double r = (double)eg * accR;
-          const double tot = v + r;
-          if (tot != 0.0) atomicAdd(&G.gradout[(size_t)ib * 2 + d], tot);
+          const float DE = d == 0 ? 1.f : 0.f, DA = d == 1 ? 1.f : 0.f;
+          const float DFJ = G.dfj[((size_t)ip * 8 + nb) * 2 + d], dal = G.dalbm[((size_t)ip * 8 + nb) * 2 + d];
+          const float dex = G.dextm[(size_t)ib * 2 + d];
+          const float dsource = (DE * ap + DA * ep) * d1 + DFJ * d2;
+          v[d] = xi * (sourcet * (albip * dex + dal) + dsource);
+          // emission e (1 - albedo) B (src/polarized/shdomsub4.f:2009-2016), no temperature unknowns
+          if (G.planck) v[d] += xi * (G.planck[ip] * (1.f - albip) * dex - G.planck[ip] * dal);
+          if (a.deltam) v[d] += dirf * a.secmu0 * xi * (singscatj * DFJ + DA * (ssp - singscatj) * ep + DE * (ssp - singscatj) * ap);
         }
       }
-      if (gl == 0 && accS != 0.0) {
-        const double bw = adj * accS;
+      gv[(2 * nb) * (GWARPS * 32)] = v[0];
+      gv[(2 * nb + 1) * (GWARPS * 32)] = v[1];
+    }
+  }
+}
+
+// One pass over the rays of a warp (eight lanes each).  Returns the ray's
+// radiance; with GRAD adds the gradient of adj times it, rtot the radiance of
+// a first pass.
+template <bool GRAD>
+__device__ double levis_traverse(const GradArgs &G, const LevisRay &ray, const float *ydir, const float *tl, double rtot,
+                                 float *gv) {
+  const RenderArgs &a = G.r;
+  const int lane = threadIdx.x & 31, k8 = lane & 7;
+  const unsigned gmask = 0xffu << (lane & 24);
+  const double cx = ray.c[0], cy = ray.c[1], cz = ray.c[2];
+  const int bitx = cx < 0, bity = cy < 0, bitz = cz < 0, ioct0 = bitx + 2 * bity + 4 * bitz;
+  const float xm = 0.5f * (a.xgrid[0] + a.xgrid[a.nx - 1]), ym = 0.5f * (a.ygrid[0] + a.ygrid[a.ny - 1]);
+  const double eps = 1.0e-5 * (a.gridpos[3 * a.gridptr[7] + 2] - a.gridpos[3 * a.gridptr[0] + 2]);
+  const double c12 = (double)0.08333333333f;
+  double xe = ray.x, ye = ray.y, ze = ray.z;
+  int cell = ray.cell;
+  int mine = -1;  // the point this lane's J, ss and gradient are of
+  float myJ = 0.f, myss = 0.f;
+  double transmit = 1.0, cumf = 0.0, racc = 0.0;
+  bool act = cell >= 0;
+  int guard = 0;
+  while (__any_sync(0xffffffffu, act)) {
+    const int c = act ? cell : 0;
+    // Lane k8 holds the corner whose grid indices have its parities (a cell
+    // without width along an axis: its corner on that side), so a corner
+    // shared with the next cell stays in its lane.
+    const int cb = k8 ^ G.cellflip[c];
+    const int *g = a.gridptr + 8 * (size_t)c;
+    const int ip = g[cb];
+    const float ext = a.text[ip];
+    // a cell without extinction adds nothing and changes no transmission
+    const unsigned cloudy = __ballot_sync(0xffffffffu, ext != 0.f);  // (every lane votes)
+    const bool run = act && (cloudy & gmask);
+    const float *P1 = a.gridpos + 3 * g[0], *P2 = a.gridpos + 3 * g[7];
+    const float p1x = P1[0], p1y = P1[1], p1z = P1[2], p2x = P2[0], p2y = P2[1], p2z = P2[2];
+    if (run && mine != ip) {
+      levis_corner<GRAD>(G, ray, ip, ydir, tl, myJ, myss, gv);
+      mine = ip;
+    }
+    __syncwarp();
+    const int cf = a.cellflags[c];
+    const bool ipinx = (cf & 1) && !((a.bcflag & 1) && ((cx > 0 && xe < xm) || (cx < 0 && xe > xm)));
+    const bool ipiny = (cf & 2) && !((a.bcflag & 2) && ((cy > 0 && ye < ym) || (cy < 0 && ye > ym)));
+    const double sox = ipinx ? 1e20 : ((bitx ? p1x : p2x) - xe) * ray.ci[0];
+    const double soy = ipiny ? 1e20 : ((bity ? p1y : p2y) - ye) * ray.ci[1];
+    const double soz = ((bitz ? p1z : p2z) - ze) * ray.ci[2];
+    const double so = fmin(sox, fmin(soy, soz));
+    if (act && so < -eps) { if (k8 == 0) atomicCAS(a.err, ERR_NONE, ERR_RAY_SO); act = false; }
+    // Positions, path lengths, trilinear weights and the sums of weighted
+    // corner values are FP64: the weight terms of the gradient are of the
+    // size of the interpolated extinction, which cancels to nearly zero
+    // beside clouds and in the extrapolating open-boundary edge cells.
+    // Each lane forms the weight of its own corner only.
+    if (__any_sync(0xffffffffu, run)) {
+      const float delx = p2x - p1x, dely = p2y - p1y, delz = p2z - p1z;
+      const double idx = delx <= 0.f ? 1.0 : 1.0 / delx, idy = dely <= 0.f ? 1.0 : 1.0 / dely, idz = 1.0 / delz;
+      const bool hx = cb & 1, hy = cb & 2, hz = cb & 4;
+      // Rounded as the reference's: the position first, then its coordinate in
+      // the cell.  Where a ray enters through one face and leaves through
+      // another, the corner on neither has weight zero at both ends, and
+      // whether that is exactly zero decides if the cell counts.
+      auto weight = [&](double s) {
+        const double u = (fma(s, cx, xe) - p1x) * idx, v = (fma(s, cy, ye) - p1y) * idy, w = (fma(s, cz, ze) - p1z) * idz;
+        return (hz ? w : 1 - w) * (hy ? v : 1 - v) * (hx ? u : 1 - u);
+      };
+      const double eD = run ? (double)ext : 0.0, jD = run ? (double)(myJ * ext) : 0.0;
+      const double ss8 = (double)(myss * ext);  // this corner's single scatter x extinction
+      double w1 = weight(0.0);
+      double e1 = ray_sum(w1 * eD), s1 = fmax(0.0, ray_sum(w1 * jD));
+      const double wn = weight(so), en = ray_sum(wn * eD);
+      int ntau = 0;
+      if (run) ntau = max(1, 1 + (int)(so * 0.5 * (e1 + en) / a.tautol));
+      const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)ntau);
+      const double dels = ntau > 1 ? so / ntau : so;
+      double accG = 0.0, accS = 0.0, accR = 0.0;  // per-cell weights of this lane's corner
+      for (int it = 1; it <= nmax; ++it) {
+        const bool last = it >= ntau;
+        const double w0 = last ? wn : weight(it * dels);
+        const double e0 = last ? en : 0.0;
+        const double es = nmax > 1 ? ray_sum(w0 * eD) : en;
+        const double e0_ = last ? e0 : es;
+        const double s0 = fmax(0.0, ray_sum(w0 * jD));
+        if (it <= ntau) {
+          const double ex = 0.5 * (e0_ + e1);
+          if (ex != 0.0) {
+            // abscell / ext = dels (1 - tau/2 (1 - tau/3)): no quotient by the extinction
+            const double tau = ex * dels, poly = 1.0 - 0.5 * tau * (1.0 - 0.33333333333 * tau);
+            const double transcell = 1.0 - tau * poly, dp = dels * poly;
+            const double k = c12 * dels * (1.0 - 0.05 * (e1 - e0_) * dels);
+            const double fn = transmit * dp * (0.5 * (s0 + s1) + k * (e0_ * s1 - e1 * s0));
+            if (GRAD) {
+              accG += transmit * dp * (0.5 * (w0 + w1) + k * (e0_ * w1 - e1 * w0));
+              // the single scatter is interpolated with each corner's term
+              // clamped at zero (SINGSCAT0/1 of ADJOINT_INTEGRATE_1RAY); the
+              // trilinear weights go negative where open-boundary edge cells
+              // extrapolate beyond the cell
+              const double g0 = fmax(0.0, w0 * ss8), g1 = fmax(0.0, w1 * ss8);
+              accS += transmit * dp * (0.5 * (g0 + g1) + k * (e0_ * g1 - e1 * g0));
+              // radiance still to come from the start (r1 / transmit) and from
+              // the end of this interval (r0 / transmit)
+              const double r1 = rtot - cumf, r0 = (r1 - fn) / transcell;
+              accR += dp * (0.5 * (r0 * w0 + r1 * w1) + k * (e0_ * r1 * w1 - e1 * r0 * w0));
+            }
+            cumf += fn;
+            racc += fn;
+            transmit *= transcell;
+          } else {
+            accS = 0.0;
+          }
+          e1 = e0_; s1 = s0; w1 = w0;
+        }
+      }
+      if (GRAD && run) {
+        // source-gradient and attenuation terms of this lane's corner
+        const double ag = ray.adj * accG, ar = -ray.adj * accR;
+        if (ag != 0.0 || ar != 0.0) {
+          const float4 *xw = reinterpret_cast<const float4 *>(G.optinterpwt + (size_t)ip * 8);
+          const float4 xa = xw[0], xb = xw[1];
+          const float xs[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+#pragma unroll
+          for (int nb = 0; nb < 8; ++nb) {
+            if (xs[nb] == 0.f) continue;
+            const int ib = G.interpptr[(size_t)ip * 8 + nb];
+            const float2 de = *reinterpret_cast<const float2 *>(G.dextm + (size_t)ib * 2);
+            const double t0 = ag * (double)gv[(2 * nb) * (GWARPS * 32)] + (double)(de.x * xs[nb]) * ar;
+            const double t1 = ag * (double)gv[(2 * nb + 1) * (GWARPS * 32)] + (double)(de.y * xs[nb]) * ar;
+            if (t0 != 0.0) atomicAdd(&G.gradout[(size_t)ib * 2], t0);
+            if (t1 != 0.0) atomicAdd(&G.gradout[(size_t)ib * 2 + 1], t1);
+          }
+        }
+        const double bw = ray.adj * accS;
         if (bw != 0.0) atomicAdd(&G.beam[ip], bw);
       }
     }
-    int iface, jface;
-    bool openbc;
-    if (sox <= soz && sox <= soy) { iface = 1 - bitx; jface = 0; openbc = (cf & 1) && (a.bcflag & 1); }
-    else if (soy <= soz) { iface = 3 - bity; jface = 1; openbc = (cf & 2) && (a.bcflag & 2); }
-    else { iface = 5 - bitz; jface = 2; openbc = false; }
-    const int nxt = a.neighptr[6 * (size_t)cell + iface];
-    int kface = iface, kc = cell;
-    if (openbc) { kface = iface ^ 1; kc = nxt; iface = -1; }
-    if (nxt >= 0) {
-      const float *q = a.gridpos + 3 * a.gridptr[8 * (size_t)nxt + ioct0];
-      if (jface == 0) xn = q[0]; else if (jface == 1) yn = q[1]; else zn = q[2];
-    }
-    if (transmit < a.transcut) {
-      validrad = true;
-    } else if (nxt < 0 && iface >= 4) {
-      validrad = true;
-      const int *gk = a.gridptr + 8 * (size_t)kc;
-      float xs[4], ys[4], rb[4], dr[4];
-      int bp[4];
+    if (act) {
+      int iface, jface;
+      bool openbc;
+      if (sox <= soz && sox <= soy) { iface = 1 - bitx; jface = 0; openbc = (cf & 1) && (a.bcflag & 1); }
+      else if (soy <= soz) { iface = 3 - bity; jface = 1; openbc = (cf & 2) && (a.bcflag & 2); }
+      else { iface = 5 - bitz; jface = 2; openbc = false; }
+      const int nxt = a.neighptr[6 * (size_t)c + iface];
+      int kface = iface, kc = c;
+      if (openbc) { kface = iface ^ 1; kc = nxt; iface = -1; }
+      double xn = xe + so * cx, yn = ye + so * cy, zn = ze + so * cz;
+      if (nxt >= 0) {
+        const float *q = a.gridpos + 3 * a.gridptr[8 * (size_t)nxt + ioct0];
+        if (jface == 0) xn = q[0]; else if (jface == 1) yn = q[1]; else zn = q[2];
+      }
+      if (transmit < a.transcut) {
+        act = false;
+      } else if (nxt < 0 && iface >= 4) {
+        act = false;
+        const int *gk = a.gridptr + 8 * (size_t)kc;
+        float xs[4], ys[4], rb[4], dr[4];
+        int bp[4];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int q = gk[c_face[kface][k]];
-        bp[k] = q; xs[k] = a.gridpos[3 * q]; ys[k] = a.gridpos[3 * q + 1]; dr[k] = 0.f;
-        if ((float)mu2 < 0.f) rb[k] = a.skyrad;
-        else {
-          const int bi = a.bot_index[q];
-          rb[k] = bi >= 0 ? a.bcrad_bot[bi] : 0.f;
-          if (bi >= 0) dr[k] = 0.318309886f * G.botalb[bi] * a.dirflux[q];
+        for (int k = 0; k < 4; ++k) {
+          const int q = gk[c_face[kface][k]];
+          bp[k] = q; xs[k] = a.gridpos[3 * q]; ys[k] = a.gridpos[3 * q + 1]; dr[k] = 0.f;
+          if (ray.mu < 0.f) rb[k] = a.skyrad;
+          else {
+            const int bi = a.bot_index[q];
+            rb[k] = bi >= 0 ? a.bcrad_bot[bi] : 0.f;
+            if (bi >= 0) dr[k] = 0.318309886f * G.botalb[bi] * a.dirflux[q];
+          }
         }
+        const double uu = (xs[1] - xs[0] > 0) ? (xn - xs[0]) / (xs[1] - xs[0]) : 0.0;
+        const double vv = (ys[2] - ys[0] > 0) ? (yn - ys[0]) / (ys[2] - ys[0]) : 0.0;
+        const double bi4[4] = {(1 - uu) * (1 - vv), uu * (1 - vv), (1 - uu) * vv, uu * vv};
+        const float radbnd = (float)(bi4[0] * rb[0] + bi4[1] * rb[1] + bi4[2] * rb[2] + bi4[3] * rb[3]);
+        racc += transmit * radbnd;
+        if (GRAD) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (k8 == k) {
+              const double bw = ray.adj * transmit * bi4[k] * (double)dr[k];
+              if (bw != 0.0) atomicAdd(&G.beam[bp[k]], bw);
+            }
+        }
+      } else {
+        cell = nxt;
+        if (cell < 0 || ++guard >= (1 << 22)) act = false;
       }
-      const double uu = (xs[1] - xs[0] > 0) ? (xn - xs[0]) / (xs[1] - xs[0]) : 0.0;
-      const double vv = (ys[2] - ys[0] > 0) ? (yn - ys[0]) / (ys[2] - ys[0]) : 0.0;
-      const double bi4[4] = {(1 - uu) * (1 - vv), uu * (1 - vv), (1 - uu) * vv, uu * vv};
-      const float radbnd = (float)(bi4[0] * rb[0] + bi4[1] * rb[1] + bi4[2] * rb[2] + bi4[3] * rb[3]);
-      racc += transmit * radbnd;
-      if (GRAD && lane < 4) {
-        const double bw = adj * transmit * bi4[lane] * (double)dr[lane];
-        if (bw != 0.0) atomicAdd(&G.beam[bp[lane]], bw);
-      }
-    } else {
-      cell = nxt;
+      xe = xn; ye = yn; ze = zn;
     }
-    xe = xn; ye = yn; ze = zn;
   }
-  if (rtot_out) *rtot_out = racc;
+  return racc;
 }
 
-// Pass A then pass B for each ray (one warp per ray).
+// Per cell, which of its low corner's grid indices are odd (0 along an axis
+// on which the cell has no width): bits x, y, z.
+__global__ void k_cell_flip(const int *__restrict__ gridptr, int ncells, int ny1, int nz, uint8_t *__restrict__ flip) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= ncells) return;
+  const int lo = gridptr[8 * (size_t)c], hi = gridptr[8 * (size_t)c + 7];
+  const int z0 = lo % nz, y0 = lo / nz % ny1, x0 = lo / nz / ny1, z1 = hi % nz, y1 = hi / nz % ny1, x1 = hi / nz / ny1;
+  flip[c] = (uint8_t)((x0 != x1 ? x0 & 1 : 0) | (y0 != y1 ? (y0 & 1) << 1 : 0) | (z0 != z1 ? (z0 & 1) << 2 : 0));
+}
+
+// Pass A then pass B for the rays of a warp.  Dynamic shared memory: per ray
+// the functions of its direction (nlm + 4 floats, so that the four rays of a
+// warp read different banks) and t_l (32 floats).
 __global__ void __launch_bounds__(GWARPS * 32) k_levis_adjoint(GradArgs G) {
-  __shared__ float ydir_s[GWARPS][RNLM];
-  __shared__ float tl_s[GWARPS][64];
+  extern __shared__ __align__(16) float gsm[];
+  __shared__ float gvs[16 * GWARPS * 32];
   const RenderArgs &a = G.r;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int ray = blockIdx.x * GWARPS + w;
-  if (ray >= a.nrays) return;
-  if (G.adj[ray] == 0.0) return;
-  float *ydir = ydir_s[w], *tl = tl_s[w];
-  ylm_dir_warp(ydir, (float)a.cammu[ray], (float)a.camphi[ray], a.ml, a.mm, lane);
-  __syncwarp();
-  for (int l = lane; l <= a.ml; l += 32) {
-    int me = min(l, a.mm), j0 = (l <= a.mm) ? l * l : (2 * a.mm + 1) * l - a.mm * a.mm - a.mm;
-    float s = 0.f;
-    for (int k = 0; k < 2 * me + 1; ++k) s += ydir[j0 + k] * a.ylmsun[j0 + k];
-    tl[l] = s;
+  const int k8 = threadIdx.x & 7, lr = threadIdx.x >> 3;
+  const int ystr = ((a.nlm + 3) & ~3) + 4;
+  float *ydir = gsm + lr * ystr, *tl = gsm + GWARPS * GRAYS * ystr + lr * 32;
+  const LevisRay ray = levis_ray(G, blockIdx.x * (GWARPS * GRAYS) + lr);
+  if (ray.cell >= 0) {
+    const int i = blockIdx.x * (GWARPS * GRAYS) + lr;
+    ylm_dir_lanes(ydir, (float)a.cammu[i], (float)a.camphi[i], a.ml, a.mm, k8, 8);
   }
   __syncwarp();
-  double rtot = 0.0;
-  levis_traverse<false>(G, ray, ydir, tl, 0.0, &rtot);
-  levis_traverse<true>(G, ray, ydir, tl, rtot, nullptr);
+  if (ray.cell >= 0)
+    for (int l = k8; l <= a.ml; l += 8) {
+      const int me = min(l, a.mm), j0 = (l <= a.mm) ? l * l : (2 * a.mm + 1) * l - a.mm * a.mm - a.mm;
+      float s = 0.f;
+      for (int k = 0; k < 2 * me + 1; ++k) s += ydir[j0 + k] * a.ylmsun[j0 + k];
+      tl[l] = s;
+    }
+  __syncwarp();
+  const double rtot = levis_traverse<false>(G, ray, ydir, tl, 0.0, nullptr);
+  levis_traverse<true>(G, ray, ydir, tl, rtot, gvs + threadIdx.x);
 }
 
 // Direct-beam term: for each point with a non-zero beam weight, the sun
 // path's d(optical path)/d(extinction) per property corner, cell by cell
-// (the path of DIRECT_BEAM_PROP).
+// (the path of DIRECT_BEAM_PROP).  The weights are summed per property point
+// (one atomic per corner); k_levis_beam_add turns the sums into both
+// unknowns' derivatives.
 struct BeamArgs {
   const float *gridpos, *zlev;
   const double *beam;
-  const float *dextm;
-  double *gradout;
+  double *sunpath;  // [ng] sum over points of beam weight times d(optical path)/d(extinction)
   int npts, npx, npy, npz, bcflag, ipflag;
   float delx, dely, solarmu, solaraz;
 };
@@ -533,33 +541,30 @@ __global__ void k_levis_beam(BeamArgs b) {
     const double ax = 1.0 / (x1 - x0), ay = 1.0 / (y1 - y0), az = 1.0 / (z1 - z0);
     const double u0 = (xe - x0) * ax, v0 = (ye - y0) * ay, w0 = (ze - z0) * az;
     const double du = (xp - x0) * ax - u0, dv = (yp - y0) * ay - v0, dw = (zp - z0) * az - w0;
-    const double u0m = 1 - u0, v0m = 1 - v0, w0m = 1 - w0;
-    const double uv = u0 * v0, umv = u0m * v0, uvm = u0 * v0m, umvm = u0m * v0m;
-    const double uw = u0 * w0, umw = u0m * w0, uwm = u0 * w0m, umwm = u0m * w0m;
-    const double vw = v0 * w0, vmw = v0m * w0, vwm = v0 * w0m, vmwm = v0m * w0m;
-    const double A[8] = {u0m * vmwm, u0 * vmwm, u0m * vwm, u0 * vwm, u0m * vmw, u0 * vmw, u0m * vw, u0 * vw};
-    const double B[8] = {-du * vmwm - dv * umwm - dw * umvm, du * vmwm - dv * uwm - dw * uvm,
-                         -du * vwm + dv * umwm - dw * umv,   du * vwm + dv * uwm - dw * uv,
-                         -du * vmw - dv * umw + dw * umvm,   du * vmw - dv * uw + dw * uvm,
-                         -du * vw + dv * umw + dw * umv,     du * vw + dv * uw + dw * uv};
-    const double VW = dv * dw, vwu = VW * u0, vwum = VW * u0m, UW = du * dw, uwv = UW * v0, uwvm = UW * v0m;
-    const double UV = du * dv, uvw = UV * w0, uvwm = UV * w0m;
-    const double C[8] = {vwum + uwvm + uvwm, vwu - uwvm - uvwm, -vwum + uwv - uvwm, -vwu - uwv + uvwm,
-                         -vwum - uwvm + uvw, -vwu + uwvm - uvw, vwum - uwv - uvw,   vwu + uwv + uvw};
-    const double sgn[8] = {-1, 1, 1, -1, 1, -1, -1, 1}, ddd = du * dv * dw;
+    // the path integral of each corner's trilinear weight: a cubic along the
+    // segment, exact with the two-point Gauss rule
+    constexpr double t1 = 0.21132486540518713, t2 = 0.78867513459481287;
+    const double ua = fma(t1, du, u0), va = fma(t1, dv, v0), wa = fma(t1, dw, w0);
+    const double ub = fma(t2, du, u0), vb = fma(t2, dv, v0), wb = fma(t2, dw, w0);
+    const double h = 0.5 * so;
+    const double a00 = (1 - va) * (1 - wa) * h, a10 = va * (1 - wa) * h, a01 = (1 - va) * wa * h, a11 = va * wa * h;
+    const double b00 = (1 - vb) * (1 - wb) * h, b10 = vb * (1 - wb) * h, b01 = (1 - vb) * wb * h, b11 = vb * wb * h;
+    const double path[8] = {(1 - ua) * a00 + (1 - ub) * b00, ua * a00 + ub * b00, (1 - ua) * a10 + (1 - ub) * b10, ua * a10 + ub * b10,
+                            (1 - ua) * a01 + (1 - ub) * b01, ua * a01 + ub * b01, (1 - ua) * a11 + (1 - ub) * b11, ua * a11 + ub * b11};
     const int ptrs[8] = {I1, I2, I3, I4, I1 + 1, I2 + 1, I3 + 1, I4 + 1};
 #pragma unroll
     for (int c = 0; c < 8; ++c) {
-      const float dpath = (float)(so * (A[c] + 0.5 * B[c] + 0.3333333333333333 * C[c] + sgn[c] * 0.25 * ddd));
-      if (dpath == 0.f) continue;
-#pragma unroll
-      for (int d = 0; d < 2; ++d) {
-        const double v = -(double)b.dextm[(size_t)ptrs[c] * 2 + d] * dpath * weight;
-        if (v != 0.0) atomicAdd(&b.gradout[(size_t)ptrs[c] * 2 + d], v);
-      }
+      const float dpath = (float)path[c];
+      if (dpath != 0.f) atomicAdd(&b.sunpath[ptrs[c]], weight * dpath);
     }
     xe = xp + xoffs; ye = yp + yoffs; ze = zp;
   }
+}
+
+__global__ void k_levis_beam_add(const double *__restrict__ sunpath, const float *__restrict__ dextm, int ng, double *gradout) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= 2 * ng) return;
+  gradout[i] -= (double)dextm[i] * sunpath[i >> 1];
 }
 
 }  // namespace shdom
