@@ -2804,7 +2804,7 @@ struct RenderArgs {
   const double *cammu, *camphi;
   float *out;
   int *err;
-  int nrays, nx, ny, nz, nlm, nl, ml, mm, bcflag, ipflag, numphase, nscatangle, deltam;
+  int nrays, nx, ny, nz, ny1, nlm, nl, ml, mm, bcflag, ipflag, numphase, nscatangle, deltam;
   // RENDER's SINGLESCATTER (the source is the exact single scatter of the
   // direct beam only) and NOSURFACE (no boundary radiance is added)
   int single_scatter = 0, nosurface = 0;
@@ -2814,17 +2814,19 @@ struct RenderArgs {
 
 // Reflected radiance of bottom point bi toward (mu2, phi2) (the BRDF branch
 // of FIND_BOUNDARY_RADIANCE, src/polarized/shdomsub2.f:2748-2863): the
-// warp sums the downward ordinates; every lane gets the Stokes vector.
-__device__ __noinline__ void brdf_radiance_warp(const RenderArgs &a, int bi, float mu2, float phi2, int lane, int nst, float out[3]) {
+// group of step lanes (mask) sums the downward ordinates; every lane of it
+// gets the Stokes vector.
+__device__ __noinline__ void brdf_radiance_lanes(const RenderArgs &a, int bi, float mu2, float phi2, int first, int step, unsigned mask,
+                                                 int nst, float out[3]) {
   const float *par = a.botpar + (size_t)bi * a.nsfcpar;
   const int p = a.botp[bi];
   const float *row = a.raddo + (size_t)p * a.ord_ps;
   float acc[3] = {0.f, 0.f, 0.f}, R[3][3];
-  if (lane == 0) {
+  if (first == 0) {
     surface_brdf_d(a.brdf, par, mu2, phi2, a.solarmu, a.solaraz, R);
     for (int k = 0; k < nst; ++k) acc[k] = 0.318309886f * R[k][0] * a.dirflux[p];
   }
-  for (int d = lane; d < a.nbrdf_dn; d += 32) {
+  for (int d = first; d < a.nbrdf_dn; d += step) {
     const BrdfOrd i = a.brdf_dn[d];
     surface_brdf_d(a.brdf, par, mu2, phi2, i.mu, i.phi, R);
     const int ci = (int)i.col, oi = (int)i.off;
@@ -2840,7 +2842,7 @@ __device__ __noinline__ void brdf_radiance_warp(const RenderArgs &a, int bi, flo
   }
   for (int k = 0; k < 3; ++k) {
     float v = acc[k];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    for (int o = step >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
     out[k] = v;
   }
 }
@@ -2886,14 +2888,8 @@ __device__ int locate_cell(const RenderArgs &a, double &x0, double &y0, double z
   return (iz - 1) + (nz - 1) * (iy - 1) + (nz - 1) * nyc * (ix - 1);
 }
 
-constexpr int RWARPS = 4;     // rays (warps) per block
 constexpr int RNLM = 1024;    // max spherical-harmonic terms for the per-ray tables
 
-// One warp per ray (RENDER / INTEGRATE_1RAY / COMPUTE_SOURCE_1CELL_UNPOL /
-// FIND_BOUNDARY_RADIANCE, src/polarized/shdomsub4.f:93-286,
-// src/polarized/shdomsub2.f:2311-2863, :3046-3192).  The spherical-harmonic
-// dot products of the new cell corners are split over groups of four lanes;
-// the path integration is evaluated uniformly by all lanes.
 // Real spherical harmonics Y_lm of one direction (mu, phi) into y[NLM] (the
 // j(l, m) term order of the solver), this lane running the upward l
 // recurrence of the normalised Wigner d^l_{m0}(mu) for m = first, first +
@@ -2926,244 +2922,6 @@ __device__ __forceinline__ void ylm_dir_lanes(float *y, float x, float phf, int 
   }
 }
 
-// The ray's direction for the cell walk, in FP32: direction cosines,
-// their inverses (1e6 where a cosine is below 1e-6 and set to zero, as the
-// reference's INTEGRATE_1RAY) and the octant bits.
-struct RayDir {
-  float c[3], ci[3];
-  int bit[3], ioct;
-};
-__device__ __forceinline__ RayDir ray_dir(double mu2, double phi2) {
-  const double pi = 3.141592653589793;
-  const double st = sqrt(1.0 - mu2 * mu2);
-  double c[3] = {st * cos(phi2 - pi), st * sin(phi2 - pi), -mu2};
-  RayDir r;
-  for (int k = 0; k < 3; ++k) {
-    double ci;
-    if (fabs(c[k]) > 1e-6) ci = 1.0 / c[k]; else { c[k] = 0.0; ci = 1e6; }
-    r.c[k] = (float)c[k]; r.ci[k] = (float)ci; r.bit[k] = c[k] < 0;
-  }
-  r.ioct = r.bit[0] + 2 * r.bit[1] + 4 * r.bit[2];
-  return r;
-}
-
-template <bool BRDF>
-__global__ void __launch_bounds__(RWARPS * 32) k_render(RenderArgs a) {
-  __shared__ float ydir[RWARPS][RNLM];
-  __shared__ float tl[RWARPS][64];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int ray = blockIdx.x * RWARPS + w;
-  if (ray >= a.nrays) return;
-  const double pi = 3.141592653589793;
-  double x0 = a.camx[ray], y0 = a.camy[ray], z0 = a.camz[ray], mu2 = a.cammu[ray], phi2 = a.camphi[ray];
-  const double muray = -mu2, phiray = phi2 - pi;
-  const float ztop = a.zgrid[a.nz - 1];
-  if (z0 > ztop) {
-    if (muray >= 0.0) { if (lane == 0) a.out[ray] = 0.f; return; }
-    double r = (ztop - z0) / muray;
-    x0 += r * sqrt(1 - muray * muray) * cos(phiray);
-    y0 += r * sqrt(1 - muray * muray) * sin(phiray);
-    z0 = ztop;
-  } else if (z0 < a.zgrid[0]) {
-    if (lane == 0) { atomicCAS(a.err, ERR_NONE, ERR_RAY_BELOW); a.out[ray] = 0.f; }
-    return;
-  }
-  // Y_lm in the ray direction: lane m runs the l recurrence of its m
-  ylm_dir_lanes(ydir[w], (float)mu2, (float)phi2, a.ml, a.mm, lane, 32);
-  __syncwarp();
-  // t_l = sum_m Ydir(l,m) Ysun(l,m)
-  for (int l = lane; l <= a.ml; l += 32) {
-    int me = min(l, a.mm), j0 = (l <= a.mm) ? l * l : (2 * a.mm + 1) * l - a.mm * a.mm - a.mm;
-    float s = 0.f;
-    for (int k = 0; k < 2 * me + 1; ++k) s += ydir[w][j0 + k] * a.ylmsun[j0 + k];
-    tl[w][l] = s;
-  }
-  __syncwarp();
-  // single-scatter phase table interpolation parameters
-  int sj = 0;
-  float sf = 0.f;
-  if (a.deltam) {
-    double cosscat = (double)a.solarmu * mu2 + sqrt((1.0 - (double)a.solarmu * a.solarmu) * (1.0 - mu2 * mu2)) * cos((double)a.solaraz - phi2);
-    cosscat = fmax(fmin(1.0, cosscat), -1.0);
-    float F = (float)((a.nscatangle - 1) * (acos(cosscat) / pi) + 1);
-    int J = min(a.nscatangle - 1, (int)F);
-    sf = F - J; sj = J - 1;
-  }
-  RayDir rd = ray_dir(mu2, phi2);
-  const int ioct0 = rd.ioct;
-  const float xm = 0.5f * (a.xgrid[0] + a.xgrid[a.nx - 1]), ym = 0.5f * (a.ygrid[0] + a.ygrid[a.ny - 1]);
-  double xe = x0, ye = y0, ze = z0;
-  int cell = locate_cell(a, xe, ye, ze);
-  // the position as the cell's low corner (grid coordinates) plus an FP32 offset
-  float lx, ly, lz;
-  if (cell >= 0) {
-    const float *P = a.gridpos + 3 * a.gridptr[8 * (size_t)cell];
-    lx = (float)(xe - P[0]); ly = (float)(ye - P[1]); lz = (float)(ze - P[2]);
-  }
-  const float eps = 1.0e-5f * (a.gridpos[3 * a.gridptr[7] + 2] - a.gridpos[3 * a.gridptr[0] + 2]);
-  const int maxcross = 500 * max(a.nx, max(a.ny, a.nz));
-  int oldp[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
-  float osrc[8] = {0};
-  float ext8[8], src8[8];
-  double radacc = 0.0, transmit = 1.0;
-  const float inv_tautol = 1.0f / a.tautol;
-  int ngrid = 0;
-  bool validrad = false;
-  const int grp = lane >> 2, gl = lane & 3;  // 8 groups of 4 lanes, one corner per group
-  while (!validrad && cell >= 0) {
-    ++ngrid;
-    const int *g = a.gridptr + 8 * (size_t)cell;
-    int mypt = g[grp];
-    // reuse corners already evaluated for the previous cell
-    int reuse = -1;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) if (oldp[k] == mypt) reuse = k;
-    float cval = 0.f, cext = a.text[mypt];
-    const bool need = reuse < 0;
-    const int ns = (need && !a.single_scatter) ? a.ns[mypt] : 0;
-    float s = 0.f;
-    {
-      const float *S = a.source + (size_t)mypt * a.nlm;
-      for (int j = gl; j < ns; j += 4) s += S[j] * ydir[w][j];
-    }
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    if (!need) {
-      cval = osrc[reuse];
-    } else {
-      if (a.deltam) {
-        const float da = a.dirflux[mypt] * a.secmu0;
-        const float *cf = a.coef + (size_t)mypt * a.nl;
-        if (ns > 0) {
-          int ls = a.lofj[ns - 1];
-          float sub = 0.f;
-          for (int l = 0; l <= ls; ++l) sub += cf[l] * tl[w][l];
-          s -= da * sub;
-        }
-        float add = 0.f;
-        for (int q = a.tms_ptr[mypt]; q < a.tms_ptr[mypt + 1]; ++q) {
-          int iph = a.tms_iph[q];
-          float ss = (1.f - sf) * a.phasetab[(size_t)sj * a.numphase + iph] + sf * a.phasetab[(size_t)(sj + 1) * a.numphase + iph];
-          add += a.tms_w[q] * ss;
-        }
-        s += da * add;
-      }
-      cval = s * cext;
-    }
-    // gather the 8 corners from the groups
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      src8[k] = __shfl_sync(0xffffffffu, cval, 4 * k);
-      ext8[k] = __shfl_sync(0xffffffffu, cext, 4 * k);
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { oldp[k] = g[k]; osrc[k] = src8[k]; }
-    const int ip1 = g[0], ip2 = g[7];
-    const float *P1 = a.gridpos + 3 * ip1, *P2 = a.gridpos + 3 * ip2;
-    const float delx = P2[0] - P1[0], dely = P2[1] - P1[1], delz = P2[2] - P1[2];
-    const float idx = delx <= 0.f ? 1.f : 1.f / delx, idy = dely <= 0.f ? 1.f : 1.f / dely, idz = 1.f / delz;
-    // The geometry of the step runs in FP32 on cell-relative offsets (an
-    // offset from the cell's own corner keeps FP32's relative precision on
-    // the cell size); only the two ray accumulators stay FP64.  The
-    // trilinear weights are cell-relative coordinates in [0, 1].
-    auto tri = [&](const float *v, float u, float vv, float ww) {
-      const float a0 = fmaf(u, v[1] - v[0], v[0]), a1 = fmaf(u, v[3] - v[2], v[2]);
-      const float a2 = fmaf(u, v[5] - v[4], v[4]), a3 = fmaf(u, v[7] - v[6], v[6]);
-      const float b0 = fmaf(vv, a1 - a0, a0), b1 = fmaf(vv, a3 - a2, a2);
-      return fmaf(ww, b1 - b0, b0);
-    };
-    const float u0 = lx * idx, v0 = ly * idy, w0 = lz * idz;
-    float srcext1 = fmaxf(0.f, tri(src8, u0, v0, w0));
-    float ext1 = tri(ext8, u0, v0, w0);
-    const int cf = a.cellflags[cell];
-    const float cx = rd.c[0], cy = rd.c[1], cz = rd.c[2];
-    bool ipinx = (cf & 1) && !((a.bcflag & 1) && ((cx > 0 && P1[0] + lx < xm) || (cx < 0 && P1[0] + lx > xm)));
-    bool ipiny = (cf & 2) && !((a.bcflag & 2) && ((cy > 0 && P1[1] + ly < ym) || (cy < 0 && P1[1] + ly > ym)));
-    const float *Po = a.gridpos + 3 * g[7 - ioct0];
-    const float sox = ipinx ? 1e20f : ((Po[0] - P1[0]) - lx) * rd.ci[0];
-    const float soy = ipiny ? 1e20f : ((Po[1] - P1[1]) - ly) * rd.ci[1];
-    const float soz = ((Po[2] - P1[2]) - lz) * rd.ci[2];
-    const float so = fminf(sox, fminf(soy, soz));
-    if (so < -eps) { if (lane == 0) atomicCAS(a.err, ERR_NONE, ERR_RAY_SO); break; }
-    const float lxn = fmaf(so, cx, lx), lyn = fmaf(so, cy, ly), lzn = fmaf(so, cz, lz);
-    // per unit path length, the cell-relative coordinates move by (du, dv, dw)
-    const float du = cx * idx, dv = cy * idy, dw = cz * idz;
-    const float sof = so;
-    float extn = tri(ext8, fmaf(sof, du, u0), fmaf(sof, dv, v0), fmaf(sof, dw, w0));
-    const float taugrid = so * 0.5f * (ext1 + extn);
-    int ntau = max(1, 1 + (int)(taugrid * inv_tautol));
-    const float delsf = sof / (float)ntau;
-    // the cell's source integral and transmission from its entry, in FP32;
-    // folded into the FP64 ray accumulators once per cell
-    float cacc = 0.f, ctr = 1.f;
-    for (int it = 1; it <= ntau; ++it) {
-      const float sf_ = it * delsf;
-      const float uu_ = fmaf(sf_, du, u0), vv_ = fmaf(sf_, dv, v0), ww_ = fmaf(sf_, dw, w0);
-      float ext0 = tri(ext8, uu_, vv_, ww_);
-      float srcext0 = fmaxf(0.f, tri(src8, uu_, vv_, ww_));
-      float ext = 0.5f * (ext0 + ext1);
-      float absc, trc, src;
-      if (ext != 0.f) {
-        float tau = ext * delsf;
-        absc = tau * (1.f - 0.5f * tau * (1.f - 0.33333333333f * tau));
-        trc = 1.f - absc;
-        src = (0.5f * (srcext0 + srcext1) + 0.08333333333f * (ext0 * srcext1 - ext1 * srcext0) * delsf *
-                                                (1.f - 0.05f * (ext1 - ext0) * delsf)) / ext;
-      } else { absc = 0.f; trc = 1.f; src = 0.f; }
-      cacc = fmaf(ctr * src, absc, cacc);
-      ctr *= trc;
-      ext1 = ext0; srcext1 = srcext0;
-    }
-    radacc += transmit * (double)cacc;
-    transmit *= (double)ctr;
-    int iface, jface;
-    bool openbc;
-    if (sox <= soz && sox <= soy) { iface = 1 - rd.bit[0]; jface = 0; openbc = (cf & 1) && (a.bcflag & 1); }
-    else if (soy <= soz) { iface = 3 - rd.bit[1]; jface = 1; openbc = (cf & 2) && (a.bcflag & 2); }
-    else { iface = 5 - rd.bit[2]; jface = 2; openbc = false; }
-    int nxt = a.neighptr[6 * (size_t)cell + iface];
-    int kface = iface, kc = cell;
-    if (openbc) { kface = iface ^ 1; kc = nxt; iface = -1; }
-    if (transmit < a.transcut || ngrid > maxcross) {
-      validrad = true;
-    } else if (nxt < 0 && iface >= 4) {
-      validrad = true;
-      const int *gk = a.gridptr + 8 * (size_t)kc;
-      float xs[4], ys[4], rb[4];
-      for (int k = 0; k < 4; ++k) {
-        int q = gk[c_face[kface][k]];
-        xs[k] = a.gridpos[3 * q]; ys[k] = a.gridpos[3 * q + 1];
-        if ((float)mu2 < 0.f) rb[k] = a.skyrad;
-        else {
-          int bi = a.bot_index[q];
-          rb[k] = bi >= 0 ? a.bcrad_bot[bi] : 0.f;
-          if constexpr (BRDF) {
-            if (bi >= 0) {
-              float o[3];
-              brdf_radiance_warp(a, bi, (float)mu2, (float)phi2, lane, 1, o);
-              rb[k] = o[0];
-            }
-          }
-        }
-      }
-      float uu = (xs[1] - xs[0] > 0) ? ((P1[0] - xs[0]) + lxn) / (xs[1] - xs[0]) : 0.f;
-      float vv = (ys[2] - ys[0] > 0) ? ((P1[1] - ys[0]) + lyn) / (ys[2] - ys[0]) : 0.f;
-      if (!a.nosurface)
-        radacc += transmit * ((1 - uu) * (1 - vv) * rb[0] + uu * (1 - vv) * rb[1] + (1 - uu) * vv * rb[2] + uu * vv * rb[3]);
-    } else {
-      // into the next cell: offsets from its corner, the crossed face's
-      // coordinate taken from the grid
-      const float *Pn = a.gridpos + 3 * a.gridptr[8 * (size_t)nxt];
-      const float *q = a.gridpos + 3 * a.gridptr[8 * (size_t)nxt + ioct0];
-      lx = jface == 0 ? q[0] - Pn[0] : (P1[0] - Pn[0]) + lxn;
-      ly = jface == 1 ? q[1] - Pn[1] : (P1[1] - Pn[1]) + lyn;
-      lz = jface == 2 ? q[2] - Pn[2] : (P1[2] - Pn[2]) + lzn;
-      cell = nxt;
-    }
-  }
-  if (lane == 0) a.out[ray] = (float)radacc;
-}
-
 // Wigner d^n_{m m1}(x) at n = max(m, m1), m, m1 >= 0 (double precision).
 __device__ __forceinline__ double wig_start_d(double x, int m, int m1) {
   if (m == m1) return pow(0.5 * (1.0 + x), (double)m);
@@ -3175,12 +2933,12 @@ __device__ __forceinline__ double wig_start_d(double x, int m, int m1) {
 
 // The five generalized spherical functions a polarized ray needs (YLMALL,
 // src/polarized/shdomsub2.f:4244-4354, elements 1 I-I, 2 Q-Q, 3 U-U, 5 I-Q,
-// 6 Q-U) at one direction: y[e * nlm + j], e = 0..4.  Lane m runs the upward
-// recurrences in l of d^l_{m0}(x), d^l_{m2}(x) and d^l_{m2}(-x) in double
-// precision.
-__device__ void ylm6_dir_warp(float *y, int nlm, double x, double phi, int ml, int mm, int lane) {
+// 6 Q-U) at one direction: y[e * nlm + j], e = 0..4 (nlm: the row stride).
+// This lane runs the upward recurrences in l of d^l_{m0}(x), d^l_{m2}(x) and
+// d^l_{m2}(-x) for m = first, first + step, ... in double precision.
+__device__ void ylm6_dir_lanes(float *y, int nlm, double x, double phi, int ml, int mm, int first, int step) {
   const double fct = 0.3989422804014327;  // 1/sqrt(2 pi)
-  for (int m = lane; m <= mm; m += 32) {
+  for (int m = first; m <= mm; m += step) {
     double c = 1.0, sn = 0.0;
     if (m > 0) sincos(m * phi, &sn, &c);
     // d^l_{m0}
@@ -3229,258 +2987,461 @@ __device__ void ylm6_dir_warp(float *y, int nlm, double x, double phi, int ml, i
   }
 }
 
-// Polarized ray integration (INTEGRATE_1RAY with the polarized
-// COMPUTE_SOURCE_1CELL, src/polarized/shdomsub2.f:2311-2863, :2868-3042,
-// and ROTATE_POL_PLANE :3277-3316): as k_render, with the I, Q, U sources
-// of each corner and a Stokes vector along the ray.  Dynamic shared memory:
-// the five generalized functions (5 nlm floats) per warp.  out[ray][3].
-template <bool BRDF>
-__global__ void __launch_bounds__(RWARPS * 32) k_render_pol(RenderArgs a) {
-  extern __shared__ float rsm[];
-  __shared__ float tl[RWARPS][3][64];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int ray = blockIdx.x * RWARPS + w;
-  if (ray >= a.nrays) return;
+constexpr int RGRAYS = 4;     // rays per warp, eight lanes each
+constexpr int RLEG = 64;      // Legendre terms of the per-ray single-scatter series at most
+
+// Geometry of the base grid for a ray walk, without its pointer tables: a
+// cell is (x, y, z) cell coordinates; along an axis its corners are
+// consecutive grid lines (periodic), consecutive or the same edge line
+// (open: the edge cells have no width), or the same line (independent
+// pixel).
+struct WalkAxis {
+  int n, nc, kind;  // grid lines, cells, 0 periodic, 1 open, 2 independent pixel
+  __device__ __forceinline__ int lo(int j) const { return kind == 1 ? max(0, j - 1) : j; }
+  __device__ __forceinline__ int hi(int j) const { return kind == 1 ? min(n - 1, j) : kind == 0 ? j + 1 : j; }
+  __device__ __forceinline__ bool edge(int j) const { return kind == 2 || (kind == 1 && (j == 0 || j == nc - 1)); }
+  __device__ __forceinline__ int down(int j) const { return kind == 2 ? j : j > 0 ? j - 1 : kind == 1 ? 0 : nc - 1; }
+  __device__ __forceinline__ int up(int j) const { return kind == 2 ? j : j < nc - 1 ? j + 1 : kind == 1 ? j : 0; }
+};
+
+// The source (I, or I, Q, U) times extinction of grid point ip in a ray's
+// direction: the series over its terms, with delta-M the truncated single
+// scatter replaced by the exact one (TMS).  Y: the direction's functions (one
+// row, or the five generalized ones), tl: their series with the sun's, pv:
+// the single-scatter values of the phase functions at the ray's scattering
+// angle (two rows for NST = 3), null when they are too many to keep.  What
+// depends on the point alone is loaded before any of it is used, and the
+// series in batches, since the latency of these loads is the kernel's.
+template <int NST>
+__device__ __forceinline__ void corner_source(const RenderArgs &a, int ip, float ext, const float *Y, int ldy, const float *tl,
+                                              const float *pv, int sj, float sf, float cos22, float sin22, float *out) {
+  constexpr int NB = NST == 3 ? 4 : 8;  // 16-byte loads per row in a batch
   const int nlm = a.nlm;
-  float *Y = rsm + (size_t)w * 5 * nlm;
-  const double pi = 3.141592653589793;
-  double x0 = a.camx[ray], y0 = a.camy[ray], z0 = a.camz[ray], mu2 = a.cammu[ray], phi2 = a.camphi[ray];
-  const double muray = -mu2, phiray = phi2 - pi;
-  const float ztop = a.zgrid[a.nz - 1];
-  if (z0 > ztop) {
-    if (muray >= 0.0) { if (lane < 3) a.out[(size_t)ray * 3 + lane] = 0.f; return; }
-    double r = (ztop - z0) / muray;
-    x0 += r * sqrt(1 - muray * muray) * cos(phiray);
-    y0 += r * sqrt(1 - muray * muray) * sin(phiray);
-    z0 = ztop;
-  } else if (z0 < a.zgrid[0]) {
-    if (lane == 0) atomicCAS(a.err, ERR_NONE, ERR_RAY_BELOW);
-    if (lane < 3) a.out[(size_t)ray * 3 + lane] = 0.f;
-    return;
-  }
-  ylm6_dir_warp(Y, nlm, (double)(float)mu2, (double)(float)phi2, a.ml, a.mm, lane);
-  __syncwarp();
-  // TMS subtraction series: t_k(l) = sum_m Y_k(l, m) Ysun(l, m) for k = I-I, Q-Q, Q-U
-  for (int l = lane; l <= a.ml; l += 32) {
-    const int me = min(l, a.mm), j0 = (l <= a.mm) ? l * l : (2 * a.mm + 1) * l - a.mm * a.mm - a.mm;
-    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-    for (int k = 0; k < 2 * me + 1; ++k) {
-      const float ys = a.ylmsun[j0 + k];
-      s0 += Y[j0 + k] * ys; s1 += Y[nlm + j0 + k] * ys; s2 += Y[4 * nlm + j0 + k] * ys;
+  const int ns = a.single_scatter ? 0 : a.ns[ip];
+  const float da = a.dirflux[ip] * a.secmu0;
+  int t0 = 0, t1 = 0;
+  if (a.deltam) { t0 = a.tms_ptr[ip]; t1 = a.tms_ptr[ip + 1]; }
+  const float *S = a.source + (size_t)ip * NST * nlm;
+  const float *c1 = a.coef + (size_t)ip * a.nl, *cb1 = NST == 3 ? a.coefp + ((size_t)ip * 3 + 2) * a.nl : nullptr;
+  const bool vec = (nlm & 3) == 0 && (a.nl & 3) == 0;
+  float s[3] = {0.f, 0.f, 0.f}, t[3] = {0.f, 0.f, 0.f};
+  if (vec) {
+    float p[NST][4];
+#pragma unroll
+    for (int k = 0; k < NST; ++k) p[k][0] = p[k][1] = p[k][2] = p[k][3] = 0.f;
+    const float4 ca = *reinterpret_cast<const float4 *>(c1);
+    float4 cp = make_float4(0.f, 0.f, 0.f, 0.f);
+    if constexpr (NST == 3) cp = *reinterpret_cast<const float4 *>(cb1);
+    for (int j0 = 0; j0 < nlm; j0 += 4 * NB) {  // terms past ns are stored as zero
+      float4 v[NST][NB];
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+        if (j0 + 4 * i < nlm)
+#pragma unroll
+          for (int k = 0; k < NST; ++k) v[k][i] = *reinterpret_cast<const float4 *>(S + k * nlm + j0 + 4 * i);
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+        if (j0 + 4 * i < nlm) {
+          const float4 x = v[0][i], y = *reinterpret_cast<const float4 *>(Y + j0 + 4 * i);
+          p[0][0] = fmaf(x.x, y.x, p[0][0]); p[0][1] = fmaf(x.y, y.y, p[0][1]);
+          p[0][2] = fmaf(x.z, y.z, p[0][2]); p[0][3] = fmaf(x.w, y.w, p[0][3]);
+          if constexpr (NST == 3) {
+            const float4 q = v[1][i], u = v[2][i];
+            const float *yj = Y + j0 + 4 * i;
+            const float4 y1 = *reinterpret_cast<const float4 *>(yj + ldy), y2 = *reinterpret_cast<const float4 *>(yj + 2 * ldy);
+            const float4 y3 = *reinterpret_cast<const float4 *>(yj + 3 * ldy), y4 = *reinterpret_cast<const float4 *>(yj + 4 * ldy);
+            p[1][0] = fmaf(q.x, y1.x, fmaf(u.x, y3.x, p[1][0])); p[1][1] = fmaf(q.y, y1.y, fmaf(u.y, y3.y, p[1][1]));
+            p[1][2] = fmaf(q.z, y1.z, fmaf(u.z, y3.z, p[1][2])); p[1][3] = fmaf(q.w, y1.w, fmaf(u.w, y3.w, p[1][3]));
+            p[2][0] = fmaf(q.x, y4.x, fmaf(u.x, y2.x, p[2][0])); p[2][1] = fmaf(q.y, y4.y, fmaf(u.y, y2.y, p[2][1]));
+            p[2][2] = fmaf(q.z, y4.z, fmaf(u.z, y2.z, p[2][2])); p[2][3] = fmaf(q.w, y4.w, fmaf(u.w, y2.w, p[2][3]));
+          }
+        }
+      if (j0 + 4 * NB >= ns) break;
     }
-    tl[w][0][l] = s0; tl[w][1][l] = s1; tl[w][2][l] = s2;
+#pragma unroll
+    for (int k = 0; k < NST; ++k) s[k] = ns > 0 ? (p[k][0] + p[k][1]) + (p[k][2] + p[k][3]) : 0.f;
+    if (a.deltam && ns > 0) {
+      const int ls = a.lofj[ns - 1];
+      for (int l = 0; l <= ls; l += 4) {
+        const float4 c4 = l == 0 ? ca : *reinterpret_cast<const float4 *>(c1 + l);
+        const float4 x = *reinterpret_cast<const float4 *>(tl + l);
+        t[0] = fmaf(c4.x, x.x, t[0]);
+        if (l + 1 <= ls) t[0] = fmaf(c4.y, x.y, t[0]);
+        if (l + 2 <= ls) t[0] = fmaf(c4.z, x.z, t[0]);
+        if (l + 3 <= ls) t[0] = fmaf(c4.w, x.w, t[0]);
+        if constexpr (NST == 3) {
+          const float4 b4 = l == 0 ? cp : *reinterpret_cast<const float4 *>(cb1 + l);
+          const float4 x1 = *reinterpret_cast<const float4 *>(tl + RLEG + l), x2 = *reinterpret_cast<const float4 *>(tl + 2 * RLEG + l);
+          t[1] = fmaf(b4.x, x1.x, t[1]); t[2] = fmaf(b4.x, x2.x, t[2]);
+          if (l + 1 <= ls) { t[1] = fmaf(b4.y, x1.y, t[1]); t[2] = fmaf(b4.y, x2.y, t[2]); }
+          if (l + 2 <= ls) { t[1] = fmaf(b4.z, x1.z, t[1]); t[2] = fmaf(b4.z, x2.z, t[2]); }
+          if (l + 3 <= ls) { t[1] = fmaf(b4.w, x1.w, t[1]); t[2] = fmaf(b4.w, x2.w, t[2]); }
+        }
+      }
+    }
+  } else {
+    for (int j = 0; j < ns; ++j) {
+      s[0] = fmaf(S[j], Y[j], s[0]);
+      if constexpr (NST == 3) {
+        const float q = S[nlm + j], u = S[2 * nlm + j];
+        s[1] = fmaf(q, Y[ldy + j], fmaf(u, Y[3 * ldy + j], s[1]));
+        s[2] = fmaf(q, Y[4 * ldy + j], fmaf(u, Y[2 * ldy + j], s[2]));
+      }
+    }
+    if (a.deltam && ns > 0) {
+      const int ls = a.lofj[ns - 1];
+      for (int l = 0; l <= ls; ++l) {
+        t[0] = fmaf(c1[l], tl[l], t[0]);
+        if constexpr (NST == 3) { t[1] = fmaf(cb1[l], tl[RLEG + l], t[1]); t[2] = fmaf(cb1[l], tl[2 * RLEG + l], t[2]); }
+      }
+    }
   }
-  __syncwarp();
-  int sj = 0;
-  float sf = 0.f, cos22 = 1.f, sin22 = 0.f;
+  if (a.deltam) {
+    float add0 = 0.f, add1 = 0.f;
+#pragma unroll 4
+    for (int q = t0; q < t1; ++q) {
+      const float w = a.tms_w[q];
+      const int iph = a.tms_iph[q];
+      float f0, f1 = 0.f;
+      if (pv) {
+        f0 = pv[iph];
+        if constexpr (NST == 3) f1 = pv[a.numphase + iph];
+      } else {
+        const size_t o0 = (size_t)sj * a.numphase + iph, o1 = o0 + a.numphase;
+        f0 = (1.f - sf) * a.phasetab[o0] + sf * a.phasetab[o1];
+        if constexpr (NST == 3) f1 = (1.f - sf) * a.phasetab2[o0] + sf * a.phasetab2[o1];
+      }
+      add0 += w * f0;
+      if constexpr (NST == 3) add1 += w * f1;
+    }
+    s[0] += da * (add0 - t[0]);
+    if constexpr (NST == 3) { s[1] += da * (add1 * cos22 - t[1]); s[2] += da * (add1 * sin22 - t[2]); }
+  }
+#pragma unroll
+  for (int k = 0; k < NST; ++k) out[k] = s[k] * ext;
+}
+
+// What a ray's eight lanes need of its description, formed by one lane.
+struct RaySetup {
+  float lx, ly, lz, c[3], ci[3], mu, phi, sf, cos22, sin22;
+  int cell, sj;  // cell < 0: the ray crosses nothing
+};
+constexpr int RPHASE = 32;  // phase functions whose single-scatter values a ray keeps at most
+
+template <int NST>
+__device__ RaySetup ray_setup(const RenderArgs &a, int ray) {
+  const double pi = 3.141592653589793;
+  RaySetup r;
+  r.cell = -1; r.sj = 0; r.sf = 0.f; r.cos22 = 1.f; r.sin22 = 0.f;
+  r.lx = r.ly = r.lz = 0.f;
+  double x0 = a.camx[ray], y0 = a.camy[ray], z0 = a.camz[ray];
+  const double mu2 = a.cammu[ray], phi2 = a.camphi[ray], st = sqrt(1.0 - mu2 * mu2);
+  double sn, cn;
+  sincos(phi2 - pi, &sn, &cn);
+  r.mu = (float)mu2; r.phi = (float)phi2;
+  // direction cosines, their inverses (1e6 where a cosine is below 1e-6 and
+  // set to zero, as the reference's INTEGRATE_1RAY)
+  const double c[3] = {st * cn, st * sn, -mu2};
+  for (int k = 0; k < 3; ++k) {
+    const bool on = fabs(c[k]) > 1e-6;
+    r.c[k] = on ? (float)c[k] : 0.f;
+    r.ci[k] = on ? (float)(1.0 / c[k]) : 1e6f;
+  }
+  // single-scatter phase table interpolation, and the rotation of its
+  // polarization to the outgoing meridional plane
   if (a.deltam) {
     double cosscat = (double)a.solarmu * mu2 + sqrt((1.0 - (double)a.solarmu * a.solarmu) * (1.0 - mu2 * mu2)) * cos((double)a.solaraz - phi2);
     cosscat = fmax(fmin(1.0, cosscat), -1.0);
-    float F = (float)((a.nscatangle - 1) * (acos(cosscat) / pi) + 1);
-    int J = min(a.nscatangle - 1, (int)F);
-    sf = F - J; sj = J - 1;
-    // rotation of the single-scatter polarization to the outgoing meridional plane
-    const float smu = a.solarmu, mu2f = (float)mu2, dphi = a.solaraz - (float)phi2;
-    const double sin_scat = sqrt(fmax(0.0, 1.0 - cosscat * cosscat));
-    const double st1 = sqrt(1.0 - (double)(smu * smu)), st2 = sqrt(1.0 - (double)(mu2f * mu2f));
-    double sp, cp;
-    sincos((double)dphi, &sp, &cp);
-    double sin2, cos2;
-    if (sin_scat == 0.0) { sin2 = 0.0; cos2 = -1.0; }
-    else { sin2 = st1 * sp / sin_scat; cos2 = (st2 * smu - st1 * mu2f * cp) / sin_scat; }
-    cos22 = (float)(1.0 - 2.0 * sin2 * sin2);
-    sin22 = (float)(2.0 * sin2 * cos2);
+    const float F = (float)((a.nscatangle - 1) * (acos(cosscat) / pi) + 1);
+    const int J = min(a.nscatangle - 1, (int)F);
+    r.sf = F - J; r.sj = J - 1;
+    if constexpr (NST == 3) {
+      const float smu = a.solarmu, mu2f = (float)mu2, dphi = a.solaraz - (float)phi2;
+      const double sin_scat = sqrt(fmax(0.0, 1.0 - cosscat * cosscat));
+      const double st1 = sqrt(1.0 - (double)(smu * smu)), st2 = sqrt(1.0 - (double)(mu2f * mu2f));
+      double sp, cp;
+      sincos((double)dphi, &sp, &cp);
+      double sin2, cos2;
+      if (sin_scat == 0.0) { sin2 = 0.0; cos2 = -1.0; }
+      else { sin2 = st1 * sp / sin_scat; cos2 = (st2 * smu - st1 * mu2f * cp) / sin_scat; }
+      r.cos22 = (float)(1.0 - 2.0 * sin2 * sin2);
+      r.sin22 = (float)(2.0 * sin2 * cos2);
+    }
   }
-  RayDir rd = ray_dir(mu2, phi2);
-  const int ioct0 = rd.ioct;
-  const float xm = 0.5f * (a.xgrid[0] + a.xgrid[a.nx - 1]), ym = 0.5f * (a.ygrid[0] + a.ygrid[a.ny - 1]);
-  double xe = x0, ye = y0, ze = z0;
-  int cell = locate_cell(a, xe, ye, ze);
-  // the position as the cell's low corner (grid coordinates) plus an FP32 offset (as k_render)
-  float lx, ly, lz;
-  if (cell >= 0) {
-    const float *P = a.gridpos + 3 * a.gridptr[8 * (size_t)cell];
-    lx = (float)(xe - P[0]); ly = (float)(ye - P[1]); lz = (float)(ze - P[2]);
+  const float ztop = a.zgrid[a.nz - 1];
+  if (z0 > ztop) {
+    if (-mu2 >= 0.0) return r;
+    const double d = (ztop - z0) / -mu2;
+    x0 += d * st * cn;
+    y0 += d * st * sn;
+    z0 = ztop;
+  } else if (z0 < a.zgrid[0]) {
+    atomicCAS(a.err, ERR_NONE, ERR_RAY_BELOW);
+    return r;
   }
-  const float eps = 1.0e-5f * (a.gridpos[3 * a.gridptr[7] + 2] - a.gridpos[3 * a.gridptr[0] + 2]);
-  const int maxcross = 500 * max(a.nx, max(a.ny, a.nz));
-  int oldp[8] = {-1, -1, -1, -1, -1, -1, -1, -1};
-  float osrc[3][8] = {{0}};
-  float ext8[8], src8[3][8];
-  double radacc[3] = {0.0, 0.0, 0.0}, transmit = 1.0;
+  r.cell = locate_cell(a, x0, y0, z0);
+  // the position as the cell's low corner (grid coordinates) plus an FP32 offset
+  if (r.cell >= 0) {
+    const float *P = a.gridpos + 3 * a.gridptr[8 * (size_t)r.cell];
+    r.lx = (float)(x0 - P[0]); r.ly = (float)(y0 - P[1]); r.lz = (float)(z0 - P[2]);
+  }
+  return r;
+}
+
+// Ray integration (RENDER / INTEGRATE_1RAY / COMPUTE_SOURCE_1CELL /
+// FIND_BOUNDARY_RADIANCE, src/polarized/shdomsub4.f:93-286,
+// src/polarized/shdomsub2.f:2311-3192, ROTATE_POL_PLANE :3277-3316), for I
+// (NST = 1, out[ray]) or I, Q, U (NST = 3, out[ray][3]).
+//
+// Eight lanes per ray, four rays per warp.  A lane holds the cell corner
+// whose grid indices have its parities (in a cell without width along an
+// axis, the corner on its side), so a corner shared with the next cell stays
+// in its lane, and evaluates that corner's series by itself; cells without
+// extinction add nothing and their corners are not evaluated.  The cell's
+// geometry is arithmetic on cell coordinates, and the next cell's extinction
+// is on its way while this one is integrated.  The sub-steps of a cell go to
+// the eight lanes, whose (source, transmission) pairs are composed in order.
+// Geometry in FP32 on offsets from the cell's low corner; the two ray
+// accumulators are FP64, folded once per cell.  Where all rays of a block
+// have one direction (a parallel view) its functions are formed once.
+//
+// What bounds it: %RENDER%
+template <int NST, bool BRDF>
+__global__ void __launch_bounds__(128) k_render(RenderArgs a) {
+  extern __shared__ __align__(16) float rsm[];
+  __shared__ RaySetup setup[16];
+  constexpr int NY = NST == 3 ? 5 : 1;
+  const int lane = threadIdx.x & 31, k8 = lane & 7, lr = threadIdx.x >> 3, nrb = blockDim.x >> 3;
+  const int b0 = blockIdx.x * nrb, ray = b0 + lr;
+  // shared memory: per ray NY rows of functions (padded so that a warp's rays
+  // read different banks), the single-scatter series and phase values, then the grid lines
+  const int ldy = (a.nlm + 3) & ~3, ystr = NY * ldy + 4;
+  const bool keep = a.numphase <= RPHASE;
+  float *tls = rsm + nrb * ystr, *pvs = tls + nrb * NST * RLEG, *xg = pvs + nrb * NST * RPHASE, *yg = xg + a.nx + 1, *zg = yg + a.ny + 1;
+  // one lane per ray forms its setup (the FP64 trigonometry), the other warps fetch the grid lines
+  bool same = true;
+  if ((int)threadIdx.x < nrb) {
+    const int i = min(b0 + (int)threadIdx.x, a.nrays - 1);
+    setup[threadIdx.x] = ray_setup<NST>(a, i);
+    same = a.cammu[i] == a.cammu[b0] && a.camphi[i] == a.camphi[b0];
+  }
+  for (int i = threadIdx.x; i <= a.nx; i += blockDim.x) xg[i] = a.xgrid[i];
+  for (int i = threadIdx.x; i <= a.ny; i += blockDim.x) yg[i] = a.ygrid[i];
+  for (int i = threadIdx.x; i < a.nz; i += blockDim.x) zg[i] = a.zgrid[i];
+  const bool one = __syncthreads_and(same);  // one direction for the whole block
+  const RaySetup ry = setup[lr];
+  bool act = ray < a.nrays && ry.cell >= 0;
+  // the direction's functions: lane m runs the l recurrence of its m
+  const int set = one ? 0 : lr;
+  float *Y = rsm + set * ystr, *tl = tls + set * NST * RLEG, *pv = pvs + set * NST * RPHASE;
+  const int first = one ? (int)threadIdx.x : k8, step = one ? (int)blockDim.x : 8;
+  if constexpr (NST == 3) ylm6_dir_lanes(Y, ldy, (double)ry.mu, (double)ry.phi, a.ml, a.mm, first, step);
+  else ylm_dir_lanes(Y, ry.mu, ry.phi, a.ml, a.mm, first, step);
+  const int sj = ry.sj;
+  const float sf = ry.sf, cos22 = ry.cos22, sin22 = ry.sin22;
+  if (keep && a.deltam)
+    for (int i = first; i < a.numphase; i += step) {
+      const size_t o0 = (size_t)sj * a.numphase + i, o1 = o0 + a.numphase;
+      pv[i] = (1.f - sf) * a.phasetab[o0] + sf * a.phasetab[o1];
+      if constexpr (NST == 3) pv[a.numphase + i] = (1.f - sf) * a.phasetab2[o0] + sf * a.phasetab2[o1];
+    }
+  const float *pvk = keep ? pv : nullptr;
+  __syncthreads();
+  // TMS subtraction series: t(l) = sum_m Y(l, m) Ysun(l, m) (for I-I, Q-Q and Q-U)
+  for (int l = first; l <= a.ml; l += step) {
+    const int me = min(l, a.mm), j0 = (l <= a.mm) ? l * l : (2 * a.mm + 1) * l - a.mm * a.mm - a.mm;
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f;
+    for (int k = j0; k < j0 + 2 * me + 1; ++k) {
+      const float ys = a.ylmsun[k];
+      s0 += Y[k] * ys;
+      if constexpr (NST == 3) { s1 += Y[ldy + k] * ys; s2 += Y[4 * ldy + k] * ys; }
+    }
+    tl[l] = s0;
+    if constexpr (NST == 3) { tl[RLEG + l] = s1; tl[2 * RLEG + l] = s2; }
+  }
+  __syncthreads();
+  const float cx = ry.c[0], cy = ry.c[1], cz = ry.c[2];
+  const bool bx = cx < 0.f, by = cy < 0.f, bz = cz < 0.f;
+  const float xm = 0.5f * (xg[0] + xg[a.nx - 1]), ym = 0.5f * (yg[0] + yg[a.ny - 1]);
+  const WalkAxis AX{(a.bcflag & 1) || (a.ipflag & 1) ? a.nx : a.nx + 1, (a.bcflag & 1) ? a.nx + 1 : a.nx,
+                    (a.ipflag & 1) ? 2 : (a.bcflag & 1) ? 1 : 0};
+  const WalkAxis AY{(a.bcflag & 2) || (a.ipflag & 2) ? a.ny : a.ny + 1, (a.bcflag & 2) ? a.ny + 1 : a.ny,
+                    (a.ipflag & 2) ? 2 : (a.bcflag & 2) ? 1 : 0};
+  const int ny1 = a.ny1, nz = a.nz;
+  const int cell0 = act ? ry.cell : 0;
+  int jz = cell0 % (nz - 1), jy = cell0 / (nz - 1) % AY.nc, jx = cell0 / (nz - 1) / AY.nc;
+  float lx = ry.lx, ly = ry.ly, lz = ry.lz;
+  const float eps = 1.0e-5f * (zg[1] - zg[0]);
+  const int maxcross = 500 * max(a.nx, max(a.ny, nz));
   const float inv_tautol = 1.0f / a.tautol;
-  const int nl = a.nl;
-  int ngrid = 0;
-  bool validrad = false;
-  const int grp = lane >> 2, gl = lane & 3;
-  while (!validrad && cell >= 0) {
+  double radacc[NST], transmit = 1.0;
+#pragma unroll
+  for (int k = 0; k < NST; ++k) radacc[k] = 0.0;
+  int ngrid = 0, mine = -1;  // mine: the point this lane's source cv is of
+  float cv[NST];
+#pragma unroll
+  for (int k = 0; k < NST; ++k) cv[k] = 0.f;
+  // this lane's corner of a cell: its point, and which lane has corner 0
+  auto corner = [&](int px, int py, int pz, int &flip) {
+    const int xa = AX.lo(px), xb = AX.hi(px), ya = AY.lo(py), yb = AY.hi(py);
+    flip = (xa != xb ? xa & 1 : 0) | (ya != yb ? (ya & 1) << 1 : 0) | ((pz & 1) << 2);
+    const int c = k8 ^ flip;
+    return ((c & 1 ? xb : xa) * ny1 + (c & 2 ? yb : ya)) * nz + pz + (c >> 2);
+  };
+  int flip, ip = corner(jx, jy, jz, flip);
+  float ext = act ? a.text[ip] : 0.f;
+  const unsigned gmask = 0xffu << (lane & 24);
+  while (__any_sync(0xffffffffu, act)) {
     ++ngrid;
-    const int *g = a.gridptr + 8 * (size_t)cell;
-    const int mypt = g[grp];
-    int reuse = -1;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) if (oldp[k] == mypt) reuse = k;
-    const float cext = a.text[mypt];
-    const bool need = reuse < 0;
-    const int ns = (need && !a.single_scatter) ? a.ns[mypt] : 0;
-    float sI = 0.f, sQ = 0.f, sU = 0.f;
-    {
-      const float *S = a.source + (size_t)mypt * 3 * nlm;
-      for (int j = gl; j < ns; j += 4) {
-        const float si = S[j], sq = S[nlm + j], su = S[2 * nlm + j];
-        sI += si * Y[j];
-        sQ += sq * Y[nlm + j] + su * Y[3 * nlm + j];
-        sU += sq * Y[4 * nlm + j] + su * Y[2 * nlm + j];
-      }
-    }
-#pragma unroll
-    for (int o = 1; o <= 2; o <<= 1) {
-      sI += __shfl_xor_sync(0xffffffffu, sI, o);
-      sQ += __shfl_xor_sync(0xffffffffu, sQ, o);
-      sU += __shfl_xor_sync(0xffffffffu, sU, o);
-    }
-    float cv[3];
-    if (!need) {
-      cv[0] = osrc[0][reuse]; cv[1] = osrc[1][reuse]; cv[2] = osrc[2][reuse];
-    } else {
-      if (a.deltam) {
-        const float da = a.dirflux[mypt] * a.secmu0;
-        const float *c1 = a.coef + (size_t)mypt * nl, *cb1 = a.coefp + ((size_t)mypt * 3 + 2) * nl;
-        if (ns > 0) {
-          const int ls = a.lofj[ns - 1];
-          float s0 = 0.f, s1 = 0.f, s2 = 0.f;
-          for (int l = 0; l <= ls; ++l) { s0 += c1[l] * tl[w][0][l]; s1 += cb1[l] * tl[w][1][l]; s2 += cb1[l] * tl[w][2][l]; }
-          sI -= da * s0; sQ -= da * s1; sU -= da * s2;
-        }
-        float add0 = 0.f, add1 = 0.f;
-        for (int q = a.tms_ptr[mypt]; q < a.tms_ptr[mypt + 1]; ++q) {
-          const int iph = a.tms_iph[q];
-          const size_t o0 = (size_t)sj * a.numphase + iph, o1 = (size_t)(sj + 1) * a.numphase + iph;
-          add0 += a.tms_w[q] * ((1.f - sf) * a.phasetab[o0] + sf * a.phasetab[o1]);
-          add1 += a.tms_w[q] * ((1.f - sf) * a.phasetab2[o0] + sf * a.phasetab2[o1]);
-        }
-        sI += da * add0; sQ += da * add1 * cos22; sU += da * add1 * sin22;
-      }
-      cv[0] = sI * cext; cv[1] = sQ * cext; cv[2] = sU * cext;
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      ext8[k] = __shfl_sync(0xffffffffu, cext, 4 * k);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) src8[c][k] = __shfl_sync(0xffffffffu, cv[c], 4 * k);
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { oldp[k] = g[k]; osrc[0][k] = src8[0][k]; osrc[1][k] = src8[1][k]; osrc[2][k] = src8[2][k]; }
-    const int ip1 = g[0], ip2 = g[7];
-    const float *P1 = a.gridpos + 3 * ip1, *P2 = a.gridpos + 3 * ip2;
-    const float delx = P2[0] - P1[0], dely = P2[1] - P1[1], delz = P2[2] - P1[2];
-    const float idx = delx <= 0.f ? 1.f : 1.f / delx, idy = dely <= 0.f ? 1.f : 1.f / dely, idz = 1.f / delz;
-    auto tri = [&](const float *v, float u, float vv, float ww) {
-      const float a0 = fmaf(u, v[1] - v[0], v[0]), a1 = fmaf(u, v[3] - v[2], v[2]);
-      const float a2 = fmaf(u, v[5] - v[4], v[4]), a3 = fmaf(u, v[7] - v[6], v[6]);
-      const float b0 = fmaf(vv, a1 - a0, a0), b1 = fmaf(vv, a3 - a2, a2);
-      return fmaf(ww, b1 - b0, b0);
-    };
-    const float u0 = lx * idx, v0 = ly * idy, w0 = lz * idz;
-    float srcext1[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) srcext1[c] = tri(src8[c], u0, v0, w0);
-    srcext1[0] = fmaxf(0.f, srcext1[0]);
-    float ext1 = tri(ext8, u0, v0, w0);
-    const int cf = a.cellflags[cell];
-    const float cx = rd.c[0], cy = rd.c[1], cz = rd.c[2];
-    bool ipinx = (cf & 1) && !((a.bcflag & 1) && ((cx > 0 && P1[0] + lx < xm) || (cx < 0 && P1[0] + lx > xm)));
-    bool ipiny = (cf & 2) && !((a.bcflag & 2) && ((cy > 0 && P1[1] + ly < ym) || (cy < 0 && P1[1] + ly > ym)));
-    const float *Po = a.gridpos + 3 * g[7 - ioct0];
-    const float sox = ipinx ? 1e20f : ((Po[0] - P1[0]) - lx) * rd.ci[0];
-    const float soy = ipiny ? 1e20f : ((Po[1] - P1[1]) - ly) * rd.ci[1];
-    const float soz = ((Po[2] - P1[2]) - lz) * rd.ci[2];
+    const float p1x = xg[AX.lo(jx)], p1y = yg[AY.lo(jy)], p1z = zg[jz];
+    const float delx = xg[AX.hi(jx)] - p1x, dely = yg[AY.hi(jy)] - p1y, delz = zg[jz + 1] - p1z;
+    const bool ex = AX.edge(jx), ey = AY.edge(jy);
+    const bool ipinx = ex && !((a.bcflag & 1) && ((cx > 0 && p1x + lx < xm) || (cx < 0 && p1x + lx > xm)));
+    const bool ipiny = ey && !((a.bcflag & 2) && ((cy > 0 && p1y + ly < ym) || (cy < 0 && p1y + ly > ym)));
+    const float sox = ipinx ? 1e20f : ((bx ? 0.f : delx) - lx) * ry.ci[0];
+    const float soy = ipiny ? 1e20f : ((by ? 0.f : dely) - ly) * ry.ci[1];
+    const float soz = ((bz ? 0.f : delz) - lz) * ry.ci[2];
     const float so = fminf(sox, fminf(soy, soz));
-    if (so < -eps) { if (lane == 0) atomicCAS(a.err, ERR_NONE, ERR_RAY_SO); break; }
+    if (act && so < -eps) { if (k8 == 0) atomicCAS(a.err, ERR_NONE, ERR_RAY_SO); act = false; }
     const float lxn = fmaf(so, cx, lx), lyn = fmaf(so, cy, ly), lzn = fmaf(so, cz, lz);
-    const float du = cx * idx, dv = cy * idy, dw = cz * idz;
-    const float sof = so;
-    float extn = tri(ext8, fmaf(sof, du, u0), fmaf(sof, dv, v0), fmaf(sof, dw, w0));
-    const float taugrid = so * 0.5f * (ext1 + extn);
-    int ntau = max(1, 1 + (int)(taugrid * inv_tautol));
-    const float delsf = sof / (float)ntau;
-    float cacc[3] = {0.f, 0.f, 0.f}, ctr = 1.f;  // as in k_render: per cell in FP32, folded once per cell
-    for (int it = 1; it <= ntau; ++it) {
-      const float sf_ = it * delsf;
-      const float uu_ = fmaf(sf_, du, u0), vv_ = fmaf(sf_, dv, v0), ww_ = fmaf(sf_, dw, w0);
-      const float ext0 = tri(ext8, uu_, vv_, ww_);
-      float srcext0[3];
+    // the cell beyond the exit face (an open edge cell entered from inside
+    // keeps the ray; one left at the domain's side stays in place), and the
+    // offsets there, the crossed face's coordinate taken from the grid
+    const int jface = (sox <= soz && sox <= soy) ? 0 : (soy <= soz) ? 1 : 2;
+    const int nx_ = jface == 0 ? (bx ? AX.down(jx) : AX.up(jx)) : jx;
+    const int ny_ = jface == 1 ? (by ? AY.down(jy) : AY.up(jy)) : jy;
+    const int nz_ = jface == 2 ? (bz ? jz - 1 : jz + 1) : jz;
+    const bool out = nz_ < 0 || nz_ >= nz - 1;  // through the top or the bottom
+    const int mz = out ? jz : nz_;
+    const float q1x = xg[AX.lo(nx_)], q1y = yg[AY.lo(ny_)], q1z = zg[mz];
+    const float lx2 = jface == 0 ? (bx ? xg[AX.hi(nx_)] - q1x : 0.f) : (p1x - q1x) + lxn;
+    const float ly2 = jface == 1 ? (by ? yg[AY.hi(ny_)] - q1y : 0.f) : (p1y - q1y) + lyn;
+    const float lz2 = jface == 2 ? (bz ? zg[mz + 1] - q1z : 0.f) : (p1z - q1z) + lzn;
+    int flipn;
+    const int ipn = corner(nx_, ny_, mz, flipn);
+    const float extn_ = a.text[ipn];  // on its way while this cell is integrated
+    const unsigned cloudy = __ballot_sync(0xffffffffu, ext != 0.f);
+    const bool run = act && (cloudy & gmask);
+    if (__any_sync(0xffffffffu, run)) {
+      if (run && mine != ip) {
+        corner_source<NST>(a, ip, ext, Y, ldy, tl, pvk, sj, sf, cos22, sin22, cv);
+        mine = ip;
+      }
+      __syncwarp();
+      float ext8[8], src8[NST][8];
 #pragma unroll
-      for (int c = 0; c < 3; ++c) srcext0[c] = tri(src8[c], uu_, vv_, ww_);
-      srcext0[0] = fmaxf(0.f, srcext0[0]);
-      const float ext = 0.5f * (ext0 + ext1);
-      float absc, trc;
-      if (ext != 0.f) {
-        const float tau = ext * delsf;
-        absc = tau * (1.f - 0.5f * tau * (1.f - 0.33333333333f * tau));
-        trc = 1.f - absc;
-        const float iext = 1.f / ext, corr = delsf * (1.f - 0.05f * (ext1 - ext0) * delsf);
+      for (int c = 0; c < 8; ++c) {
+        ext8[c] = __shfl_sync(0xffffffffu, ext, c ^ flip, 8);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          const float src = (0.5f * (srcext0[c] + srcext1[c]) + 0.08333333333f * (ext0 * srcext1[c] - ext1 * srcext0[c]) * corr) * iext;
-          cacc[c] = fmaf(ctr * src, absc, cacc[c]);
+        for (int k = 0; k < NST; ++k) src8[k][c] = __shfl_sync(0xffffffffu, cv[k], c ^ flip, 8);
+      }
+      const float idx = delx <= 0.f ? 1.f : 1.f / delx, idy = dely <= 0.f ? 1.f : 1.f / dely, idz = 1.f / delz;
+      auto tri = [&](const float *v, float u, float vv, float ww) {
+        const float a0 = fmaf(u, v[1] - v[0], v[0]), a1 = fmaf(u, v[3] - v[2], v[2]);
+        const float a2 = fmaf(u, v[5] - v[4], v[4]), a3 = fmaf(u, v[7] - v[6], v[6]);
+        const float b0 = fmaf(vv, a1 - a0, a0), b1 = fmaf(vv, a3 - a2, a2);
+        return fmaf(ww, b1 - b0, b0);
+      };
+      // the trilinear weights are cell-relative coordinates in [0, 1], moving by (du, dv, dw) per unit path
+      const float u0 = lx * idx, v0 = ly * idy, w0 = lz * idz, du = cx * idx, dv = cy * idy, dw = cz * idz;
+      float ec = tri(ext8, u0, v0, w0), sc[NST];  // at the start of the lanes' sub-steps
+#pragma unroll
+      for (int k = 0; k < NST; ++k) sc[k] = tri(src8[k], u0, v0, w0);
+      sc[0] = fmaxf(0.f, sc[0]);
+      const float exit = tri(ext8, fmaf(so, du, u0), fmaf(so, dv, v0), fmaf(so, dw, w0));
+      const int ntau = run ? max(1, 1 + (int)(so * 0.5f * (ec + exit) * inv_tautol)) : 0;
+      const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)ntau);
+      const float dels = so / (float)max(ntau, 1);
+      // the cell's source integral and transmission from its entry, in FP32
+      float cacc[NST], ctr = 1.f;
+#pragma unroll
+      for (int k = 0; k < NST; ++k) cacc[k] = 0.f;
+      for (int base = 0; base < nmax; base += 8) {
+        const int it = base + k8 + 1;
+        const float t = it * dels;
+        const float uu = fmaf(t, du, u0), vv = fmaf(t, dv, v0), ww = fmaf(t, dw, w0);
+        const float e0 = tri(ext8, uu, vv, ww);
+        float s0[NST], s1[NST], A[NST], T = 1.f;
+#pragma unroll
+        for (int k = 0; k < NST; ++k) { s0[k] = tri(src8[k], uu, vv, ww); A[k] = 0.f; }
+        s0[0] = fmaxf(0.f, s0[0]);
+        float e1 = __shfl_up_sync(0xffffffffu, e0, 1, 8);
+        if (k8 == 0) e1 = ec;
+#pragma unroll
+        for (int k = 0; k < NST; ++k) {
+          s1[k] = __shfl_up_sync(0xffffffffu, s0[k], 1, 8);
+          if (k8 == 0) s1[k] = sc[k];
         }
-      } else { trc = 1.f; }
-      ctr *= trc;
-      ext1 = ext0;
+        const float em = 0.5f * (e0 + e1);
+        if (it <= ntau && em != 0.f) {
+          const float tau = em * dels, absc = tau * (1.f - 0.5f * tau * (1.f - 0.33333333333f * tau));
+          T = 1.f - absc;
+          const float corr = dels * (1.f - 0.05f * (e1 - e0) * dels);
 #pragma unroll
-      for (int c = 0; c < 3; ++c) srcext1[c] = srcext0[c];
+          for (int k = 0; k < NST; ++k)
+            A[k] = (0.5f * (s0[k] + s1[k]) + 0.08333333333f * (e0 * s1[k] - e1 * s0[k]) * corr) / em * absc;
+        }
+        if (base + 8 < nmax) {
+          ec = __shfl_sync(0xffffffffu, e0, 7, 8);
+#pragma unroll
+          for (int k = 0; k < NST; ++k) sc[k] = __shfl_sync(0xffffffffu, s0[k], 7, 8);
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) {
+          const float Tp = __shfl_xor_sync(0xffffffffu, T, o);
+          const bool later = k8 & o;
+#pragma unroll
+          for (int k = 0; k < NST; ++k) {
+            const float Ap = __shfl_xor_sync(0xffffffffu, A[k], o);
+            A[k] = later ? fmaf(Tp, A[k], Ap) : fmaf(T, Ap, A[k]);
+          }
+          T *= Tp;
+        }
+#pragma unroll
+        for (int k = 0; k < NST; ++k) cacc[k] = fmaf(ctr, A[k], cacc[k]);
+        ctr *= T;
+      }
+      if (run) {
+#pragma unroll
+        for (int k = 0; k < NST; ++k) radacc[k] += transmit * (double)cacc[k];
+        transmit *= (double)ctr;
+      }
     }
+    if (act) {
+      if (transmit < a.transcut || ngrid > maxcross) {
+        act = false;
+      } else if (out) {
+        // the boundary radiance at the exit point; unpolarized sky and
+        // Lambertian surface, a BRDF surface polarizes
+        act = false;
+        if (!a.nosurface) {
+          const int xa = AX.lo(jx), xb = AX.hi(jx), ya = AY.lo(jy), yb = AY.hi(jy), zz = bz ? jz : jz + 1;
+          const float uu = delx > 0 ? lxn / delx : 0.f, vv = dely > 0 ? lyn / dely : 0.f;
 #pragma unroll
-    for (int c = 0; c < 3; ++c) radacc[c] += transmit * (double)cacc[c];
-    transmit *= (double)ctr;
-    int iface, jface;
-    bool openbc;
-    if (sox <= soz && sox <= soy) { iface = 1 - rd.bit[0]; jface = 0; openbc = (cf & 1) && (a.bcflag & 1); }
-    else if (soy <= soz) { iface = 3 - rd.bit[1]; jface = 1; openbc = (cf & 2) && (a.bcflag & 2); }
-    else { iface = 5 - rd.bit[2]; jface = 2; openbc = false; }
-    int nxt = a.neighptr[6 * (size_t)cell + iface];
-    int kface = iface, kc = cell;
-    if (openbc) { kface = iface ^ 1; kc = nxt; iface = -1; }
-    if (transmit < a.transcut || ngrid > maxcross) {
-      validrad = true;
-    } else if (nxt < 0 && iface >= 4) {
-      validrad = true;  // unpolarized sky and Lambertian surface (I only); a BRDF surface polarizes
-      const int *gk = a.gridptr + 8 * (size_t)kc;
-      float xs[4], ys[4], rb[3][4];
-      for (int k = 0; k < 4; ++k) {
-        int q = gk[c_face[kface][k]];
-        xs[k] = a.gridpos[3 * q]; ys[k] = a.gridpos[3 * q + 1];
-        rb[1][k] = rb[2][k] = 0.f;
-        if ((float)mu2 < 0.f) rb[0][k] = a.skyrad;
-        else {
-          int bi = a.bot_index[q];
-          rb[0][k] = bi >= 0 ? a.bcrad_bot[bi] : 0.f;
-          if constexpr (BRDF) {
-            if (bi >= 0) {
-              float o[3];
-              brdf_radiance_warp(a, bi, (float)mu2, (float)phi2, lane, 3, o);
-              rb[0][k] = o[0]; rb[1][k] = o[1]; rb[2][k] = o[2];
+          for (int k = 0; k < 4; ++k) {
+            const int q = ((k & 1 ? xb : xa) * ny1 + (k & 2 ? yb : ya)) * nz + zz;
+            const float w = (k & 1 ? uu : 1 - uu) * (k & 2 ? vv : 1 - vv);
+            float rb[3] = {a.skyrad, 0.f, 0.f};
+            if (ry.mu >= 0.f) {
+              const int bi = a.bot_index[q];
+              rb[0] = bi >= 0 ? a.bcrad_bot[bi] : 0.f;
+              if constexpr (BRDF)
+                if (bi >= 0) brdf_radiance_lanes(a, bi, ry.mu, ry.phi, k8, 8, gmask, NST, rb);
             }
+#pragma unroll
+            for (int c = 0; c < NST; ++c) radacc[c] += transmit * (double)(w * rb[c]);
           }
         }
       }
-      float uu = (xs[1] - xs[0] > 0) ? ((P1[0] - xs[0]) + lxn) / (xs[1] - xs[0]) : 0.f;
-      float vv = (ys[2] - ys[0] > 0) ? ((P1[1] - ys[0]) + lyn) / (ys[2] - ys[0]) : 0.f;
-      if (!a.nosurface)
-        for (int c = 0; c < 3; ++c)
-          radacc[c] += transmit * ((1 - uu) * (1 - vv) * rb[c][0] + uu * (1 - vv) * rb[c][1] + (1 - uu) * vv * rb[c][2] +
-                                   uu * vv * rb[c][3]);
-    } else {
-      const float *Pn = a.gridpos + 3 * a.gridptr[8 * (size_t)nxt];
-      const float *q = a.gridpos + 3 * a.gridptr[8 * (size_t)nxt + ioct0];
-      lx = jface == 0 ? q[0] - Pn[0] : (P1[0] - Pn[0]) + lxn;
-      ly = jface == 1 ? q[1] - Pn[1] : (P1[1] - Pn[1]) + lyn;
-      lz = jface == 2 ? q[2] - Pn[2] : (P1[2] - Pn[2]) + lzn;
-      cell = nxt;
     }
+    jx = nx_; jy = ny_; jz = mz; lx = lx2; ly = ly2; lz = lz2;
+    ip = ipn; flip = flipn; ext = extn_;
   }
-  if (lane < 3) a.out[(size_t)ray * 3 + lane] = (float)radacc[lane];
+  if (ray < a.nrays && k8 < NST) {
+    double v = radacc[0];
+    if constexpr (NST == 3) v = k8 == 0 ? radacc[0] : k8 == 1 ? radacc[1] : radacc[2];
+    a.out[(size_t)ray * NST + k8] = (float)v;
+  }
 }
 
 __global__ void k_bcrad_bottom(const int *botp, int nbot, const float *botalb, const float *dirflux,
@@ -5159,7 +5120,7 @@ static shdom::RenderArgs render_args(Handle &H, int nrays, const float *camx, co
   a.ns = H.ns.p; a.lofj = H.lofj.p; a.tms_ptr = H.tms_ptr.p; a.tms_iph = H.tms_iph.p; a.tms_w = H.tms_w.p;
   a.phasetab = H.phasetab.p; a.ylmsun = H.ylmsun.p; a.botp = H.botp.p; a.bcrad_bot = H.bcrad.p;
   a.bot_index = H.bot_index.p; a.camx = camx; a.camy = camy; a.camz = camz; a.cammu = cammu; a.camphi = camphi;
-  a.out = out; a.err = H.errflag.p; a.nrays = nrays; a.nx = P.nx; a.ny = P.ny; a.nz = P.nz; a.nlm = P.nlm;
+  a.out = out; a.err = H.errflag.p; a.nrays = nrays; a.nx = P.nx; a.ny = P.ny; a.nz = P.nz; a.ny1 = P.ny1; a.nlm = P.nlm;
   a.nl = P.ml + 1; a.ml = P.ml; a.mm = P.mm; a.bcflag = P.bcflag; a.ipflag = P.ipflag; a.numphase = P.numphase;
   a.nscatangle = P.nscatangle; a.deltam = P.prob.deltam; a.solarmu = P.prob.solarmu; a.solaraz = P.prob.solaraz;
   a.secmu0 = 1.0f / std::fabs(P.prob.solarmu); a.skyrad = P.skyrad_bc; a.tautol = P.prob.tautol;
@@ -5190,22 +5151,22 @@ static int render_impl(shdom_handle *hh, int nrays, const float *camx, const flo
   shdom::RenderArgs a = render_args(H, nrays, camx, camy, camz, cammu, camphi, out);
   a.single_scatter = H.render_single_scatter; a.nosurface = H.render_nosurface;
   if (P.nlm > shdom::RNLM || P.ml + 1 > 64) return fail(hh, "render: too many spherical-harmonic terms");
-  int blocks = (nrays + shdom::RWARPS - 1) / shdom::RWARPS;
-  if (blocks > 0) {
-    if (H.nst == 3) {
-      const size_t smem = (size_t)shdom::RWARPS * 5 * P.nlm * sizeof(float);
-      if (P.brdf) {
-        CK(cudaFuncSetAttribute(shdom::k_render_pol<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        shdom::k_render_pol<true><<<blocks, shdom::RWARPS * 32, smem, stream>>>(a);
-      } else {
-        CK(cudaFuncSetAttribute(shdom::k_render_pol<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        shdom::k_render_pol<false><<<blocks, shdom::RWARPS * 32, smem, stream>>>(a);
-      }
-    } else if (P.brdf) {
-      shdom::k_render<true><<<blocks, shdom::RWARPS * 32, 0, stream>>>(a);
-    } else {
-      shdom::k_render<false><<<blocks, shdom::RWARPS * 32, 0, stream>>>(a);
-    }
+  if (nrays > 0) {
+    auto kernel = H.nst == 3 ? (P.brdf ? shdom::k_render<3, true> : shdom::k_render<3, false>)
+                             : (P.brdf ? shdom::k_render<1, true> : shdom::k_render<1, false>);
+    // four warps a block, fewer where the rays' functions would not leave
+    // room for a second block on the SM, or where the rays are few
+    auto smem = [&](int warps) {
+      const size_t per = (size_t)(H.nst == 3 ? 5 : 1) * ((P.nlm + 3) & ~3) + 4 + (size_t)H.nst * (shdom::RLEG + shdom::RPHASE);
+      return sizeof(float) * ((size_t)warps * shdom::RGRAYS * per + P.nx + P.ny + P.nz + 2);
+    };
+    int warps = 4;
+    while (warps > 1 && (smem(warps) > 100 * 1024 || (long long)nrays < (long long)warps * shdom::RGRAYS * H.nsm)) warps >>= 1;
+    const size_t bytes = smem(warps);
+    if (bytes > 220 * 1024) return fail(hh, "render: too many spherical-harmonic terms");
+    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    const int per = warps * shdom::RGRAYS;
+    kernel<<<(nrays + per - 1) / per, warps * 32, bytes, stream>>>(a);
     H.launches += 1;
   }
   CK(cudaGetLastError());
