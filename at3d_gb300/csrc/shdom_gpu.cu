@@ -6,7 +6,7 @@
 //                   k_tc_gemm, or the factorized k_sh_to_do)
 //   2. sweeps     : downward ordinates, Lambertian bottom, upward ordinates;
 //                   with open boundaries the boundary-plane chains
-//                   (k_sweep_p1s), then the plane march (k_sweep_march);
+//                   (k_sweep_p1c), then the plane march (k_sweep_march);
 //                   else boundary-plane chains (k_sweep_p1) beside the
 //                   source pass (k_sweep_prep), then the wavefront levels
 //                   (k_sweep_levels, or one k_sweep per level); grids whose
@@ -623,7 +623,6 @@ constexpr int P1_THREADS = 512;
 constexpr int P1_SPLIT = 4;
 constexpr int P1_STAGE = 2;
 constexpr int P1_SEGCAP = 512;  // level segments of a phase-1 group kept in shared memory
-constexpr int P1S_THREADS = 512;  // threads of a block-local phase-1 block (256: 0.47 -> 0.50 ms per hemisphere)
 
 __global__ void __launch_bounds__(P1_THREADS) k_sweep_p1(SweepArgs a, const Seg *__restrict__ p1segs,
                                                          const int *__restrict__ p1off) {
@@ -816,126 +815,123 @@ __global__ void __launch_bounds__(P1_THREADS) k_sweep_p1r(SweepArgs a, const Seg
   }
 }
 
-// Phase 1 with block-local radiances.  A phase-1 point's corners are
-// preset boundary points (final before phase 1) or phase-1 points of the
-// same ordinates, i.e. of the same (octant, class) group.  Each group's
-// phase-1 points are numbered in level order (slots); a block owns a slice
-// of the group's columns and keeps the slice's radiances of all the
-// group's phase-1 points in shared memory, so a level reads its corners
-// from there.  k_p1_prep_s folds the boundary corners into radsrc and
-// turns the other corners into slots (q[k] = slot, or -1).
-struct P1Blk {
-  int grp, cbeg, ncs, nslots;  // group, its column slice [cbeg, cbeg + ncs), the group's phase-1 points
+// Phase 1 column by column.  A phase-1 point's corners are preset boundary
+// points (final before phase 1) or phase-1 points of the same ordinates, i.e.
+// of the same (octant, class) group.  Each group's phase-1 points are
+// numbered in level order (slots).
+//  * k_p1_prep_c: every (column, slot)'s trace in one parallel pass (traces
+//    depend on the source only) as a 32-byte record at [column][slot]: the
+//    known part (with the preset corners folded in), the weights and slots of
+//    up to four other corners, the point.
+//  * k_sweep_p1c: one block per column keeps the radiances of the column's
+//    phase-1 points in shared memory; a level is a few shared-memory reads per
+//    point and a block barrier.  Each thread copies its own records of the
+//    next levels into a ring of shared memory, so that their latency is off
+//    the chain of levels.
+//
+// What bounds it: the chain of levels (about 0.25 us each with two columns an
+// SM: 189 levels and 177 columns at 128x128x64 0.116 ms a hemisphere), and for
+// the records the scattered reads of the edge planes (0.25 ms there).  Blocks
+// of several columns with a level's records loaded one level ahead took
+// 0.28 ms at 128x128x64, 0.127 against 0.025 at 64x64x32 and 0.118 against
+// 0.020 at 45x37x29 (12 x 24): few blocks, and a load's latency per level.
+struct P1Col {
+  int col, cs, b, cls;       // column, its place in the group, the group's octant and class
+  int grp, n, pt0;           // group, its slots, its first entry of the slot tables
+  int lev0, nlev;            // its first entry of the level offsets, its levels
+  long long rec;             // the column's first record
 };
+struct __align__(16) P1Rec {
+  float radsrc, w[4];
+  uint16_t q[4];
+  int pt;
+};
+static_assert(sizeof(P1Rec) == 32, "phase-1 records");
 
-__global__ void __launch_bounds__(256) k_p1_prep_s(SweepArgs a, const Seg *__restrict__ segs, int nseg, int n,
-                                                   const int *__restrict__ seggrp, const int *__restrict__ p1slot,
-                                                   TraceRec *__restrict__ out) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    const int si = irr_seg_find(segs, nseg, j);
-    const Seg g = segs[si];
-    const int li = j - g.irr0, task = li / g.ncol, slot = li - task * g.ncol;
-    const int pt = (int)__ldg(a.tasks + g.t0 + task), col = g.col0 + slot;
-    const IrrRec rec = a.irr[j];
+__global__ void __launch_bounds__(256) k_p1_prep_c(SweepArgs a, const P1Col *__restrict__ cols, const int *__restrict__ pts,
+                                                   const int *__restrict__ irr0, const int *__restrict__ p1slot,
+                                                   P1Rec *__restrict__ out) {
+  const P1Col C = cols[blockIdx.y];
+  const int hb = (C.b & 4) ? 2 : 1, col = C.col;
+  const int *slots = p1slot + (size_t)C.grp * a.npts;
+  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < C.n; s += gridDim.x * blockDim.x) {
+    const int pt = __ldg(pts + C.pt0 + s);
+    const IrrRec rec = a.irr[__ldg(irr0 + C.pt0 + s) + C.cs];
     Trace t;
     if (rec.g.w > 0.5f) {
       RegLoad x;
       rec_load(a, rec, pt, col, x, false);
-      t = reg_trace(x, g.b, pt);
+      t = reg_trace(x, C.b, pt);
       t.q[0] = rec.q.x; t.q[1] = rec.q.y; t.q[2] = rec.q.z; t.q[3] = rec.q.w;
     } else {
-      t = trace_general(a, g.b, g.cls, pt, col, true);
+      t = trace_general(a, C.b, C.cls, pt, col, true);
       if (t.status != ERR_NONE) atomicCAS(a.err, ERR_NONE, t.status);
     }
-    const int hb = (g.b & 4) ? 2 : 1;
-    const int *slots = p1slot + (size_t)seggrp[si] * a.npts;
     const float f[4] = {(1.f - t.u) * (1.f - t.v), (1.f - t.u) * t.v, t.u * (1.f - t.v), t.u * t.v};
-    TraceRec r;
-    r.radsrc = t.radsrc; r.tr = t.tr; r.u = t.u; r.v = t.v;
-    int sl[4] = {-1, -1, -1, -1};
+    P1Rec r;
+    r.radsrc = t.radsrc;
+    r.pt = pt;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const float w = t.tr * f[k];
-      if (w == 0.f) continue;
-      if (a.bnd[t.q[k]] & hb) {
-        r.radsrc += w * a.raddo[a.at(t.q[k], col)];  // preset: final
-      } else {
-        sl[k] = slots[t.q[k]];
-        if (sl[k] < 0) atomicCAS(a.err, ERR_NONE, ERR_SWEEP_NOFACE);  // not a phase-1 point of the group
+      float w = t.tr * f[k];
+      int q = 0;
+      if (w != 0.f) {
+        if (a.bnd[t.q[k]] & hb) {
+          r.radsrc += w * a.raddo[a.at(t.q[k], col)];  // preset: final
+          w = 0.f;
+        } else {
+          q = slots[t.q[k]];
+          if (q < 0 || q >= s) { atomicCAS(a.err, ERR_NONE, ERR_SWEEP_NOFACE); q = 0; w = 0.f; }  // not an earlier phase-1 point of the group
+        }
       }
+      r.w[k] = w;
+      r.q[k] = (uint16_t)q;
     }
-    r.q = make_int4(sl[0], sl[1], sl[2], sl[3]);
-    out[j] = r;
+    out[C.rec + s] = r;
   }
 }
 
-__global__ void __launch_bounds__(P1S_THREADS) k_sweep_p1s(SweepArgs a, const Seg *__restrict__ p1segs,
-                                                          const int *__restrict__ p1off, const P1Blk *__restrict__ blks,
-                                                          const int *__restrict__ segbase,
-                                                          const TraceRec *__restrict__ recs) {
-  extern __shared__ float sv[];  // [slot][column of the slice]
-  __shared__ Seg ssg[P1_SEGCAP];
-  __shared__ int sbase[P1_SEGCAP];
-  const P1Blk B = blks[blockIdx.x];
-  const int s0 = p1off[B.grp], s1 = p1off[B.grp + 1], ncs = B.ncs;
-  for (int t = threadIdx.x; t < s1 - s0; t += blockDim.x) { ssg[t] = p1segs[s0 + t]; sbase[t] = segbase[s0 + t]; }
+__global__ void __launch_bounds__(512) k_sweep_p1c(SweepArgs a, const P1Col *__restrict__ cols, const int *__restrict__ levs,
+                                                   const P1Rec *__restrict__ recs, int depth, int maxtask) {
+  extern __shared__ __align__(16) unsigned char p1m[];
+  P1Rec *ring = reinterpret_cast<P1Rec *>(p1m);                      // [depth][maxtask]
+  float *val = reinterpret_cast<float *>(ring + (size_t)depth * maxtask);  // [slot]
+  const P1Col C = cols[blockIdx.x];
+  int *lev = reinterpret_cast<int *>(val + C.n);                     // [nlev + 1]
+  const int tid = threadIdx.x;
+  const P1Rec *rec = recs + C.rec;
+  float *rado = a.raddo + (size_t)C.col * a.cs;
+  for (int i = tid; i <= C.nlev; i += blockDim.x) lev[i] = __ldg(levs + C.lev0 + i);
+  if (tid == 0) val[0] = 0.f;  // read with weight zero
   __syncthreads();
-  TraceRec sr[P1_STAGE];
-  int spt[P1_STAGE];
-  auto rec_of = [&](const Seg &g, int ii, int &pt, int &col, int &slot, int &c) {
-    const int task = ii / ncs;
-    c = ii - task * ncs;
-    pt = (int)__ldg(a.tasks + g.t0 + task);
-    col = g.col0 + B.cbeg + c;
-    slot = task;
-    return g.irr0 + task * g.ncol + B.cbeg + c;
-  };
-  auto combine = [&](const TraceRec &R, int pt, int col, int slot, int c) {
-    float rad = R.radsrc;
-    if (R.tr != 0.f) {
-      const float u = R.u, v = R.v;
-      const float f0 = (1.f - u) * (1.f - v), f1 = (1.f - u) * v, f2 = u * (1.f - v), f3 = u * v;
-      float acc = 0.f;
-      if (R.q.x >= 0) acc += f0 * sv[R.q.x * ncs + c];
-      if (R.q.y >= 0) acc += f1 * sv[R.q.y * ncs + c];
-      if (R.q.z >= 0) acc += f2 * sv[R.q.z * ncs + c];
-      if (R.q.w >= 0) acc += f3 * sv[R.q.w * ncs + c];
-      rad += R.tr * acc;
-    }
-    sv[slot * ncs + c] = rad;
-    a.raddo[a.at(pt, col)] = rad;
-  };
-  auto stage = [&](int si) {
-    if (si >= s1) return;
-    const Seg &g = ssg[si - s0];
-    const int items = g.ntask * ncs;
-#pragma unroll
-    for (int k = 0; k < P1_STAGE; ++k) {
-      const int ii = threadIdx.x + k * blockDim.x;
-      if (ii < items) {
-        int col, slot, c;
-        sr[k] = recs[rec_of(g, ii, spt[k], col, slot, c)];
+  auto fetch = [&](int l, int d) {  // this thread's records of level l (an empty group past the last)
+    if (l < C.nlev) {
+      const int l0 = lev[l], m = lev[l + 1] - l0;
+      for (int i = tid; i < m; i += blockDim.x) {
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(ring + (size_t)d * maxtask + i);
+        const P1Rec *src = rec + l0 + i;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n cp.async.cg.shared.global [%0 + 16], [%1 + 16], 16;" ::"r"(dst), "l"(src) : "memory");
       }
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  stage(s0);
-  for (int si = s0; si < s1; ++si) {
-    const Seg &g = ssg[si - s0];
-    const int items = g.ntask * ncs, base = sbase[si - s0];
-#pragma unroll
-    for (int k = 0; k < P1_STAGE; ++k) {
-      const int ii = threadIdx.x + k * blockDim.x;
-      if (ii < items) {
-        const int task = ii / ncs, c = ii - task * ncs;
-        combine(sr[k], spt[k], g.col0 + B.cbeg + c, base + task, c);
-      }
+  // groups are counted in steps of two in flight at least: depth levels minus one are always committed
+  for (int l = 0; l < depth - 1; ++l) fetch(l, l);
+  int d = 0, dn = depth - 1;
+  for (int l = 0; l < C.nlev; ++l) {
+    if (depth >= 8) asm volatile("cp.async.wait_group 6;" ::: "memory");
+    else if (depth >= 4) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const int l0 = lev[l], m = lev[l + 1] - l0;
+    for (int i = tid; i < m; i += blockDim.x) {
+      const P1Rec r = ring[(size_t)d * maxtask + i];
+      const float x = r.radsrc + (r.w[0] * val[r.q[0]] + r.w[1] * val[r.q[1]] + r.w[2] * val[r.q[2]] + r.w[3] * val[r.q[3]]);
+      val[l0 + i] = x;
+      rado[(size_t)r.pt * a.ps] = x;
     }
-    for (int ii = threadIdx.x + P1_STAGE * blockDim.x; ii < items; ii += blockDim.x) {
-      int pt, col, slot, c;
-      const int j = rec_of(g, ii, pt, col, slot, c);
-      combine(recs[j], pt, col, base + slot, c);
-    }
-    stage(si + 1);  // the next level's records, which do not depend on this level
+    fetch(l + depth - 1, dn);
+    if (++d == depth) d = 0;
+    if (++dn == depth) dn = 0;
     __syncthreads();
   }
 }
@@ -3205,7 +3201,11 @@ __device__ RaySetup ray_setup(const RenderArgs &a, int ray) {
 // accumulators are FP64, folded once per cell.  Where all rays of a block
 // have one direction (a parallel view) its functions are formed once.
 //
-// What bounds it: %RENDER%
+// What bounds it: latency (a corner's loads, then the dependent chain of a
+// cell; 14 warps an SM issue 31% of the cycles), then issue slots.  Measured
+// for 36,864 rays against one warp per ray: 64x64x32 0.73 against 2.12 ms,
+// 128x128x64 (256 terms) 2.8 against 4.9, polarized 64x64x40 3.0 against
+// 11.0; 169 rays at 32x32x24 0.21 ms either way (the chain of one ray).
 template <int NST, bool BRDF>
 __global__ void __launch_bounds__(128) k_render(RenderArgs a) {
   extern __shared__ __align__(16) float rsm[];
@@ -3566,12 +3566,14 @@ struct DevGeom {
   DBuf<IrrRec> irr[2];
   bool irr_built = false;
   bool seq_checked = false, seq_lex[2] = {false, false};  // the walk's order per hemisphere (k_seq_check)
-  // block-local phase 1 (setup_p1s): per hemisphere, built once per grid and device
-  bool p1s_built = false, p1s_ok[2] = {false, false};
-  DBuf<P1Blk> p1blk[2];
-  DBuf<int> p1base[2], p1grp[2], p1slot[2];
-  int np1blk[2] = {0, 0};
-  size_t p1smem[2] = {0, 0};
+  // phase 1 column by column (setup_p1c): per hemisphere, built once per grid
+  // and device: the columns; per group and slot its point and first record of
+  // the general-trace table, the level offsets; [group][point] slot or -1
+  bool p1c_built = false, p1c_ok[2] = {false, false};
+  DBuf<P1Col> p1cols[2];
+  DBuf<int> p1pts[2], p1irr0[2], p1lev[2], p1slot[2];
+  struct P1Shape { int ncols = 0, threads = 0, depth = 0, maxtask = 0, maxn = 0; long long recs = 0; size_t smem = 0; };
+  P1Shape p1shape[2];
   std::mutex mu;  // guards the one-time builds of irr and of the phase-1 tables
 };
 static std::mutex g_devgeom_mu;
@@ -3660,11 +3662,7 @@ struct Handle {
   bool seq[2] = {false, false};  // reference-order sweep engine per hemisphere
   DBuf<TraceRec> seqrec;            // its trace records, [ordinate][rank] of one hemisphere
   DBuf<TraceRec> p1rec;             // phase-1 trace records ahead of the plane march, [irr entry]
-  bool p1s[2] = {false, false};     // phase 1 with block-local radiances (k_sweep_p1s)
-  DBuf<P1Blk> p1blk[2];
-  int np1blk[2] = {0, 0};
-  size_t p1smem[2] = {0, 0};
-  DBuf<int> p1base[2], p1grp[2], p1slot[2];  // per segment: first slot, group; [group][point]: slot or -1
+  bool p1c[2] = {false, false};     // phase 1 column by column (k_sweep_p1c; its records in p1rec)
   // plane-march phase 2 per hemisphere (k_sweep_march): one cluster per
   // column, the x and y classes' columns first
   bool march[2] = {false, false};
@@ -4015,7 +4013,7 @@ static long long plan_device_bytes(const Plan &P) {
     for (int h = 0; h < 2; ++h)
       if (!P.march[h].empty()) {
         n1 = std::max<long long>(n1, (long long)P.nirr[h]);
-        b += 4LL * P.npts * std::max(0, (int)P.p1off[h].size() - 1) + 8LL * (long long)P.p1segs[h].size();
+        b += 4LL * P.npts * std::max(0, (int)P.p1off[h].size() - 1) + 8LL * (long long)P.p1segs[h].size() + 8LL * (long long)P.tasks[h].size();
       }
     b += 32LL * n1;
   }
@@ -4166,79 +4164,76 @@ static void setup_march(Handle &H) {
   }
 }
 
-// Block-local phase 1 (k_sweep_p1s) for each marching hemisphere whose
-// phase-1 groups fit: a group's phase-1 points are numbered in level order,
-// and a block takes as many of its columns as keep the slice's radiances
-// of all those points in kP1SmemCap bytes (and a level's items within four
-// per thread).  Otherwise the hemisphere keeps k_sweep_p1r.
-constexpr size_t kP1SmemCap = 192 * 1024;
-
-static void setup_p1s(Handle &H) {
+// Phase 1 column by column (k_sweep_p1c) for each marching hemisphere whose
+// groups fit: a column's radiances, level offsets and a ring of two levels'
+// records in shared memory, slots in 16 bits.  Otherwise the hemisphere keeps
+// k_sweep_p1r.
+static void setup_p1c(Handle &H) {
   Plan &P = H.P;
   int dev = 0, maxsm = 0;
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  const size_t static_smem = sizeof(Seg) * P1_SEGCAP + sizeof(int) * P1_SEGCAP;
-  if ((size_t)maxsm >= kP1SmemCap + static_smem)
-    CK(cudaFuncSetAttribute(k_sweep_p1s, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(maxsm - static_smem)));
+  CK(cudaFuncSetAttribute(k_sweep_p1c, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
   DevGeom &G = *H.geom;
   std::lock_guard<std::mutex> lk(G.mu);
-  if (!G.p1s_built) {
+  if (!G.p1c_built) {
     for (int h = 0; h < 2; ++h) {
-      G.p1s_ok[h] = false;
+      G.p1c_ok[h] = false;
       const std::vector<int> &off = P.p1off[h];
       const int ng1 = (int)off.size() - 1;
-      if (!H.march[h] || ng1 <= 0 || (size_t)maxsm < kP1SmemCap + static_smem) continue;
+      if (!H.march[h] || ng1 <= 0) continue;
       const std::vector<Seg> &sg = P.p1segs[h];
-      std::vector<int> base(sg.size(), 0), grp(sg.size(), 0), nslots(ng1, 0);
+      std::vector<int> pts, irr0, lev, slot((size_t)ng1 * P.npts, -1);
+      std::vector<P1Col> cols;
+      long long rec = 0;
+      int maxtask = 1, maxn = 0, maxlev = 0;
       bool ok = true;
       for (int g = 0; g < ng1 && ok; ++g) {
-        if (off[g + 1] - off[g] > P1_SEGCAP) ok = false;
-        for (int si = off[g]; si < off[g + 1]; ++si) {
-          base[si] = nslots[g];
-          grp[si] = g;
-          nslots[g] += sg[si].ntask;
-          if (sg[si].col0 != sg[off[g]].col0 || sg[si].ncol != sg[off[g]].ncol) ok = false;
-        }
-        if ((size_t)nslots[g] * sizeof(float) > kP1SmemCap) ok = false;
-      }
-      if (!ok) continue;
-      std::vector<P1Blk> blks;
-      size_t smem = 0;
-      for (int g = 0; g < ng1; ++g) {
         if (off[g + 1] == off[g]) continue;
         const Seg &s0 = sg[off[g]];
-        int maxtask = 0;
-        for (int si = off[g]; si < off[g + 1]; ++si) maxtask = std::max(maxtask, sg[si].ntask);
-        int ncs = (int)std::min<size_t>(kP1SmemCap / ((size_t)nslots[g] * sizeof(float)), (size_t)s0.ncol);
-        ncs = std::max(1, std::min(ncs, 4 * P1S_THREADS / std::max(1, maxtask)));
-        for (int c0 = 0; c0 < s0.ncol; c0 += ncs) {
-          const int nc = std::min(ncs, s0.ncol - c0);
-          blks.push_back(P1Blk{g, c0, nc, nslots[g]});
-          smem = std::max(smem, (size_t)nslots[g] * nc * sizeof(float));
+        P1Col C{};
+        C.b = s0.b; C.cls = s0.cls; C.grp = g; C.pt0 = (int)pts.size(); C.lev0 = (int)lev.size(); C.nlev = off[g + 1] - off[g];
+        for (int si = off[g]; si < off[g + 1]; ++si) {
+          const Seg &q = sg[si];
+          if (q.col0 != s0.col0 || q.ncol != s0.ncol || q.b != s0.b || q.cls != s0.cls) ok = false;
+          lev.push_back((int)pts.size() - C.pt0);
+          for (int t = 0; t < q.ntask; ++t) {
+            const int pt = (int)P.tasks[h][q.t0 + t];
+            slot[(size_t)g * P.npts + pt] = (int)pts.size() - C.pt0;
+            pts.push_back(pt);
+            irr0.push_back(q.irr0 + t * q.ncol);
+          }
+          maxtask = std::max(maxtask, q.ntask);
+        }
+        C.n = (int)pts.size() - C.pt0;
+        lev.push_back(C.n);
+        maxn = std::max(maxn, C.n);
+        maxlev = std::max(maxlev, C.nlev);
+        for (int c = 0; c < s0.ncol; ++c) {
+          C.col = s0.col0 + c; C.cs = c; C.rec = rec;
+          if (P.col_cz[C.col] == 0.f) continue;  // padding ordinate
+          cols.push_back(C);
+          rec += C.n;
         }
       }
-      std::vector<int> slot((size_t)ng1 * P.npts, -1);
-      for (int g = 0; g < ng1; ++g)
-        for (int si = off[g]; si < off[g + 1]; ++si)
-          for (int t = 0; t < sg[si].ntask; ++t) slot[(size_t)g * P.npts + P.tasks[h][sg[si].t0 + t]] = base[si] + t;
-      G.p1blk[h].upload(blks);
-      G.p1base[h].upload(base);
-      G.p1grp[h].upload(grp);
+      int depth = 0;
+      for (int d : {8, 4, 2})
+        if (!depth && 32 * (size_t)d * maxtask + 4 * ((size_t)maxn + maxlev + 1) <= (size_t)maxsm) depth = d;
+      if (!ok || cols.empty() || !depth || maxn > 65535) continue;
+      // the columns with the longest chains first
+      std::stable_sort(cols.begin(), cols.end(), [](const P1Col &x, const P1Col &y) { return x.nlev > y.nlev; });
+      G.p1cols[h].upload(cols);
+      G.p1pts[h].upload(pts);
+      G.p1irr0[h].upload(irr0);
+      G.p1lev[h].upload(lev);
       G.p1slot[h].upload(slot);
-      G.np1blk[h] = (int)blks.size();
-      G.p1smem[h] = smem;
-      G.p1s_ok[h] = true;
+      G.p1shape[h] = {(int)cols.size(), std::min(512, (std::max(64, maxtask) + 31) / 32 * 32), depth, maxtask, maxn, rec,
+                      32 * (size_t)depth * maxtask + 4 * ((size_t)maxn + maxlev + 1)};
+      G.p1c_ok[h] = true;
     }
-    G.p1s_built = true;
+    G.p1c_built = true;
   }
-  for (int h = 0; h < 2; ++h) {
-    H.p1s[h] = G.p1s_ok[h] && H.march[h];
-    if (!H.p1s[h]) continue;
-    H.p1blk[h].view(G.p1blk[h]); H.p1base[h].view(G.p1base[h]);
-    H.p1grp[h].view(G.p1grp[h]); H.p1slot[h].view(G.p1slot[h]);
-    H.np1blk[h] = G.np1blk[h]; H.p1smem[h] = G.p1smem[h];
-  }
+  for (int h = 0; h < 2; ++h) H.p1c[h] = G.p1c_ok[h] && H.march[h];
 }
 
 static void upload_plan(Handle &H) {
@@ -4598,7 +4593,7 @@ static void build_irr(Handle &H) {
     }
     for (int h = 0; h < 2; ++h) H.irr[h].view(G.irr[h]);
   }
-  setup_p1s(H);
+  setup_p1c(H);
   if ((!H.march[0] && !H.seq[0] && P.seg_off[0].size() > 1) || (!H.march[1] && !H.seq[1] && P.seg_off[1].size() > 1))
     H.sweepw.alloc((size_t)P.npts * H.ldo);
   {  // phase-1 trace records ahead of the plane march
@@ -4676,15 +4671,15 @@ static void sweep_hemisphere(Handle &H, int hemi) {
     if (ng1 > 0) {
       const int n1 = H.p2_irr_j0[hemi];
       const int blocks = std::min((n1 + 255) / 256, H.nsm * 8);
-      if (H.p1s[hemi]) {
-        if (n1 > 0) {
-          k_p1_prep_s<<<blocks, 256, 0, H.stream>>>(a, H.irrsegs[hemi].p, H.p2_irrseg0[hemi], n1, H.p1grp[hemi].p,
-                                                    H.p1slot[hemi].p, H.p1rec.p);
-          CK(cudaGetLastError());
-          H.launches += 1;
-        }
-        k_sweep_p1s<<<H.np1blk[hemi], P1S_THREADS, H.p1smem[hemi], H.stream>>>(
-            a, H.p1segs[hemi].p, H.p1off[hemi].p, H.p1blk[hemi].p, H.p1base[hemi].p, H.p1rec.p);
+      if (H.p1c[hemi]) {
+        const DevGeom &G = *H.geom;
+        const DevGeom::P1Shape &L = G.p1shape[hemi];
+        P1Rec *rec = reinterpret_cast<P1Rec *>(H.p1rec.p);
+        k_p1_prep_c<<<dim3((L.maxn + 255) / 256, L.ncols), 256, 0, H.stream>>>(a, G.p1cols[hemi].p, G.p1pts[hemi].p, G.p1irr0[hemi].p,
+                                                                               G.p1slot[hemi].p, rec);
+        CK(cudaGetLastError());
+        k_sweep_p1c<<<L.ncols, L.threads, L.smem, H.stream>>>(a, G.p1cols[hemi].p, G.p1lev[hemi].p, rec, L.depth, L.maxtask);
+        H.launches += 1;
       } else {
         if (n1 > 0) {
           k_p1_prep<<<blocks, 256, 0, H.stream>>>(a, H.irrsegs[hemi].p, H.p2_irrseg0[hemi], n1, H.p1rec.p);
