@@ -2726,6 +2726,174 @@ __global__ void __launch_bounds__(256) k_source_pol(SourceArgs a) {
   }
 }
 
+// x added to the pair (hi, lo), hi + lo exact to 48 bits (Knuth's two-sum):
+// the sums over points in a few FP32 operations, since one FP64 operation
+// holds the pipe of an SM for 16 cycles.
+__device__ __forceinline__ void two_sum(float &hi, float &lo, float x) {
+  const float s = hi + x, b = s - hi;
+  lo += (hi - (s - b)) + (x - b);
+  hi = s;
+}
+
+// COMPUTE_SOURCE and the next RADIANCE_TRUNCATION as k_source / k_source_pol,
+// for rows of up to 256 terms, a multiple of four: LPP lanes per point (so 16
+// lanes take a row of 64 terms and a warp two points), four consecutive terms
+// per lane and pass, NP passes.  A lane's terms are the same for every point,
+// so their degrees and sun values stay in registers; the point's coefficients
+// are spread over its lanes.  The terms wait in registers for the truncation
+// and each row is written once.  list: the points (null: all).  Points whose
+// coefficients are all zero and that do not emit keep a zero source, no terms
+// and a radiance truncation of 4 in every iteration, so after the first pass
+// the list leaves them out where the handle knows them (H.compact).
+//
+// What bounds it: memory (five rows per point).  Measured against a warp per
+// point, every point, FP64 sums: 64x64x32 with 64 terms and 20% cloud 28
+// against 104 us, 128x128x64 with 256 terms and 30% cloud 0.43 against 0.76
+// ms, 64x64x40 with 3 x 64 terms 0.11 against 0.32.
+template <int NST, int LPP, int NP>
+__global__ void __launch_bounds__(256) k_source_v(SourceArgs a, const int *__restrict__ list, int n) {
+  const int lane = threadIdx.x & 31, gl = lane % LPP, sub = lane / LPP;
+  constexpr int PPW = 32 / LPP;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int nlm = a.nlm, nl = a.nl;
+  int lj[NP][4];
+  float yv[NP][4];
+#pragma unroll
+  for (int s = 0; s < NP; ++s)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int j = 4 * (gl + s * LPP) + q;
+      lj[s][q] = j < nlm ? a.lofj[j] : 0;
+      yv[s][q] = j < nlm ? a.ylmsun[j] : 0.f;
+    }
+  float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+  const bool trunc = !a.fixsh || a.first;
+  for (int i0 = warp * PPW; i0 < n; i0 += nwarps * PPW) {
+    const bool on = i0 + sub < n;
+    const int i = on ? i0 + sub : n - 1, p = list ? __ldg(list + i) : i;
+    const float cv = gl < nl ? a.coef[(size_t)p * nl + gl] : 0.f;
+    float cp[3] = {0.f, 0.f, 0.f};
+    if constexpr (NST == 3)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) cp[k] = gl < nl ? a.coefp[((size_t)p * 3 + k) * nl + gl] : 0.f;
+    const float f0 = a.dirflux[p] * a.secmu0, th = a.thermal ? 3.544907703f * a.thermal[p] : 0.f;
+    const int nrp = a.nr[p], nsold = a.ns[p], nsmin = min(nsold, a.nso[p]);
+    float *S = a.source + (size_t)p * NST * nlm, *D = a.delsource + (size_t)p * NST * nlm;
+    const float *R = a.radiance + (size_t)p * NST * nlm;
+    float jt[NST][NP][4], sum[4] = {0.f, 0.f, 0.f, 0.f}, r00 = 0.f;
+    int last = 0;
+#pragma unroll
+    for (int s = 0; s < NP; ++s) {
+      const int j = 4 * (gl + s * LPP);
+      const bool in = j < nlm;
+      const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 r4[NST], s4[NST], d4[NST];
+#pragma unroll
+      for (int k = 0; k < NST; ++k) {
+        r4[k] = in && j < nrp ? *reinterpret_cast<const float4 *>(R + k * nlm + j) : z4;
+        s4[k] = in && !a.first && j < nsold ? *reinterpret_cast<const float4 *>(S + k * nlm + j) : z4;
+        d4[k] = in && !a.first && a.accel && j < nsmin ? *reinterpret_cast<const float4 *>(D + k * nlm + j) : z4;
+      }
+      if (s == 0) r00 = r4[0].x;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float c = __shfl_sync(0xffffffffu, cv, lj[s][q], LPP);
+        const float ri = j + q < nrp ? (&r4[0].x)[q] : 0.f;
+        if constexpr (NST == 1) {
+          jt[0][s][q] = f0 * c * yv[s][q];
+          if (j + q == 0) jt[0][s][q] += th;
+          if (j + q < nrp) jt[0][s][q] += c * ri;
+        } else {
+          const float ca2 = __shfl_sync(0xffffffffu, cp[0], lj[s][q], LPP), ca3 = __shfl_sync(0xffffffffu, cp[1], lj[s][q], LPP),
+                      cb1 = __shfl_sync(0xffffffffu, cp[2], lj[s][q], LPP);
+          const float rq = j + q < nrp ? (&r4[1].x)[q] : 0.f, ru = j + q < nrp ? (&r4[2].x)[q] : 0.f;
+          const float ys = f0 * yv[s][q];
+          jt[0][s][q] = c * ys + c * ri + cb1 * rq;
+          if (j + q == 0) jt[0][s][q] += th;
+          jt[1][s][q] = j + q >= 4 ? cb1 * ri + ca2 * rq + cb1 * ys : 0.f;
+          jt[2][s][q] = j + q >= 4 ? ca3 * ru : 0.f;
+        }
+      }
+      if (!a.first) {
+#pragma unroll
+        for (int k = 0; k < NST; ++k) {
+          float dnew[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float so = (&s4[k].x)[q], dn = jt[k][s][q] - so, dd = (&d4[k].x)[q];
+            dnew[q] = j + q < nsold ? dn : 0.f;
+            if (j + q < (a.accel ? nsmin : nsold)) {
+              sum[0] += dn * dd; sum[1] += dd * dd; sum[2] += dn * dn; sum[3] += so * so;
+            }
+          }
+          if (on && in && a.accel) *reinterpret_cast<float4 *>(D + k * nlm + j) = make_float4(dnew[0], dnew[1], dnew[2], dnew[3]);
+        }
+      }
+      if (trunc)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          bool big = fabsf(jt[0][s][q]) > a.shacc;
+          if constexpr (NST == 3) big = big || fabsf(jt[1][s][q]) > a.shacc || fabsf(jt[2][s][q]) > a.shacc;
+          if (j + q < nlm && big) last = j + q + 1;
+        }
+    }
+    if (on && !a.first)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) two_sum(hi[k], lo[k], sum[k]);
+    int nsnew = nsold, nrnext;
+    if (trunc) {
+#pragma unroll
+      for (int o = LPP / 2; o > 0; o >>= 1) last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
+      const int ls = last > 0 ? a.lofj[last - 1] : 0;
+      nsnew = last == 0 ? 0 : (ls <= a.mm) ? ls * (ls + 1) + ls + 1 : (2 * a.mm + 1) * ls - a.mm * a.mm + a.mm + 1;
+      // next radiance truncation
+      const float r0 = __shfl_sync(0xffffffffu, r00, 0, LPP);
+      const unsigned big = __ballot_sync(0xffffffffu, gl >= 1 && gl < nl && cv * r0 > a.shacc) >> (sub * LPP);
+      const unsigned mine = LPP == 32 ? big : big & ((1u << (LPP & 31)) - 1u);
+      int lr = mine ? 31 - __clz(mine) : 1;
+      lr = min(lr, a.lofj[max(1, nsnew) - 1] + a.ml / 8 + 2);
+      if (a.highorder) lr = a.ml;
+      nrnext = (lr <= a.mm) ? lr * (lr + 1) + lr + 1 : (2 * a.mm + 1) * lr - a.mm * a.mm + a.mm + 1;
+    } else {
+      nrnext = max(4, nsnew);
+    }
+    if (a.highorder && a.fixsh && !a.first) nrnext = nlm;
+    if (on) {
+#pragma unroll
+      for (int s = 0; s < NP; ++s) {
+        const int j = 4 * (gl + s * LPP);
+        if (j < nlm)
+#pragma unroll
+          for (int k = 0; k < NST; ++k)
+            *reinterpret_cast<float4 *>(S + k * nlm + j) =
+                make_float4(j < nsnew ? jt[k][s][0] : 0.f, j + 1 < nsnew ? jt[k][s][1] : 0.f,
+                            j + 2 < nsnew ? jt[k][s][2] : 0.f, j + 3 < nsnew ? jt[k][s][3] : 0.f);
+      }
+      if (gl == 0) {
+        a.ns[p] = nsnew;
+        if (a.first) a.nso[p] = nsnew;
+        else if (a.accel) a.nso[p] = nsold;
+        a.nr[p] = nrnext;
+      }
+    }
+  }
+  if (!a.first) {
+    __shared__ double sred[4][8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      double t = (double)hi[k] + (double)lo[k];
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) sred[k][threadIdx.x >> 5] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+      double t = 0;
+      for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += sred[threadIdx.x][k];
+      atomicAdd(&a.red[threadIdx.x], t);
+    }
+  }
+}
+
 struct AccelState {
   double a;        // acceleration parameter of the last iteration
   float solcrit;
@@ -2762,6 +2930,43 @@ __global__ void k_accelerate(float *source, const float *delsource, const int *n
   for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < total; t += (size_t)gridDim.x * blockDim.x) {
     int p = (int)(t / row), j = (int)(t - (size_t)p * row) % nlm;
     if (j < min(ns[p], nso[p])) source[t] += a * delsource[t];
+  }
+}
+
+// ACCELERATE_SOLUTION (src/polarized/shdomsub1.f:1807-1831) on the listed
+// points (null: all), rows of nst * nlm values (Stokes rows of nlm terms, a
+// multiple of four), one row per group of LPP lanes; with packed, the rows are
+// also copied there in list order, for the compacted transform of the next
+// iteration.
+template <int LPP>
+__global__ void __launch_bounds__(256) k_accelerate_v(float *__restrict__ source, const float *__restrict__ delsource,
+                                                      const int *__restrict__ ns, const int *__restrict__ nso,
+                                                      const int *__restrict__ list, int n, int nlm, int nst,
+                                                      const AccelState *st, float *__restrict__ packed) {
+  const float a = st ? st->accelpar : 0.f;
+  const bool acc = a > 0.f;
+  if (!acc && !packed) return;
+  const int gl = threadIdx.x % LPP, row = nst * nlm;
+  const int ngrp = gridDim.x * (blockDim.x / LPP);
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) / LPP; i < n; i += ngrp) {
+    const int p = list ? __ldg(list + i) : i;
+    const int m = acc ? min(ns[p], nso[p]) : 0;
+    float *S = source + (size_t)p * row;
+    const float *D = delsource + (size_t)p * row;
+    float *C = packed ? packed + (size_t)i * row : nullptr;
+    for (int j = 4 * gl; j < row; j += 4 * LPP) {
+      const int jt = j % nlm;  // (nlm is a multiple of four: no Stokes row is straddled)
+      float4 s = *reinterpret_cast<const float4 *>(S + j);
+      if (jt < m) {
+        const float4 d = *reinterpret_cast<const float4 *>(D + j);
+        s.x += a * d.x;
+        if (jt + 1 < m) s.y += a * d.y;
+        if (jt + 2 < m) s.z += a * d.z;
+        if (jt + 3 < m) s.w += a * d.w;
+        *reinterpret_cast<float4 *>(S + j) = s;
+      }
+      if (C) *reinterpret_cast<float4 *>(C + j) = s;
+    }
   }
 }
 
@@ -4399,6 +4604,15 @@ static void upload_plan(Handle &H) {
   CK(cudaStreamSynchronize(cudaStreamLegacy));
 }
 
+// Lanes per point of the row kernels (k_source_v, k_accelerate_v): four terms
+// per lane, half a warp for rows of up to 64 terms (a whole one there leaves
+// half its lanes idle), up to 256 terms; 0 where they do not apply (rows not
+// a multiple of four, or more degrees than lanes to hold their coefficients).
+static int row_lanes(const Plan &P) {
+  const int lpp = P.nlm <= 64 ? 16 : 32;
+  return (P.nlm & 3) == 0 && P.nlm <= 256 && P.ml + 1 <= lpp ? lpp : 0;
+}
+
 static void launch_source(Handle &H, int first, int fixsh) {
   Plan &P = H.P;
   SourceArgs a;
@@ -4410,10 +4624,54 @@ static void launch_source(Handle &H, int first, int fixsh) {
   a.first = first; a.fixsh = fixsh; a.accel = P.prob.accelflag; a.highorder = P.prob.highorderrad;
   a.coefp = H.nst == 3 ? H.coefp.p : nullptr;
   CK(cudaMemsetAsync(H.red.p, 0, 4 * sizeof(double), H.stream));
-  int blocks = std::min((P.npts + 7) / 8, 152 * 16);
-  if (H.nst == 3) k_source_pol<<<blocks, 256, 0, H.stream>>>(a);
-  else k_source<<<blocks, 256, 0, H.stream>>>(a);
-  H.launches += 1;
+  const int lpp = row_lanes(P);
+  if (lpp) {
+    // after the first pass the points without a source are left out
+    const bool some = H.compact && !first && P.prob.shacc >= 0.f;
+    const int *list = some ? H.heavy.p : nullptr;
+    const int n = some ? H.nheavy : P.npts;
+    const int blocks = std::min((n + 8 * (32 / lpp) - 1) / (8 * (32 / lpp)), H.nsm * 8);
+    const bool two = P.nlm > 4 * lpp;
+    if (n > 0) {
+      if (H.nst == 3) (lpp == 16 ? k_source_v<3, 16, 1> : two ? k_source_v<3, 32, 2> : k_source_v<3, 32, 1>)<<<blocks, 256, 0, H.stream>>>(a, list, n);
+      else (lpp == 16 ? k_source_v<1, 16, 1> : two ? k_source_v<1, 32, 2> : k_source_v<1, 32, 1>)<<<blocks, 256, 0, H.stream>>>(a, list, n);
+      H.launches += 1;
+    }
+  } else {
+    const int blocks = std::min((P.npts + 7) / 8, H.nsm * 16);
+    if (H.nst == 3) k_source_pol<<<blocks, 256, 0, H.stream>>>(a);
+    else k_source<<<blocks, 256, 0, H.stream>>>(a);
+    H.launches += 1;
+  }
+  CK(cudaGetLastError());
+}
+
+// The series acceleration of the source, and the packed rows of the next
+// compacted transform; with first, the packed rows of the first source only.
+static void launch_accelerate(Handle &H, bool first) {
+  Plan &P = H.P;
+  const AccelState *st = first ? nullptr : H.accel.p;
+  float *packed = H.compact && H.nheavy > 0 ? H.src_c.p : nullptr;
+  if (const int lpp = row_lanes(P)) {
+    const int *list = H.compact ? H.heavy.p : nullptr;
+    const int n = H.compact ? H.nheavy : P.npts;
+    if (n <= 0 || (first && !packed)) return;
+    const int blocks = std::min((n + 256 / lpp - 1) / (256 / lpp), H.nsm * 16);
+    (lpp == 16 ? k_accelerate_v<16> : k_accelerate_v<32>)<<<blocks, 256, 0, H.stream>>>(
+        H.source.p, H.delsource.p, H.ns.p, H.nso.p, list, n, P.nlm, H.nst, st, packed);
+    H.launches += 1;
+  } else {
+    if (!first) {
+      const int blocks = (int)std::min<size_t>(((size_t)P.npts * H.nst * P.nlm + 255) / 256, 152 * 64);
+      k_accelerate<<<blocks, 256, 0, H.stream>>>(H.source.p, H.delsource.p, H.ns.p, H.nso.p, P.npts, P.nlm, H.accel.p, H.nst);
+      H.launches += 1;
+    }
+    if (packed) {
+      const int rows = (int)std::min<long long>(((long long)H.nheavy * (P.nlm / 4) + 255) / 256, 152 * 16);
+      k_gather_rows<<<rows, 256, 0, H.stream>>>(H.source.p, H.heavy.p, H.nheavy, P.nlm, packed);
+      H.launches += 1;
+    }
+  }
   CK(cudaGetLastError());
 }
 
@@ -4467,9 +4725,9 @@ static void transform(Handle &H, int dir) {
       if (H.nheavy > 0) {
         const long long q = (long long)H.nheavy * (rowlen / 4);
         const int gb = (int)std::min<long long>((q + 255) / 256, 152 * 16);
-        if (!g.Aord) {
-          k_gather_rows<<<gb, 256, 0, H.stream>>>(dir == 0 ? H.source.p : H.raddo.p, H.heavy.p, H.nheavy, rowlen,
-                                                   dir == 0 ? H.src_c.p : H.rad_c.p);
+        // (the source rows are already packed: launch_accelerate)
+        if (dir == 1 && !g.Aord) {
+          k_gather_rows<<<gb, 256, 0, H.stream>>>(H.raddo.p, H.heavy.p, H.nheavy, rowlen, H.rad_c.p);
           CK(cudaGetLastError());
           H.launches += 1;
         }
@@ -4982,6 +5240,7 @@ int shdom_init_solution(shdom_handle *hh) {
     shdom::AccelState st{0.0, 1.0f, 0.0f};
     CK(cudaMemcpyAsync(H.accel.p, &st, sizeof(st), cudaMemcpyHostToDevice, H.stream));
     shdom::launch_source(H, 1, 0);
+    shdom::launch_accelerate(H, true);
     CK(cudaStreamSynchronize(H.stream));
     H.initialized = true;
     H.iters = 0;
@@ -5008,7 +5267,7 @@ int shdom_solution_iterations(shdom_handle *hh, int maxiter, int *iters, float *
     H.ktimes[0] = H.ktimes[1] = 0.f;
     H.klaunches[0] = H.klaunches[1] = 0;
     bool fixsh = false;
-    const int nlm = P.nlm, nang = P.nang;
+    const int nang = P.nang;
     {  // SOLUTION_ITERATIONS starts every call with no acceleration pending
       double zero = 0.0;
       CK(cudaMemcpyAsync(&H.accel.p->a, &zero, sizeof(double), cudaMemcpyHostToDevice, H.stream));
@@ -5038,10 +5297,8 @@ int shdom_solution_iterations(shdom_handle *hh, int maxiter, int *iters, float *
       if (timed) CK(cudaEventRecord(ev[3], H.stream));
       shdom::launch_source(H, 0, fix ? 1 : 0);
       shdom::k_accel_param<<<1, 1, 0, H.stream>>>(H.red.p, H.accel.p, P.prob.accelflag);
-      H.launches += 2;
-      int blocks = (int)std::min<size_t>(((size_t)P.npts * H.nst * nlm + 255) / 256, 152 * 64);
-      shdom::k_accelerate<<<blocks, 256, 0, H.stream>>>(H.source.p, H.delsource.p, H.ns.p, H.nso.p, P.npts, nlm, H.accel.p,
-                                                        H.nst);
+      H.launches += 1;
+      shdom::launch_accelerate(H, false);
     };
     const bool graphed = H.sweep_mode == 2;
     while (H.iters < maxiter && H.solcrit > P.prob.solacc) {
