@@ -94,9 +94,10 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr) {
   d |= (uint64_t)2 << 61;            // 128-byte swizzle
   return d;
 }
-__device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
-  asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p; }" ::"r"(dtmem),
-               "l"(a), "l"(b), "r"(idesc), "r"(accum));
+// A from tensor memory (row i of the tile in lane i, one element per column), B by descriptor.
+__device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accum) {
+  asm volatile("{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p; }" ::"r"(dtmem),
+               "r"(a), "l"(b), "r"(idesc), "r"(accum));
 }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -110,6 +111,15 @@ __device__ __forceinline__ void tmem_ld16(uint32_t ta, uint32_t *r) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(ta));
+}
+// 16 registers of each lane into 16 columns of this warp's 32 tensor-memory
+// lanes (async; complete after tcgen05.wait::st).
+__device__ __forceinline__ void tmem_st16(uint32_t ta, const uint32_t *r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(ta)
+      : "memory");
 }
 // Orders later uses of 16 registers after the preceding volatile asm (the wait).
 __device__ __forceinline__ void reg_fence16(uint32_t *r) {
@@ -133,10 +143,10 @@ __device__ __forceinline__ void reg_fence16(uint32_t *r) {
 //   warp 1 lane 0  MMA issuer: the chunk's 3 (or 1) x BK/8 tcgen05.mma into a
 //                  FRESH accumulator (tensor-memory buffer g % 2, BN columns);
 //                  warp 1 also owns the tensor-memory allocation;
-//   warps 2..5     split: one row of the chunk per thread, into TF32 high (in
-//                  place) and low parts (and, for the ordinate-to-harmonic
-//                  direction, the row's ordinates into the two hemispheric
-//                  flux sums in FP32);
+//   warps 2..5     split: one row of the chunk per thread, into TF32 high and
+//                  low parts in tensor memory, from where the MMA takes them
+//                  (and, for the ordinate-to-harmonic direction, the row's
+//                  ordinates into the two hemispheric flux sums in FP32);
 //   warps 6..13    accumulate: read chunk g's partial product from tensor
 //                  memory and add it into FP32 registers (each thread: one
 //                  row, half of the BN columns); after a tile's last chunk,
@@ -144,16 +154,30 @@ __device__ __forceinline__ void reg_fence16(uint32_t *r) {
 //                  next tile).
 // Summing the per-chunk partial products on the CUDA cores (round to
 // nearest) keeps the tensor-core accumulation chains 32 K-elements long.
+//
+// What bounds it: the results' stores and the chain load - split - products -
+// sum of a chunk; the tensor cores are busy 15-30% of the time.  A's parts lie
+// in tensor memory (64 columns a stage beside the two accumulators), which
+// takes their writes and the products' reads of A off shared memory and leaves
+// room for a fourth stage of B; a lane's results of mode 1, neighbouring
+// columns of its own row, go out 16 bytes at a time.  Measured against A's
+// parts in shared memory and 4-byte stores of those results: harmonics from
+// ordinates 1.17 -> 0.84 ms (128x128x64, 512 ordinates, 30% cloud), 0.35 ->
+// 0.20 ms (64x64x40, I, Q, U), 88 -> 50 us (45x37x29, 12 x 24 ordinates);
+// ordinates from harmonics 0.66 -> 0.58 ms, 0.17 -> 0.16, 46 -> 34 us.
 template <int BN, bool KM>
 struct Cfg {
   static constexpr int HALF = BN / 2;
   static constexpr int A_BYTES = BM * BK * 4, B_BYTES = BN * BK * 4;
-  static constexpr int STAGE = 2 * A_BYTES + 2 * B_BYTES;
+  static constexpr int STAGE = (KM ? 0 : A_BYTES) + 2 * B_BYTES;
   static constexpr int kFluxTab = 16 * 1024;  // down and up flux weights, K padded to 32 (K <= 2048)
   static constexpr int RAW = 4, kRaw = KM ? RAW * A_BYTES : 0;  // raw A tiles (KM)
   static constexpr int kRoom = (227 * 1024 - 2048 - kFluxTab - kRaw) / STAGE;
   static constexpr int S = kRoom > 4 ? 4 : kRoom;
-  static constexpr uint32_t TCOLS = 2 * BN <= 256 ? 256u : 512u;
+  // tensor memory: two accumulators, then S stages of A (high and low parts, BK columns each)
+  static constexpr int ACOL = 256, ASTAGE = 2 * BK;
+  static constexpr uint32_t TCOLS = 512;
+  static_assert(2 * BN <= ACOL && ACOL + S * ASTAGE <= 512, "tensor memory");
   static constexpr size_t smem() { return (size_t)S * STAGE + 256 + kFluxTab + kRaw + 1024; }
 };
 constexpr int kThreads = 448;
@@ -179,6 +203,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
                                                          int ntiles, Epilogue g) {
   using C = Cfg<BN, KM>;
   constexpr int S = C::S, HALF = C::HALF, A_BYTES = C::A_BYTES, B_BYTES = C::B_BYTES, STAGE = C::STAGE;
+  constexpr int BOFF = KM ? 0 : A_BYTES;  // a stage: A as loaded (not KM), B high, B low
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base0 = saddr(smem_raw);
   const uint32_t pad = (1024u - (base0 & 1023u)) & 1023u;
@@ -241,8 +266,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
         const uint32_t st = sbase + s * STAGE;
         mbar_expect_tx(full0 + 8 * s, (KM ? 0 : A_BYTES) + 2 * B_BYTES);
         if (!KM) tma_load(st, &tmA, full0 + 8 * s, kx, m0);
-        tma_load(st + 2 * A_BYTES, &tmBh, full0 + 8 * s, kx, n0);
-        tma_load(st + 2 * A_BYTES + B_BYTES, &tmBl, full0 + 8 * s, kx, n0);
+        tma_load(st + BOFF, &tmBh, full0 + 8 * s, kx, n0);
+        tma_load(st + BOFF + B_BYTES, &tmBl, full0 + 8 * s, kx, n0);
         issued = gc + 1;
       }
       // Every load issued has landed before the shared memory is released:
@@ -261,15 +286,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
       for (int gc = 0; gc < G; ++gc) {
         const int s = gc % S, b = gc & 1;
         if (*abort_flag) break;
+        if (KM && !mbar_wait(full0 + 8 * s, (gc / S) & 1, g.wait_limit)) { *abort_flag = 1; break; }
         if (!mbar_wait(split0 + 8 * s, (gc / S) & 1, g.wait_limit)) { *abort_flag = 1; break; }
         if (gc >= 2 && !mbar_wait(acce0 + 8 * b, ((gc >> 1) - 1) & 1, g.wait_limit)) { *abort_flag = 1; break; }
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t st = sbase + s * STAGE, dt = tmem + (uint32_t)(b * BN);
+        const uint32_t at = tmem + (uint32_t)(C::ACOL + s * C::ASTAGE);
 #pragma unroll
         for (int ks = 0; ks < BK / 8; ++ks) {
           const uint32_t off = ks * 32;  // 8 tf32 elements
-          const uint64_t dah = sdesc(st + off), dal = sdesc(st + A_BYTES + off);
-          const uint64_t dbh = sdesc(st + 2 * A_BYTES + off), dbl = sdesc(st + 2 * A_BYTES + B_BYTES + off);
+          const uint32_t dah = at + ks * 8, dal = dah + BK;
+          const uint64_t dbh = sdesc(st + BOFF + off), dbl = sdesc(st + BOFF + B_BYTES + off);
           if (g.split) {
             // small terms first, while the fresh accumulator is small
             mma_tf32(dt, dal, dbh, idesc, ks > 0 ? 1u : 0u);
@@ -289,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
     }
   } else if (warp < 6) {
     // ---------------------------------------------------------- split
-    const int srow = tid - 64;  // 0..127
+    const int srow = (warp & 3) * 32 + lane;  // a warp reaches the tensor-memory lanes of its number mod 4
     const int swz = srow & 7;
     float fd = 0.f, fu = 0.f;
     bool flux = false;
@@ -312,13 +339,20 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
         }
         const float *ap = arow_pt >= 0 ? g.Aord + (size_t)(c * BK) * g.acs + arow_pt : g.Aord;
         const int kn = arow_pt >= 0 ? min(BK, K - c * BK) : 0;
-        uint32_t d = saddr(raw + (gc % RAW) * (BK * BM));
+        const uint32_t d = saddr(raw + (gc % RAW) * (BK * BM));
+        if (kn == BK) {
 #pragma unroll
-        for (int u = 0; u < BK; ++u) {
-          const bool in = u < kn;
-          asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + u * (BM * 4)),
-                       "l"(in ? ap + (size_t)u * g.acs : g.Aord), "r"(in ? 4 : 0)
-                       : "memory");
+          for (int u = 0; u < BK; ++u) {
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + u * (BM * 4)), "l"(ap) : "memory");
+            ap += g.acs;
+          }
+        } else {  // the last chunk of a row, or a row past the end: zero fill
+          for (int u = 0; u < BK; ++u) {
+            const bool in = u < kn;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d + u * (BM * 4)),
+                         "l"(in ? ap + (size_t)u * g.acs : g.Aord), "r"(in ? 4 : 0)
+                         : "memory");
+          }
         }
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
@@ -336,23 +370,37 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
           v[u] = make_float4(rw[(4 * u) * BM], rw[(4 * u + 1) * BM], rw[(4 * u + 2) * BM], rw[(4 * u + 3) * BM]);
         fetch(gc + RAW - 1);  // into the tile read a chunk ago
       }
-      const bool go = !*abort_flag && mbar_wait(full0 + 8 * s, (gc / S) & 1, g.wait_limit);
+      // A's place in tensor memory is free once the stage's last products are
+      // done: the loads of a later chunk have waited for that; KM, which takes A
+      // past them, waits itself while B is on its way
+      bool go = !*abort_flag;
+      if (!KM) go = go && mbar_wait(full0 + 8 * s, (gc / S) & 1, g.wait_limit);
+      else if (gc >= S) go = go && mbar_wait(empty0 + 8 * s, ((gc / S) - 1) & 1, g.wait_limit);
       if (!__all_sync(0xffffffffu, go)) { *abort_flag = 1; break; }
-      uint8_t *arow = smem + s * STAGE + (srow >> 3) * 1024 + swz * 128;
       if (!KM) {
+        // u is the logical 16-byte unit of the row; (u ^ swz) its place in the 128-byte swizzle row
+        const uint8_t *arow = smem + s * STAGE + (srow >> 3) * 1024 + swz * 128;
 #pragma unroll
         for (int u = 0; u < 8; ++u) v[u] = *reinterpret_cast<const float4 *>(arow + ((u ^ swz) << 4));
       }
+      if (KM || gc >= S) asm volatile("tcgen05.fence::after_thread_sync;");
+      const uint32_t at = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(C::ACOL + s * C::ASTAGE);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        // u is the logical 16-byte unit of the row; (u ^ swz) its place in the 128-byte swizzle row
-        float4 h, l;
-        h.x = tf32_rna_bits(v[u].x); l.x = tf32_rna_bits(v[u].x - h.x);
-        h.y = tf32_rna_bits(v[u].y); l.y = tf32_rna_bits(v[u].y - h.y);
-        h.z = tf32_rna_bits(v[u].z); l.z = tf32_rna_bits(v[u].z - h.z);
-        h.w = tf32_rna_bits(v[u].w); l.w = tf32_rna_bits(v[u].w - h.w);
-        *reinterpret_cast<float4 *>(arow + ((u ^ swz) << 4)) = h;
-        *reinterpret_cast<float4 *>(arow + A_BYTES + ((u ^ swz) << 4)) = l;
+      for (int hf = 0; hf < 2; ++hf) {
+        uint32_t h[16], l[16];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const float4 q = v[4 * hf + u];
+          const float x[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float hi = tf32_rna_bits(x[e]);
+            h[4 * u + e] = __float_as_uint(hi);
+            l[4 * u + e] = __float_as_uint(tf32_rna_bits(x[e] - hi));
+          }
+        }
+        tmem_st16(at + 16 * hf, h);
+        tmem_st16(at + BK + 16 * hf, l);
       }
       if (flux) {
         // down / up weights of the chunk's 32 ordinates (zero past K): broadcast reads
@@ -365,7 +413,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
           fu = fmaf(b.x, v[u].x, fu); fu = fmaf(b.y, v[u].y, fu); fu = fmaf(b.z, v[u].z, fu); fu = fmaf(b.w, v[u].w, fu);
         }
       }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;");
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(split0 + 8 * s) : "memory");
       if (flux && c == KB - 1) {
@@ -399,17 +448,19 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
       if (!__all_sync(0xffffffffu, go)) { *abort_flag = 1; break; }
       asm volatile("tcgen05.fence::after_thread_sync;");
       const uint32_t ta = tmem + ((uint32_t)(lg * 32) << 16) + (uint32_t)(b * BN + half * HALF);
-      // two loads in flight per wait
+      // two loads in flight per wait where the registers allow it (at BN = 128
+      // the sums take 64 of a thread's 128)
+      constexpr int LD = HALF > 48 ? 16 : 32;
 #pragma unroll
-      for (int c0 = 0; c0 < HALF; c0 += 32) {
-        uint32_t r[32];
+      for (int c0 = 0; c0 < HALF; c0 += LD) {
+        uint32_t r[LD];
         tmem_ld16(ta + (uint32_t)c0, r);
-        if (c0 + 16 < HALF) tmem_ld16(ta + (uint32_t)(c0 + 16), r + 16);
+        if (LD > 16 && c0 + 16 < HALF) tmem_ld16(ta + (uint32_t)(c0 + 16), r + LD - 16);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         reg_fence16(r);
-        if (c0 + 16 < HALF) reg_fence16(r + 16);
+        if (LD > 16 && c0 + 16 < HALF) reg_fence16(r + LD - 16);
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
+        for (int j = 0; j < LD; ++j)
           if (c0 + j < HALF) acc[c0 + j] += __uint_as_float(r[j]);
       }
       asm volatile("tcgen05.fence::before_thread_sync;");
@@ -424,11 +475,15 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
           const int cb = n0 + half * HALF;
           if (g.mode == 0 && g.ccs) {
             // ordinate-major: a warp's rows are consecutive (or nearly), so each column is one line
-            float *out = g.C + row;
+            float *out = g.C + (size_t)cb * g.ccs + row;
+            const int nc = g.N - cb;
+            if (!g.stk && nc >= HALF) {
 #pragma unroll
-            for (int j = 0; j < HALF; ++j) {
-              const int col = cb + j;
-              if (col < g.N) out[(size_t)col * g.ccs] = g.stk && g.stk[col] ? acc[j] : fmaxf(acc[j], 0.f);
+              for (int j = 0; j < HALF; ++j, out += g.ccs) *out = fmaxf(acc[j], 0.f);
+            } else {
+#pragma unroll
+              for (int j = 0; j < HALF; ++j, out += g.ccs)
+                if (j < nc) *out = g.stk && g.stk[cb + j] ? acc[j] : fmaxf(acc[j], 0.f);
             }
           } else if (g.mode == 0) {
             float *out = g.C + (size_t)row * g.ldc;
@@ -452,13 +507,27 @@ __global__ void __launch_bounds__(kThreads, 1) k_tc_gemm(const __grid_constant__
               }
             }
           } else {
-            const int nrp = g.nr[row];
-            float *out = g.R + (size_t)row * (g.ldr ? g.ldr : g.nlm);
+            const int nrp = g.nr[row], ldr = g.ldr ? g.ldr : g.nlm;
+            float *out = g.R + (size_t)row * ldr + cb;
+            int jt = cb < g.nlm ? cb : cb % g.nlm;
+            // a lane's columns are consecutive but its neighbours' are a row away:
+            // as many bytes per store as the rows' alignment allows
+            const bool wide = (ldr & 3) == 0;
 #pragma unroll
-            for (int j = 0; j < HALF; ++j) {
-              const int col = cb + j;
-              const int jt = col < g.nlm ? col : col % g.nlm;
-              if (col < g.N) out[col] = (jt < nrp) ? acc[j] : 0.f;
+            for (int j = 0; j < HALF; j += 4) {
+              float v[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                v[e] = jt < nrp ? acc[j + e] : 0.f;
+                if (++jt == g.nlm) jt = 0;
+              }
+              if (wide && cb + j + 3 < g.N) {
+                *reinterpret_cast<float4 *>(out + j) = make_float4(v[0], v[1], v[2], v[3]);
+              } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                  if (cb + j + e < g.N) out[j + e] = v[e];
+              }
             }
           }
         }
