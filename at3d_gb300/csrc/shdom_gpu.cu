@@ -356,20 +356,6 @@ __device__ __forceinline__ Trace reg_trace(const RegLoad &x, int b, int pt_unuse
   return t;
 }
 
-__device__ __forceinline__ Trace trace_regular(const SweepArgs &a, int b, int pt, int col) {
-  RegLoad x;
-  reg_load(a, b, pt, col, x, false);
-  Trace t = reg_trace(x, b, pt);
-  const int iface = (int)x.g.w;
-  const int ox = (b & 1) ? -a.nz * a.ny1 : a.nz * a.ny1, oy = (b & 2) ? -a.nz : a.nz, oz = (b & 4) ? -1 : 1;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int d = c_face[iface][k] ^ b;
-    t.q[k] = pt + ((d & 1) ? ox : 0) + ((d & 2) ? oy : 0) + ((d & 4) ? oz : 0);
-  }
-  return t;
-}
-
 // Exit of a backward trace from (xe, ye, ze) through one cell of a 3D grid
 // (the geometry step of BACK_INT_GRID3D): the face's four corners, the next
 // cell, the path length and the bilinear face coordinates; the position is
@@ -447,7 +433,11 @@ __device__ __forceinline__ IrrRec trace_geom1(const SweepArgs &a, int b, int cls
 
 // General trace (any point); with use_level the level of the ordinate's
 // face class must also precede the point's (level-synchronous execution).
-__device__ __forceinline__ Trace trace_general(const SweepArgs &a, int b, int cls, int pt, int col, bool use_level) {
+// NST columns of one direction, dc apart (I, Q, U: the first is I), share
+// the cell walk; rs holds each column's radsrc (t.radsrc is the first's).
+template <int NST>
+__device__ __forceinline__ Trace trace_general(const SweepArgs &a, int b, int cls, int pt, int col, int dc, bool use_level,
+                                               float *rs) {
   Trace t;
   t.radsrc = 0.f; t.tr = 1.f; t.status = ERR_SWEEP_STEPS; t.u = 0.f; t.v = 0.f;
   t.q[0] = t.q[1] = t.q[2] = t.q[3] = pt; t.f[0] = t.f[1] = t.f[2] = t.f[3] = 0.f;
@@ -461,9 +451,10 @@ __device__ __forceinline__ Trace trace_general(const SweepArgs &a, int b, int cl
   int cell = a.start[(size_t)b * n + pt];
   float xe = a.gridpos[3 * pt], ye = a.gridpos[3 * pt + 1], ze = a.gridpos[3 * pt + 2];
   float ext1 = a.text[pt];
-  float srcext1 = ext1 * a.srcdo[a.at(pt, col)];
-  float rad = 0.f, tr = 1.f;
-  const bool clamp = !a.stk || !a.stk[col];
+  float srcext1[NST], rad[NST], tr = 1.f;
+#pragma unroll
+  for (int st = 0; st < NST; ++st) { srcext1[st] = ext1 * a.srcdo[a.at(pt, col + st * dc)]; rad[st] = 0.f; rs[st] = 0.f; }
+  const bool clamp0 = !a.stk || !a.stk[col];
   for (int guard = 0; guard < 65536; ++guard) {
     if (cell < 0) break;
     const int *g = a.gridptr + 8 * (size_t)cell;
@@ -487,16 +478,24 @@ __device__ __forceinline__ Trace trace_general(const SweepArgs &a, int b, int cl
     }
     const float e1 = a.text[i1], e2 = a.text[i2], e3 = a.text[i3], e4 = a.text[i4];
     const float ext0 = f1 * e1 + f2 * e2 + f3 * e3 + f4 * e4;
-    const float srcext0 = f1 * a.srcdo[a.at(i1, col)] * e1 + f2 * a.srcdo[a.at(i2, col)] * e2 +
-                          f3 * a.srcdo[a.at(i3, col)] * e3 + f4 * a.srcdo[a.at(i4, col)] * e4;
-    float radsrc, transcell;
-    cell_source(ext0, srcext0, ext1, srcext1, so, radsrc, transcell, clamp);
-    rad += tr * radsrc;
+    float transcell = 1.f;
+#pragma unroll
+    for (int st = 0; st < NST; ++st) {
+      const int cl = col + st * dc;
+      const float srcext0 = f1 * a.srcdo[a.at(i1, cl)] * e1 + f2 * a.srcdo[a.at(i2, cl)] * e2 +
+                            f3 * a.srcdo[a.at(i3, cl)] * e3 + f4 * a.srcdo[a.at(i4, cl)] * e4;
+      float radsrc;
+      cell_source(ext0, srcext0, ext1, srcext1[st], so, radsrc, transcell, st == 0 && clamp0);
+      rad[st] += tr * radsrc;
+      srcext1[st] = srcext0;
+    }
     tr *= transcell;
     auto ok = [&](int q) { return (a.bnd[q] & hb) || (rk[q] < rP && (!use_level || lv[q] < lP)); };
     const bool valid = ok(i1) && ok(i2) && ok(i3) && ok(i4);
     if (nxt < 0 || (tr <= a.transmin && valid)) {
-      t.radsrc = rad; t.tr = tr;
+#pragma unroll
+      for (int st = 0; st < NST; ++st) rs[st] = rad[st];
+      t.radsrc = rad[0]; t.tr = tr;
       t.q[0] = i1; t.q[1] = i2; t.q[2] = i3; t.q[3] = i4;
       t.f[0] = f1; t.f[1] = f2; t.f[2] = f3; t.f[3] = f4;
       t.u = fu; t.v = fv;
@@ -504,15 +503,48 @@ __device__ __forceinline__ Trace trace_general(const SweepArgs &a, int b, int cl
       if (!valid) t.tr = 0.f;
       return t;
     }
-    ext1 = ext0; srcext1 = srcext0; cell = nxt;
+    ext1 = ext0; cell = nxt;
   }
   t.radsrc = 0.f; t.tr = 0.f;
   return t;
 }
 
-__device__ __forceinline__ Trace trace_point(const SweepArgs &a, int b, int pt, int col) {
-  if (a.regular[(size_t)b * a.npts + pt]) return trace_regular(a, b, pt, col);
-  return trace_general(a, b, 3, pt, col, false);
+// Trace of any point, in no order but the reference's: as trace_general,
+// with regular points by their table.
+template <int NST>
+__device__ __forceinline__ Trace trace_point(const SweepArgs &a, int b, int pt, int col, int dc, float *rs) {
+  if (!a.regular[(size_t)b * a.npts + pt]) return trace_general<NST>(a, b, 3, pt, col, dc, false, rs);
+  RegLoad x;
+  reg_load(a, b, pt, col, x, false);
+  const int iface = (int)x.g.w;
+  const int ox = (b & 1) ? -a.nz * a.ny1 : a.nz * a.ny1, oy = (b & 2) ? -a.nz : a.nz, oz = (b & 4) ? -1 : 1;
+  int q[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int d = c_face[iface][k] ^ b;
+    q[k] = pt + ((d & 1) ? ox : 0) + ((d & 2) ? oy : 0) + ((d & 4) ? oz : 0);
+  }
+  float s[NST][5];  // the other columns' sources
+#pragma unroll
+  for (int st = 1; st < NST; ++st) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s[st][k] = __ldg(a.srcdo + a.at(q[k], col + st * dc));
+    s[st][4] = __ldg(a.srcdo + a.at(pt, col + st * dc));
+  }
+  Trace t = reg_trace(x, b, pt);
+  rs[0] = t.radsrc;
+#pragma unroll
+  for (int st = 1; st < NST; ++st) {
+    RegLoad y = x;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) y.s[k] = s[st][k];
+    y.s1 = s[st][4];
+    y.clamp = false;
+    rs[st] = reg_trace(y, b, pt).radsrc;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) t.q[k] = q[k];
+  return t;
 }
 
 // Level-synchronous sweep of one hemisphere in three parts.
@@ -586,7 +618,8 @@ __global__ void __launch_bounds__(256) k_sweep_prep_irr(SweepArgs a, const Seg *
       const Trace t = reg_trace(x, g.b, pt);
       out = make_float2(t.radsrc, t.tr);
     } else {
-      const Trace t = trace_general(a, g.b, g.cls, pt, col, true);
+      float rs[1];
+      const Trace t = trace_general<1>(a, g.b, g.cls, pt, col, 0, true, rs);
       if (t.status != ERR_NONE) atomicCAS(a.err, ERR_NONE, t.status);
       out = make_float2(t.radsrc, t.tr);
       IrrRec r;
@@ -691,7 +724,8 @@ __global__ void __launch_bounds__(P1_THREADS) k_sweep_p1(SweepArgs a, const Seg 
         rad = t.radsrc;
         if (t.tr != 0.f) rad += t.tr * (t.f[0] * y.r[0] + t.f[1] * y.r[1] + t.f[2] * y.r[2] + t.f[3] * y.r[3]);
       } else {
-        const Trace t = trace_general(a, g.b, g.cls, pt, col, true);
+        float rs[1];
+      const Trace t = trace_general<1>(a, g.b, g.cls, pt, col, 0, true, rs);
         if (t.status != ERR_NONE) atomicCAS(a.err, ERR_NONE, t.status);
         rad = t.radsrc;
         if (t.tr != 0.f)
@@ -733,7 +767,8 @@ __global__ void __launch_bounds__(256) k_p1_prep(SweepArgs a, const Seg *__restr
       t = reg_trace(x, g.b, pt);
       t.q[0] = rec.q.x; t.q[1] = rec.q.y; t.q[2] = rec.q.z; t.q[3] = rec.q.w;
     } else {
-      t = trace_general(a, g.b, g.cls, pt, col, true);
+      float rs[1];
+      t = trace_general<1>(a, g.b, g.cls, pt, col, 0, true, rs);
       if (t.status != ERR_NONE) atomicCAS(a.err, ERR_NONE, t.status);
     }
     TraceRec r;
@@ -864,7 +899,8 @@ __global__ void __launch_bounds__(256) k_p1_prep_c(SweepArgs a, const P1Col *__r
       t = reg_trace(x, C.b, pt);
       t.q[0] = rec.q.x; t.q[1] = rec.q.y; t.q[2] = rec.q.z; t.q[3] = rec.q.w;
     } else {
-      t = trace_general(a, C.b, C.cls, pt, col, true);
+      float rs[1];
+      t = trace_general<1>(a, C.b, C.cls, pt, col, 0, true, rs);
       if (t.status != ERR_NONE) atomicCAS(a.err, ERR_NONE, t.status);
     }
     const float f[4] = {(1.f - t.u) * (1.f - t.v), (1.f - t.u) * t.v, t.u * (1.f - t.v), t.u * t.v};
@@ -1521,7 +1557,9 @@ constexpr double kMarchRow = 33, kMarchPlane = 184, kMarchIdle = 20, kMarchIpc =
 // cycles, 18 to 20 runs a window).  Measured per hemisphere, against one
 // thread walking item by item: 32x32x24 with 45 ordinates 0.177 against
 // 1.175 ms, 64x64x40 with 135 columns (I, Q, U) 0.97 against 7.57 ms; the
-// records 0.08 against 0.13 and 1.1 against 2.2 ms.  Tried: the rank order
+// records 0.08 against 0.13 and 0.74 against 2.2 ms (one thread per column:
+// 1.14; most of it is the cell walks at the wrap-around).  Tried: two items
+// per lane, runs of up to 64 (1.18 ms at 64x64x40); the rank order
 // with a scan of (v_(i-1), v_(i-2)) pairs for the interleaved rows (0.45 ms
 // at 32x32x24: 12 dependent steps a run) and with one late item per run
 // added afterwards (0.53 ms).
@@ -1549,37 +1587,53 @@ __device__ __forceinline__ int seq_point(const SweepArgs &a, int b, int r, const
 // Whether every corner of the hemisphere's traces comes earlier in the lex walk (bad counts those that do not).
 __global__ void __launch_bounds__(256) k_seq_check(SweepArgs a, const int *__restrict__ col_oct, int col_begin, int *bad) {
   const int col = col_begin + blockIdx.y;
-  if (a.col_cz[col] == 0.f) return;
+  if (a.col_cz[col] == 0.f || (a.stk && a.stk[col])) return;  // Q and U go the ways of I
   const int b = __ldg(col_oct + col) - 1, hb = (b & 4) ? 2 : 1;
   for (int pt = blockIdx.x * blockDim.x + threadIdx.x; pt < a.npts; pt += gridDim.x * blockDim.x) {
     if (a.bnd[pt] & hb) continue;
-    const Trace t = trace_point(a, b, pt, col);
+    float rs[1];
+    const Trace t = trace_point<1>(a, b, pt, col, 0, rs);
     const int r = seq_place(a, b, pt, true);
     for (int k = 0; k < 4; ++k)
       if (!(a.bnd[t.q[k]] & hb) && t.f[k] != 0.f && seq_place(a, b, t.q[k], true) >= r) atomicAdd(bad, 1);
   }
 }
 
+// One thread per direction and point: the NST columns of a direction (I, Q,
+// U) share their cells, faces and places.  A group of n directions has its n
+// columns of I, then of Q, then of U.
+template <int NST>
 __global__ void __launch_bounds__(256) k_seq_prep(SweepArgs a, const int *__restrict__ col_oct, int col_begin, int lex,
                                                    TraceRec *__restrict__ rec) {
   const int n = a.npts;
   const int col = col_begin + blockIdx.y;
   if (a.col_cz[col] == 0.f) return;  // padding ordinate
+  int dc = 0;
+  if (NST > 1) {
+    if (a.stk[col]) return;
+    int lo = col, hi = col;
+    while (lo > col_begin && a.stk[lo - 1] == 0) --lo;
+    while (hi < a.nang && a.stk[hi] == 0) ++hi;
+    dc = hi - lo;
+  }
   const int b = __ldg(col_oct + col) - 1, hb = (b & 4) ? 2 : 1;
   TraceRec *crec = rec + (size_t)blockIdx.y * n;
   for (int pt = blockIdx.x * blockDim.x + threadIdx.x; pt < n; pt += gridDim.x * blockDim.x) {
     const int r = seq_place(a, b, pt, lex);
     if (r < 0) continue;
     TraceRec x;
+    float rs[NST];
     if (a.bnd[pt] & hb) {  // preset boundary point: its own value
-      x.radsrc = a.raddo[a.at(pt, col)]; x.tr = 0.f; x.u = 0.f; x.v = 0.f;
+#pragma unroll
+      for (int st = 0; st < NST; ++st) rs[st] = a.raddo[a.at(pt, col + st * dc)];
+      x.tr = 0.f; x.u = 0.f; x.v = 0.f;
       x.q = make_int4(-1, -1, -1, -1);
     } else {
       // a regular trace's corners are upwind neighbours: their places follow from the point's
       const bool near = lex && a.regular[(size_t)b * n + pt];
-      const Trace t = trace_point(a, b, pt, col);
+      const Trace t = trace_point<NST>(a, b, pt, col, dc, rs);
       if (t.status != ERR_NONE) atomicCAS(a.err, ERR_NONE, t.status);
-      x.radsrc = t.radsrc; x.tr = t.tr; x.u = t.u; x.v = t.v;
+      x.tr = t.tr; x.u = t.u; x.v = t.v;
       int iface = 0;
       if (near) {
         const int iz = pt % a.nz, layer = (b & 4) ? iz - 1 : iz;
@@ -1591,7 +1645,8 @@ __global__ void __launch_bounds__(256) k_seq_prep(SweepArgs a, const int *__rest
         const float w = t.tr * t.f[k];
         if (w == 0.f) continue;
         if (a.bnd[t.q[k]] & hb) {
-          x.radsrc += w * a.raddo[a.at(t.q[k], col)];
+#pragma unroll
+          for (int st = 0; st < NST; ++st) rs[st] += w * a.raddo[a.at(t.q[k], col + st * dc)];
         } else if (near) {
           const int dlt = c_face[iface][k] ^ b;
           rq[k] = r - (dlt & 1) - ((dlt & 2) ? a.nx1 : 0) - ((dlt & 4) ? a.nx1 * a.ny1 : 0);
@@ -1602,7 +1657,11 @@ __global__ void __launch_bounds__(256) k_seq_prep(SweepArgs a, const int *__rest
       }
       x.q = make_int4(rq[0], rq[1], rq[2], rq[3]);
     }
-    crec[r] = x;
+#pragma unroll
+    for (int st = 0; st < NST; ++st) {
+      x.radsrc = rs[st];
+      crec[(size_t)st * dc * n + r] = x;
+    }
   }
 }
 
@@ -4908,7 +4967,9 @@ static void sweep_hemisphere(Handle &H, int hemi) {
     const int c0 = hemi ? P.ncol_down : 0, nc = hemi ? P.nang - P.ncol_down : P.ncol_down;
     if (nc > 0) {
       const int lex = H.geom->seq_lex[hemi];
-      k_seq_prep<<<dim3(std::min((P.npts + 255) / 256, H.nsm), nc), 256, 0, H.stream>>>(a, H.col_oct.p, c0, lex, H.seqrec.p);
+      const dim3 grid(std::min((P.npts + 255) / 256, H.nsm), nc);
+      if (H.nst == 3) k_seq_prep<3><<<grid, 256, 0, H.stream>>>(a, H.col_oct.p, c0, lex, H.seqrec.p);
+      else k_seq_prep<1><<<grid, 256, 0, H.stream>>>(a, H.col_oct.p, c0, lex, H.seqrec.p);
       CK(cudaGetLastError());
       k_sweep_seq<<<nc, SEQW, kSeqSmem, H.stream>>>(a, H.col_oct.p, H.order.p, c0, lex, H.seqrec.p);
       CK(cudaGetLastError());
