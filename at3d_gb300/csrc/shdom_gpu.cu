@@ -866,7 +866,8 @@ __global__ void __launch_bounds__(P1_THREADS) k_sweep_p1r(SweepArgs a, const Seg
 //
 // What bounds it: the chain of levels (about 0.25 us each with two columns an
 // SM: 189 levels and 177 columns at 128x128x64 0.116 ms a hemisphere), and for
-// the records the scattered reads of the edge planes (0.25 ms there).  Blocks
+// the records the faces' records and the edge planes' fields (0.17 ms there;
+// with the points in level order, not in memory order, 0.25).  Blocks
 // of several columns with a level's records loaded one level ahead took
 // 0.28 ms at 128x128x64, 0.127 against 0.025 at 64x64x32 and 0.118 against
 // 0.020 at 45x37x29 (12 x 24): few blocks, and a load's latency per level.
@@ -883,15 +884,17 @@ struct __align__(16) P1Rec {
 };
 static_assert(sizeof(P1Rec) == 32, "phase-1 records");
 
-__global__ void __launch_bounds__(256) k_p1_prep_c(SweepArgs a, const P1Col *__restrict__ cols, const int *__restrict__ pts,
-                                                   const int *__restrict__ irr0, const int *__restrict__ p1slot,
-                                                   P1Rec *__restrict__ out) {
+// tasks: a group's (point, first face record, slot), in point order, so that
+// a warp reads the fields along z; a record is a whole sector wherever it goes.
+__global__ void __launch_bounds__(256) k_p1_prep_c(SweepArgs a, const P1Col *__restrict__ cols, const int4 *__restrict__ tasks,
+                                                   const int *__restrict__ p1slot, P1Rec *__restrict__ out) {
   const P1Col C = cols[blockIdx.y];
   const int hb = (C.b & 4) ? 2 : 1, col = C.col;
   const int *slots = p1slot + (size_t)C.grp * a.npts;
-  for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < C.n; s += gridDim.x * blockDim.x) {
-    const int pt = __ldg(pts + C.pt0 + s);
-    const IrrRec rec = a.irr[__ldg(irr0 + C.pt0 + s) + C.cs];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < C.n; i += gridDim.x * blockDim.x) {
+    const int4 task = __ldg(tasks + C.pt0 + i);
+    const int pt = task.x, s = task.z;
+    const IrrRec rec = a.irr[task.y + C.cs];
     Trace t;
     if (rec.g.w > 0.5f) {
       RegLoad x;
@@ -3835,7 +3838,8 @@ struct DevGeom {
   // the general-trace table, the level offsets; [group][point] slot or -1
   bool p1c_built = false, p1c_ok[2] = {false, false};
   DBuf<P1Col> p1cols[2];
-  DBuf<int> p1pts[2], p1irr0[2], p1lev[2], p1slot[2];
+  DBuf<int> p1lev[2], p1slot[2];
+  DBuf<int4> p1tasks[2];
   struct P1Shape { int ncols = 0, threads = 0, depth = 0, maxtask = 0, maxn = 0; long long recs = 0; size_t smem = 0; };
   P1Shape p1shape[2];
   std::mutex mu;  // guards the one-time builds of irr and of the phase-1 tables
@@ -4447,7 +4451,8 @@ static void setup_p1c(Handle &H) {
       const int ng1 = (int)off.size() - 1;
       if (!H.march[h] || ng1 <= 0) continue;
       const std::vector<Seg> &sg = P.p1segs[h];
-      std::vector<int> pts, irr0, lev, slot((size_t)ng1 * P.npts, -1);
+      std::vector<int4> tasks;
+      std::vector<int> lev, slot((size_t)ng1 * P.npts, -1);
       std::vector<P1Col> cols;
       long long rec = 0;
       int maxtask = 1, maxn = 0, maxlev = 0;
@@ -4456,20 +4461,21 @@ static void setup_p1c(Handle &H) {
         if (off[g + 1] == off[g]) continue;
         const Seg &s0 = sg[off[g]];
         P1Col C{};
-        C.b = s0.b; C.cls = s0.cls; C.grp = g; C.pt0 = (int)pts.size(); C.lev0 = (int)lev.size(); C.nlev = off[g + 1] - off[g];
+        C.b = s0.b; C.cls = s0.cls; C.grp = g; C.pt0 = (int)tasks.size(); C.lev0 = (int)lev.size(); C.nlev = off[g + 1] - off[g];
         for (int si = off[g]; si < off[g + 1]; ++si) {
           const Seg &q = sg[si];
           if (q.col0 != s0.col0 || q.ncol != s0.ncol || q.b != s0.b || q.cls != s0.cls) ok = false;
-          lev.push_back((int)pts.size() - C.pt0);
+          lev.push_back((int)tasks.size() - C.pt0);
           for (int t = 0; t < q.ntask; ++t) {
             const int pt = (int)P.tasks[h][q.t0 + t];
-            slot[(size_t)g * P.npts + pt] = (int)pts.size() - C.pt0;
-            pts.push_back(pt);
-            irr0.push_back(q.irr0 + t * q.ncol);
+            const int sl = (int)tasks.size() - C.pt0;
+            slot[(size_t)g * P.npts + pt] = sl;
+            tasks.push_back(make_int4(pt, q.irr0 + t * q.ncol, sl, 0));
           }
           maxtask = std::max(maxtask, q.ntask);
         }
-        C.n = (int)pts.size() - C.pt0;
+        C.n = (int)tasks.size() - C.pt0;
+        std::sort(tasks.begin() + C.pt0, tasks.end(), [](const int4 &x, const int4 &y) { return x.x < y.x; });
         lev.push_back(C.n);
         maxn = std::max(maxn, C.n);
         maxlev = std::max(maxlev, C.nlev);
@@ -4487,8 +4493,7 @@ static void setup_p1c(Handle &H) {
       // the columns with the longest chains first
       std::stable_sort(cols.begin(), cols.end(), [](const P1Col &x, const P1Col &y) { return x.nlev > y.nlev; });
       G.p1cols[h].upload(cols);
-      G.p1pts[h].upload(pts);
-      G.p1irr0[h].upload(irr0);
+      G.p1tasks[h].upload(tasks);
       G.p1lev[h].upload(lev);
       G.p1slot[h].upload(slot);
       G.p1shape[h] = {(int)cols.size(), std::min(512, (std::max(64, maxtask) + 31) / 32 * 32), depth, maxtask, maxn, rec,
@@ -4994,7 +4999,7 @@ static void sweep_hemisphere(Handle &H, int hemi) {
         const DevGeom &G = *H.geom;
         const DevGeom::P1Shape &L = G.p1shape[hemi];
         P1Rec *rec = reinterpret_cast<P1Rec *>(H.p1rec.p);
-        k_p1_prep_c<<<dim3((L.maxn + 255) / 256, L.ncols), 256, 0, H.stream>>>(a, G.p1cols[hemi].p, G.p1pts[hemi].p, G.p1irr0[hemi].p,
+        k_p1_prep_c<<<dim3((L.maxn + 255) / 256, L.ncols), 256, 0, H.stream>>>(a, G.p1cols[hemi].p, G.p1tasks[hemi].p,
                                                                                G.p1slot[hemi].p, rec);
         CK(cudaGetLastError());
         k_sweep_p1c<<<L.ncols, L.threads, L.smem, H.stream>>>(a, G.p1cols[hemi].p, G.p1lev[hemi].p, rec, L.depth, L.maxtask);
