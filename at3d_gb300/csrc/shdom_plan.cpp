@@ -99,16 +99,21 @@ const int kGoodNFFT[256] = {
 
 const int kFace[6][4] = {{0, 2, 4, 6}, {1, 3, 5, 7}, {0, 1, 4, 5}, {2, 3, 6, 7}, {0, 1, 2, 3}, {4, 5, 6, 7}};
 
+// f(b, e) over [0, n) on host threads, at least grain items each: about as
+// many as take 0.1 ms, since starting a thread takes 25 us.  (A medium of
+// 24x24x16 points, all threads for each of its seven passes: 2.5 ms, 1.8 of
+// them for the starts.)
 template <class F>
-void parallel_for(int n, F f) {
-  int nt = std::max(1u, std::min(32u, std::thread::hardware_concurrency()));
-  if (n < 4096 || nt == 1) { f(0, n); return; }
+void parallel_for(int n, int grain, F f) {
+  const int nt = std::min({32, (int)std::max(1u, std::thread::hardware_concurrency()), n / std::max(1, grain)});
+  if (nt < 2) { f(0, n); return; }
   std::vector<std::thread> th;
-  int chunk = (n + nt - 1) / nt;
-  for (int t = 0; t < nt; ++t) {
-    int b = t * chunk, e = std::min(n, b + chunk);
+  const int chunk = (n + nt - 1) / nt;
+  for (int t = 1; t < nt; ++t) {
+    const int b = t * chunk, e = std::min(n, b + chunk);
     if (b < e) th.emplace_back(f, b, e);
   }
+  f(0, std::min(n, chunk));
   for (auto &x : th) x.join();
 }
 
@@ -677,7 +682,7 @@ bool build_medium(const shdom_problem &p, Plan &P) {
   HostVec<float> temp(therm ? npts : 0);  // TEMP of the grid points (TRILIN_INTERP_PROP)
   bool bad = false;
   for (int ipa = 0; ipa < npart; ++ipa) {
-    parallel_for(npts, [&](int b, int e) {
+    parallel_for(npts, 1024, [&](int b, int e) {
       std::vector<std::pair<float, int>> srt(nq);
       for (int ipt = b; ipt < e; ++ipt) {
         float x = P.gridpos[3 * ipt], y = P.gridpos[3 * ipt + 1], z = P.gridpos[3 * ipt + 2];
@@ -746,7 +751,7 @@ bool build_medium(const shdom_problem &p, Plan &P) {
     return f;
   };
   if (p.deltam) {  // per point, the species in order (the additions of the serial loops)
-    parallel_for(npts, [&](int b, int e) {
+    parallel_for(npts, 16384, [&](int b, int e) {
       for (int ipt = b; ipt < e; ++ipt) {
         float s = 0.f;
         for (int ipa = 0; ipa < npart; ++ipa) s += ext[(size_t)ipa * npts + ipt];
@@ -771,7 +776,7 @@ bool build_medium(const shdom_problem &p, Plan &P) {
   if (therm) {
     P.thermal.clear(); P.thermal.resize(npts);      // written for every point below
     P.planckpt.clear(); P.planckpt.resize(npts);
-    parallel_for(npts, [&](int b, int e) {
+    parallel_for(npts, 4096, [&](int b, int e) {
       for (int ipt = b; ipt < e; ++ipt) {
         const float bb = planck_fn(temp[ipt], P.unitc, p.wavelen, p.waveno);
         P.planckpt[ipt] = bb;
@@ -810,7 +815,7 @@ bool build_medium(const shdom_problem &p, Plan &P) {
   // number of single-scatter entries of each point, then (after the prefix
   // sum) the entries themselves
   HostVec<int> tcnt(npts);  // written for every point
-  parallel_for(npts, [&](int pb, int pe) {
+  parallel_for(npts, 1024, [&](int pb, int pe) {
     std::vector<double> ltp(nstleg == 6 ? 3 * nl : 0);
     std::vector<float> ltp1(nstleg == 6 ? 3 * nl : 0);
     std::vector<float> lt1(nleg + 1);
@@ -877,7 +882,7 @@ bool build_medium(const shdom_problem &p, Plan &P) {
   // scattering points: the coefficient row is non-zero exactly when its l = 0 term (the albedo) is
   P.scat.assign(npts, 0);
   // a point has a source when it scatters or (thermal source) emits
-  parallel_for(npts, [&](int b, int e) {
+  parallel_for(npts, 65536, [&](int b, int e) {
     for (int ipt = b; ipt < e; ++ipt)
       P.scat[ipt] = P.coef[(size_t)ipt * nl] != 0.f || (!P.thermal.empty() && P.thermal[ipt] != 0.f);
   });
@@ -885,7 +890,7 @@ bool build_medium(const shdom_problem &p, Plan &P) {
   P.tms_iph.clear(); P.tms_iph.resize(P.tms_ptr[npts]);  // every entry is written below
   P.tms_w.clear(); P.tms_w.resize(P.tms_ptr[npts]);
   // exact single scatter: weight (albedo * ext_ipa / ext) / (1 - f) per phase function
-  parallel_for(npts, [&](int pb, int pe) {
+  parallel_for(npts, 8192, [&](int pb, int pe) {
     for (int ipt = pb; ipt < pe; ++ipt) {
       int w0 = P.tms_ptr[ipt];
       const float etot = P.total_ext[ipt];
@@ -911,7 +916,7 @@ bool build_medium(const shdom_problem &p, Plan &P) {
   const float pif = (float)std::acos(-1.0f);
   const float c0 = std::sqrt(1.0f / pif), c1 = std::sqrt(3.0f / (4 * pif));
   const int ncol = P.nx1 * P.ny1;
-  parallel_for(ncol, [&](int cb, int ce) {
+  parallel_for(ncol, 2048 / nz, [&](int cb, int ce) {
     std::vector<double> lo(2 * nlay + 3), up(2 * nlay + 3), dg(2 * nlay + 3), rhs(2 * nlay + 3);
     std::vector<float> od(nlay), al(nlay), as(nlay);
     for (int col = cb; col < ce; ++col) {
