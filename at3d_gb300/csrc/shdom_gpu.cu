@@ -4198,12 +4198,10 @@ static void setup_tc(Handle &H) {
     H.tc_bh[dir].upload(bh);
     H.tc_bl[dir].upload(bl);
     const float *a = dir == 0 ? H.source.p : H.raddo.p;
-    if (dir == 1 && H.ord_major)  // A does not come by TMA (KM)
-      make_map(&H.tm_a[1], H.source.p, (uint64_t)nsh, (uint64_t)P.npts, (uint64_t)nsh, tc::BM);
-    else
-      make_map(&H.tm_a[dir], a, (uint64_t)K, (uint64_t)P.npts, (uint64_t)lda, tc::BM);
     make_map(&H.tm_bh[dir], H.tc_bh[dir].p, (uint64_t)kpad, (uint64_t)npad, (uint64_t)kpad, (uint32_t)bn);
     make_map(&H.tm_bl[dir], H.tc_bl[dir].p, (uint64_t)kpad, (uint64_t)npad, (uint64_t)kpad, (uint32_t)bn);
+    if (dir == 1 && H.ord_major) H.tm_a[1] = H.tm_bh[1];  // A does not come by TMA (KM): not read
+    else make_map(&H.tm_a[dir], a, (uint64_t)K, (uint64_t)P.npts, (uint64_t)lda, tc::BM);
     H.tc_bn[dir] = bn; H.tc_ntiles[dir] = ntiles; H.tc_kpad[dir] = kpad;
     tc_attr(bn);
     H.tc_ok[dir] = true;
