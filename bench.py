@@ -39,9 +39,9 @@ NWAVE = 4
 # from an ncu capture of that kernel on the 96x96x48 field (2.195 GB for
 # 73.5M point-ordinates).
 LEVELS_DRAM_BYTES_PER_ITEM = 29.9
-# The same for one k_sweep_march launch, from an ncu capture of that kernel
-# on the 96x96x48 field (1.846 GB for 78.3M point-ordinates).
-MARCH_DRAM_BYTES_PER_ITEM = 23.6
+# The same for a hemisphere's two k_sweep_march launches (0.743 GB for the
+# 78.3M point-ordinates of the 96x96x48 field).
+MARCH_DRAM_BYTES_PER_ITEM = 9.5
 
 
 def scenes(args):
@@ -220,7 +220,7 @@ def gb300_arm(args, rank, ws):
         alg = 12.0 * items                     # (radsrc, tr) read + radiance write per point-ordinate
         per_item = LEVELS_DRAM_BYTES_PER_ITEM
         kernel, p1_name, p2_name = "k_sweep_levels", "phase1_and_source_pass", "level_pass"
-    p2_ms = sweep_parts[1] / nsweeps           # mean CUDA-event time of one phase-2 launch
+    p2_ms = sweep_parts[1] / nsweeps           # mean CUDA-event time of one hemisphere's phase 2
     achieved = alg / (p2_ms / 1e3) / 1e9
     # DRAM bytes per launch from ncu (96x96x48 capture, bytes per point-ordinate), scaled
     traffic = per_item * items if per_item else None
