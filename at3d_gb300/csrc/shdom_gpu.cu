@@ -915,14 +915,14 @@ __global__ void __launch_bounds__(256) k_p1_prep_c(SweepArgs a, const P1Col *__r
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       float w = t.tr * f[k];
-      int q = 0;
+      int q = C.n;  // no corner: the slot that stays zero
       if (w != 0.f) {
         if (a.bnd[t.q[k]] & hb) {
           r.radsrc += w * a.raddo[a.at(t.q[k], col)];  // preset: final
           w = 0.f;
         } else {
           q = slots[t.q[k]];
-          if (q < 0 || q >= s) { atomicCAS(a.err, ERR_NONE, ERR_SWEEP_NOFACE); q = 0; w = 0.f; }  // not an earlier phase-1 point of the group
+          if (q < 0 || q >= s) { atomicCAS(a.err, ERR_NONE, ERR_SWEEP_NOFACE); q = C.n; w = 0.f; }  // not an earlier phase-1 point of the group
         }
       }
       r.w[k] = w;
@@ -936,14 +936,14 @@ __global__ void __launch_bounds__(512) k_sweep_p1c(SweepArgs a, const P1Col *__r
                                                    const P1Rec *__restrict__ recs, int depth, int maxtask) {
   extern __shared__ __align__(16) unsigned char p1m[];
   P1Rec *ring = reinterpret_cast<P1Rec *>(p1m);                      // [depth][maxtask]
-  float *val = reinterpret_cast<float *>(ring + (size_t)depth * maxtask);  // [slot]
+  float *val = reinterpret_cast<float *>(ring + (size_t)depth * maxtask);  // [slot], then a zero that nobody writes
   const P1Col C = cols[blockIdx.x];
-  int *lev = reinterpret_cast<int *>(val + C.n);                     // [nlev + 1]
+  int *lev = reinterpret_cast<int *>(val + C.n + 1);                 // [nlev + 1]
   const int tid = threadIdx.x;
   const P1Rec *rec = recs + C.rec;
   float *rado = a.raddo + (size_t)C.col * a.cs;
   for (int i = tid; i <= C.nlev; i += blockDim.x) lev[i] = __ldg(levs + C.lev0 + i);
-  if (tid == 0) val[0] = 0.f;  // read with weight zero
+  if (tid == 0) val[C.n] = 0.f;  // the corners that a record does not have
   __syncthreads();
   auto fetch = [&](int l, int d) {  // this thread's records of level l (an empty group past the last)
     if (l < C.nlev) {
@@ -4491,7 +4491,7 @@ static void setup_p1c(Handle &H) {
       }
       int depth = 0;
       for (int d : {8, 4, 2})
-        if (!depth && 32 * (size_t)d * maxtask + 4 * ((size_t)maxn + maxlev + 1) <= (size_t)maxsm) depth = d;
+        if (!depth && 32 * (size_t)d * maxtask + 4 * ((size_t)maxn + maxlev + 2) <= (size_t)maxsm) depth = d;
       if (!ok || cols.empty() || !depth || maxn > 65535) continue;
       // the columns with the longest chains first
       std::stable_sort(cols.begin(), cols.end(), [](const P1Col &x, const P1Col &y) { return x.nlev > y.nlev; });
@@ -4500,7 +4500,7 @@ static void setup_p1c(Handle &H) {
       G.p1lev[h].upload(lev);
       G.p1slot[h].upload(slot);
       G.p1shape[h] = {(int)cols.size(), std::min(512, (std::max(64, maxtask) + 31) / 32 * 32), depth, maxtask, maxn, rec,
-                      32 * (size_t)depth * maxtask + 4 * ((size_t)maxn + maxlev + 1)};
+                      32 * (size_t)depth * maxtask + 4 * ((size_t)maxn + maxlev + 2)};
       G.p1c_ok[h] = true;
     }
     G.p1c_built = true;
