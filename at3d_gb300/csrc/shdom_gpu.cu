@@ -4503,6 +4503,10 @@ static void setup_p1c(Handle &H) {
                       32 * (size_t)depth * maxtask + 4 * ((size_t)maxn + maxlev + 2)};
       G.p1c_ok[h] = true;
     }
+    // the tables have landed before any handle on this grid launches a kernel
+    // that reads them (a copy from pageable memory may return before its DMA
+    // does, and the handles' non-blocking streams are not ordered after it)
+    CK(cudaStreamSynchronize(cudaStreamLegacy));
     G.p1c_built = true;
   }
   for (int h = 0; h < 2; ++h) H.p1c[h] = G.p1c_ok[h] && H.march[h];
