@@ -4117,6 +4117,29 @@ static void make_map(CUtensorMap *m, const float *base, uint64_t inner, uint64_t
   if (r != CUDA_SUCCESS) throw std::runtime_error("cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
 }
 
+// Lets a kernel be launched with as much dynamic shared memory as the current
+// device has.  The limit belongs to the kernel, not to a call: one that
+// followed each call's size could be lowered by another thread between a
+// call's setting it and its launch.
+template <class F>
+static void allow_smem(F *kernel) {
+  int dev = 0, maxsm = 0;
+  CK(cudaGetDevice(&dev));
+  CK(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  cudaFuncAttributes fa;
+  CK(cudaFuncGetAttributes(&fa, kernel));
+  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm - (int)fa.sharedSizeBytes));
+}
+
+// The kernels whose shared memory goes with a call or a handle, on a new handle's device.
+static void allow_smem_all() {
+  allow_smem(k_render<1, false>); allow_smem(k_render<1, true>);
+  allow_smem(k_render<3, false>); allow_smem(k_render<3, true>);
+  allow_smem(k_levis_adjoint);
+  allow_smem(k_sh_to_do<8>); allow_smem(k_sh_to_do<16>); allow_smem(k_sh_to_do<32>);
+  allow_smem(k_do_to_sh<8>); allow_smem(k_do_to_sh<16>); allow_smem(k_do_to_sh<32>);
+}
+
 // The tensor-core GEMM is instantiated for N tiles of 32..128 columns.
 template <int BN>
 static void tc_attr1() {
@@ -4759,10 +4782,8 @@ static void transforms_launch(Handle &H, int dir) {
   size_t smem = (size_t)P.nlm * (NMU + 1) * sizeof(float) + 8 * sizeof(float) * (dir == 0 ? (size_t)NMU * nm : (size_t)P.nang);
   int blocks = std::min((P.npts + 7) / 8, 152 * 8);
   if (dir == 0) {
-    CK(cudaFuncSetAttribute(k_sh_to_do<NMU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_sh_to_do<NMU><<<blocks, 256, smem, H.stream>>>(x, H.source.p, H.ord_major ? H.xf_rows.p : H.srcdo.p);
   } else {
-    CK(cudaFuncSetAttribute(k_do_to_sh<NMU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     k_do_to_sh<NMU><<<blocks, 256, smem, H.stream>>>(x, H.ord_major ? H.xf_rows.p : H.raddo.p, H.radiance.p);
   }
   CK(cudaGetLastError());
@@ -5187,6 +5208,7 @@ static int create_on_device(std::unique_ptr<shdom_handle> &H, int device, shdom_
     if (device >= 0) CK(cudaSetDevice(device));
     CK(cudaGetDevice(&H->h.device));
     CK(cudaStreamCreateWithFlags(&H->h.stream, cudaStreamNonBlocking));
+    shdom::allow_smem_all();
     shdom::upload_plan(H->h);
     CK(cudaMemsetAsync(H->h.errflag.p, 0, sizeof(int), H->h.stream));
     shdom::build_irr(H->h);
@@ -5489,7 +5511,6 @@ static int render_impl(shdom_handle *hh, int nrays, const float *camx, const flo
     while (warps > 1 && (smem(warps) > 100 * 1024 || (long long)nrays < (long long)warps * shdom::RGRAYS * H.nsm)) warps >>= 1;
     const size_t bytes = smem(warps);
     if (bytes > 220 * 1024) return fail(hh, "render: too many spherical-harmonic terms");
-    CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     const int per = warps * shdom::RGRAYS;
     kernel<<<(nrays + per - 1) / per, warps * 32, bytes, stream>>>(a);
     H.launches += 1;
@@ -5656,7 +5677,6 @@ static void levis_adjoint_device(Handle &H, int nrays, const float *dx, const fl
   constexpr int per = shdom::GWARPS * shdom::GRAYS;  // rays per block
   const int blocks = (nrays + per - 1) / per;
   const size_t smem = sizeof(float) * per * (((P.nlm + 3) & ~3) + 4 + 32);
-  CK(cudaFuncSetAttribute(shdom::k_levis_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   shdom::k_levis_adjoint<<<blocks, shdom::GWARPS * 32, smem, H.stream>>>(G);
   CK(cudaGetLastError());
   shdom::BeamArgs b;

@@ -7,7 +7,7 @@ import threading
 import numpy as np
 import pytest
 
-from at3d_gb300.scenes import cloud_field
+from at3d_gb300.scenes import cloud_field, polarized_blob
 
 pytestmark = pytest.mark.gpu
 
@@ -68,3 +68,42 @@ def test_handles_of_one_grid_created_at_once(rte_cls, shape):
         assert np.array_equal(a["ns"], b["ns"])
         for k in ("radiance", "fluxes"):
             assert relrms(a[k], b[k]) < 1e-6, k
+
+
+@pytest.mark.parametrize("kind", ["render", "render polarized", "gradient", "fp32 transforms"])
+def test_calls_of_different_size_at_once(rte_cls, kind):
+    """Renders, gradients and FP32 transforms need shared memory by their number
+    of terms and rays, less or more than the default limit; threads that launch
+    the same kernels with different needs must each get theirs, call after call."""
+    rng = np.random.default_rng(5)
+    handles, calls = [], []
+    for nmu, nphi, nrays, ncalls in ((32, 32, 2500, 1000), (4, 8, 2, 2500), (32, 32, 3, 1500), (4, 8, 2, 2500)):
+        kw = dict(seed=nmu, nx=7, ny=6, nz=6, nmu=nmu, nphi=nphi, boundary="open")
+        pb = polarized_blob(**kw) if kind == "render polarized" else cloud_field(nleg=128, **kw)
+        nx, ny, _ = pb.shape
+        q = ((rng.uniform(0.1, 0.9, nrays) * nx * pb.delx).astype(np.float32),
+             (rng.uniform(0.1, 0.9, nrays) * ny * pb.dely).astype(np.float32),
+             np.full(nrays, float(pb.zlevels[-1]), np.float32), rng.uniform(0.5, 1.0, nrays), rng.uniform(0.0, 6.0, nrays))
+        w = np.ones(nrays)
+        r = rte_cls.from_problem(pb)
+        if kind == "fp32 transforms":
+            r.set_transform_mode("fp32")
+            ncalls //= 25
+        r.solve(1, verbose=False)
+        handles.append(r)
+
+        def call(r=r, q=q, w=w):
+            if kind == "fp32 transforms":
+                r.solve(2, verbose=False)
+                return r.export_state()["fluxes"]
+            return r.levis_adjoint(q, w) if kind == "gradient" else r.render(*q)
+
+        def repeat(call=call, n=ncalls):
+            first = call()
+            return first, max(relrms(call(), first) for _ in range(n))
+        calls.append((call, repeat))
+    alone = [call() for call, _ in calls]
+    for a, (first, spread) in zip(alone, run_threads([repeat for _, repeat in calls])):
+        assert relrms(first, a) < 1e-6 and spread < 1e-6
+    for r in handles:
+        r.close()
