@@ -4138,6 +4138,7 @@ static void allow_smem_all() {
   allow_smem(k_levis_adjoint);
   allow_smem(k_sh_to_do<8>); allow_smem(k_sh_to_do<16>); allow_smem(k_sh_to_do<32>);
   allow_smem(k_do_to_sh<8>); allow_smem(k_do_to_sh<16>); allow_smem(k_do_to_sh<32>);
+  allow_smem(k_do_to_sh_light_om);  // 64 KB at the 2048 ordinates that setup_tc takes
 }
 
 // The tensor-core GEMM is instantiated for N tiles of 32..128 columns.
