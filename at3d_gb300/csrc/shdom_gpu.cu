@@ -74,8 +74,10 @@ __constant__ int c_face[6][4] = {{0, 2, 4, 6}, {1, 3, 5, 7}, {0, 1, 4, 5}, {2, 3
 // Legendre contraction over l for each azimuthal mode m (CMU1/CMU2) and an
 // azimuthal Fourier synthesis/analysis per zenith angle (CPHI1/CPHI2; the
 // reference's FFT branch is the same linear map).  One warp per point; for
-// the Legendre step lane t handles mode m = t - mm, for the Fourier step the
-// lanes run over azimuths (synthesis) or modes (analysis).
+// the Legendre step lane t handles mode m = t - mm (with more than 32 modes
+// also t + 32), for the Fourier step the lanes run over azimuths (synthesis)
+// or modes (analysis).  The modes m and -m are combined; up to 32 modes the
+// other one's sums come from its lane, else each lane forms both.
 struct XfArgs {
   const float *cmu;      // [nlm][nmu] (CMU1 for sh_to_do, CMU2 for do_to_sh)
   const float *cphi;     // sh_to_do: [nmu][nm][nphi0max] (CPHI1 transposed); do_to_sh: [nmu][nphi0max][nm]
@@ -104,29 +106,32 @@ __global__ void __launch_bounds__(256) k_sh_to_do(XfArgs x, const float *__restr
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-  const bool active = lane < nm;
-  const int m = lane - x.mm, ma = m < 0 ? -m : m;
-  const int partner = active ? 2 * x.mm - lane : lane;
+  const bool one = nm <= 32;
   for (int p = warp; p < x.npts; p += nwarps) {
     const float *Sp = S + (size_t)p * x.nlm;
-    float U[NMU];
+    for (int t = lane; t < ((nm + 31) & ~31); t += 32) {
+      const bool active = t < nm;
+      const int m = t - x.mm, ma = m < 0 ? -m : m;
+      auto legendre = [&](int mode, float *U) {
+        for (int l = ma; l <= x.ml; ++l) {
+          const int j = jindex(l, mode, x.mm);
+          const float sv = Sp[j];
+          const float *c = scmu + j * (NMU + 1);
 #pragma unroll
-    for (int i = 0; i < NMU; ++i) U[i] = 0.f;
-    if (active)
-      for (int l = ma; l <= x.ml; ++l) {
-        const int j = jindex(l, m, x.mm);
-        const float sv = Sp[j];
-        const float *c = scmu + j * (NMU + 1);
+          for (int i = 0; i < NMU; ++i) U[i] = fmaf(c[i], sv, U[i]);
+        }
+      };
+      float U[NMU] = {}, V[NMU] = {};
+      if (active) legendre(m, U);
+      if (!one && active) legendre(-m, V);
 #pragma unroll
-        for (int i = 0; i < NMU; ++i) U[i] = fmaf(c[i], sv, U[i]);
-      }
-#pragma unroll
-    for (int i = 0; i < NMU; ++i) {
-      const float up = __shfl_sync(0xffffffffu, U[i], partner);
-      if (active && i < x.nmu) {
-        const int me = max(0, x.nphi0[i] / 2 - 1);
-        float cs = (m == 0) ? U[i] : (m > 0 ? U[i] + up : U[i] - up);
-        sw[i * nm + lane] = (ma <= me) ? cs : 0.f;
+      for (int i = 0; i < NMU; ++i) {
+        const float up = one ? __shfl_sync(0xffffffffu, U[i], active ? 2 * x.mm - t : t) : V[i];
+        if (active && i < x.nmu) {
+          const int me = max(0, x.nphi0[i] / 2 - 1);
+          float cs = (m == 0) ? U[i] : (m > 0 ? U[i] + up : U[i] - up);
+          sw[i * nm + t] = (ma <= me) ? cs : 0.f;
+        }
       }
     }
     __syncwarp();
@@ -157,9 +162,7 @@ __global__ void __launch_bounds__(256) k_do_to_sh(XfArgs x, const float *__restr
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-  const bool active = lane < nm;
-  const int m = lane - x.mm, ma = m < 0 ? -m : m;
-  const int partner = active ? 2 * x.mm - lane : lane;
+  const bool one = nm <= 32;
   for (int p = warp; p < x.npts; p += nwarps) {
     float fd = 0.f, fu = 0.f;
     for (int c = lane; c < x.nang; c += 32) {
@@ -174,37 +177,41 @@ __global__ void __launch_bounds__(256) k_do_to_sh(XfArgs x, const float *__restr
     }
     if (lane == 0) { x.fluxes[2 * (size_t)p] = fd; x.fluxes[2 * (size_t)p + 1] = fu; }
     __syncwarp();
-    float CS[NMU];
-#pragma unroll
-    for (int i = 0; i < NMU; ++i) {
-      CS[i] = 0.f;
-      if (active && i < x.nmu) {
-        const int n0 = x.nphi0[i], me = max(0, n0 / 2 - 1);
-        if (ma <= me) {
-          const float *c = x.cphi + (size_t)i * x.nphi0max * nm + lane;
-          const int *co = x.col_of + i * x.nphi0max;
-          float s = 0.f;
-          for (int k = 0; k < n0; ++k) s = fmaf(c[k * nm], sr[co[k]], s);
-          CS[i] = s;
-        }
-      }
-    }
     const int nrp = x.nr[p];
     float *Rp = R + (size_t)p * x.nlm;
+    for (int t = lane; t < ((nm + 31) & ~31); t += 32) {
+      const bool active = t < nm;
+      const int m = t - x.mm, ma = m < 0 ? -m : m;
+      auto fourier = [&](int i, int mode) {
+        const int n0 = x.nphi0[i], me = max(0, n0 / 2 - 1);
+        float s = 0.f;
+        if (ma <= me) {
+          const float *c = x.cphi + (size_t)i * x.nphi0max * nm + x.mm + mode;
+          const int *co = x.col_of + i * x.nphi0max;
+          for (int k = 0; k < n0; ++k) s = fmaf(c[k * nm], sr[co[k]], s);
+        }
+        return s;
+      };
+      float CS[NMU];
 #pragma unroll
-    for (int i = 0; i < NMU; ++i) {
-      const float cp = __shfl_sync(0xffffffffu, CS[i], partner);
-      CS[i] = (m == 0) ? CS[i] : (m > 0 ? CS[i] - cp : cp + CS[i]);  // SUMUV(m)
-    }
-    if (active)
-      for (int l = ma; l <= x.ml; ++l) {
-        const int j = jindex(l, m, x.mm);
-        const float *c = scmu + j * (NMU + 1);
-        float v = 0.f;
+      for (int i = 0; i < NMU; ++i) CS[i] = active && i < x.nmu ? fourier(i, m) : 0.f;
 #pragma unroll
-        for (int i = 0; i < NMU; ++i) v = fmaf(c[i], CS[i], v);
-        Rp[j] = (j < nrp) ? v : 0.f;
+      for (int i = 0; i < NMU; ++i) {
+        float cp;
+        if (one) cp = __shfl_sync(0xffffffffu, CS[i], active ? 2 * x.mm - t : t);
+        else cp = active && i < x.nmu ? fourier(i, -m) : 0.f;
+        CS[i] = (m == 0) ? CS[i] : (m > 0 ? CS[i] - cp : cp + CS[i]);  // SUMUV(m)
       }
+      if (active)
+        for (int l = ma; l <= x.ml; ++l) {
+          const int j = jindex(l, m, x.mm);
+          const float *c = scmu + j * (NMU + 1);
+          float v = 0.f;
+#pragma unroll
+          for (int i = 0; i < NMU; ++i) v = fmaf(c[i], CS[i], v);
+          Rp[j] = (j < nrp) ? v : 0.f;
+        }
+    }
     __syncwarp();
   }
 }
