@@ -2797,18 +2797,6 @@ __global__ void __launch_bounds__(256) k_source_pol(SourceArgs a) {
   }
 }
 
-// x added to the pair (hi, lo), hi + lo exact to 48 bits (Knuth's two-sum):
-// the sums over points in a few FP32 operations, since one FP64 operation
-// holds the pipe of an SM for 16 cycles.  The error of such a sum against
-// 64-bit arithmetic is that of its FP32 addends (a point's terms) with pairs
-// as with FP64: 1.4e-8 to 3.2e-8 of the sum of magnitudes over 4 to 400
-// points a lane and 4 to 12 terms, the two within 1.3e-14 of each other.
-__device__ __forceinline__ void two_sum(float &hi, float &lo, float x) {
-  const float s = hi + x, b = s - hi;
-  lo += (hi - (s - b)) + (x - b);
-  hi = s;
-}
-
 // COMPUTE_SOURCE and the next RADIANCE_TRUNCATION as k_source / k_source_pol,
 // for rows of up to 256 terms, a multiple of four: LPP lanes per point (so 16
 // lanes take a row of 64 terms and a warp two points), four consecutive terms
@@ -2821,9 +2809,11 @@ __device__ __forceinline__ void two_sum(float &hi, float &lo, float x) {
 // the list leaves them out where the handle knows them (H.compact).
 //
 // What bounds it: memory (five rows per point).  Measured against a warp per
-// point, every point, FP64 sums: 64x64x32 with 64 terms and 20% cloud 28
-// against 104 us, 128x128x64 with 256 terms and 30% cloud 0.43 against 0.76
-// ms, 64x64x40 with 3 x 64 terms 0.11 against 0.32.
+// point, every point: 64x64x32 with 64 terms and 20% cloud 27 against 104 us,
+// 128x128x64 with 256 terms and 30% cloud 0.44 against 0.76 ms, 64x64x40 with
+// 3 x 64 terms 0.11 against 0.32.  The sums over points are FP64: four
+// conversions and additions a point and lane, hidden behind the rows but for
+// 0.01 ms at 128x128x64 (pairs of FP32 in their place, 48 bits: 0.43).
 template <int NST, int LPP, int NP>
 __global__ void __launch_bounds__(256) k_source_v(SourceArgs a, const int *__restrict__ list, int n) {
   const int lane = threadIdx.x & 31, gl = lane % LPP, sub = lane / LPP;
@@ -2840,7 +2830,7 @@ __global__ void __launch_bounds__(256) k_source_v(SourceArgs a, const int *__res
       lj[s][q] = j < nlm ? a.lofj[j] : 0;
       yv[s][q] = j < nlm ? a.ylmsun[j] : 0.f;
     }
-  float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+  double tot[4] = {0.0, 0.0, 0.0, 0.0};  // over points in FP64, a point's terms in FP32
   const bool trunc = !a.fixsh || a.first;
   for (int i0 = warp * PPW; i0 < n; i0 += nwarps * PPW) {
     const bool on = i0 + sub < n;
@@ -2913,7 +2903,7 @@ __global__ void __launch_bounds__(256) k_source_v(SourceArgs a, const int *__res
     }
     if (on && !a.first)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) two_sum(hi[k], lo[k], sum[k]);
+      for (int k = 0; k < 4; ++k) tot[k] += (double)sum[k];
     int nsnew = nsold, nrnext;
     if (trunc) {
 #pragma unroll
@@ -2955,7 +2945,7 @@ __global__ void __launch_bounds__(256) k_source_v(SourceArgs a, const int *__res
     __shared__ double sred[4][8];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      double t = (double)hi[k] + (double)lo[k];
+      double t = tot[k];
       for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
       if (lane == 0) sred[k][threadIdx.x >> 5] = t;
     }
