@@ -1127,16 +1127,32 @@ struct MarchUnit {
   int grp, col;
 };
 constexpr int MRING = 8;     // halo rows in flight between neighbouring strips
-constexpr int MMAXT = 512;   // threads per CTA at most
+constexpr int MMAXT = 512;   // threads per CTA at most (M_WIDE: twice as many)
 constexpr int MROWS = 16;    // rows per thread at most
 constexpr int MWAIT = tc::kWaitLimit;
 
-constexpr int MDEPTH = 4;    // planes of the x and y classes in flight from memory (a power of two)
+// Where the planes are too large for what M_XY and M_Z keep on the chip (16
+// CTAs of a cluster: about 190 points a side), the march keeps less in flight:
+// one group of layers instead of two (to about 240 a side), then single planes
+// two deep (to about 290).  M_WIDE takes more V positions than MMAXT.  A
+// hemisphere with a class that none of them takes (larger planes, more than
+// 1024 layers) keeps the level schedule, and so does the other.
+enum MarchKind {
+  M_XY,      // x and y classes: planes MDEPTH deep
+  M_Z,       // z class: four layers at a time, two such groups
+  M_Z1,      // z class: one group, loaded when the one before is stored
+  M_PLANES,  // any class: planes two deep
+  M_WIDE     // the same with up to 1024 threads
+};
+constexpr int MDEPTH = 4;    // planes of the x and y classes in flight from memory
+__host__ __device__ constexpr int march_depth(int kind) { return kind == M_XY ? MDEPTH : 2; }
+__host__ __device__ constexpr bool march_layers(int kind) { return kind == M_Z || kind == M_Z1; }
+__host__ __device__ constexpr int march_groups(int kind) { return kind == M_Z ? 2 : 1; }
 
-__host__ __device__ inline size_t march_smem_bytes(int tw, int nv, int nz, bool z) {
+__host__ __device__ inline size_t march_smem_bytes(int tw, int nv, int nz, int kind, bool z) {
   const size_t n1 = (size_t)(tw + 1) * nv, nfix = 2 * (size_t)(tw + nv);
-  return 256 + sizeof(float) * ((z ? 16 * n1 + 8 * nfix + 4 * (size_t)nz : MDEPTH * (2 * n1 + nfix)) + (size_t)MRING * nv + 16 +
-                                2 * (size_t)tw * nv + 4 * n1);
+  return 256 + sizeof(float) * ((march_layers(kind) ? march_groups(kind) * (8 * n1 + 4 * nfix) : march_depth(kind) * (2 * n1 + nfix)) +
+                                (z ? 4 * (size_t)nz : 0) + (size_t)MRING * nv + 16 + 2 * (size_t)tw * nv + 4 * n1);
 }
 
 // One float into another CTA's shared memory, 4 bytes counted on a barrier there.
@@ -1205,12 +1221,14 @@ __device__ __forceinline__ void cell_source_march(float ext0, float se0, float e
   radsrc = src * ab;
 }
 
-template <int RM, bool ZC>
+template <int RM, int KIND>
 __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp &G, int col, unsigned char *msm, int cs, int rank) {
+  constexpr int DEPTH = march_depth(KIND), NG = march_groups(KIND);
+  const bool zc = march_layers(KIND) ? true : KIND == M_XY ? false : G.cls == 2;
   const int nV = G.nV, tw = (G.nU + cs - 1) / cs, w0 = rank * tw, nrow = max(0, min(tw, G.nU - w0));
   const int N = tw * nV, N1 = N + nV, tid = threadIdx.x;
   // shared memory: barriers; the points' own values on their way from memory
-  // (x and y classes: [MDEPTH planes][s, e][tw + 1][nV]; z class: [2 groups]
+  // (planes: [DEPTH planes][s, e][tw + 1][nV]; layers: [NG groups]
   // [s, e][tw + 1][nV][4 layers]) and the final radiances of the fixed points
   // ([..][2 per row, then the two edge rows]); the z class's face geometry;
   // (source x ext, ext) pairs [2][tw + 1][nV], halo ring [MRING][nV],
@@ -1218,9 +1236,9 @@ __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp 
   // a row of fixed points.
   const int nfix = 2 * (tw + nV);
   float *own = reinterpret_cast<float *>(msm + 256);
-  float *ownr = own + (ZC ? 16 : 2 * MDEPTH) * N1;
-  float4 *sgeo = reinterpret_cast<float4 *>(ownr + (ZC ? 8 : MDEPTH) * nfix);
-  float2 *sbuf = reinterpret_cast<float2 *>(sgeo + (ZC ? a.nz : 0)) + 2;
+  float *ownr = own + (march_layers(KIND) ? 8 * NG : 2 * DEPTH) * N1;
+  float4 *sgeo = reinterpret_cast<float4 *>(ownr + (march_layers(KIND) ? 4 * NG : DEPTH) * nfix);
+  float2 *sbuf = reinterpret_cast<float2 *>(sgeo + (zc ? a.nz : 0)) + 2;
   float *halo = reinterpret_cast<float *>(sbuf + 2 * N1) + 4;
   float *rbuf = halo + MRING * nV + 4;
   const uint32_t full0 = (uint32_t)__cvta_generic_to_shared(msm), empty0 = full0 + 8 * MRING;
@@ -1230,7 +1248,7 @@ __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp 
   const int ngrp = blockDim.x / nV, gi = tid / nV, v = tid - gi * nV;
   const int R = (nrow + ngrp - 1) / ngrp, q0 = gi * R;  // rows [q0, q0 + kn) of the strip
   const int kn = gi < ngrp ? max(0, min(R, nrow - q0)) : 0;
-  const int sdv = (G.b & (ZC ? 2 : 4)) ? -1 : 1;        // V offset of the upwind neighbour
+  const int sdv = G.upv;                                // V offset of the upwind neighbour
   // the face fraction along V is u and along U is v, or the other way round;
   // from the stopping face's corners
   const bool vu = G.dv[0] != G.dv[2], vflip = G.dv[0] != 0, uflip = G.du[0] != 0;
@@ -1246,14 +1264,13 @@ __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp 
 #pragma unroll
   for (int j = 0; j < RM; ++j) {
     const int w = w0 + q0 + j, u = G.upu > 0 ? w : G.nU - 1 - w;
-    const bool f = (!ZC && v == G.zfix) || (G.xedge && G.cls != 0 && (u == 0 || u == a.nx1 - 1)) ||
-                   (G.yedge && ((G.cls == 0 && (u == 0 || u == a.ny1 - 1)) || (ZC && (v == 0 || v == a.ny1 - 1))));
+    const bool f = (zc ? G.vedge && (v == 0 || v == nV - 1) : v == G.zfix) || (G.uedge && (u == 0 || u == G.nU - 1));
     fix |= (unsigned)(f && j < kn) << j;
   }
   // where a fixed row's radiance is staged: by row at a fixed V position, else in an edge row
-  const bool vfix = ZC ? G.yedge && (v == 0 || v == a.ny1 - 1) : v == G.zfix;
+  const bool vfix = zc ? G.vedge && (v == 0 || v == nV - 1) : v == G.zfix;
   auto fixslot = [&](int j) {
-    return vfix ? 2 * (q0 + j) + (ZC && v != 0 ? 1 : 0) : 2 * tw + (w0 + q0 + j == 0 ? 0 : nV) + v;
+    return vfix ? 2 * (q0 + j) + (zc && v != 0 ? 1 : 0) : 2 * tw + (w0 + q0 + j == 0 ? 0 : nV) + v;
   };
   const bool pusher = push && q0 == 0 && kn > 0;
   const bool above = from_up && kn > 0 && q0 + kn == nrow;  // the row above this thread's last is the next strip's
@@ -1367,9 +1384,13 @@ __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp 
       p += ustep;
     }
   }
-  if constexpr (!ZC) {
-    weights(load_g(v));
-    cx = fx; cgx = gx; cw = fw; cgw = gw;
+  if constexpr (!march_layers(KIND)) {
+    if (zc) {
+      for (int i = tid; i < a.nz; i += blockDim.x) sgeo[i] = load_g(i);  // read past the first barrier
+    } else {
+      weights(load_g(v));
+      cx = fx; cgx = gx; cw = fw; cgw = gw;
+    }
     const int nl = kn + (above ? 1 : 0);
     unsigned pf = (unsigned)((G.a0 + G.da) * G.sa + p0);  // first row's point in the plane fetched next
     float *dst = own + r0off, *dfr = ownr;                 // and where its values go
@@ -1392,12 +1413,12 @@ __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp 
         pf += astep;
         dst += 2 * N1;
         dfr += nfix;
-        if ((t % MDEPTH) == 0) { dst = own + r0off; dfr = ownr; }  // slots of planes 1 .. MDEPTH, in turn
+        if ((t % DEPTH) == 0) { dst = own + r0off; dfr = ownr; }  // slots of planes 1 .. DEPTH, in turn
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
 #pragma unroll 1
-    for (int t = 1; t < MDEPTH; ++t) fetch(t);
+    for (int t = 1; t < DEPTH; ++t) fetch(t);
     unsigned pc = (unsigned)(G.a0 * G.sa + p0);  // first row's point in plane t - 1
     const float *o = own + r0off, *of = ownr;
 #pragma unroll 1
@@ -1408,26 +1429,29 @@ __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp 
           if (!((fix >> j) & 1)) rado[pc + j * ustep] = rad;
         });
       if (t < nT) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(MDEPTH - 2) : "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(DEPTH - 2) : "memory");
+        if (KIND != M_XY && zc) weights(sgeo[G.a0 + t * G.da]);
         integrate(o, nV, N1, of, 1);
+        if (KIND != M_XY && zc) { cx = fx; cgx = gx; cw = fw; cgw = gw; }
         o += 2 * N1;
         of += nfix;
-        if ((t % MDEPTH) == 0) { o = own + r0off; of = ownr; }
-        fetch(t + MDEPTH - 1);
+        if ((t % DEPTH) == 0) { o = own + r0off; of = ownr; }
+        fetch(t + DEPTH - 1);
       }
       pc += astep;
     }
   } else {
     // four layers (z & ~3 and the next three) of this thread's points at a
-    // time, staged in shared memory one group ahead; a combined radiance takes
-    // the place of its point's source, and the group is stored once its last
-    // plane is combined
+    // time, staged in shared memory one group ahead (M_Z1: when the group
+    // before is stored, in its place); a combined radiance takes the place of
+    // its point's source, and the group is stored once its last plane is combined
     const bool up = G.da > 0, vec = (a.nz & 3) == 0;
     float *const fs = own + 4 * r0off;
+    auto place = [](int zg) { return NG == 2 ? zg & 1 : 0; };
     for (int i = tid; i < a.nz; i += blockDim.x) sgeo[i] = load_g(i);
     auto stage = [&](int zg) {
       int p = p0 + 4 * zg;
-      float *d = fs + (zg & 1) * 8 * N1;
+      float *d = fs + place(zg) * 8 * N1;
 #pragma unroll
       for (int j = 0; j <= RM; ++j) {
         if (j < kn || (j == kn && above)) {
@@ -1443,7 +1467,7 @@ __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp 
           }
         }
         if (j < RM && ((fix >> j) & 1)) {
-          float *f = ownr + (zg & 1) * 4 * nfix + 4 * fixslot(j);
+          float *f = ownr + place(zg) * 4 * nfix + 4 * fixslot(j);
           if (vec) cp_async16(f, rado + p);
           else
             for (int k = 0; k < 4; ++k)
@@ -1456,7 +1480,7 @@ __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp 
     };
     auto flush = [&](int zg) {
       int p = p0 + 4 * zg;
-      const float *d = fs + (zg & 1) * 8 * N1;
+      const float *d = fs + place(zg) * 8 * N1;
 #pragma unroll
       for (int j = 0; j < RM; ++j) {
         if (j < kn && !((fix >> j) & 1)) {
@@ -1479,28 +1503,33 @@ __device__ __forceinline__ void march_column(const SweepArgs &a, const MarchGrp 
       const int zn = z + G.da, zg = zn >> 2;
       next_plane(t + 1);
       if (t > 0) {
-        float *d = fs + ((z >> 2) & 1) * 8 * N1 + (z & 3);
+        float *d = fs + place(z >> 2) * 8 * N1 + (z & 3);
         combine(t, [&](int j, float rad) { d[4 * j * nV] = rad; });
       }
       if (t + 1 == nT) { flush(z >> 2); break; }
       if (t > 0 && zg != z >> 2) flush(z >> 2);
       weights(sgeo[zn]);
       if (zg != zhave) {  // entering group zg: wait for it, then stage the one after
-        if (zg != zstaged) stage(zg);
+        if (zg != zstaged) {
+          if (NG == 1) asm volatile("cp.async.wait_group 0;" ::: "memory");  // the first plane's group, in the same place
+          stage(zg);
+        }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
-        zhave = zg;
-        zstaged = zg + (up ? 1 : -1);
-        if (zstaged >= 0 && 4 * zstaged < a.nz) stage(zstaged);
+        zhave = zstaged = zg;
+        if (NG == 2) {
+          zstaged = zg + (up ? 1 : -1);
+          if (zstaged >= 0 && 4 * zstaged < a.nz) stage(zstaged);
+        }
       }
-      integrate(fs + (zg & 1) * 8 * N1 + (zn & 3), 4 * nV, 4 * N1, ownr + (zg & 1) * 4 * nfix + (zn & 3), 4);
+      integrate(fs + place(zg) * 8 * N1 + (zn & 3), 4 * nV, 4 * N1, ownr + place(zg) * 4 * nfix + (zn & 3), 4);
       cx = fx; cgx = gx; cw = fw; cgw = gw;
       z = zn;
     }
   }
 }
 
-template <int RM, bool ZC>
-__global__ void __launch_bounds__(MMAXT) k_sweep_march(SweepArgs a, const MarchGrp *__restrict__ grps,
+template <int RM, int KIND>
+__global__ void __launch_bounds__(KIND == M_WIDE ? 2 * MMAXT : MMAXT) k_sweep_march(SweepArgs a, const MarchGrp *__restrict__ grps,
                                                        const MarchUnit *__restrict__ units, int smem_words) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
@@ -1519,7 +1548,7 @@ __global__ void __launch_bounds__(MMAXT) k_sweep_march(SweepArgs a, const MarchG
       for (int i = 0; i < MRING; ++i) tc::mbar_expect_tx(bar0 + 8 * i, 4 * G.nV);
   }
   cl.sync();
-  march_column<RM, ZC>(a, G, U.col, msm, cs, rank);
+  march_column<RM, KIND>(a, G, U.col, msm, cs, rank);
   cl.sync();  // no CTA leaves while another may still send into it or arrive on its barriers
 }
 
@@ -1529,6 +1558,11 @@ __global__ void __launch_bounds__(MMAXT) k_sweep_march(SweepArgs a, const MarchG
 // Fitted to 217 timings (six grids from 24x24x16 to 128x128x64, 1 to 16
 // CTAs per column, 64 to 512 threads; 29% rms), over which the choice is
 // within 17% of the best shape, 5% in the mean.
+// kMarchSpare: of each row that a class has less than the launch it shares
+// (64x520x32, the y class's one row a thread: 1.0, 1.5 and 2.4 us a plane in
+// kernels of 3, 6 and 16 rows).
+constexpr double kMarchSpare = 300;
+constexpr double kMarchLaunch = 8000;  // a launch by itself
 constexpr double kMarchRow = 33, kMarchPlane = 184, kMarchIdle = 20, kMarchIpc = 1.97, kMarchLat = 633, kMarchRowLat = 575;
 
 // Sequential-order sweep for grids whose wavefront is too deep (periodic
@@ -3941,8 +3975,8 @@ struct Handle {
   int tc_wait_limit = tc::kWaitLimit;  // polls of a tensor-core pipeline wait (0 only to test the abort path)
   DBuf<MarchGrp> mgrp[2];
   DBuf<MarchUnit> munit[2];
-  struct MarchLaunch { int units = 0, cs = 0, threads = 0, rows = 0; size_t smem = 0; };
-  MarchLaunch mlaunch[2][2];  // [hemisphere][x and y classes, z class]
+  struct MarchLaunch { int units = 0, cs = 0, threads = 0, rows = 0, kind = 0; size_t smem = 0; double cycles = 0; };
+  MarchLaunch mlaunch[2][3];  // [hemisphere][x and y classes or the x class, the y class by itself, the z class]
 
   bool initialized = false;
   int iters = 0;
@@ -4338,18 +4372,23 @@ static void fill_sizes(const Plan &P, shdom_sizes *o) {
 // that has one, for the x and y classes and for the z class.  A hemisphere
 // whose columns cannot be launched on this device keeps the level schedule.
 typedef void (*MarchKernel)(SweepArgs, const MarchGrp *, const MarchUnit *, int);
-constexpr int kMarchRows[6] = {1, 2, 3, 4, 6, MROWS};  // the kernel's rows per thread
-static int march_rows(int rows) {
-  int k = 0;
-  while (kMarchRows[k] < rows) ++k;
+// The kernel that takes at least this many rows per thread; rows becomes what it takes, 0 when none does.
+template <int KIND, int... RM>
+static MarchKernel march_kernel_of(int &rows) {
+  MarchKernel k = nullptr;
+  int took = 0;
+  (void)((RM >= rows && (k = k_sweep_march<RM, KIND>, took = RM, true)) || ...);
+  rows = took;
   return k;
 }
-static MarchKernel march_kernel(int rows, bool z) {
-  static const MarchKernel xy[6] = {k_sweep_march<1, false>, k_sweep_march<2, false>, k_sweep_march<3, false>,
-                                    k_sweep_march<4, false>, k_sweep_march<6, false>, k_sweep_march<MROWS, false>};
-  static const MarchKernel zz[6] = {k_sweep_march<1, true>, k_sweep_march<2, true>, k_sweep_march<3, true>,
-                                    k_sweep_march<4, true>, k_sweep_march<6, true>, k_sweep_march<MROWS, true>};
-  return (z ? zz : xy)[march_rows(rows)];
+static MarchKernel march_kernel(int kind, int &rows) {
+  switch (kind) {
+    case M_XY: return march_kernel_of<M_XY, 1, 2, 3, 4, 6, MROWS>(rows);
+    case M_Z: return march_kernel_of<M_Z, 1, 2, 3, 4, 6, MROWS>(rows);
+    case M_Z1: return march_kernel_of<M_Z1, 4, 8, MROWS>(rows);
+    case M_PLANES: return march_kernel_of<M_PLANES, 4, 8, MROWS>(rows);
+    default: return march_kernel_of<M_WIDE, 8>(rows);
+  }
 }
 
 static cudaLaunchConfig_t march_config(int units, int cs, int threads, size_t smem, cudaStream_t st, cudaLaunchAttribute *at) {
@@ -4370,8 +4409,71 @@ static bool march_stencil_ok(const MarchGrp &g) {
     const bool k1 = k & 1, k2 = k & 2;  // corner k: second in v for k1, in u for k2
     if ((g.dv[k] != g.dv[0]) != (vu ? k2 : k1) || (g.du[k] != g.du[0]) != (vu ? k1 : k2)) return false;
   }
-  const bool uend = g.cls == 0 ? g.yedge : g.xedge, vend = g.cls == 2 ? g.yedge : true;
-  return uend && vend;
+  return g.uedge && (g.cls != 2 || g.vedge);
+}
+
+// The z class with its rows along y and its positions along x, or back.
+static MarchGrp march_swap(const MarchGrp &g) {
+  MarchGrp s = g;
+  s.nU = g.nV; s.nV = g.nU; s.su = g.sv; s.sv = g.su; s.upu = g.upv; s.upv = g.upu; s.uedge = g.vedge; s.vedge = g.uedge;
+  for (int k = 0; k < 4; ++k) { s.du[k] = g.dv[k]; s.dv[k] = g.du[k]; }
+  return s;
+}
+
+// The fastest launch of a kind for the groups of some classes (a bit each:
+// x, y, or the z class), by the march's cost model; L.cycles is its estimate.
+// False when none fits.
+static bool march_shape(const Handle &H, const std::vector<MarchGrp> &grps, int classes, int kind, size_t nunits, int maxsm,
+                        int smsm, Handle::MarchLaunch &L) {
+  const int nz = H.P.nz, maxt = kind == M_WIDE ? 2 * MMAXT : MMAXT;
+  const bool z = classes == 4;
+  double best = 0;
+  bool found = false;
+  for (int cs : {1, 2, 4, 8, 16})
+    for (int nt = 64; nt <= maxt; nt += 32) {
+      size_t smem = 0;
+      int rows = 0;
+      double work = 0, longest = 0;
+      for (const MarchGrp &g : grps)
+        if ((classes >> g.cls) & 1) rows = nt < g.nV ? MROWS + 1 : std::max(rows, ((g.nU + cs - 1) / cs + nt / g.nV - 1) / (nt / g.nV));
+      if (rows > MROWS) continue;
+      for (const MarchGrp &g : grps) {
+        if (!((classes >> g.cls) & 1)) continue;
+        const int tw = (g.nU + cs - 1) / cs, ng = nt / g.nV, r = (tw + ng - 1) / ng;
+        smem = std::max(smem, march_smem_bytes(tw, g.nV, nz, kind, z));
+        // issue slots of a column's planes (cycles of one SM) and the latency of the chain of planes (cycles)
+        const double busy = std::min(nt / 32, ((tw + r - 1) / r * g.nV + 31) / 32);
+        work += (double)g.ncol * cs * g.nA * (busy * (kMarchRow * r + kMarchPlane) + (nt / 32 - busy) * kMarchIdle) / kMarchIpc;
+        longest = std::max(longest, (g.nA + 2.0 * (cs - 1)) * (kMarchLat + kMarchRowLat * r + kMarchSpare * (rows - r)));
+      }
+      if (smem > (size_t)maxsm) continue;
+      MarchKernel kn = march_kernel(kind, rows);
+      if (!kn) continue;
+      cudaFuncAttributes fa;
+      CK(cudaFuncGetAttributes(&fa, kn));
+      const int wregs = (fa.numRegs + 7) / 8 * 8 * 32 * ((nt / 32 + 3) / 4 * 4);
+      const int resident = std::min({(int)((size_t)smsm / (smem + 1024)), 65536 / wregs, 2048 / nt, 32});
+      if (resident < 1) continue;
+      const double waves = std::ceil((double)nunits * cs / ((double)resident * H.nsm));
+      const double t = std::max(work / H.nsm, waves * longest) + 0.09 * std::min(work / H.nsm, waves * longest);
+      if (found && t >= best) continue;
+      CK(cudaFuncSetAttribute(kn, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
+      if (cs > 8 && cudaFuncSetAttribute(kn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        continue;
+      }
+      cudaLaunchAttribute at;
+      cudaLaunchConfig_t cfg = march_config(1, cs, nt, smem, nullptr, &at);
+      int n = 0;  // the launch must fit on this device
+      if (cudaOccupancyMaxActiveClusters(&n, kn, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        continue;
+      }
+      best = t;
+      found = true;
+      L.cs = cs; L.threads = nt; L.rows = rows; L.kind = kind; L.smem = smem; L.cycles = t;
+    }
+  return found;
 }
 
 static void setup_march(Handle &H) {
@@ -4386,70 +4488,62 @@ static void setup_march(Handle &H) {
   if (!clus) return;
   for (int h = 0; h < 2; ++h) {
     if (P.march[h].empty() || H.seq[h]) continue;
-    std::vector<MarchUnit> units[2];
+    std::vector<MarchGrp> grps(P.march[h].begin(), P.march[h].end()), swapped(grps);
+    std::vector<MarchUnit> units[3];  // of each class
     bool ok = true;
-    for (size_t gi = 0; gi < P.march[h].size(); ++gi) {
-      const MarchGrp &g = P.march[h][gi];
+    for (size_t gi = 0; gi < grps.size(); ++gi) {
+      const MarchGrp &g = grps[gi];
       ok = ok && march_stencil_ok(g);
+      if (g.cls == 2) swapped[gi] = march_swap(g);
       for (int c = g.col0; c < g.col0 + g.ncol; ++c)
-        if (P.col_cz[c] != 0.f) units[g.cls == 2].push_back(MarchUnit{(int)gi, c});
+        if (P.col_cz[c] != 0.f) units[g.cls].push_back(MarchUnit{(int)gi, c});
     }
-    for (int k = 0; k < 2 && ok; ++k) {
-      Handle::MarchLaunch &L = H.mlaunch[h][k];
-      L.units = 0;
-      if (units[k].empty()) continue;
-      double best = 0;
-      bool found = false;
-      for (int cs : {1, 2, 4, 8, 16})
-        for (int nt = 64; nt <= MMAXT; nt += 32) {
-          size_t smem = 0;
-          int rows = 0;
-          double work = 0, longest = 0;
-          for (const MarchGrp &g : P.march[h]) {
-            if ((g.cls == 2) != (k == 1)) continue;
-            const int tw = (g.nU + cs - 1) / cs, ng = nt / g.nV;
-            if (ng < 1) { rows = MROWS + 1; break; }
-            const int r = (tw + ng - 1) / ng;
-            smem = std::max(smem, march_smem_bytes(tw, g.nV, P.nz, k == 1));
-            rows = std::max(rows, r);
-            // issue slots of a column's planes (cycles of one SM) and the latency of the chain of planes (cycles)
-            const double busy = std::min(nt / 32, ((tw + r - 1) / r * g.nV + 31) / 32);
-            work += (double)g.ncol * cs * g.nA * (busy * (kMarchRow * r + kMarchPlane) + (nt / 32 - busy) * kMarchIdle) / kMarchIpc;
-            longest = std::max(longest, (g.nA + 2.0 * (cs - 1)) * (kMarchLat + kMarchRowLat * r));
-          }
-          if (rows > MROWS || smem > (size_t)maxsm) continue;
-          cudaFuncAttributes fa;
-          CK(cudaFuncGetAttributes(&fa, march_kernel(rows, k == 1)));
-          const int wregs = (fa.numRegs + 7) / 8 * 8 * 32 * ((nt / 32 + 3) / 4 * 4);
-          const int resident = std::min({(int)((size_t)smsm / (smem + 1024)), 65536 / wregs, 2048 / nt, 32});
-          if (resident < 1) continue;
-          const double waves = std::ceil((double)units[k].size() * cs / ((double)resident * H.nsm));
-          const double t = std::max(work / H.nsm, waves * longest) + 0.09 * std::min(work / H.nsm, waves * longest);
-          if (found && t >= best) continue;
-          MarchKernel kn = march_kernel(rows, k == 1);
-          CK(cudaFuncSetAttribute(kn, cudaFuncAttributeMaxDynamicSharedMemorySize, maxsm));
-          if (cs > 8 && cudaFuncSetAttribute(kn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-            cudaGetLastError();
-            continue;
-          }
-          cudaLaunchAttribute at;
-          cudaLaunchConfig_t cfg = march_config(1, cs, nt, smem, nullptr, &at);
-          int n = 0;  // the launch must fit on this device
-          if (cudaOccupancyMaxActiveClusters(&n, kn, &cfg) != cudaSuccess || n < 1) {
-            cudaGetLastError();
-            continue;
-          }
-          best = t;
-          found = true;
-          L.cs = cs; L.threads = nt; L.rows = rows; L.smem = smem;
-        }
-      if (!found) { ok = false; break; }
-      L.units = (int)units[k].size();
+    if (!ok) continue;
+    Handle::MarchLaunch *L = H.mlaunch[h];
+    for (int k = 0; k < 3; ++k) L[k] = Handle::MarchLaunch{};
+    // The kinds that keep the most in flight first, the z class on either
+    // axis before the next kind (an iteration at 8 x 16 ordinates: 300x100x64
+    // with M_Z 4.68 ms, with M_Z1 on the other axis 4.81; 200x200x64 with M_Z1
+    // 4.74, by levels 9.2; 246x246x64 with M_PLANES 10.6, by levels 14.5).
+    auto planes = [&](int classes, size_t n, Handle::MarchLaunch &l) {
+      for (int kind : {M_XY, M_PLANES, M_WIDE})
+        if (march_shape(H, grps, classes, kind, n, maxsm, smsm, l)) { l.units = (int)n; return true; }
+      return false;
+    };
+    const size_t nx = units[0].size(), ny = units[1].size(), nzc = units[2].size();
+    // The x and y classes in one launch, whose shape is a compromise where the
+    // grid is long, or in one launch each where that is estimated faster (an
+    // iteration, one against two launches, 8 x 16 ordinates: 12x200x24 0.72
+    // and 0.64 ms, 64x520x32 7.4 and 3.4, 1010x32x64 15.7 and 7.9; it is wrong
+    // by little at 96x10x48, 0.50 and 0.51, where it takes two)
+    Handle::MarchLaunch both, one[2];
+    if (nx + ny) {
+      ok = planes(3, nx + ny, both);
+      if (nx && ny && P.nx1 != P.ny1 && planes(1, nx, one[0]) && planes(2, ny, one[1]) &&
+          (!ok || one[0].cycles + one[1].cycles + kMarchLaunch < both.cycles)) {
+        L[0] = one[0]; L[1] = one[1];
+        ok = true;
+      } else {
+        L[0] = both;
+      }
     }
-    if (!ok || (units[0].empty() && units[1].empty())) continue;
+    if (ok && nzc) {
+      ok = false;
+      for (int kind : {M_Z, M_Z1, M_PLANES, M_WIDE}) {
+        if ((ok = march_shape(H, grps, 4, kind, nzc, maxsm, smsm, L[2]))) break;
+        if ((ok = march_shape(H, swapped, 4, kind, nzc, maxsm, smsm, L[2]))) { grps = swapped; break; }
+      }
+      L[2].units = (int)nzc;
+    }
+    if (!ok || nx + ny + nzc == 0) continue;
+    // in one launch, the groups' order; longer chains first where they differ
     std::vector<MarchUnit> all(units[0]);
     all.insert(all.end(), units[1].begin(), units[1].end());
-    std::vector<MarchGrp> grps(P.march[h].begin(), P.march[h].end());
+    if (!L[1].units)
+      std::stable_sort(all.begin(), all.end(), [&](const MarchUnit &x, const MarchUnit &y) {
+        return grps[x.grp].nA != grps[y.grp].nA ? grps[x.grp].nA > grps[y.grp].nA : x.grp < y.grp;
+      });
+    all.insert(all.end(), units[2].begin(), units[2].end());
     H.mgrp[h].upload(grps);
     H.munit[h].upload(all);
     H.march[h] = true;
@@ -5044,12 +5138,12 @@ static void sweep_hemisphere(Handle &H, int hemi) {
     if (H.ktime_on) CK(cudaEventRecord(H.ev_k[hemi][1], H.stream));
     const MarchGrp *gp = H.mgrp[hemi].p;
     const MarchUnit *up = H.munit[hemi].p;
-    for (int k = 0; k < 2; ++k) {
-      const Handle::MarchLaunch &L = H.mlaunch[hemi][k];
+    for (const Handle::MarchLaunch &L : H.mlaunch[hemi]) {
       if (!L.units) continue;
       cudaLaunchAttribute at;
       cudaLaunchConfig_t cfg = march_config(L.units, L.cs, L.threads, L.smem, H.stream, &at);
-      CK(cudaLaunchKernelEx(&cfg, march_kernel(L.rows, k == 1), a, gp, up, (int)(L.smem / 4)));
+      int rows = L.rows;
+      CK(cudaLaunchKernelEx(&cfg, march_kernel(L.kind, rows), a, gp, up, (int)(L.smem / 4)));
       up += L.units;
       H.launches += 1;
     }
@@ -6017,8 +6111,11 @@ int shdom_get_sizes(shdom_handle *hh, shdom_sizes *o) {
   o->launches = hh->h.launches;
   const shdom::Handle &H = hh->h;
   o->march = H.march_off ? 0 : ((H.march[0] ? 1 : 0) | (H.march[1] ? 2 : 0));
-  auto units = [&](int h) { return H.march[h] ? H.mlaunch[h][0].units + H.mlaunch[h][1].units : 0; };
-  auto clus = [&](int h) { return H.march[h] ? H.mlaunch[h][H.mlaunch[h][0].units ? 0 : 1].cs : 0; };
+  auto units = [&](int h) { return H.march[h] ? H.mlaunch[h][0].units + H.mlaunch[h][1].units + H.mlaunch[h][2].units : 0; };
+  auto clus = [&](int h) {
+    const auto *L = H.mlaunch[h];
+    return H.march[h] ? (L[0].units ? std::max(L[0].cs, L[1].cs) : L[2].cs) : 0;
+  };
   o->march_units_down = units(0); o->march_units_up = units(1);
   o->march_cluster_down = clus(0); o->march_cluster_up = clus(1);
   return 0;

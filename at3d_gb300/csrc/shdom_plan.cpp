@@ -1370,8 +1370,11 @@ void build_march(Plan &P) {
           g.dv[k] = ((d >> iv) & 1) ? ((((b >> iv) & 1) ? -1 : 1)) : 0;
         }
         g.upu = ((b >> iu) & 1) ? -1 : 1;
+        g.upv = ((b >> iv) & 1) ? -1 : 1;
         g.zfix = h == 0 ? P.nz - 1 : 0;
         g.xedge = xopen ? 1 : 0; g.yedge = yopen ? 1 : 0;
+        g.uedge = cls == 0 ? g.yedge : g.xedge;
+        g.vedge = cls == 2 ? g.yedge : 0;
         const uint8_t *kd = &P.kind[((size_t)b * 4 + cls) * n];
         for (int p = 0; p < n && ok; ++p) {
           const int ix = p / (P.ny1 * P.nz), iy = (p / P.nz) % P.ny1, iz = p % P.nz;

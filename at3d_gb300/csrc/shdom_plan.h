@@ -100,10 +100,11 @@ struct MarchGrp {
   int nA, nU, nV, sa, su, sv;
   int a0, da;          // first plane in march order (the upwind boundary plane) and the step
   int du[4], dv[4];    // transverse offsets (0 or +-1) of the stopping face's corners, face-weight order
-  int upu;             // the sign of the U offsets: +1 when the upwind rows are at higher U
+  int upu, upv;        // the signs of the U and V offsets: +1 when the upwind rows are at higher U
   // fixed points (preset boundary or phase 1): the layer iz == zfix, and
   // with open x (y) boundaries the planes ix == 0 or nx1 - 1 (iy == 0 or ny1 - 1)
   int zfix, xedge, yedge;
+  int uedge, vedge;    // those of the two that lie along U and (z class) along V
 };
 
 struct Plan {

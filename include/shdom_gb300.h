@@ -45,7 +45,7 @@ typedef struct shdom_sizes {
     int nstokes;   /* Stokes components (1, or 3 for I, Q, U) */
     int march;     /* hemispheres swept by the plane march (bit 0 down, bit 1 up; plan: eligible, handle: in use) */
     int march_units_down, march_units_up;     /* handle: thread-block clusters of each hemisphere's march launch */
-    int march_cluster_down, march_cluster_up; /* handle: CTAs per cluster (16 or 8) */
+    int march_cluster_down, march_cluster_up; /* handle: CTAs per cluster of the x and y classes' march (1 to 16; without them the z class's) */
 } shdom_sizes;
 
 /* Builds the grid, the cell structure, the sweep schedule and the medium on

@@ -80,3 +80,38 @@ def test_cuda_core_transforms_on_ordinate_major_fields(rte_cls, scene):
     r.close()
     assert relrms(a["radiance"], b["radiance"]) < 1e-4
     assert relrms(a["fluxes"], b["fluxes"]) < 1e-5
+
+
+PLANES = {  # planes beyond what the deepest staging holds, and rows beyond a thread per position
+    "200x200x5": dict(nx=200, ny=200, nz=5),     # z class: one group of layers
+    "246x246x6": dict(nx=246, ny=246, nz=6),     # z class: single planes
+    "100x300x7": dict(nx=100, ny=300, nz=7),     # z class: positions along x
+    "1010x4x64": dict(nx=1010, ny=4, nz=64),     # y class: single planes
+    "5x6x600": dict(nx=5, ny=6, nz=600),         # x and y classes: more than 512 positions
+}
+
+
+@pytest.mark.parametrize("shape", list(PLANES))
+def test_march_of_large_planes(rte_cls, shape):
+    """Grids that march although their planes are large, with a column split
+    over several CTAs, so that rows go from one to the next."""
+    from oracle.oracle import Oracle
+    pb = cloud_field(seed=8, nmu=6, nphi=12, nleg=128, boundary="open", **PLANES[shape])
+    r = rte_cls.from_problem(pb)
+    s = r.sizes
+    assert s["march"] == 3
+    assert shape == "5x6x600" or (s["march_cluster_down"] > 1 and s["march_cluster_up"] > 1)
+    r.solve(2, verbose=False)
+    a = r.export_state()
+    r.set_sweep_mode("levels_only")
+    r.solve(2, verbose=False)
+    b = r.export_state()
+    r.close()
+    for k in ("radiance", "fluxes"):
+        assert relrms(a[k], b[k]) < 1e-5, k
+    o = Oracle(pb, fp64=False)
+    o.solve(2)
+    c = o.export()
+    assert np.array_equal(a["ns"], c["ns"]) and np.array_equal(a["nr"], c["nr"])
+    for k in ("radiance", "fluxes"):
+        assert relrms(a[k], c[k]) < 1e-4, k
