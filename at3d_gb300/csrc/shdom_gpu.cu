@@ -3509,7 +3509,10 @@ __device__ RaySetup ray_setup(const RenderArgs &a, int ray) {
 // for 36,864 rays against one warp per ray: 64x64x32 0.73 against 2.12 ms,
 // 128x128x64 (256 terms) 2.8 against 4.9, polarized 64x64x40 3.0 against
 // 11.0; 169 rays at 32x32x24 0.21 ms either way (the chain of one ray).
-template <int NST, bool BRDF>
+//
+// LINES: the grid lines are kept in shared memory; without, grids of some
+// 50,000 lines, which do not fit there, are read from memory.
+template <int NST, bool BRDF, bool LINES>
 __global__ void __launch_bounds__(128) k_render(RenderArgs a) {
   extern __shared__ __align__(16) float rsm[];
   __shared__ RaySetup setup[16];
@@ -3520,7 +3523,8 @@ __global__ void __launch_bounds__(128) k_render(RenderArgs a) {
   // read different banks), the single-scatter series and phase values, then the grid lines
   const int ldy = (a.nlm + 3) & ~3, ystr = NY * ldy + 4;
   const bool keep = a.numphase <= RPHASE;
-  float *tls = rsm + nrb * ystr, *pvs = tls + nrb * NST * RLEG, *xg = pvs + nrb * NST * RPHASE, *yg = xg + a.nx + 1, *zg = yg + a.ny + 1;
+  float *tls = rsm + nrb * ystr, *pvs = tls + nrb * NST * RLEG, *xs = pvs + nrb * NST * RPHASE, *ys = xs + a.nx + 1, *zs = ys + a.ny + 1;
+  const float *xg = LINES ? xs : a.xgrid, *yg = LINES ? ys : a.ygrid, *zg = LINES ? zs : a.zgrid;
   // one lane per ray forms its setup (the FP64 trigonometry), the other warps fetch the grid lines
   bool same = true;
   if ((int)threadIdx.x < nrb) {
@@ -3528,9 +3532,11 @@ __global__ void __launch_bounds__(128) k_render(RenderArgs a) {
     setup[threadIdx.x] = ray_setup<NST>(a, i);
     same = a.cammu[i] == a.cammu[b0] && a.camphi[i] == a.camphi[b0];
   }
-  for (int i = threadIdx.x; i <= a.nx; i += blockDim.x) xg[i] = a.xgrid[i];
-  for (int i = threadIdx.x; i <= a.ny; i += blockDim.x) yg[i] = a.ygrid[i];
-  for (int i = threadIdx.x; i < a.nz; i += blockDim.x) zg[i] = a.zgrid[i];
+  if constexpr (LINES) {
+    for (int i = threadIdx.x; i <= a.nx; i += blockDim.x) xs[i] = a.xgrid[i];
+    for (int i = threadIdx.x; i <= a.ny; i += blockDim.x) ys[i] = a.ygrid[i];
+    for (int i = threadIdx.x; i < a.nz; i += blockDim.x) zs[i] = a.zgrid[i];
+  }
   const bool one = __syncthreads_and(same);  // one direction for the whole block
   const RaySetup ry = setup[lr];
   bool act = ray < a.nrays && ry.cell >= 0;
@@ -4164,8 +4170,10 @@ static void allow_smem(F *kernel) {
 
 // The kernels whose shared memory goes with a call or a handle, on a new handle's device.
 static void allow_smem_all() {
-  allow_smem(k_render<1, false>); allow_smem(k_render<1, true>);
-  allow_smem(k_render<3, false>); allow_smem(k_render<3, true>);
+  allow_smem(k_render<1, false, true>); allow_smem(k_render<1, true, true>);
+  allow_smem(k_render<3, false, true>); allow_smem(k_render<3, true, true>);
+  allow_smem(k_render<1, false, false>); allow_smem(k_render<1, true, false>);
+  allow_smem(k_render<3, false, false>); allow_smem(k_render<3, true, false>);
   allow_smem(k_levis_adjoint);
   allow_smem(k_sh_to_do<8>); allow_smem(k_sh_to_do<16>); allow_smem(k_sh_to_do<32>);
   allow_smem(k_do_to_sh<8>); allow_smem(k_do_to_sh<16>); allow_smem(k_do_to_sh<32>);
@@ -5591,18 +5599,21 @@ static int render_impl(shdom_handle *hh, int nrays, const float *camx, const flo
   a.single_scatter = H.render_single_scatter; a.nosurface = H.render_nosurface;
   if (P.nlm > shdom::RNLM || P.ml + 1 > 64) return fail(hh, "render: too many spherical-harmonic terms");
   if (nrays > 0) {
-    auto kernel = H.nst == 3 ? (P.brdf ? shdom::k_render<3, true> : shdom::k_render<3, false>)
-                             : (P.brdf ? shdom::k_render<1, true> : shdom::k_render<1, false>);
     // four warps a block, fewer where the rays' functions would not leave
     // room for a second block on the SM, or where the rays are few
-    auto smem = [&](int warps) {
-      const size_t per = (size_t)(H.nst == 3 ? 5 : 1) * ((P.nlm + 3) & ~3) + 4 + (size_t)H.nst * (shdom::RLEG + shdom::RPHASE);
-      return sizeof(float) * ((size_t)warps * shdom::RGRAYS * per + P.nx + P.ny + P.nz + 2);
-    };
+    constexpr size_t room = 220 * 1024;
+    const size_t ray = (size_t)(H.nst == 3 ? 5 : 1) * ((P.nlm + 3) & ~3) + 4 + (size_t)H.nst * (shdom::RLEG + shdom::RPHASE);
+    const size_t lines = (size_t)P.nx + P.ny + P.nz + 2;
+    const bool keep = sizeof(float) * (shdom::RGRAYS * ray + lines) <= room;
+    auto smem = [&](int warps) { return sizeof(float) * ((size_t)warps * shdom::RGRAYS * ray + (keep ? lines : 0)); };
+    auto kernel = keep ? (H.nst == 3 ? (P.brdf ? shdom::k_render<3, true, true> : shdom::k_render<3, false, true>)
+                                     : (P.brdf ? shdom::k_render<1, true, true> : shdom::k_render<1, false, true>))
+                       : (H.nst == 3 ? (P.brdf ? shdom::k_render<3, true, false> : shdom::k_render<3, false, false>)
+                                     : (P.brdf ? shdom::k_render<1, true, false> : shdom::k_render<1, false, false>));
     int warps = 4;
     while (warps > 1 && (smem(warps) > 100 * 1024 || (long long)nrays < (long long)warps * shdom::RGRAYS * H.nsm)) warps >>= 1;
     const size_t bytes = smem(warps);
-    if (bytes > 220 * 1024) return fail(hh, "render: too many spherical-harmonic terms");
+    if (bytes > room) return fail(hh, "render: too many spherical-harmonic terms");
     const int per = warps * shdom::RGRAYS;
     kernel<<<(nrays + per - 1) / per, warps * 32, bytes, stream>>>(a);
     H.launches += 1;

@@ -3,7 +3,7 @@ mixtures where their split can go wrong: fewer rays than a warp or a block
 takes, one more than a block, blocks of one direction and of many, rays that
 start inside the medium and look up or down, rays of weight zero, rows of
 harmonics that are not a multiple of four; and the ordinate-to-harmonic
-transform with such rows.
+transform with such rows; and a grid with more lines than fit on the chip.
 
 Compared with the FP64 oracle on the state of 3 iterations (I, Q, U: the FP32
 one), to the 1e-4 relative RMS that the solve, the render and the gradient
@@ -90,3 +90,23 @@ def test_adjoint_lanes(solved, n, mixed):
     gb = o.levis_adjoint(0, rays, w, nthreads=4).reshape(ga.shape)
     for d in range(2):
         assert relrms(ga[..., d], gb[..., d]) < 1e-4, d
+
+
+def test_render_of_a_grid_of_many_lines():
+    """57,000 cells along x: the rays read the grid's lines from memory.  The
+    rays stay near its start, where positions in FP32 are as fine as elsewhere."""
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from at3d_gb300.solver import RTE
+    from oracle.oracle import Oracle
+    pb = cloud_field(seed=15, nx=57000, ny=2, nz=3, nmu=4, nphi=8, nleg=128, boundary="open")
+    near = cloud_field(seed=16, nx=20, ny=2, nz=3, nmu=4, nphi=8, nleg=128, boundary="open")
+    pb.species[0].extinction[:20] = near.species[0].extinction
+    r = RTE.from_problem(pb)
+    r.solve(1, verbose=False)
+    o = Oracle(pb, fp64=True)
+    o.solve(1)
+    rays = list(some_rays(near, 33, True))
+    assert relrms(r.render(*rays), o.render(*rays, nthreads=4)) < 1e-4
+    r.close()
