@@ -501,7 +501,7 @@ __device__ __forceinline__ Trace trace_general(const SweepArgs &a, int b, int cl
     tr *= transcell;
     auto ok = [&](int q) { return (a.bnd[q] & hb) || (rk[q] < rP && (!use_level || lv[q] < lP)); };
     const bool valid = ok(i1) && ok(i2) && ok(i3) && ok(i4);
-    if (nxt < 0 || (tr <= a.transmin && valid)) {
+    if (nxt < 0 || (valid && (a.is1d || tr <= a.transmin))) {
 #pragma unroll
       for (int st = 0; st < NST; ++st) rs[st] = rad[st];
       t.radsrc = rad[0]; t.tr = tr;

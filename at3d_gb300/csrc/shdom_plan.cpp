@@ -388,16 +388,16 @@ void sweep_order(Plan &P, int ioct) {
 
 // Trace back from point pt along one ordinate with the reference's validity
 // rule (a face is usable when all four corners precede pt in the sweep order
-// or are preset boundary points); returns the corners of the stopping face.
+// or are preset boundary points), at TRANSMIN 1; returns the corners of the
+// stopping face, the first usable one.
 bool trace_final_face(const Plan &P, int ioct, int pt, double cx, double cy, double cz, int hemi_bnd,
-                      double transmin, int face_out[4]) {
+                      int face_out[4]) {
   const int b = ioct - 1;
   const int *rk = &P.rank[(size_t)b * P.npts];
   double cxinv = cx != 0 ? 1.0 / cx : 1e6, cyinv = cy != 0 ? 1.0 / cy : 1e6, czinv = 1.0 / cz;
   int bitx = cx < 0, bity = cy < 0, bitz = cz < 0;
   int cell = P.startcell[(size_t)b * P.npts + pt];
   double xe = P.gridpos[3 * pt], ye = P.gridpos[3 * pt + 1], ze = P.gridpos[3 * pt + 2];
-  double transmit = 1.0;
   const float *gp = P.gridpos.data();
   for (int guard = 0; guard < 1000000; ++guard) {
     if (cell < 0) return false;
@@ -429,7 +429,7 @@ bool trace_final_face(const Plan &P, int ioct, int pt, double cx, double cy, dou
     }
     bool valid = true;
     for (int k = 0; k < 4; ++k) valid = valid && ((P.bnd[f[k]] & hemi_bnd) || rk[f[k]] < rk[pt]);
-    if (nxt < 0 || (transmit <= transmin && valid)) {
+    if (nxt < 0 || valid) {
       if (!valid) return false;
       for (int k = 0; k < 4; ++k) face_out[k] = f[k];
       return true;
@@ -1121,6 +1121,13 @@ bool build_schedule(const shdom_problem &p, Plan &P) {
     th.emplace_back([&, ioct]() {
       sweep_order(P, ioct);
       const int b = ioct - 1;
+      if (transmin < 1.0 && !P.is1d) {
+        // which face a trace stops on depends on the medium, so no schedule
+        // of the grid's holds: the hemisphere is swept in the reference order
+        // (a 1D trace stops on the first usable point whatever TRANSMIN is)
+        deep[b] = 1;
+        return;
+      }
       const int hemi_bnd = (b & 4) ? 2 : 1;  // trace down: bottom points preset
       const int *rk = &P.rank[(size_t)b * n];
       const int *sc = &P.startcell[(size_t)b * n];
@@ -1131,7 +1138,7 @@ bool build_schedule(const shdom_problem &p, Plan &P) {
         if (P.bnd[pt] & hemi_bnd) continue;
         int cell = sc[pt];
         const int *g = &P.gridptr[8 * (size_t)cell];
-        bool fast = transmin >= 1.0 && !P.is1d && g[b] == pt && P.cellflags[cell] == 0;
+        bool fast = !P.is1d && g[b] == pt && P.cellflags[cell] == 0;
         for (int k = 0; k < 8 && fast; ++k) {
           if (k == b) continue;
           int q = g[k];
@@ -1158,7 +1165,7 @@ bool build_schedule(const shdom_problem &p, Plan &P) {
               int f[4];
               double tcx, tcy, tcz;
               trace_dir(P.mu[P.col_imu[c]], P.phi[(size_t)P.col_imu[c] * P.nphi0max + P.col_iphi[c]], tcx, tcy, tcz);
-              if (!trace_final_face(P, ioct, pt, tcx, tcy, tcz, hemi_bnd, transmin, f)) {
+              if (!trace_final_face(P, ioct, pt, tcx, tcy, tcz, hemi_bnd, f)) {
                 errs[b] = "sweep planning: trace found no valid face (BACK_INT_GRID: INEXTCELL=0)";
                 return;
               }
