@@ -2577,6 +2577,7 @@ struct SourceArgs {
   const int *lofj;
   float *source, *delsource;
   int *ns, *nso, *nr;     // nr is read (current) and rewritten (next)
+  int *nrr;               // the current one kept: the truncation of the radiance as it stands
   double *red;            // [4] deljdot, deljold, deljnew, jnorm
   int npts, nlm, nl, ml, mm;
   float secmu0, shacc;
@@ -2705,6 +2706,7 @@ __global__ void __launch_bounds__(256) k_source(SourceArgs a) {
       a.ns[p] = nsnew;
       if (!a.first && a.accel) a.nso[p] = nsold;
       if (a.first) a.nso[p] = nsnew;
+      a.nrr[p] = nrp;
       a.nr[p] = nrnext;
     }
   }
@@ -2809,6 +2811,7 @@ __global__ void __launch_bounds__(256) k_source_pol(SourceArgs a) {
       a.ns[p] = nsnew;
       if (!a.first && a.accel) a.nso[p] = nsold;
       if (a.first) a.nso[p] = nsnew;
+      a.nrr[p] = nrp;
       a.nr[p] = nrnext;
     }
   }
@@ -2971,6 +2974,7 @@ __global__ void __launch_bounds__(256) k_source_v(SourceArgs a, const int *__res
         a.ns[p] = nsnew;
         if (a.first) a.nso[p] = nsnew;
         else if (a.accel) a.nso[p] = nsold;
+        a.nrr[p] = nrp;
         a.nr[p] = nrnext;
       }
     }
@@ -3946,7 +3950,7 @@ struct Handle {
   DBuf<int> tms_ptr, tms_iph;
   // state
   DBuf<float> source, delsource, radiance, srcdo, raddo, fluxes, bcrad;
-  DBuf<int> ns, nso, nr, errflag;
+  DBuf<int> ns, nso, nr, nrr, errflag;
   DBuf<double> red;
   DBuf<AccelState> accel;
   int ldo = 0;  // columns of srcdo/raddo: nang rounded up to 4 (16-byte rows for TMA)
@@ -4334,7 +4338,7 @@ static long long plan_device_bytes(const Plan &P) {
   b += vbytes(P.tms_iph) + vbytes(P.tms_w) + vbytes(P.phasetab) + vbytes(P.botalb) + vbytes(P.rad0);
   b += vbytes(P.thermal) + vbytes(P.botplanck) + vbytes(P.planckpt);
   const long long ldo = (P.nang + 3) & ~3;
-  b += 4LL * P.npts * (3LL * P.nst * P.nlm + 2 + 3) + 8LL * ((P.npts + 31) & ~31) * ldo + 4LL * (long long)P.botp.size() + 64;
+  b += 4LL * P.npts * (3LL * P.nst * P.nlm + 2 + 4) + 8LL * ((P.npts + 31) & ~31) * ldo + 4LL * (long long)P.botp.size() + 64;
   if (P.nst == 3) b += vbytes(P.col_stk) + vbytes(P.coefp) + vbytes(P.phasetab2) + 8LL * P.nlm * 3 * P.nang;
   {  // gathered rows of the scattering points for the compacted transforms
     long long nh = 0;
@@ -4789,7 +4793,7 @@ static void upload_plan(Handle &H) {
   H.srcdo.alloc(nd); H.raddo.alloc(nd);
   H.srcdo.zero(H.stream); H.raddo.zero(H.stream);
   H.fluxes.alloc((size_t)P.npts * 2); H.bcrad.alloc(std::max<size_t>(1, P.botp.size()));
-  H.ns.alloc(P.npts); H.nso.alloc(P.npts); H.nr.alloc(P.npts); H.errflag.alloc(1);
+  H.ns.alloc(P.npts); H.nso.alloc(P.npts); H.nr.alloc(P.npts); H.nrr.alloc(P.npts); H.errflag.alloc(1);
   H.red.alloc(4); H.accel.alloc(1);
   setup_tc(H);
   // the uploads are legacy-stream copies from pageable memory, which may
@@ -4812,7 +4816,7 @@ static void launch_source(Handle &H, int first, int fixsh) {
   SourceArgs a;
   a.coef = H.coef.p; a.dirflux = H.dirflux.p; a.radiance = H.radiance.p; a.ylmsun = H.ylmsun.p; a.lofj = H.lofj.p;
   a.thermal = H.thermal.n ? H.thermal.p : nullptr;
-  a.source = H.source.p; a.delsource = H.delsource.p; a.ns = H.ns.p; a.nso = H.nso.p; a.nr = H.nr.p; a.red = H.red.p;
+  a.source = H.source.p; a.delsource = H.delsource.p; a.ns = H.ns.p; a.nso = H.nso.p; a.nr = H.nr.p; a.nrr = H.nrr.p; a.red = H.red.p;
   a.npts = P.npts; a.nlm = P.nlm; a.nl = P.ml + 1; a.ml = P.ml; a.mm = P.mm;
   a.secmu0 = 1.0f / std::fabs(P.prob.solarmu); a.shacc = P.prob.shacc;
   a.first = first; a.fixsh = fixsh; a.accel = P.prob.accelflag; a.highorder = P.prob.highorderrad;
@@ -5766,7 +5770,7 @@ static void levis_adjoint_device(Handle &H, int nrays, const float *dx, const fl
   shdom::Plan &P = H.P;
   shdom::GradArgs G;
   G.r = render_args(H, nrays, dx, dy, dz, dmu, dphi, nullptr);
-  G.radiance = H.radiance.p; G.nr = H.nr.p; G.interpptr = H.g_interpptr.p; G.optinterpwt = H.g_optwt.p;
+  G.radiance = H.radiance.p; G.nr = H.nrr.p; G.interpptr = H.g_interpptr.p; G.optinterpwt = H.g_optwt.p;
   G.dextm = H.g_dextm.p; G.dalbm = H.g_dalbm.p; G.dfj = H.g_dfj.p; G.alb_sp = H.g_albsp.p;
   G.planck = H.planckpt.n ? H.planckpt.p : nullptr;
   G.sj_ptr = H.g_sjptr.p; G.sj_iph = H.g_sjiph.p; G.sj_w = H.g_sjw.p; G.legent_u = H.g_legu.p; G.legent_s = H.g_legs.p;
@@ -6046,7 +6050,7 @@ int shdom_export_state(shdom_handle *hh, float *source, int *ns, float *radiance
     if (source) CK(cudaMemcpy(source, H.source.p, nf * sizeof(float), cudaMemcpyDeviceToHost));
     if (radiance) CK(cudaMemcpy(radiance, H.radiance.p, nf * sizeof(float), cudaMemcpyDeviceToHost));
     if (ns) CK(cudaMemcpy(ns, H.ns.p, P.npts * sizeof(int), cudaMemcpyDeviceToHost));
-    if (nr) CK(cudaMemcpy(nr, H.nr.p, P.npts * sizeof(int), cudaMemcpyDeviceToHost));
+    if (nr) CK(cudaMemcpy(nr, H.nrr.p, P.npts * sizeof(int), cudaMemcpyDeviceToHost));
     if (fluxes) CK(cudaMemcpy(fluxes, H.fluxes.p, (size_t)P.npts * 2 * sizeof(float), cudaMemcpyDeviceToHost));
     if (dirflux) CK(cudaMemcpy(dirflux, H.dirflux.p, (size_t)P.npts * sizeof(float), cudaMemcpyDeviceToHost));
   } catch (const std::exception &e) {
