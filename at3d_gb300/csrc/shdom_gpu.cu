@@ -6111,6 +6111,9 @@ int shdom_set_transform_mode(shdom_handle *hh, int mode) {
   Handle &H = hh->h;
   DevGuard dg(H.device);
   try {
+    if (mode != H.xf_mode)
+      for (auto &g : H.iter_graph)  // captured launches are of the old arithmetic
+        if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     H.xf_mode = mode;
     shdom::alloc_xf_rows(H);
   } catch (const std::exception &e) {

@@ -1,0 +1,55 @@
+"""Modes changed on a handle that has already solved: the calls that follow
+equal those of a handle that had the mode from the start (to the 1e-6 relative
+RMS of sums in another order; the transform arithmetics themselves differ by
+1e-5 and more)."""
+import numpy as np
+import pytest
+
+from at3d_gb300.scenes import cloud_blob, cloud_field
+
+pytestmark = pytest.mark.gpu
+
+
+def relrms(a, b):
+    a = np.asarray(a, np.float64); b = np.asarray(b, np.float64)
+    return float(np.sqrt(np.mean((a - b) ** 2)) / max(np.sqrt(np.mean(b ** 2)), 1e-300))
+
+
+@pytest.fixture(scope="module")
+def rte_cls():
+    import torch
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from at3d_gb300.solver import RTE
+    return RTE
+
+
+SCENES = {
+    "open": lambda: cloud_field(seed=71, nx=11, ny=9, nz=8, nmu=8, nphi=16, nleg=64, boundary="open"),
+    "periodic": lambda: cloud_blob(seed=72, nx=9, ny=8, nz=7),
+}
+
+
+def solved(r, iters=3):
+    r.solve(iters, verbose=False)
+    return r.export_state()["radiance"]
+
+
+@pytest.mark.parametrize("scene", list(SCENES))
+def test_transform_mode_after_a_captured_iteration(rte_cls, scene):
+    """An iteration replayed from a graph is captured again for another transform arithmetic."""
+    pb = SCENES[scene]()
+    r = rte_cls.from_problem(pb)
+    r.set_sweep_mode("graph")
+    got = {}
+    for mode in ("tf32", "fp32", "tf32x3"):
+        r.set_transform_mode(mode)
+        got[mode] = solved(r)
+    r.close()
+    for mode, a in got.items():
+        r = rte_cls.from_problem(pb)
+        r.set_transform_mode(mode)
+        b = solved(r)
+        r.close()
+        assert relrms(a, b) < 1e-6, mode
+    assert relrms(got["tf32"], got["fp32"]) > 1e-5
