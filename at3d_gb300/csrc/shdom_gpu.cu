@@ -5623,9 +5623,17 @@ static int render_impl(shdom_handle *hh, int nrays, const float *camx, const flo
     H.launches += 1;
   }
   CK(cudaGetLastError());
-  if (stream != H.stream) {  // the handle's buffers are in use on the caller's stream until this event
-    if (!H.ev_ext) CK(cudaEventCreateWithFlags(&H.ev_ext, cudaEventDisableTiming));
-    CK(cudaEventRecord(H.ev_ext, stream));
+  if (stream != H.stream) {
+    // the handle's buffers are in use on the caller's stream until this
+    // event: what the handle does next (a new solve on it, say) comes after.
+    // (A launch captured into a caller's graph is the caller's to order.)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (stream) CK(cudaStreamIsCapturing(stream, &cap));
+    if (cap == cudaStreamCaptureStatusNone) {
+      if (!H.ev_ext) CK(cudaEventCreateWithFlags(&H.ev_ext, cudaEventDisableTiming));
+      CK(cudaEventRecord(H.ev_ext, stream));
+      CK(cudaStreamWaitEvent(H.stream, H.ev_ext, 0));
+    }
   }
   return 0;
 }

@@ -128,7 +128,8 @@ int shdom_render(shdom_handle *h, int nrays, const float *camx, const float *cam
 
 /* Same as shdom_render with device-resident ray and output buffers, launched
  * on the given CUDA stream (cudaStream_t passed as void*, NULL = legacy
- * default stream).  Asynchronous: returns after the launch. */
+ * default stream).  Asynchronous: returns after the launch; later calls on
+ * the handle that change its state are ordered after it on the device. */
 int shdom_render_device(shdom_handle *h, int nrays, const float *camx, const float *camy,
                         const float *camz, const double *cammu, const double *camphi,
                         float *stokes_out, void *stream);

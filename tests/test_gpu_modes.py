@@ -1,7 +1,10 @@
-"""Modes changed on a handle that has already solved: the calls that follow
+"""What a handle has done before, and has under way, does not change what comes after.
+
+Modes changed on a handle that has already solved: the calls that follow
 equal those of a handle that had the mode from the start (to the 1e-6 relative
 RMS of sums in another order; the transform arithmetics themselves differ by
-1e-5 and more)."""
+1e-5 and more).  A solve that starts while images of the last one are being
+rendered on the caller's streams leaves those images as they are."""
 import numpy as np
 import pytest
 
@@ -53,3 +56,33 @@ def test_transform_mode_after_a_captured_iteration(rte_cls, scene):
         r.close()
         assert relrms(a, b) < 1e-6, mode
     assert relrms(got["tf32"], got["fp32"]) > 1e-5
+
+
+def test_solve_while_images_render(rte_cls):
+    import torch
+    from at3d_gb300.scenes import orthographic_views
+    pb = cloud_field(seed=73, nx=48, ny=48, nz=24, nmu=8, nphi=16, nleg=64, boundary="open")
+    r = rte_cls.from_problem(pb)
+    r.solve(4, verbose=False)
+    rays = [torch.as_tensor(np.ascontiguousarray(v), dtype=torch.float32 if i < 3 else torch.float64).cuda()
+            for i, v in enumerate(orthographic_views(pb, 96, 96))]
+    n = rays[0].numel()
+
+    def render(stream):
+        out = torch.zeros(n, dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        r.render_device(*(v.data_ptr() for v in rays), out.data_ptr(), n, stream.cuda_stream)
+        return out
+
+    streams = [torch.cuda.Stream() for _ in range(2)] + [torch.cuda.default_stream()]
+    want = render(streams[0])
+    torch.cuda.synchronize()
+    want = want.cpu().numpy()
+    for _ in range(3):
+        for s in streams:
+            r.solve(4, verbose=False)
+            got = render(s)
+            r.solve(1, verbose=False)  # resets the solution while the image is on its way
+            torch.cuda.synchronize()
+            assert relrms(got.cpu().numpy(), want) < 1e-6
+    r.close()
