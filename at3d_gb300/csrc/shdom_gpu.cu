@@ -3959,6 +3959,11 @@ struct Handle {
   // the reference order), else point-major for the level schedule
   bool ord_major = false;
   size_t ord_ps = 0, ord_cs = 0;  // strides of a point and of a column
+  void set_strides(bool om) {
+    ord_major = om;
+    ord_ps = om ? 1 : ldo;
+    ord_cs = om ? ((size_t)P.npts + 31) & ~(size_t)31 : 1;
+  }
   DBuf<float> xf_rows;            // ordinate-major: point-major rows for the CUDA-core transforms
   // tensor-core transforms, per direction (0: SH -> DO, 1: DO -> SH)
   int xf_mode = 0;  // 0: 3xTF32 tensor cores, 1: single TF32 product, 2: CUDA-core factorized
@@ -4269,11 +4274,10 @@ static void setup_tc(Handle &H) {
       }
     H.tc_bh[dir].upload(bh);
     H.tc_bl[dir].upload(bl);
-    const float *a = dir == 0 ? H.source.p : H.raddo.p;
+    const float *a = H.source.p;
     make_map(&H.tm_bh[dir], H.tc_bh[dir].p, (uint64_t)kpad, (uint64_t)npad, (uint64_t)kpad, (uint32_t)bn);
     make_map(&H.tm_bl[dir], H.tc_bl[dir].p, (uint64_t)kpad, (uint64_t)npad, (uint64_t)kpad, (uint32_t)bn);
-    if (dir == 1 && H.ord_major) H.tm_a[1] = H.tm_bh[1];  // A does not come by TMA (KM): not read
-    else make_map(&H.tm_a[dir], a, (uint64_t)K, (uint64_t)P.npts, (uint64_t)lda, tc::BM);
+    if (dir == 0) make_map(&H.tm_a[0], a, (uint64_t)K, (uint64_t)P.npts, (uint64_t)lda, tc::BM);
     H.tc_bn[dir] = bn; H.tc_ntiles[dir] = ntiles; H.tc_kpad[dir] = kpad;
     tc_attr(bn);
     H.tc_ok[dir] = true;
@@ -4300,14 +4304,25 @@ static void setup_tc(Handle &H) {
       if (H.nheavy > 0) {
         H.src_c.alloc((size_t)H.nheavy * P.nlm);
         make_map(&H.tm_ac[0], H.src_c.p, (uint64_t)P.nlm, (uint64_t)H.nheavy, (uint64_t)P.nlm, tc::BM);
-        if (H.ord_major) {
-          H.tm_ac[1] = H.tm_a[1];
-        } else {
-          H.rad_c.alloc((size_t)H.nheavy * H.ldo);
-          make_map(&H.tm_ac[1], H.rad_c.p, (uint64_t)P.nang, (uint64_t)H.nheavy, (uint64_t)H.ldo, tc::BM);
-        }
       }
     }
+  }
+}
+
+// The ordinate-to-harmonic operand of the fields' layout: ordinate-major, the
+// kernel reads A itself (KM; the maps are not read), else by TMA, gathered
+// first when only the scattering points' rows are needed.
+static void setup_tc_rows(Handle &H) {
+  Plan &P = H.P;
+  if (!H.tc_ok[1]) return;
+  if (H.ord_major) {
+    H.tm_a[1] = H.tm_ac[1] = H.tm_bh[1];
+    return;
+  }
+  make_map(&H.tm_a[1], H.raddo.p, (uint64_t)P.nang, (uint64_t)P.npts, (uint64_t)H.ldo, tc::BM);
+  if (H.compact && H.nheavy > 0) {
+    if (!H.rad_c.p) H.rad_c.alloc((size_t)H.nheavy * H.ldo);
+    make_map(&H.tm_ac[1], H.rad_c.p, (uint64_t)P.nang, (uint64_t)H.nheavy, (uint64_t)H.ldo, tc::BM);
   }
 }
 
@@ -4784,10 +4799,8 @@ static void upload_plan(Handle &H) {
   // one hemisphere that the march cannot take puts both on the level schedule
   for (int h = 0; h < 2; ++h)
     if (!H.march[h] && !H.seq[h] && (P.seg_off[h].size() > 1 || P.p1off[h].size() > 1)) H.march[0] = H.march[1] = false;
-  H.ord_major = H.march[0] || H.march[1] || (H.seq[0] && H.seq[1]);
   const size_t npad = ((size_t)P.npts + 31) & ~(size_t)31;
-  H.ord_ps = H.ord_major ? 1 : H.ldo;
-  H.ord_cs = H.ord_major ? npad : 1;
+  H.set_strides(H.march[0] || H.march[1] || (H.seq[0] && H.seq[1]));
   const size_t nf = (size_t)P.npts * H.nst * P.nlm, nd = npad * H.ldo;
   H.source.alloc(nf); H.delsource.alloc(nf); H.radiance.alloc(nf);
   H.srcdo.alloc(nd); H.raddo.alloc(nd);
@@ -4796,6 +4809,7 @@ static void upload_plan(Handle &H) {
   H.ns.alloc(P.npts); H.nso.alloc(P.npts); H.nr.alloc(P.npts); H.nrr.alloc(P.npts); H.errflag.alloc(1);
   H.red.alloc(4); H.accel.alloc(1);
   setup_tc(H);
+  setup_tc_rows(H);
   // the uploads are legacy-stream copies from pageable memory, which may
   // return before their DMA lands; the handle's non-blocking stream is not
   // ordered after them
@@ -5005,6 +5019,27 @@ static void alloc_xf_rows(Handle &H) {
     H.xf_rows.alloc((size_t)H.P.npts * H.ldo);
     H.xf_rows.zero(H.stream);
   }
+}
+
+// Turns the ordinate fields' layout (the level schedule takes one point's
+// columns at a time: ordinate-major, its pass takes twice as long at 96x96x48).
+// The radiances go along, through the source's field, which every iteration
+// forms anew but for the points without a source, whose rows are zero.
+static void set_layout(Handle &H, bool ord_major) {
+  if (ord_major == H.ord_major) return;
+  const int n = H.P.npts, c = H.P.nang, tiles = ((n + 31) / 32) * ((c + 31) / 32);
+  const size_t ps = H.ord_ps, cs = H.ord_cs;
+  H.set_strides(ord_major);
+  H.srcdo.zero(H.stream);
+  if (ord_major) k_transpose<<<tiles, 256, 0, H.stream>>>(H.raddo.p, ps, H.srcdo.p, H.ord_cs, n, c);
+  else k_transpose<<<tiles, 256, 0, H.stream>>>(H.raddo.p, cs, H.srcdo.p, H.ord_ps, c, n);
+  CK(cudaGetLastError());
+  H.launches += 1;
+  std::swap(H.raddo.p, H.srcdo.p);  // (of one size, both the handle's own)
+  H.srcdo.zero(H.stream);
+  setup_tc_rows(H);
+  alloc_xf_rows(H);
+  CK(cudaStreamSynchronize(H.stream));  // renders on other streams read them
 }
 
 static SweepArgs sweep_args(Handle &H, int hemi) {
@@ -6076,11 +6111,13 @@ int shdom_set_sweep_mode(shdom_handle *hh, int mode) {
     const bool levels_only = mode == 3;
     if (levels_only != H.march_off) {
       H.march_off = levels_only;
+      const bool march = H.march[0] || H.march[1];
       // the level schedule's source pass needs its (radsrc, tr) table
-      if (levels_only && !H.sweepw.p && (H.march[0] || H.march[1])) {
+      if (levels_only && !H.sweepw.p && march) {
         CK(cudaStreamSynchronize(H.stream));
         H.sweepw.alloc((size_t)H.P.npts * H.ldo);
       }
+      if (march) shdom::set_layout(H, !levels_only);
       for (auto &g : H.iter_graph)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     }

@@ -86,3 +86,39 @@ def test_solve_while_images_render(rte_cls):
             torch.cuda.synchronize()
             assert relrms(got.cpu().numpy(), want) < 1e-6
     r.close()
+
+
+@pytest.mark.parametrize("transforms", ["tf32x3", "fp32"])
+@pytest.mark.parametrize("kind", ["field", "blob", "polarized", "RPV surface"])
+def test_level_schedule_and_back(rte_cls, kind, transforms):
+    """The plane march switched off and on between calls: the fields' layout
+    turns, and the radiances at the surface and the top go along (to the 1e-5
+    relative RMS of the march against the levels)."""
+    from at3d_gb300.scenes import polarized_blob
+    kw = dict(seed=74, nx=11, ny=10, nz=9, boundary="open")
+    pb = polarized_blob(**kw) if kind == "polarized" else cloud_blob(**kw) if kind == "blob" else cloud_field(nmu=8, nphi=16, nleg=64, **kw)
+    pb.skyrad = 0.05
+    if kind == "RPV surface":
+        pb.surface_brdf, pb.surface_params, pb.surface_delx, pb.surface_dely = "R", np.tile(np.float32([0.1, 0.8, -0.1]), (2, 2, 1)), 1.0, 1.0
+    rng = np.random.default_rng(9)
+    n = 20
+    rays = ((rng.uniform(0.1, 0.9, n) * 11 * pb.delx).astype(np.float32), (rng.uniform(0.1, 0.9, n) * 10 * pb.dely).astype(np.float32),
+            np.full(n, float(pb.zlevels[-1]), np.float32), rng.uniform(0.3, 1.0, n), rng.uniform(0.0, 6.0, n))
+    r, q = rte_cls.from_problem(pb), rte_cls.from_problem(pb)
+    for h in (r, q):
+        h.set_transform_mode(transforms)
+        h.solve(2, verbose=False)
+    image = r.render(*rays)
+    for step, mode in enumerate(("levels_only", "persistent", "levels_only", "graph")):
+        r.set_sweep_mode(mode)
+        assert r.sizes["march"] == (0 if mode == "levels_only" else 3)
+        assert relrms(r.render(*rays), image) < 1e-6  # the surface's radiances are where they were
+        for h in (r, q):
+            h.solve(3 + step, init_solution=False, verbose=False)
+        a, b = r.export_state(), q.export_state()
+        for k in ("radiance", "fluxes"):
+            assert relrms(a[k], b[k]) < 1e-5, (k, mode)
+        image = r.render(*rays)
+        assert relrms(image, q.render(*rays)) < 1e-5
+    r.close()
+    q.close()
