@@ -29,10 +29,12 @@
 #include <cmath>
 #include <cstring>
 #include <cstdlib>
+#include <exception>
 #include <list>
 #include <map>
 #include <memory>
 #include <mutex>
+#include <system_error>
 #include <thread>
 
 namespace shdom {
@@ -107,14 +109,28 @@ template <class F>
 void parallel_for(int n, int grain, F f) {
   const int nt = std::min({32, (int)std::max(1u, std::thread::hardware_concurrency()), n / std::max(1, grain)});
   if (nt < 2) { f(0, n); return; }
-  std::vector<std::thread> th;
   const int chunk = (n + nt - 1) / nt;
+  std::vector<std::thread> th;
+  std::vector<std::exception_ptr> err(nt);
+  auto part = [&](int t) {  // (an exception goes back to the caller, out of no thread)
+    try {
+      if (const int b = t * chunk; b < n) f(b, std::min(n, b + chunk));
+    } catch (...) {
+      err[t] = std::current_exception();
+    }
+  };
+  th.reserve(nt);
   for (int t = 1; t < nt; ++t) {
-    const int b = t * chunk, e = std::min(n, b + chunk);
-    if (b < e) th.emplace_back(f, b, e);
+    try {
+      th.emplace_back(part, t);
+    } catch (const std::system_error &) {  // no more threads: here
+      part(t);
+    }
   }
-  f(0, std::min(n, chunk));
+  part(0);
   for (auto &x : th) x.join();
+  for (auto &e : err)
+    if (e) std::rethrow_exception(e);
 }
 
 // d^l_{m0}(x) * sqrt(l + 1/2), l = 0..lmax, by the standard upward recurrence
@@ -1114,87 +1130,86 @@ bool build_schedule(const shdom_problem &p, Plan &P) {
   std::vector<int> octs = P.is1d ? std::vector<int>{1, 5} : std::vector<int>{1, 2, 3, 4, 5, 6, 7, 8};
   const double transmin = p.transmin;
   bool ok = true;
-  std::vector<std::thread> th;
   std::vector<std::string> errs(8);
   std::vector<int> deep(8, 0);  // octants whose wavefront is too deep for level scheduling
-  for (int ioct : octs) {
-    th.emplace_back([&, ioct]() {
-      sweep_order(P, ioct);
-      const int b = ioct - 1;
-      if (transmin < 1.0 && !P.is1d) {
-        // which face a trace stops on depends on the medium, so no schedule
-        // of the grid's holds: the hemisphere is swept in the reference order
-        // (a 1D trace stops on the first usable point whatever TRANSMIN is)
-        deep[b] = 1;
-        return;
+  auto plan_octant = [&](int ioct) {
+    sweep_order(P, ioct);
+    const int b = ioct - 1;
+    if (transmin < 1.0 && !P.is1d) {
+      // which face a trace stops on depends on the medium, so no schedule
+      // of the grid's holds: the hemisphere is swept in the reference order
+      // (a 1D trace stops on the first usable point whatever TRANSMIN is)
+      deep[b] = 1;
+      return;
+    }
+    const int hemi_bnd = (b & 4) ? 2 : 1;  // trace down: bottom points preset
+    const int *rk = &P.rank[(size_t)b * n];
+    const int *sc = &P.startcell[(size_t)b * n];
+    std::vector<int> order(n), corners;
+    for (int i = 0; i < n; ++i) order[rk[i]] = i;
+    for (int r = 0; r < n; ++r) {
+      int pt = order[r];
+      if (P.bnd[pt] & hemi_bnd) continue;
+      int cell = sc[pt];
+      const int *g = &P.gridptr[8 * (size_t)cell];
+      bool fast = !P.is1d && g[b] == pt && P.cellflags[cell] == 0;
+      for (int k = 0; k < 8 && fast; ++k) {
+        if (k == b) continue;
+        int q = g[k];
+        if (q == pt || !((P.bnd[q] & hemi_bnd) || rk[q] < r)) fast = false;
       }
-      const int hemi_bnd = (b & 4) ? 2 : 1;  // trace down: bottom points preset
-      const int *rk = &P.rank[(size_t)b * n];
-      const int *sc = &P.startcell[(size_t)b * n];
-      std::vector<int> order(n), corners;
-      for (int i = 0; i < n; ++i) order[rk[i]] = i;
-      for (int r = 0; r < n; ++r) {
-        int pt = order[r];
-        if (P.bnd[pt] & hemi_bnd) continue;
-        int cell = sc[pt];
-        const int *g = &P.gridptr[8 * (size_t)cell];
-        bool fast = !P.is1d && g[b] == pt && P.cellflags[cell] == 0;
-        for (int k = 0; k < 8 && fast; ++k) {
-          if (k == b) continue;
-          int q = g[k];
-          if (q == pt || !((P.bnd[q] & hemi_bnd) || rk[q] < r)) fast = false;
-        }
-        if (fast) P.regular.mut()[(size_t)b * n + pt] = 1;
-        for (int cls = 0; cls < 4; ++cls) {
-          const int nc = P.cls_ncol[b][cls], c0 = P.cls_col0[b][cls];
-          if (nc == 0) continue;
-          int *lv = &P.level.mut()[((size_t)b * 4 + cls) * n];
-          uint8_t *kd = &P.kind.mut()[((size_t)b * 4 + cls) * n];
-          // the corners the point's traces for this class end on
-          corners.clear();
-          if (fast) {
-            if (cls < 3) {
-              const int bit = (b >> cls) & 1;
-              const int iface = 2 * cls + 1 - bit;
-              for (int k = 0; k < 4; ++k) corners.push_back(g[kFace[iface][k]]);
-            } else {
-              for (int k = 0; k < 8; ++k) if (k != b) corners.push_back(g[k]);
-            }
+      if (fast) P.regular.mut()[(size_t)b * n + pt] = 1;
+      for (int cls = 0; cls < 4; ++cls) {
+        const int nc = P.cls_ncol[b][cls], c0 = P.cls_col0[b][cls];
+        if (nc == 0) continue;
+        int *lv = &P.level.mut()[((size_t)b * 4 + cls) * n];
+        uint8_t *kd = &P.kind.mut()[((size_t)b * 4 + cls) * n];
+        // the corners the point's traces for this class end on
+        corners.clear();
+        if (fast) {
+          if (cls < 3) {
+            const int bit = (b >> cls) & 1;
+            const int iface = 2 * cls + 1 - bit;
+            for (int k = 0; k < 4; ++k) corners.push_back(g[kFace[iface][k]]);
           } else {
-            for (int c = c0; c < c0 + nc; ++c) {
-              int f[4];
-              double tcx, tcy, tcz;
-              trace_dir(P.mu[P.col_imu[c]], P.phi[(size_t)P.col_imu[c] * P.nphi0max + P.col_iphi[c]], tcx, tcy, tcz);
-              if (!trace_final_face(P, ioct, pt, tcx, tcy, tcz, hemi_bnd, f)) {
-                errs[b] = "sweep planning: trace found no valid face (BACK_INT_GRID: INEXTCELL=0)";
-                return;
-              }
-              for (int k = 0; k < 4; ++k) corners.push_back(f[k]);
+            for (int k = 0; k < 8; ++k) if (k != b) corners.push_back(g[k]);
+          }
+        } else {
+          for (int c = c0; c < c0 + nc; ++c) {
+            int f[4];
+            double tcx, tcy, tcz;
+            trace_dir(P.mu[P.col_imu[c]], P.phi[(size_t)P.col_imu[c] * P.nphi0max + P.col_iphi[c]], tcx, tcy, tcz);
+            if (!trace_final_face(P, ioct, pt, tcx, tcy, tcz, hemi_bnd, f)) {
+              errs[b] = "sweep planning: trace found no valid face (BACK_INT_GRID: INEXTCELL=0)";
+              return;
             }
-          }
-          // A general-trace point whose corners are all preset or phase-1
-          // points is a phase-1 point (boundary-plane chains); any other
-          // point is phase 2, where phase-1 corners count as level 0.
-          bool one = !fast;
-          int m1 = 0, m2 = 0;
-          for (int q : corners) {
-            if (P.bnd[q] & hemi_bnd) continue;
-            if (kd[q] == 3) m1 = std::max(m1, lv[q]);
-            else { one = false; m2 = std::max(m2, lv[q] - Plan::kPhase2); }
-          }
-          if (one) { kd[pt] = 3; lv[pt] = m1 + 1; }
-          else { kd[pt] = fast ? 1 : 2; lv[pt] = Plan::kPhase2 + m2 + 1; }
-          if (lv[pt] >= 2 * Plan::kPhase2 - 1 || (one && lv[pt] >= Plan::kPhase2)) {
-            // (periodic grids chain whole rows through the wrap-around) the
-            // hemisphere is swept in the reference order instead
-            deep[b] = 1;
-            return;
+            for (int k = 0; k < 4; ++k) corners.push_back(f[k]);
           }
         }
+        // A general-trace point whose corners are all preset or phase-1
+        // points is a phase-1 point (boundary-plane chains); any other
+        // point is phase 2, where phase-1 corners count as level 0.
+        bool one = !fast;
+        int m1 = 0, m2 = 0;
+        for (int q : corners) {
+          if (P.bnd[q] & hemi_bnd) continue;
+          if (kd[q] == 3) m1 = std::max(m1, lv[q]);
+          else { one = false; m2 = std::max(m2, lv[q] - Plan::kPhase2); }
+        }
+        if (one) { kd[pt] = 3; lv[pt] = m1 + 1; }
+        else { kd[pt] = fast ? 1 : 2; lv[pt] = Plan::kPhase2 + m2 + 1; }
+        if (lv[pt] >= 2 * Plan::kPhase2 - 1 || (one && lv[pt] >= Plan::kPhase2)) {
+          // (periodic grids chain whole rows through the wrap-around) the
+          // hemisphere is swept in the reference order instead
+          deep[b] = 1;
+          return;
+        }
       }
-    });
-  }
-  for (auto &t : th) t.join();
+    }
+  };
+  parallel_for((int)octs.size(), 1, [&](int b, int e) {
+    for (int i = b; i < e; ++i) plan_octant(octs[i]);
+  });
   for (auto &e : errs) if (!e.empty()) { P.err = e; ok = false; }
   if (!ok) return false;
   for (int hemi = 0; hemi < 2; ++hemi) {
