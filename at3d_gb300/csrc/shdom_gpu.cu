@@ -1114,8 +1114,8 @@ __global__ void __launch_bounds__(256) k_sweep_levels(SweepArgs a, const Seg *__
 // the cell integral alone remain), the latency of a plane on small ones.
 // Measured per hemisphere, x and y classes plus z class, against the
 // point-major march with a cluster barrier per plane that it replaced:
-// 128x128x64 16 x 32 0.76 + 0.58 against 2.46 ms, 96x96x48 0.33 + 0.27
-// against 0.91, 64x64x32 8 x 16 0.060 + 0.045 against 0.276, 12x12x10
+// 128x128x64 16 x 32 0.75 + 0.58 against 2.46 ms, 96x96x48 0.33 + 0.27
+// against 0.91, 64x64x32 8 x 16 0.056 + 0.036 against 0.276, 12x12x10
 // 0.014 + 0.014 against 0.099.  DRAM at 96x96x48: 1.2 times the bytes of the
 // source and the radiance, each once (2.9 times before).  Tried on the way:
 // fences in place of st.async (a plane waits for its global stores: 1.8
@@ -3509,7 +3509,7 @@ __device__ RaySetup ray_setup(const RenderArgs &a, int ray) {
 // have one direction (a parallel view) its functions are formed once.
 //
 // What bounds it: latency (a corner's loads, then the dependent chain of a
-// cell; 14 warps an SM issue 31% of the cycles), then issue slots.  Measured
+// cell; 14 warps an SM issue 40% of the cycles), then issue slots.  Measured
 // for 36,864 rays against one warp per ray: 64x64x32 0.73 against 2.12 ms,
 // 128x128x64 (256 terms) 2.8 against 4.9, polarized 64x64x40 3.0 against
 // 11.0; 169 rays at 32x32x24 0.21 ms either way (the chain of one ray).

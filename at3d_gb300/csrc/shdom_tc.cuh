@@ -132,7 +132,8 @@ __device__ __forceinline__ void reg_fence16(uint32_t *r) {
 // (row tile, N tile) grid, N tile fastest, so the N tiles of one row tile
 // run at the same time on neighbouring CTAs and A comes from DRAM once.  A
 // tile is a 128-row block of A against a BN-column block of B (BN a
-// multiple of 32, at most 128 so that the FP32 sums stay in registers).
+// multiple of 32, at most 128 so that the FP32 sums stay in registers, but for
+// 80 bytes a thread that spill at 128).
 // The chunks of all the CTA's tiles form one pipeline, so loads for the
 // next tile start while the current one is in the tensor cores and its
 // results are stored.
