@@ -5014,8 +5014,8 @@ static void transform(Handle &H, int dir) {
 
 // Point-major rows for the CUDA-core transforms of ordinate-major fields
 // (the FP32 mode, and directions without a tensor-core transform).
-static void alloc_xf_rows(Handle &H) {
-  if (H.ord_major && !H.xf_rows.p && (H.xf_mode == 2 || !H.tc_ok[0] || !H.tc_ok[1])) {
+static void alloc_xf_rows(Handle &H, bool ord_major, int xf_mode) {
+  if (ord_major && !H.xf_rows.p && (xf_mode == 2 || !H.tc_ok[0] || !H.tc_ok[1])) {
     H.xf_rows.alloc((size_t)H.P.npts * H.ldo);
     H.xf_rows.zero(H.stream);
   }
@@ -5027,6 +5027,9 @@ static void alloc_xf_rows(Handle &H) {
 // forms anew but for the points without a source, whose rows are zero.
 static void set_layout(Handle &H, bool ord_major) {
   if (ord_major == H.ord_major) return;
+  // what can fail comes first
+  if (!ord_major && H.tc_ok[1] && H.compact && H.nheavy > 0 && !H.rad_c.p) H.rad_c.alloc((size_t)H.nheavy * H.ldo);
+  alloc_xf_rows(H, ord_major, H.xf_mode);
   const int n = H.P.npts, c = H.P.nang, tiles = ((n + 31) / 32) * ((c + 31) / 32);
   const size_t ps = H.ord_ps, cs = H.ord_cs;
   H.set_strides(ord_major);
@@ -5038,7 +5041,6 @@ static void set_layout(Handle &H, bool ord_major) {
   std::swap(H.raddo.p, H.srcdo.p);  // (of one size, both the handle's own)
   H.srcdo.zero(H.stream);
   setup_tc_rows(H);
-  alloc_xf_rows(H);
   CK(cudaStreamSynchronize(H.stream));  // renders on other streams read them
 }
 
@@ -5351,7 +5353,7 @@ static int create_on_device(std::unique_ptr<shdom_handle> &H, int device, shdom_
     shdom::upload_plan(H->h);
     CK(cudaMemsetAsync(H->h.errflag.p, 0, sizeof(int), H->h.stream));
     shdom::build_irr(H->h);
-    shdom::alloc_xf_rows(H->h);
+    shdom::alloc_xf_rows(H->h, H->h.ord_major, H->h.xf_mode);
   } catch (const std::exception &e) {
     return fail(nullptr, e.what());
   }
@@ -6110,7 +6112,6 @@ int shdom_set_sweep_mode(shdom_handle *hh, int mode) {
   try {
     const bool levels_only = mode == 3;
     if (levels_only != H.march_off) {
-      H.march_off = levels_only;
       const bool march = H.march[0] || H.march[1];
       // the level schedule's source pass needs its (radsrc, tr) table
       if (levels_only && !H.sweepw.p && march) {
@@ -6118,6 +6119,7 @@ int shdom_set_sweep_mode(shdom_handle *hh, int mode) {
         H.sweepw.alloc((size_t)H.P.npts * H.ldo);
       }
       if (march) shdom::set_layout(H, !levels_only);
+      H.march_off = levels_only;  // only now: an allocation that failed leaves the mode as it was
       for (auto &g : H.iter_graph)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     }
@@ -6159,8 +6161,8 @@ int shdom_set_transform_mode(shdom_handle *hh, int mode) {
     if (mode != H.xf_mode)
       for (auto &g : H.iter_graph)  // captured launches are of the old arithmetic
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
+    shdom::alloc_xf_rows(H, H.ord_major, mode);
     H.xf_mode = mode;
-    shdom::alloc_xf_rows(H);
   } catch (const std::exception &e) {
     return fail(hh, e.what());
   }
