@@ -4541,13 +4541,14 @@ static void setup_march(Handle &H) {
     // The x and y classes in one launch, whose shape is a compromise where the
     // grid is long, or in one launch each where that is estimated faster (an
     // iteration, one against two launches, 8 x 16 ordinates: 12x200x24 0.72
-    // and 0.64 ms, 64x520x32 7.4 and 3.4, 1010x32x64 15.7 and 7.9; it is wrong
-    // by little at 96x10x48, 0.50 and 0.51, where it takes two)
+    // and 0.64 ms, 16x400x16 1.27 and 1.01, 64x520x32 7.4 and 3.4; where it
+    // prefers one, 96x10x48 0.50 and 0.51, 81x55x24 0.49 and 0.58; the choice
+    // was the faster one on all of 34 grids tried)
     Handle::MarchLaunch both, one[2];
     if (nx + ny) {
       ok = planes(3, nx + ny, both);
       if (nx && ny && P.nx1 != P.ny1 && planes(1, nx, one[0]) && planes(2, ny, one[1]) &&
-          (!ok || one[0].cycles + one[1].cycles + kMarchLaunch < both.cycles)) {
+          (!ok || one[0].cycles + one[1].cycles + kMarchLaunch < 0.95 * both.cycles)) {
         L[0] = one[0]; L[1] = one[1];
         ok = true;
       } else {
