@@ -2846,11 +2846,13 @@ __global__ void __launch_bounds__(256) k_source_pol(SourceArgs a) {
 // the list leaves them out where the handle knows them (H.compact).
 //
 // What bounds it: memory (five rows per point).  Measured against a warp per
-// point, every point: 64x64x32 with 64 terms and 20% cloud 27 against 104 us,
+// point, every point: 64x64x32 with 64 terms and 20% cloud 20 against 104 us,
 // 128x128x64 with 256 terms and 30% cloud 0.44 against 0.76 ms, 64x64x40 with
-// 3 x 64 terms 0.11 against 0.32.  The sums over points are FP64: four
-// conversions and additions a point and lane, hidden behind the rows but for
-// 0.01 ms at 128x128x64 (pairs of FP32 in their place, 48 bits: 0.43).
+// 3 x 64 terms 0.11 against 0.32.  The sums over points are FP64, of
+// which one warp operation holds the SM's pipe for 16 cycles; a warp's four are
+// added up together, six additions in place of twenty (at 64x64x32 with the
+// stores of unchanged truncations left out 31 -> 20 us, at 81x55x24 with a
+// source everywhere 51 -> 37; three FP32 numbers a sum instead 28 and 46).
 template <int NST, int LPP, int NP>
 __global__ void __launch_bounds__(256) k_source_v(SourceArgs a, const int *__restrict__ list, int n) {
   const int lane = threadIdx.x & 31, gl = lane % LPP, sub = lane / LPP;
@@ -2878,7 +2880,7 @@ __global__ void __launch_bounds__(256) k_source_v(SourceArgs a, const int *__res
 #pragma unroll
       for (int k = 0; k < 3; ++k) cp[k] = gl < nl ? a.coefp[((size_t)p * 3 + k) * nl + gl] : 0.f;
     const float f0 = a.dirflux[p] * a.secmu0, th = a.thermal ? 3.544907703f * a.thermal[p] : 0.f;
-    const int nrp = a.nr[p], nsold = a.ns[p], nsmin = min(nsold, a.nso[p]);
+    const int nrp = a.nr[p], nsold = a.ns[p], nsoold = a.nso[p], nsmin = min(nsold, nsoold);
     float *S = a.source + (size_t)p * NST * nlm, *D = a.delsource + (size_t)p * NST * nlm;
     const float *R = a.radiance + (size_t)p * NST * nlm;
     float jt[NST][NP][4], sum[4] = {0.f, 0.f, 0.f, 0.f}, r00 = 0.f;
@@ -2971,22 +2973,27 @@ __global__ void __launch_bounds__(256) k_source_v(SourceArgs a, const int *__res
                             j + 2 < nsnew ? jt[k][s][2] : 0.f, j + 3 < nsnew ? jt[k][s][3] : 0.f);
       }
       if (gl == 0) {
-        a.ns[p] = nsnew;
-        if (a.first) a.nso[p] = nsnew;
-        else if (a.accel) a.nso[p] = nsold;
+        // (most truncations stay as they are, and a store of one is a sector of its own)
+        const int nsonew = a.first ? nsnew : a.accel ? nsold : nsoold;
+        if (nsnew != nsold) a.ns[p] = nsnew;
+        if (nsonew != nsoold) a.nso[p] = nsonew;
+        if (nrnext != nrp) a.nr[p] = nrnext;
         a.nrr[p] = nrp;
-        a.nr[p] = nrnext;
       }
     }
   }
   if (!a.first) {
     __shared__ double sred[4][8];
+    // a lane has two of the sums after the first exchange, one after the second
+    const bool o1 = lane & 1, o2 = lane & 2;
+    double t0 = o1 ? tot[1] : tot[0], t1 = o1 ? tot[3] : tot[2];
+    t0 += __shfl_xor_sync(0xffffffffu, o1 ? tot[0] : tot[1], 1);
+    t1 += __shfl_xor_sync(0xffffffffu, o1 ? tot[2] : tot[3], 1);
+    double t = o2 ? t1 : t0;
+    t += __shfl_xor_sync(0xffffffffu, o2 ? t0 : t1, 2);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      double t = tot[k];
-      for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (lane == 0) sred[k][threadIdx.x >> 5] = t;
-    }
+    for (int o = 4; o < 32; o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane < 4) sred[lane][threadIdx.x >> 5] = t;
     __syncthreads();
     if (threadIdx.x < 4) {
       double t = 0;
